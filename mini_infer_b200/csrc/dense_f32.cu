@@ -4,71 +4,91 @@
 // of rows and wherever a row lies in its tile, so a token's result does not depend on how many other
 // tokens share its step: the float32 path gives the same bits for every way of cutting and batching the
 // work.  (A library product picks other kernels, and other orders of summation, for other row counts.)
-// CUDA cores only, no reduced-precision mode: this path exists to show faults that bfloat16 hides, not to
-// be fast.  The reference runs every dense product in FP16 through cuBLAS (src/layers/mlp.cpp:120-130).
+// CUDA cores only, no reduced-precision mode: this path exists to show faults that bfloat16 hides.
+// The reference runs every dense product in FP16 through cuBLAS (src/layers/mlp.cpp:120-130).
 
-#include "common.cuh"
+#include "f32_tiles.cuh"
 
 namespace mi {
 
-constexpr int DF_BM = 64, DF_BN = 64, DF_BK = 16;
+// One of several independent products (a head, say) is blockIdx.z; its operands lie sA, sW, sC apart.
+struct DenseF32 {
+    const float* A; const float* W; float* C;
+    int T, N, K, lda, ldc;
+    int64_t sA, sW, sC;
+};
 
-template <bool VEC>
-__global__ void __launch_bounds__(256)
-dense_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C, int T, int N,
-                 int K, int lda, int ldc, int64_t sA, int64_t sW, int64_t sC) {
-    // blockIdx.z: one of several independent products (a head, say) whose operands lie sA, sW, sC apart
-    A += blockIdx.z * sA; W += blockIdx.z * sW; C += blockIdx.z * sC;
-    __shared__ float As[DF_BK][DF_BM + 4];
-    __shared__ float Ws[DF_BK][DF_BN + 4];
-    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    const int row0 = blockIdx.y * DF_BM, n0 = blockIdx.x * DF_BN;
-    float acc[4][4];
+template <int BN, bool VEC>
+__global__ void __launch_bounds__(f32t::THREADS, 3)
+dense_f32_wide_kernel(DenseF32 g) {
+    constexpr int TN = BN / 16;
+    const float* A = g.A + blockIdx.z * g.sA;
+    const float* W = g.W + blockIdx.z * g.sW;
+    float* C = g.C + blockIdx.z * g.sC;
+    const int row0 = blockIdx.y * f32t::BM, n0 = blockIdx.x * BN;
+    const f32t::WidePlace<BN> at(blockIdx.x + blockIdx.y);
+    unsigned long long acc[8][TN / 2];
+    const int rows = min(f32t::BM, g.T - row0);
+    f32t::wide_tile<BN, VEC>(
+        acc, [&](int r) { return r < rows ? A + (int64_t)(row0 + r) * g.lda : nullptr; },
+        [&](int n) { return n0 + n < g.N ? W + (int64_t)(n0 + n) * g.K : nullptr; }, rows, g.K, at);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        if (at.r_lo + i >= rows) break;
+        float* c = C + (int64_t)(row0 + at.r_lo + i) * g.ldc;
+#pragma unroll
+        for (int j = 0; j < TN / 2; ++j) {
+            const float2 v = f32t::halves_of(acc[i][j]);
+            const int n = n0 + (j < TN / 4 ? at.c_lo + 2 * j : BN / 2 + at.c_lo + 2 * (j - TN / 4));
+            if (n < g.N) c[n] = v.x;
+            if (n + 1 < g.N) c[n + 1] = v.y;
+        }
+    }
+}
+
+__global__ void __launch_bounds__(f32t::THREADS)
+dense_f32_narrow_kernel(DenseF32 g) {
+    const float* A = g.A + blockIdx.z * g.sA;
+    const float* W = g.W + blockIdx.z * g.sW;
+    float* C = g.C + blockIdx.z * g.sC;
+    const int n0 = blockIdx.x * f32t::NN, row0 = blockIdx.y * f32t::NM;
+    const int rows = min(f32t::NM, g.T - row0);
+    float acc[1][4];
+    f32t::narrow_tile<1>(
+        acc, [&](int r) { return r < rows ? A + (int64_t)(row0 + r) * g.lda : nullptr; },
+        [&](int n) { return n0 + n < g.N ? W + (int64_t)(n0 + n) * g.K : nullptr; }, rows, g.K, A);
+    const int r = (threadIdx.x >> 5) * 4, n = n0 + (threadIdx.x & 31);
+    if (n >= g.N) return;
 #pragma unroll
     for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
-    for (int k0 = 0; k0 < K; k0 += DF_BK) {
-        if (VEC) {                                          // K % 4 == 0 and 16-byte aligned operands
-            const int r = tid >> 2, c = (tid & 3) * 4;
-            float4 a = make_float4(0.f, 0.f, 0.f, 0.f), w = a;
-            if (k0 + c < K) {
-                if (row0 + r < T) a = __ldg(reinterpret_cast<const float4*>(A + (int64_t)(row0 + r) * lda + k0 + c));
-                if (n0 + r < N) w = __ldg(reinterpret_cast<const float4*>(W + (int64_t)(n0 + r) * K + k0 + c));
-            }
-            As[c][r] = a.x; As[c + 1][r] = a.y; As[c + 2][r] = a.z; As[c + 3][r] = a.w;
-            Ws[c][r] = w.x; Ws[c + 1][r] = w.y; Ws[c + 2][r] = w.z; Ws[c + 3][r] = w.w;
-        } else {
-            for (int idx = tid; idx < DF_BM * DF_BK; idx += 256) {
-                const int r = idx / DF_BK, c = idx % DF_BK;
-                const bool kin = k0 + c < K;
-                As[c][r] = (kin && row0 + r < T) ? A[(int64_t)(row0 + r) * lda + k0 + c] : 0.f;
-                Ws[c][r] = (kin && n0 + r < N) ? W[(int64_t)(n0 + r) * K + k0 + c] : 0.f;
-            }
-        }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < DF_BK; ++kk) {                // k beyond K holds zeros: fma(0, 0, acc) == acc
-            float a[4], w[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) { a[i] = As[kk][ty * 4 + i]; w[i] = Ws[kk][tx * 4 + i]; }
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], w[j], acc[i][j]);
-        }
-        __syncthreads();
+        if (r + i < rows) C[(int64_t)(row0 + r + i) * g.ldc + n] = acc[0][i];
+}
+
+// Which form: up to DF_NARROW_ROWS rows a product is bound by reading W, and the narrow tiles keep more of it in flight;
+// above, wide tiles of 128 columns, or of 64 where those of 128 would leave SMs without one.
+constexpr int DF_NARROW_ROWS = 16, DF_SMS = 148;
+
+static int dense_f32_launch(const DenseF32& g, int batch, bool vec, cudaStream_t stream, const char* what) {
+    const int64_t tiles_y = ((int64_t)g.T + f32t::BM - 1) / f32t::BM;
+    if (tiles_y > 65535) { set_last_error("dense product (float32): %d rows exceed the grid limit", g.T); return kBadShape; }
+    if (vec && g.T <= DF_NARROW_ROWS) {
+        const size_t smem = f32t::narrow_smem(1);
+        cudaFuncSetAttribute(dense_f32_narrow_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        dense_f32_narrow_kernel<<<dim3((g.N + f32t::NN - 1) / f32t::NN, 1, batch), f32t::THREADS, smem, stream>>>(g);
+        return finish_launch(what);
     }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int r = row0 + ty * 4 + i;
-        if (r >= T) continue;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int n = n0 + tx * 4 + j;
-            if (n < N) C[(int64_t)r * ldc + n] = acc[i][j];
-        }
+    const int64_t wide = tiles_y * ((g.N + 127) / 128) * batch;
+    const bool half = wide < DF_SMS;
+    const int bn = half ? 64 : 128;
+    const dim3 grid((g.N + bn - 1) / bn, (unsigned)tiles_y, batch);
+    if (half) {
+        if (vec) dense_f32_wide_kernel<64, true><<<grid, f32t::THREADS, 0, stream>>>(g);
+        else dense_f32_wide_kernel<64, false><<<grid, f32t::THREADS, 0, stream>>>(g);
+    } else {
+        if (vec) dense_f32_wide_kernel<128, true><<<grid, f32t::THREADS, 0, stream>>>(g);
+        else dense_f32_wide_kernel<128, false><<<grid, f32t::THREADS, 0, stream>>>(g);
     }
+    return finish_launch(what);
 }
 
 }  // namespace mi
@@ -77,13 +97,8 @@ extern "C" int mi_dense_f32(const float* A, const float* W, float* C, int T, int
     using namespace mi;
     if (T <= 0 || N <= 0) return kOk;
     if (K <= 0) { set_last_error("dense product (float32): inner size %d", K); return kBadShape; }
-    const int64_t tiles_y = ((int64_t)T + DF_BM - 1) / DF_BM;
-    if (tiles_y > 65535) { set_last_error("dense product (float32): %d rows exceed the grid limit", T); return kBadShape; }
-    const dim3 grid((N + DF_BN - 1) / DF_BN, (unsigned)tiles_y);
     const bool vec = (K % 4 == 0) && (((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W)) & 15) == 0);
-    if (vec) dense_f32_kernel<true><<<grid, 256, 0, stream>>>(A, W, C, T, N, K, K, N, 0, 0, 0);
-    else dense_f32_kernel<false><<<grid, 256, 0, stream>>>(A, W, C, T, N, K, K, N, 0, 0, 0);
-    return finish_launch("dense_f32");
+    return dense_f32_launch(DenseF32{A, W, C, T, N, K, K, N, 0, 0, 0}, 1, vec, stream, "dense_f32");
 }
 
 // `batch` products at once: C_b[T, N] = A_b[T, K] . W_b[N, K]^T with rows of A and C `lda` and `ldc` floats
@@ -97,12 +112,7 @@ extern "C" int mi_dense_f32_batched(const float* A, const float* W, float* C, in
         set_last_error("batched dense product (float32): inner size %d, rows %d and %d apart, %d products", K, lda, ldc, batch);
         return kBadShape;
     }
-    const int64_t tiles_y = ((int64_t)T + DF_BM - 1) / DF_BM;
-    if (tiles_y > 65535) { set_last_error("batched dense product (float32): %d rows exceed the grid limit", T); return kBadShape; }
-    const dim3 grid((N + DF_BN - 1) / DF_BN, (unsigned)tiles_y, batch);
     const bool vec = (K % 4 == 0) && (lda % 4 == 0) && (sA % 4 == 0) && (sW % 4 == 0) &&
                      (((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W)) & 15) == 0);
-    if (vec) dense_f32_kernel<true><<<grid, 256, 0, stream>>>(A, W, C, T, N, K, lda, ldc, sA, sW, sC);
-    else dense_f32_kernel<false><<<grid, 256, 0, stream>>>(A, W, C, T, N, K, lda, ldc, sA, sW, sC);
-    return finish_launch("dense_f32_batched");
+    return dense_f32_launch(DenseF32{A, W, C, T, N, K, lda, ldc, sA, sW, sC}, batch, vec, stream, "dense_f32_batched");
 }

@@ -1,0 +1,113 @@
+"""The forms of the 32-bit path's kernels (wide and narrow tiles of the products, staged tokens of the router, warps of
+eight queries of the attention): every form against float64 within the bound of a chain of additions, and the same bits
+from every form."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+UNIT = 2.0 ** -24
+
+
+def F():
+    from mini_infer_b200.ops import functional
+    return functional
+
+
+def rnd(*shape, seed=0, scale=1.0):
+    return (torch.randn(*shape, generator=torch.Generator().manual_seed(seed)) * scale).to(DEV)
+
+
+def within_chain(out, a, w):
+    """A chain of K fused multiply-adds is off by at most K units of sum |a||w|."""
+    ref = a.double() @ w.double().T
+    bound = a.shape[1] * UNIT * (a.double().abs() @ w.double().abs().T) + 1e-30
+    assert bool(((out.double() - ref).abs() <= bound).all())
+
+
+# rows: one, the narrow form's last, one more, a warp's and a tile's edges; columns and inner sizes that fill no tile
+@pytest.mark.parametrize("T", [1, 16, 17, 64, 65, 200])
+@pytest.mark.parametrize("N,K", [(33, 4), (64, 68), (129, 100), (320, 63), (200, 2050), (19200, 36)])
+def test_dense_forms(T, N, K):
+    a, w = rnd(T, K, seed=1), rnd(N, K, seed=2)
+    out = F().dense_f32(a, w)
+    within_chain(out, a, w)
+    for lo, hi in ((0, min(T, 5)), (T - 1, T), (max(0, T - 20), T)):
+        assert torch.equal(F().dense_f32(a[lo:hi].contiguous(), w), out[lo:hi])
+
+
+def test_dense_rows_that_are_not_aligned():
+    flat, w = rnd(40 * 64 + 1, seed=3), rnd(70, 64, seed=4)
+    a = flat[1:].view(40, 64)
+    assert torch.equal(F().dense_f32(a, w), F().dense_f32(a.clone(), w))
+
+
+@pytest.mark.parametrize("counts", [[0, 1, 0, 16, 17], [64, 65, 0, 0, 3], [3] * 40 + [0, 8], [200, 0, 15]])
+@pytest.mark.parametrize("nout,K", [(32, 64), (45, 68), (130, 36), (70, 33)])
+@pytest.mark.parametrize("paired", [False, True])
+def test_grouped_forms(counts, nout, K, paired):
+    E, n, T = len(counts), sum(counts), 50
+    x, w = rnd(T, K, seed=5), rnd(E, (2 if paired else 1) * nout, K, seed=6)
+    gather = torch.randint(0, T, (n,), generator=torch.Generator().manual_seed(7)).to(torch.int32).to(DEV)
+    offsets = torch.tensor([sum(counts[:e]) for e in range(E + 1)], dtype=torch.int32, device=DEV)
+    scale = rnd(n, seed=8).abs() if paired else None
+    out = F().grouped_gemm_plain(x, gather, w, offsets, n, paired, torch.float32, row_scale=scale)
+    for e in range(E):
+        lo, hi = int(offsets[e]), int(offsets[e + 1])
+        if lo == hi:
+            continue
+        rows = x[gather[lo:hi].long()].contiguous()
+        z = F().dense_f32(rows, w[e].contiguous())
+        within_chain(z, rows, w[e])
+        if not paired:
+            assert torch.equal(out[lo:hi], z)
+            # whatever else is in the step: the expert's rows one by one
+            one = F().grouped_gemm_plain(rows[-1:].contiguous(), None, w[e:e + 1].contiguous(),
+                                         torch.tensor([0, 1], dtype=torch.int32, device=DEV), 1, False, torch.float32)
+            assert torch.equal(one[0], out[hi - 1])
+        else:
+            g, u = (z.double() * scale[lo:hi, None].double()).chunk(2, 1)
+            ref = g * torch.sigmoid(g) * u
+            assert bool(((out[lo:hi].double() - ref).abs() <= 16 * UNIT * (g.abs() + 1) * u.abs() + 1e-30).all())
+
+
+@pytest.mark.parametrize("T", [33, 40, 77, 512])
+@pytest.mark.parametrize("H,E,gated", [(64, 5, True), (1028, 16, False), (2048, 60, True), (2052, 33, True)])
+def test_router_of_many_tokens_adds_as_that_of_few(T, H, E, gated):
+    x, w, g = rnd(T, H, seed=9), rnd(E, H, seed=10, scale=0.05), rnd(H, seed=11, scale=0.05) if gated else None
+    whole = F().moe_router(x, w, g, 2, False, want_probs=True)
+    few = [F().moe_router(x[lo:lo + 8].contiguous(), w, g, 2, False, want_probs=True) for lo in range(0, T, 8)]
+    for i, got in enumerate(whole):
+        if got is not None:
+            assert torch.equal(got, torch.cat([f[i] for f in few]))
+
+
+@pytest.mark.parametrize("d,nh,nkv,page,window", [(64, 4, 2, 16, 0), (128, 2, 1, 16, 0), (128, 3, 3, 8, 40), (64, 2, 2, 32, 17)])
+def test_attention_of_every_cut(d, nh, nkv, page, window):
+    lengths, S = [1, 7, 8, 33, 64, 95], 95
+    k, v = rnd(1, S, nkv, d, seed=12)[0], rnd(1, S, nkv, d, seed=13)[0]
+    q = rnd(S, nh, d, seed=14)
+    pages = -(-S // page)
+    order = list(range(pages))[::-1]
+    kc, vc = torch.zeros(pages, nkv, page, d, device=DEV), torch.zeros(pages, nkv, page, d, device=DEV)
+    for p in range(S):
+        kc[order[p // page], :, p % page], vc[order[p // page], :, p % page] = k[p], v[p]
+    i32 = lambda t: torch.tensor(t, dtype=torch.int32, device=DEV)
+    table = i32([order])
+    whole = F().attention(q, kc, vc, table, i32([0, S]), i32([S]), S, window)
+    at = torch.arange(S, device=DEV)
+    seen = (at[None] <= at[:, None]) & ((at[None] > at[:, None] - window) if window else torch.ones(S, S, dtype=torch.bool, device=DEV))
+    for h in range(nh):
+        s = (q[:, h].double() @ k[:, h // (nh // nkv)].double().T) * d ** -0.5
+        ref = torch.softmax(s.masked_fill(~seen, -torch.inf), -1) @ v[:, h // (nh // nkv)].double()
+        assert float((whole[:, h].double() - ref).abs().max()) <= 3e-6 * float(ref.abs().max())
+    lo = 0
+    for hi in lengths:              # the same prompt in portions
+        out = F().attention(q[lo:hi].contiguous(), kc, vc, table, i32([0, hi - lo]), i32([hi]), hi - lo, window)
+        assert torch.equal(out, whole[lo:hi])
+        lo = hi
+    # several requests in one step, one of them with one token
+    two = F().attention(torch.cat([q[94:95], q[30:64]]).contiguous(), kc, vc, table.expand(2, -1).contiguous(), i32([0, 1, 35]),
+                        i32([95, 64]), 34, window)
+    assert torch.equal(two, torch.cat([whole[94:95], whole[30:64]]))
