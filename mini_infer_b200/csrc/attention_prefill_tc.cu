@@ -2,21 +2,26 @@
 // of prompts of a ragged batch over the paged cache, flash-attention style, with both products on
 // tcgen05.mma and their accumulators in tensor memory.
 //
-// Block = 128 queries of one head; two blocks share an SM, so that one's softmax runs beside the
-// other's tensor-core work.  Key tiles of 64, aligned to absolute positions, arrive page by page
-// through TMA (128-byte swizzle) into rings of three K and two V tiles.  Per key tile:
+// Block = 256 queries of one head as two query tiles of 128 that read the same key tiles: one's softmax runs beside
+// the other's tensor-core work.  Key tiles of 64, aligned to absolute positions, arrive page by page
+// through TMA (128-byte swizzle) into rings of K and V tiles as deep as shared memory allows.  Per key and query tile:
 //   S = Q K^T    A = Q tile (K-major), B = K tile (K-major), accumulator S[buf] in tensor memory
-//   softmax      one thread per query row (a row is a lane of tensor memory, so the row maximum and
-//                sum need no exchange between threads): the row of S comes to registers with
+//   softmax      two threads per query row, 32 keys each (a row is a lane of tensor memory; the two
+//                threads sit in two warps of the same lane quarter): the row of S comes to registers with
 //                tcgen05.ld, P = exp2(s - reference) is rounded to bfloat16 and written over S in
 //                place with tcgen05.st (two keys per 32-bit column); the reference follows the
 //                running maximum only when that moved by more than 8 (P stays below 2^8), and only
-//                then O is scaled in place (tcgen05.ld / .st)
+//                then O is scaled in place (tcgen05.ld / .st).  The two halves' maxima meet in shared
+//                memory, their sums once, at the end
 //   O += P V     A = P straight from tensor memory, B = V tile as it lies in the cache (keys x head,
 //                i.e. MN-major), accumulator O in tensor memory
-//   warp 0    TMA producer (Q once; K and V tiles of every key tile, one copy per page and 64 columns)
-//   warp 1    allocates tensor memory, issues the MMAs
-//   warps 2-5 softmax and epilogue, one lane quarter of tensor memory each
+//   warps 0-7, 8-15  softmax and epilogue of the first and the second query tile
+//   warps 16, 17     TMA producers of K (and Q) and of V, one copy per page and 64 columns
+//   warps 18, 19     issue the MMAs of the first and the second query tile (18 allocates tensor memory)
+// What bounds it is the chain of one key tile (wait, load, maximum, exponentials, store, hand-over, product), so
+// every part of the chain is kept off the producers' way: page numbers are looked up a tile ahead, K and V have a warp
+// each, and a block that has the SM to itself keeps four and more tiles of each on their way (two blocks of one query
+// tile per SM, with one producer and rings of three K and two V tiles: 1.9 us a key tile).
 // S is double-buffered, so the next tile's S = Q K^T runs beside this tile's softmax.  Masking is positional: key j is visible from the
 // query at position p iff j <= p and (window == 0 or j > p - window or j < keep_first) and j < kv_len; with chunks
 // instead of a window iff j <= p and j lies in p's chunk (or j < keep_first): see AttnForm, which also gives the added
@@ -35,12 +40,46 @@ namespace pt {
 
 using namespace mi::tc;
 
-constexpr int BQ = 128;            // queries per block (MMA M)
+constexpr int BQ = 128;            // queries per tile (MMA M)
+// query tiles per block: two, but one where the queries of two would leave no room for rings
+constexpr int query_tiles(int dk) { return dk > 192 ? 1 : 2; }
 constexpr int BN = 64;             // keys per tile
-constexpr int NK = 3;              // stages of the K ring (unless a form chooses others)
-constexpr int NV = 2;              // stages of the V ring
-constexpr int HALF_BYTES = 128 * 64 * 2;   // a tile of 128 rows x 64 columns: 16 KiB (Q, P)
+constexpr int HK = BN / 2;         // keys of a tile that a softmax thread takes
+constexpr int THREADS = 640;       // 2 x 8 softmax warps, two producers, two that issue MMAs
+constexpr int HALF_BYTES = 128 * 64 * 2;   // a tile of 128 rows x 64 columns: 16 KiB (Q)
 constexpr int KV_HALF = BN * 64 * 2;       // a tile of BN keys x 64 columns: 8 KiB
+// behind the tiles: barriers and words, then the halves' maxima of two tiles in turn, per query tile [2][2][BQ] floats
+constexpr int WORDS = 512;
+constexpr int tail(int dk) { return WORDS + query_tiles(dk) * 2 * 2 * BQ * 4; }
+constexpr int SMEM_MAX = 227 * 1024;
+constexpr int SMS = 148;
+// Stages of the rings: as many K and V tiles as fit beside the queries (8 of each at most).
+constexpr int stages(int dk, int dv) {
+    const int per = (dk / 64 + dv / 64) * KV_HALF, room = SMEM_MAX - tail(dk) - query_tiles(dk) * (dk / 64) * HALF_BYTES;
+    return room / per < 8 ? room / per : 8;
+}
+constexpr size_t smem_bytes(int dk, int dv) {
+    return (size_t)query_tiles(dk) * (dk / 64) * HALF_BYTES + (size_t)stages(dk, dv) * (dk / 64 + dv / 64) * KV_HALF + tail(dk);
+}
+static_assert(stages(256, 128) >= 3 && stages(192, 128) >= 3, "rings of three stages at the largest sizes");
+// Which query tiles share a block (and its key tiles):
+//   kSingle      one alone, where the tiles of all heads and requests find an SM each (or two do not fit): a chain by
+//                itself takes 0.80 us a key tile, two beside each other 1.05 us
+//   kApart       the last but i and the first but i, where the pairs find an SM each and all earlier keys are seen: no
+//                block has two long ones (2,048 queries of 16 heads, 128 blocks: 36 us, 45 us with neighbours)
+//   kNeighbours  2 i and 2 i + 1, whose keys are nearly the same, so that both chains run to the end (8,192 queries of 16
+//                heads: 263 us, 353 us apart)
+enum QueryTiles : int { kSingle = 0, kApart = 1, kNeighbours = 2 };
+inline QueryTiles query_order(int64_t rows, int heads, int requests, int dk, bool bounded) {
+    const int64_t tiles = (rows + BQ - 1) / BQ, each = (int64_t)heads * requests;
+    if (query_tiles(dk) == 1 || tiles * each <= SMS) return kSingle;
+    return !bounded && (tiles + 1) / 2 * each <= SMS ? kApart : kNeighbours;
+}
+// blocks along x: the query tiles of the longest portion, for every head
+inline unsigned grid_x(int64_t rows, int heads, QueryTiles order) {
+    const int64_t tiles = (rows + BQ - 1) / BQ;
+    return (unsigned)((order == kSingle ? tiles : (tiles + 1) / 2) * heads);
+}
 
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
     __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
@@ -72,9 +111,39 @@ __device__ __forceinline__ float fast_exp2(float x) {
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-__device__ __forceinline__ void mbar_arrive_after_tmem(uint64_t* bar) {
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    mbar_arrive(bar);
+// Barrier `id` of the two warps that share a lane quarter of a query tile; whether `ok` held for all of their threads.
+__device__ __forceinline__ bool pair_and(int id, bool ok) {
+    uint32_t all;
+    asm volatile("{\n .reg .pred p, q;\n setp.ne.u32 p, %1, 0;\n barrier.cta.red.and.pred q, %2, 64, p;\n selp.u32 %0, 1, 0, q;\n}"
+                 : "=r"(all) : "r"((uint32_t)ok), "r"(id) : "memory");
+    return all != 0;
+}
+// one lane of a converged warp
+__device__ __forceinline__ bool elect_one() {
+    uint32_t is;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(is));
+    return is != 0;
+}
+// two multiply-adds, two additions in one instruction (each rounded as by itself)
+__device__ __forceinline__ float2 fma_two(float2 a, float b, float c) {
+    float2 r;
+    asm("{\n .reg .b64 x, y, z;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %4};\n mov.b64 z, {%5, %5};\n"
+        " fma.rn.f32x2 x, x, y, z;\n mov.b64 {%0, %1}, x;\n}"
+        : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b), "f"(c));
+    return r;
+}
+__device__ __forceinline__ float2 add_two(float2 a, float2 b) {
+    float2 r;
+    asm("{\n .reg .b64 x, y;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n add.rn.f32x2 x, x, y;\n mov.b64 {%0, %1}, x;\n}"
+        : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+}
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+          "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+        : "memory");
 }
 
 struct Maps {
@@ -105,78 +174,93 @@ __device__ __forceinline__ float fast_tanh(float x) {
     return 1.0f - __fdividef(2.0f, fast_exp2(x * 2.8853900817779268f) + 1.0f);
 }
 
-template <int DK, int DV, bool CAPPED = false, bool LOGISTIC = false, bool UNFOLDED = false, int NK = pt::NK, int NV = pt::NV>
-__global__ void __launch_bounds__(192, 2)
+template <int DK, int DV, bool CAPPED = false, bool LOGISTIC = false, bool UNFOLDED = false>
+__global__ void __launch_bounds__(THREADS, 1)
 attn_prefill_tc_kernel(const __grid_constant__ Maps maps, const int* __restrict__ block_table,
                        const int* __restrict__ q_start, const int* __restrict__ kv_len,
                        __nv_bfloat16* __restrict__ out, int nh, int nkv, int page_size, int max_pages,
                        int window, float scale_log2, int* __restrict__ status, int keep_first, int hpq,
-                       float cap_in, float cap_out, int sink, const float* __restrict__ head_bias, Unfolded uf, AttnForm form) {
+                       float cap_in, float cap_out, int sink, const float* __restrict__ head_bias, Unfolded uf, AttnForm form,
+                       QueryTiles order) {
     constexpr int DKH = DK / 64, DVH = DV / 64;           // 64-column halves of a key and of a value row
-    constexpr uint32_t TMEM_COLS = 256;                   // S[0], S[1] (BN columns each), O (D): two blocks share an SM
-    constexpr uint32_t COL_S = 0, COL_O = 2 * BN;
+    constexpr int NS = stages(DK, DV), QT = query_tiles(DK);
+    constexpr uint32_t TMEM_COLS = 512;                   // per query tile S[0], S[1] (BN columns each), O (128)
+    constexpr uint32_t COL_O = 2 * BN, COL_TILE = 256;
     // instruction descriptors: D float32, A and B bfloat16, M = 128
     constexpr uint32_t IDESC_S = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((128u >> 4) << 24);
     constexpr uint32_t IDESC_PV = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(DV >> 3) << 17) |
                                   ((128u >> 4) << 24);    // B (the V tile) MN-major
     extern __shared__ __align__(1024) uint8_t smem[];     // tiles first (the swizzle wants 1024-byte alignment)
-    uint8_t* sQ = smem;                                   // DKH halves of [128 queries][64]
-    uint8_t* sK = sQ + DKH * HALF_BYTES;                  // NK stages of DKH halves of [BN keys][64]
-    uint8_t* sV = sK + NK * DKH * KV_HALF;                // NV stages of DVH halves for V
-    uint64_t* bars = reinterpret_cast<uint64_t*>(sV + NV * DVH * KV_HALF);
-    uint64_t* q_full = bars;                              // then the barriers and a few words
-    uint64_t* k_full = bars + 1;
-    uint64_t* v_full = k_full + NK;
-    uint64_t* k_empty = v_full + NV;
-    uint64_t* v_empty = k_empty + NK;
-    uint64_t* s_full = v_empty + NV;
-    uint64_t* p_full = s_full + 2;                        // per S/P buffer: the softmax may be a tile ahead
-    uint64_t* o_done = p_full + 2;
-    uint32_t* tmem_base_p = reinterpret_cast<uint32_t*>(o_done + 1);
+    uint8_t* sQ = smem;                                   // per query tile DKH halves of [128 queries][64]
+    uint8_t* sK = sQ + QT * DKH * HALF_BYTES;             // NS stages of DKH halves of [BN keys][64]
+    uint8_t* sV = sK + NS * DKH * KV_HALF;                // NS stages of DVH halves for V
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sV + NS * DVH * KV_HALF);
+    uint64_t* k_full = bars;
+    uint64_t* v_full = k_full + NS;
+    uint64_t* k_empty = v_full + NS;
+    uint64_t* v_empty = k_empty + NS;
+    uint64_t* q_full = v_empty + NS;                      // the rest per query tile
+    uint64_t* s_full = q_full + QT;                       // [QT][2]
+    uint64_t* p_full = s_full + QT * 2;                   // [QT][2] per S/P buffer: the softmax may be a tile ahead
+    uint64_t* o_done = p_full + QT * 2;
+    uint32_t* tmem_base_p = reinterpret_cast<uint32_t*>(o_done + QT);
     int* abort_p = reinterpret_cast<int*>(tmem_base_p + 1);
-    int* tile_pages = abort_p + 1;                        // BN / 8 entries
+    float* halves = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(bars) + WORDS);      // [QT][2 in turn][2][BQ]
+    static_assert((4 * 8 + QT * 6) * 8 + 8 <= WORDS, "barriers and words");
 
-    // later query tiles see more keys: they are launched first, so that the short ones fill the tail
-    const int b = blockIdx.z, h = blockIdx.y, qt = gridDim.x - 1 - blockIdx.x;
+    // later queries see more keys: those of all heads are launched first, so that the short ones fill the tail
+    const int b = blockIdx.z, h = blockIdx.x % nh, step = blockIdx.x / nh;
     const int q0 = q_start[b] * hpq, q_len = (q_start[b + 1] - q_start[b]) * hpq;      // in rows
-    if (qt * BQ >= q_len) return;                         // uniform for the whole block
+    const int n_q = (q_len + BQ - 1) / BQ, n_blocks = order == kSingle ? n_q : (n_q + 1) / 2;
+    if (step >= n_blocks) return;                         // uniform for the whole block
     const int kvl = kv_len[b];
+    const bool bounded = window > 0 || form.chunk > 0;    // keys before some position are out of sight
+    const int tile_a = order == kNeighbours ? 2 * (n_blocks - 1 - step) : n_q - 1 - step;
+    const int tile_b = order == kSingle ? tile_a : min(order == kApart ? step : tile_a + 1, n_q - 1);
+    const int tiles_q = tile_a == tile_b ? 1 : 2;
     const int hk = h / (nh / nkv);
     const int dh = UNFOLDED ? (uf.d16 + 3) / 4 : DKH;     // halves of the unrotated part
     int kv_base = 0;                                      // first row of the request's context in the maps
     if constexpr (UNFOLDED) for (int i = 0; i < b; ++i) kv_base += kv_len[i];
-    const int nq = min(BQ, q_len - qt * BQ);
-    const int p_lo = kvl - q_len / hpq + (qt * BQ) / hpq; // position of the tile's first query (hpq divides BQ)
-    const int p_hi = p_lo + (nq - 1) / hpq;
-    const bool bounded = window > 0 || form.chunk > 0;    // keys before some position are out of sight
-    const int k_begin = (first_visible(p_lo, window, form.chunk) / BN) * BN;
-    const int k_end = min(kvl, p_hi + 1);
+    const int pos0 = kvl - q_len / hpq;                   // position of the portion's first query (hpq divides BQ)
+    auto row_of = [&](int t) { return (t ? tile_b : tile_a) * BQ; };                   // a query tile's first row,
+    auto rows_of = [&](int t) { return min(BQ, q_len - row_of(t)); };                  // its number of rows,
+    auto last_of = [&](int t) { return pos0 + (row_of(t) + rows_of(t) - 1) / hpq; };   // its last position
+    const int blk_lo = pos0 + min(row_of(0), row_of(1)) / hpq, blk_hi = max(last_of(0), last_of(1));
+    // Both query tiles read the same key tiles, each up to its last position.
+    const int k_begin = (first_visible(blk_lo, window, form.chunk) / BN) * BN;
+    const int k_end = min(kvl, blk_hi + 1);
     // Behind a window the first keep_first keys of a request stay visible: tiles over [0, sink_end) come
     // before the window's tiles.  Keys between the two are seen by no query of this block (k_begin is not
     // above any query's window).
     const int sink_end = bounded ? min(min(keep_first, k_begin), k_end) : 0;
     const int n_sink = (sink_end + BN - 1) / BN;
     const int n_tiles = n_sink + (k_end - k_begin + BN - 1) / BN;  // >= 1: the query's own key is visible
+    auto tiles_of = [&](int t) { return n_sink + (min(kvl, last_of(t) + 1) - k_begin + BN - 1) / BN; };
     auto tile_start = [&](int j) { return j < n_sink ? j * BN : k_begin + (j - n_sink) * BN; };
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     volatile int* abort_flag = abort_p;
 
     if (threadIdx.x == 0) {
         *abort_p = (smem_u32(smem) & 1023u) ? 10 : 0;     // misplaced tiles: nothing is issued
-        mbar_init(q_full, 1);
-        for (int s = 0; s < NK; ++s) { mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], 1); }
-        for (int s = 0; s < NV; ++s) { mbar_init(&v_full[s], 1); mbar_init(&v_empty[s], 1); }
-        for (int s = 0; s < 2; ++s) { mbar_init(&s_full[s], 1); mbar_init(&p_full[s], 128); }
-        mbar_init(o_done, 1);
+        for (int s = 0; s < NS; ++s) {
+            mbar_init(&k_full[s], 1); mbar_init(&v_full[s], 1);
+            mbar_init(&k_empty[s], tiles_q); mbar_init(&v_empty[s], tiles_q);     // every query tile has read it
+        }
+        for (int t = 0; t < QT; ++t) {
+            mbar_init(&q_full[t], 1);
+            for (int s = 0; s < 2; ++s) { mbar_init(&s_full[2 * t + s], 1); mbar_init(&p_full[2 * t + s], 8); }
+            mbar_init(&o_done[t], 1);
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    // Key and value stages start as zeros: rows that no copy fills (pages a window has released, the
-    // end of the last tile) are masked in S, and P = 0 times a finite stale value is 0.
-    for (int i = threadIdx.x; i < (NK * DKH + NV * DVH) * KV_HALF / 16; i += blockDim.x)
-        reinterpret_cast<uint4*>(sK)[i] = make_uint4(0u, 0u, 0u, 0u);
+    // Value stages start as zeros: rows that no copy fills (pages a window has released, the end of the last
+    // tile) meet P = 0, and zero times a finite stale value is 0.  (What K holds there is masked in S.)
+    for (int i = threadIdx.x; i < NS * DVH * KV_HALF / 16; i += THREADS)
+        reinterpret_cast<uint4*>(sV)[i] = make_uint4(0u, 0u, 0u, 0u);
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    if (warp == 1) {
+    if (warp == 18) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
                      ::"r"(smem_u32(tmem_base_p)), "r"(TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -186,146 +270,174 @@ attn_prefill_tc_kernel(const __grid_constant__ Maps maps, const int* __restrict_
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_base_p;
 
-    if (warp == 0) {
-        if (lane == 0) {
-            mbar_expect_tx(q_full, DKH * HALF_BYTES);
-            for (int hh = 0; hh < DKH; ++hh)
-                tma_load_2d(sQ + hh * HALF_BYTES, &maps.q, h * DK + hh * 64, q0 + qt * BQ, q_full);
+    if (warp == 16 || warp == 17) {
+        // producers: warp 16 the K tiles (and Q), warp 17 the V tiles
+        const bool is_k = warp == 16;
+        if (is_k && lane == 0) {
+            for (int t = 0; t < tiles_q; ++t) {
+                mbar_expect_tx(&q_full[t], DKH * HALF_BYTES);
+                for (int hh = 0; hh < DKH; ++hh)
+                    tma_load_2d(sQ + (t * DKH + hh) * HALF_BYTES, &maps.q, h * DK + hh * 64, q0 + row_of(t), &q_full[t]);
+            }
         }
         const int* table = block_table + (int64_t)b * max_pages;
-        const int pages_per_tile = BN / page_size;
+        const int pages_per_tile = BN / page_size, halves_n = is_k ? DKH : DVH;
         const uint32_t page_bytes = (uint32_t)page_size * 128u;
-        // One tile of K or of V: wait for its stage, look its pages up, copy those that exist (inside the
-        // request, not released by a window).  A K stage is free once S = Q K^T of two tiles before has
-        // run, a V stage once O += P V of two tiles before has: K runs a tile ahead of V.
-        auto load_tile = [&](int j, bool is_k) -> bool {
-            const int ns = is_k ? NK : NV;
-            const int halves = is_k ? DKH : DVH;
-            const int items = pages_per_tile * halves;    // page x 64-column half: one copy each
-            const int s = j % ns;
-            const uint32_t parity = ((j / ns) & 1) ^ 1;
-            const int k0 = tile_start(j);
-            int my_page = -1;                             // looked up before the wait: the latencies overlap
-            if (lane < pages_per_tile) {
-                const int kpos = k0 + lane * page_size;
-                if (kpos < kvl) my_page = UNFOLDED ? 0 : table[kpos / page_size];
-            }
+        // one copy per page and 64-column half: lane = page * halves + half (at most 8 x 4)
+        const int pg = lane / halves_n, hh = lane - pg * halves_n;
+        const bool mine = pg < pages_per_tile;
+        // the lane's page of tile j: inside the request and not released by a window, else -1
+        auto page_of = [&](int j) {
+            const int kpos = tile_start(j) + pg * page_size;
+            return !mine || j >= n_tiles || kpos >= kvl ? -1 : (UNFOLDED ? 0 : __ldg(table + kpos / page_size));
+        };
+        uint64_t* full = is_k ? k_full : v_full;
+        uint64_t* empty = is_k ? k_empty : v_empty;
+        uint8_t* base = is_k ? sK : sV;
+        int page = page_of(0);
+        for (int j = 0; j < n_tiles; ++j) {
+            const int next_page = page_of(j + 1);         // on its way while this tile's stage is waited for
+            const int s = j % NS;
             bool ok = true;
-            if (lane == 0) ok = mbar_wait(is_k ? &k_empty[s] : &v_empty[s], parity, abort_flag, is_k ? 11 : 21);
-            if (!__shfl_sync(0xffffffffu, ok, 0)) return false;
-            const unsigned have = __ballot_sync(0xffffffffu, my_page >= 0);
-            if (lane < pages_per_tile) tile_pages[lane] = my_page;
-            uint64_t* bar = is_k ? &k_full[s] : &v_full[s];
-            if (lane == 0) mbar_expect_tx(bar, (uint32_t)__popc(have) * page_bytes * halves);
+            if (lane == 0) ok = mbar_wait(&empty[s], ((j / NS) & 1) ^ 1, abort_flag, is_k ? 11 : 21);
+            if (!__shfl_sync(0xffffffffu, ok, 0)) break;
+            const unsigned have = __ballot_sync(0xffffffffu, page >= 0);
+            if (lane == 0) mbar_expect_tx(&full[s], (uint32_t)__popc(have) * page_bytes);
             __syncwarp();
-            for (int it = lane; it < items; it += 32) {
-                const int pg = it / halves, hh = it - pg * halves;
-                const int page = tile_pages[pg];
-                if (page < 0) continue;
-                uint8_t* dst = (is_k ? sK : sV) + (size_t)s * halves * KV_HALF + hh * KV_HALF + (size_t)pg * page_bytes;
+            if (page >= 0) {
+                uint8_t* dst = base + (size_t)s * halves_n * KV_HALF + hh * KV_HALF + (size_t)pg * page_bytes;
                 if constexpr (UNFOLDED) {
-                    const int row = kv_base + k0 + pg * page_size;
-                    if (!is_k) tma_load_2d(dst, &maps.v, h * uf.e + hh * 64, row, bar);
-                    else if (hh < dh) tma_load_2d(dst, &maps.k, h * uf.d + hh * 64, row, bar);
-                    else tma_load_2d(dst, &maps.kr, (hh - dh) * 64, row, bar);
+                    const int row = kv_base + tile_start(j) + pg * page_size;
+                    if (!is_k) tma_load_2d(dst, &maps.v, h * uf.e + hh * 64, row, &full[s]);
+                    else if (hh < dh) tma_load_2d(dst, &maps.k, h * uf.d + hh * 64, row, &full[s]);
+                    else tma_load_2d(dst, &maps.kr, (hh - dh) * 64, row, &full[s]);
                 } else {
-                    const int row = (page * nkv + hk) * page_size;
-                    tma_load_2d(dst, is_k ? &maps.k : &maps.v, hh * 64, row, bar);
+                    tma_load_2d(dst, is_k ? &maps.k : &maps.v, hh * 64, (page * nkv + hk) * page_size, &full[s]);
                 }
             }
-            __syncwarp();                                 // tile_pages is rewritten by the next call
-            return true;
-        };
-        constexpr int AHEAD = NK > 2 ? 2 : 1;             // K runs two tiles ahead of V (one with two stages)
-        for (int i = 0; i < n_tiles + AHEAD; ++i) {
-            if (i < n_tiles && !load_tile(i, true)) break;
-            if (i >= AHEAD && !load_tile(i - AHEAD, false)) break;
+            page = next_page;
         }
-    } else if (warp == 1) {
-        if (lane == 0) {
-            bool ok = *abort_flag == 0 && mbar_wait(q_full, 0, abort_flag, 12);
+    } else if (warp >= 18) {
+        // The whole warp walks through this, one lane issues: what describes the products stays in uniform registers
+        // (a single lane's branch moved every descriptor there product by product: 850 cycles for the eight of S).
+        const int t = warp - 18;
+        if (t < tiles_q) {
+            bool ok = *abort_flag == 0 && mbar_wait(&q_full[t], 0, abort_flag, 12);
+            const int n_mine = tiles_of(t);
+            const uint32_t tmem_t = tmem_base + t * COL_TILE;
             // descriptors of the tile origins; an offset of b bytes inside a tile adds b / 16 to the address field
-            const uint64_t dq = umma_desc(smem_u32(sQ));
+            const uint64_t dq = umma_desc(smem_u32(sQ + (size_t)t * DKH * HALF_BYTES));
+            const uint64_t dk0 = umma_desc(smem_u32(sK)), dv0 = umma_desc_mn(smem_u32(sV), KV_HALF);
             // S of tile j goes to buffer j & 1.  P of tile j overwrites S of tile j in place (bfloat16, two
             // keys per 32-bit column) and is the A operand of O += P V straight from tensor memory; S of
             // tile j + 2 goes to the same buffer and is issued once O += P V of tile j is complete.
-            auto issue_s = [&](int j) -> bool {
-                const int s = j % NK, buf = j & 1;
-                if (!mbar_wait(&k_full[s], (j / NK) & 1, abort_flag, 13)) return false;
+            auto issue_s = [&](int j) {                   // its K tile is there
+                const int s = j % NS, buf = j & 1;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint64_t dks = umma_desc(smem_u32(sK + (size_t)s * DKH * KV_HALF));
+                const uint64_t dks = dk0 + (uint32_t)((s * DKH * KV_HALF) >> 4);
+                if (elect_one()) {
 #pragma unroll
-                for (int kk = 0; kk < DK / 16; ++kk) {
-                    // columns that neither part fills are left out (what lies in K there is another head's)
-                    if (UNFOLDED && !(kk < dh * 4 ? kk < uf.d16 : kk - dh * 4 < uf.r16)) continue;
-                    const uint32_t sub = (uint32_t)(kk & 3) * 32;
-                    umma_bf16(tmem_base + COL_S + buf * BN, dq + (((uint32_t)(kk >> 2) * HALF_BYTES + sub) >> 4),
-                              dks + (((uint32_t)(kk >> 2) * KV_HALF + sub) >> 4), IDESC_S, kk > 0 ? 1u : 0u);
+                    for (int kk = 0; kk < DK / 16; ++kk) {
+                        // columns that neither part fills are left out (what lies in K there is another head's)
+                        if (UNFOLDED && !(kk < dh * 4 ? kk < uf.d16 : kk - dh * 4 < uf.r16)) continue;
+                        const uint32_t sub = (uint32_t)(kk & 3) * 32;
+                        umma_bf16(tmem_t + buf * BN, dq + (((uint32_t)(kk >> 2) * HALF_BYTES + sub) >> 4),
+                                  dks + (((uint32_t)(kk >> 2) * KV_HALF + sub) >> 4), IDESC_S, kk > 0 ? 1u : 0u);
+                    }
+                    umma_commit(&s_full[2 * t + buf]);
+                    umma_commit(&k_empty[s]);             // this query tile has read the K stage once these MMAs have run
                 }
-                umma_commit(&s_full[buf]);
-                umma_commit(&k_empty[s]);                 // the K stage is free once these MMAs have read it
-                return true;
+                __syncwarp();
             };
-            if (ok) ok = issue_s(0);
-            if (ok && n_tiles > 1) ok = issue_s(1);
-            for (int j = 0; j < n_tiles && ok; ++j) {
-                const int s = j % NV, buf = j & 1;
-                ok = mbar_wait(&p_full[buf], (j >> 1) & 1, abort_flag, 15) &&
-                     mbar_wait(&v_full[s], (j / NV) & 1, abort_flag, 16);
+            auto k_there = [&](int j) { return mbar_wait(&k_full[j % NS], (j / NS) & 1, abort_flag, 13); };
+            for (int j = 0; j < 2 && j < n_mine && ok; ++j) {
+                ok = __all_sync(0xffffffffu, k_there(j));
+                if (ok) issue_s(j);
+            }
+            for (int j = 0; j < n_mine && ok; ++j) {
+                const int s = j % NS, buf = j & 1;
+                ok = mbar_wait(&v_full[s], (j / NS) & 1, abort_flag, 16) &&
+                     mbar_wait(&p_full[2 * t + buf], (j >> 1) & 1, abort_flag, 15);
+                ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint64_t dvs = umma_desc_mn(smem_u32(sV + (size_t)s * DVH * KV_HALF), KV_HALF);
+                const uint64_t dvs = dv0 + (uint32_t)((s * DVH * KV_HALF) >> 4);
+                if (elect_one()) {
 #pragma unroll
-                for (int ks = 0; ks < BN / 16; ++ks)     // 16 keys of P are 8 columns of tensor memory
-                    umma_bf16_tmem_a(tmem_base + COL_O, tmem_base + COL_S + buf * BN + ks * 8,
-                                     dvs + (((uint32_t)ks * 2048) >> 4), IDESC_PV, (j > 0 || ks > 0) ? 1u : 0u);
-                umma_commit(&v_empty[s]);                 // the V stage is free once these MMAs have read it
-                umma_commit(o_done);                      // O holds tile j
-                if (j + 2 < n_tiles) ok = mbar_wait(o_done, j & 1, abort_flag, 14) && issue_s(j + 2);
+                    for (int ks = 0; ks < BN / 16; ++ks) // 16 keys of P are 8 columns of tensor memory
+                        umma_bf16_tmem_a(tmem_t + COL_O, tmem_t + buf * BN + ks * 8,
+                                         dvs + (((uint32_t)ks * 2048) >> 4), IDESC_PV, (j > 0 || ks > 0) ? 1u : 0u);
+                    umma_commit(&o_done[t]);              // O holds tile j
+                    umma_commit(&v_empty[s]);             // ... and has read the V stage
+                }
+                __syncwarp();
+                if (j + 2 < n_mine) {
+                    ok = k_there(j + 2) && mbar_wait(&o_done[t], j & 1, abort_flag, 14);
+                    ok = __all_sync(0xffffffffu, ok);
+                    if (ok) issue_s(j + 2);
+                }
+            }
+            // key tiles that only the other query tile reads: passed on as they arrive
+            for (int j = n_mine; j < n_tiles && ok; ++j) {
+                const int s = j % NS;
+                ok = k_there(j) && mbar_wait(&v_full[s], (j / NS) & 1, abort_flag, 16);
+                ok = __all_sync(0xffffffffu, ok);
+                if (ok && elect_one()) { mbar_arrive(&k_empty[s]); mbar_arrive(&v_empty[s]); }
+                __syncwarp();
             }
         }
-    } else {
-        // softmax and epilogue: thread = query row = tensor-memory lane
-        const int quarter = warp & 3;
-        const int r = quarter * 32 + lane;
-        const uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16);
+    } else if ((warp >> 3) < tiles_q) {
+        // softmax and epilogue: two threads to a query row (= lane of tensor memory), one half of a tile's keys each
+        const int t = warp >> 3, quarter = warp & 3, half = (warp >> 2) & 1, my0 = half * HK;
+        const int r = quarter * 32 + lane, pair_id = 1 + 4 * t + quarter;
+        const uint32_t lane_addr = tmem_base + t * COL_TILE + ((uint32_t)(quarter * 32) << 16);
+        const int tile_row0 = row_of(t), nq = rows_of(t), n_mine = tiles_of(t);
+        const int p_lo = pos0 + tile_row0 / hpq;          // position of the tile's first query
+        const int p_hi = p_lo + (nq - 1) / hpq;
         const int p_row = p_lo + r / hpq;                 // position of this thread's query
         const int vis_hi = min(p_row, kvl - 1);           // last visible key
         const int vis_lo = first_visible(p_row, window, form.chunk);   // first visible key
+        const int tile_vis_lo = first_visible(p_hi, window, form.chunk);
+        float* meet = halves + t * 4 * BQ;                // [2 in turn][2 halves][BQ]
         float m_ref = sink ? (form.sink_score ? form.sink_score[h] * 1.4426950408889634f : 0.f) : -INFINITY;   // reference of the exponentials, in log2 units
-        float l_run = sink ? 1.f : 0.f;
-        bool ok = true;
-        for (int j = 0; j < n_tiles; ++j) {
+        float l_run = sink && half == 0 ? 1.f : 0.f;
+        bool ok = true, together = true;                  // until both halves leave early, at a meeting
+        for (int j = 0; j < n_mine; ++j) {
             const int buf = j & 1;
-            const int k0 = tile_start(j);
-            ok = mbar_wait(&s_full[buf], (j >> 1) & 1, abort_flag, 17);
+            const int k0 = tile_start(j) + my0;
+            ok = ok && mbar_wait(&s_full[2 * t + buf], (j >> 1) & 1, abort_flag, 17);
             ok = __all_sync(0xffffffffu, ok);             // tcgen05.ld and .st are warp-wide: all lanes or none
-            if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            // the whole row of S to registers; the buffer is free for the tile after next at once
-            uint32_t v[BN];
-            const uint32_t s_addr = lane_addr + COL_S + buf * BN;
+            // the half's row of S to registers; once both halves have it, its place may take P
+            uint32_t v[HK];
+            const uint32_t s_addr = lane_addr + buf * BN;
+            if (ok) {
+                tmem_ld32(s_addr + my0, v);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            } else {
 #pragma unroll
-            for (int c0 = 0; c0 < BN; c0 += 32) tmem_ld32(s_addr + c0, *reinterpret_cast<uint32_t(*)[32]>(&v[c0]));
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                for (int i = 0; i < HK; ++i) v[i] = 0u;
+            }
             if constexpr (CAPPED) {
 #pragma unroll
-                for (int i = 0; i < BN; ++i)
+                for (int i = 0; i < HK; ++i)
                     v[i] = __float_as_uint(fast_tanh(__uint_as_float(v[i]) * cap_in) * cap_out);
             }
-            // does any (row, key) of this tile need the mask?
-            const bool masked = (k0 + BN - 1 > p_lo) || (k0 + BN > kvl) || (bounded && k0 < first_visible(p_hi, window, form.chunk));
+            // does any (row, key) of this half need the mask?
+            const bool masked = (k0 + HK - 1 > p_lo) || (k0 + HK > kvl) || (bounded && k0 < tile_vis_lo);
             // below a row's window only kept first keys are visible: of a tile of kept first keys those below
             // sink_end (such a tile lies below every window, so it is always masked key by key), of a window's
             // tile those below keep_first
             const int keep_lim = j < n_sink ? sink_end : keep_first;
-            uint32_t pk[BN / 2];
+            uint32_t pk[HK / 2];
             float alpha = 1.f;
             if constexpr (LOGISTIC) {
+                ok = together = pair_and(pair_id, ok);    // both halves have read S (or one gave up: both leave)
+                if (!ok) break;
                 // logistic(x) = 1 / (1 + 2^(-x log2 e)); the exponent is bounded so that the power stays finite
                 const float hb = head_bias[h] * 1.4426950408889634f;
 #pragma unroll
-                for (int i = 0; i < BN; i += 2) {
+                for (int i = 0; i < HK; i += 2) {
                     float w0 = __fdividef(1.0f, 1.0f + fast_exp2(fminf(-fmaf(__uint_as_float(v[i]), scale_log2, hb), 80.f)));
                     float w1 = __fdividef(1.0f, 1.0f + fast_exp2(fminf(-fmaf(__uint_as_float(v[i + 1]), scale_log2, hb), 80.f)));
                     if (masked) {
@@ -336,46 +448,52 @@ attn_prefill_tc_kernel(const __grid_constant__ Maps maps, const int* __restrict_
                     pk[i >> 1] = pack_bf16(w0, w1);
                 }
             } else {
-            float mxs[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};   // four chains, not one of BN steps
-            if (masked) {
+                float mxs[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};   // four chains, not one of HK steps
+                if (masked) {
 #pragma unroll
-                for (int i = 0; i < BN; ++i) {
-                    const int kj = k0 + i;
-                    if (kj > vis_hi || (kj < vis_lo && kj >= keep_lim)) v[i] = 0xff800000u;   // -inf
-                    mxs[i & 3] = fmaxf(mxs[i & 3], __uint_as_float(v[i]));
+                    for (int i = 0; i < HK; ++i) {
+                        const int kj = k0 + i;
+                        if (kj > vis_hi || (kj < vis_lo && kj >= keep_lim)) v[i] = 0xff800000u;   // -inf
+                    }
                 }
-            } else {
 #pragma unroll
-                for (int i = 0; i < BN; ++i) mxs[i & 3] = fmaxf(mxs[i & 3], __uint_as_float(v[i]));
-            }
-            // the scale is positive: the maximum of the scaled scores is the scaled maximum
-            const float mx = fmaxf(fmaxf(mxs[0], mxs[1]), fmaxf(mxs[2], mxs[3])) * scale_log2;
-            // the reference follows the maximum only when that moved by more than 8: exponentials stay
-            // below 2^8, and O needs scaling only then
-            if (mx > m_ref + 8.f || (m_ref == -INFINITY && mx > -INFINITY)) {
-                alpha = m_ref == -INFINITY ? 0.f : fast_exp2(m_ref - mx);
-                m_ref = mx;
-            }
-            const float base = m_ref == -INFINITY ? 0.f : m_ref;
-            float sums[4] = {0.f, 0.f, 0.f, 0.f};
+                for (int i = 0; i < HK; ++i) mxs[i & 3] = fmaxf(mxs[i & 3], __uint_as_float(v[i]));
+                // the scale is positive: the maximum of the scaled scores is the scaled maximum
+                const float mine = fmaxf(fmaxf(mxs[0], mxs[1]), fmaxf(mxs[2], mxs[3])) * scale_log2;
+                float* at = meet + buf * 2 * BQ + r;      // (the other half has read this place two barriers ago)
+                at[half * BQ] = mine;
+                ok = together = pair_and(pair_id, ok);    // both halves have read S and left their maxima (or one gave
+                if (!ok) break;                           // up: both leave)
+                const float mx = fmaxf(mine, at[(half ^ 1) * BQ]);
+                // the reference follows the maximum only when that moved by more than 8: exponentials stay
+                // below 2^8, and O needs scaling only then
+                if (mx > m_ref + 8.f || (m_ref == -INFINITY && mx > -INFINITY)) {
+                    alpha = m_ref == -INFINITY ? 0.f : fast_exp2(m_ref - mx);
+                    m_ref = mx;
+                }
+                const float base = m_ref == -INFINITY ? 0.f : m_ref;
+                float2 sums[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll
-            for (int i = 0; i < BN; i += 2) {
-                const float e0 = fast_exp2(fmaf(__uint_as_float(v[i]), scale_log2, -base));
-                const float e1 = fast_exp2(fmaf(__uint_as_float(v[i + 1]), scale_log2, -base));
-                sums[(i >> 1) & 3] += e0 + e1;
-                pk[i >> 1] = pack_bf16(e0, e1);
+                for (int i = 0; i < HK; i += 2) {
+                    float2 e = fma_two(make_float2(__uint_as_float(v[i]), __uint_as_float(v[i + 1])), scale_log2, -base);
+                    e.x = fast_exp2(e.x); e.y = fast_exp2(e.y);
+                    sums[(i >> 1) & 1] = add_two(sums[(i >> 1) & 1], e);
+                    pk[i >> 1] = pack_bf16(e.x, e.y);
+                }
+                l_run = l_run * alpha + ((sums[0].x + sums[0].y) + (sums[1].x + sums[1].y));
             }
-            l_run = l_run * alpha + ((sums[0] + sums[1]) + (sums[2] + sums[3]));
-            }
-            // O is scaled only after the O += P V of tile j - 1 is complete
+            // O is scaled only after O += P V of tile j - 1.  (S of tile j was issued after that of tile j - 2 was
+            // complete and that of tile j waits for this warp: the barrier is in phase j - 1 or j, which its
+            // parity tells apart, so the phases before need not have been followed one by one.)
             const bool rescale = !LOGISTIC && j > 0 && !__all_sync(0xffffffffu, alpha == 1.f);
-            if (rescale) ok = mbar_wait(o_done, (j - 1) & 1, abort_flag, 18);
-            ok = __all_sync(0xffffffffu, ok);
-            if (!ok) break;
             if (rescale) {
+                ok = mbar_wait(&o_done[t], (j - 1) & 1, abort_flag, 18);
+                ok = __all_sync(0xffffffffu, ok);
+            }
+            if (ok && rescale) {
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll 1
-                for (int c0 = 0; c0 < DV; c0 += 32) {
+                for (int c0 = half * (DV / 2); c0 < (half + 1) * (DV / 2); c0 += 32) {
                     uint32_t o[32];
                     tmem_ld32(lane_addr + COL_O + c0, o);
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
@@ -383,37 +501,37 @@ attn_prefill_tc_kernel(const __grid_constant__ Maps maps, const int* __restrict_
                     for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
                     tmem_st32(lane_addr + COL_O + c0, o);
                 }
-                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-            }
-            // Follow the O += P V barrier phase by phase, and do so BEFORE this tile's P is handed over:
-            // O += P V of tile j cannot complete before every thread has arrived below, so the barrier
-            // cannot run a second phase ahead of a thread that has not yet seen tile j - 1 complete (a
-            // parity wait that falls two phases behind never returns).  The product of tile j - 1 was
-            // issued a tile ago, so this seldom waits.
-            if (j > 0) {
-                ok = mbar_wait(o_done, (j - 1) & 1, abort_flag, 19);
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok) break;
             }
             // P over S in place: 64 keys are 32 columns of two bfloat16 each
-            tmem_st32(s_addr, pk);
-            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-            mbar_arrive_after_tmem(&p_full[buf]);
+            if (ok) {
+                tmem_st16(s_addr + half * (HK / 2), pk);
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&p_full[2 * t + buf]);
+            }
         }
-        if (ok) {
-            ok = mbar_wait(o_done, (n_tiles - 1) & 1, abort_flag, 20);
+        if (together) {
+            // the last two products in turn: a parity tells only neighbouring phases apart
+            ok = ok && (n_mine < 2 || mbar_wait(&o_done[t], (n_mine - 2) & 1, abort_flag, 19)) &&
+                 mbar_wait(&o_done[t], (n_mine - 1) & 1, abort_flag, 20);
             ok = __all_sync(0xffffffffu, ok);
+            // the halves' sums meet where the maxima of a tile more would
+            float* at = meet + (n_mine & 1) * 2 * BQ + r;
+            at[half * BQ] = l_run;
+            ok = pair_and(pair_id, ok);
+            l_run = at[0] + at[BQ];
         }
         if (ok) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             float inv = LOGISTIC ? 1.f : (l_run > 0.f ? 1.f / l_run : 0.f);
-            if (form.gate && r < nq) inv *= head_gate(form, q0 + qt * BQ + r, h);
+            if (form.gate && r < nq) inv *= head_gate(form, q0 + tile_row0 + r, h);
             const int ev = UNFOLDED ? uf.e : DV;          // columns of a value (a multiple of 8)
-            __nv_bfloat16* dst = out + ((int64_t)(q0 + qt * BQ + r) * nh + h) * ev;
+            __nv_bfloat16* dst = out + ((int64_t)(q0 + tile_row0 + r) * nh + h) * ev;
             const float* gt = UNFOLDED && uf.gate && r < nq
-                                  ? uf.gate + (int64_t)(q0 + qt * BQ + r) * uf.ldg + uf.gcol + h * ev : nullptr;
+                                  ? uf.gate + (int64_t)(q0 + tile_row0 + r) * uf.ldg + uf.gcol + h * ev : nullptr;
 #pragma unroll 1
-            for (int c0 = 0; c0 < DV; c0 += 32) {
+            for (int c0 = half * (DV / 2); c0 < (half + 1) * (DV / 2); c0 += 32) {
                 uint32_t o[32];
                 tmem_ld32(lane_addr + COL_O + c0, o);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
@@ -439,7 +557,7 @@ attn_prefill_tc_kernel(const __grid_constant__ Maps maps, const int* __restrict_
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (warp == 1) {
+    if (warp == 18) {
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
     }
     if (threadIdx.x == 0 && *abort_p != 0) atomicMax(status, *abort_p);
@@ -519,18 +637,18 @@ int mi_attn_prefill_tc(const void* q, const void* k_cache, const void* v_cache, 
         set_last_error("prefill attention (tcgen05): cuTensorMapEncodeTiled failed");
         return kLaunchFailed;
     }
-    const dim3 grid((max_q_len + pt::BQ - 1) / pt::BQ, nh, B);
+    const pt::QueryTiles order = pt::query_order(max_q_len, nh, B, d, window > 0 || chunk > 0);
+    const dim3 grid(pt::grid_x(max_q_len, nh, order), 1, B);
     const float scale_log2 = scale * 1.4426950408889634f;
-    const int dh = d / 64;
-    const size_t smem = (size_t)dh * pt::HALF_BYTES + (size_t)(pt::NK + pt::NV) * dh * pt::KV_HALF + 256;
+    const size_t smem = d == 64 ? pt::smem_bytes(64, 64) : pt::smem_bytes(128, 128);
     const float cap_in = cap > 0.f ? scale / cap : 0.f, cap_out = cap > 0.f ? cap / scale : 0.f;
 #define MI_PT(DD, CC)                                                                                     \
     do {                                                                                                  \
         auto kern = pt::attn_prefill_tc_kernel<DD, DD, CC>;                                               \
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);               \
-        kern<<<grid, 192, smem, stream>>>(maps, block_table, q_start, kv_len, (__nv_bfloat16*)out, nh,    \
+        kern<<<grid, pt::THREADS, smem, stream>>>(maps, block_table, q_start, kv_len, (__nv_bfloat16*)out, nh,    \
                                           nkv, page_size, max_pages, window, scale_log2, status,          \
-                                          keep_first, 1, cap_in, cap_out, sink, nullptr, pt::Unfolded{}, form);           \
+                                          keep_first, 1, cap_in, cap_out, sink, nullptr, pt::Unfolded{}, form, order);           \
     } while (0)
     if (cap > 0.f) { if (d == 64) MI_PT(64, true); else MI_PT(128, true); }
     else { if (d == 64) MI_PT(64, false); else MI_PT(128, false); }
@@ -572,17 +690,17 @@ int mi_attn_prefill_tc_logistic(const void* q, const void* k_cache, const void* 
         set_last_error("prefill attention (tcgen05): cuTensorMapEncodeTiled failed");
         return kLaunchFailed;
     }
-    const dim3 grid((max_q_len + pt::BQ - 1) / pt::BQ, nh, B);
+    const pt::QueryTiles order = pt::query_order(max_q_len, nh, B, dk, window > 0);
+    const dim3 grid(pt::grid_x(max_q_len, nh, order), 1, B);
     const float scale_log2 = scale * 1.4426950408889634f;
-    const size_t smem = (size_t)(dk / 64) * pt::HALF_BYTES +
-                        (size_t)(pt::NK * (dk / 64) + pt::NV * (dv / 64)) * pt::KV_HALF + 256;
 #define MI_PTL(KK, VV)                                                                                    \
     do {                                                                                                  \
         auto kern = pt::attn_prefill_tc_kernel<KK, VV, false, true>;                                      \
+        const size_t smem = pt::smem_bytes(KK, VV);                                                       \
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);               \
-        kern<<<grid, 192, smem, stream>>>(maps, block_table, q_start, kv_len, (__nv_bfloat16*)out, nh,    \
+        kern<<<grid, pt::THREADS, smem, stream>>>(maps, block_table, q_start, kv_len, (__nv_bfloat16*)out, nh,    \
                                           nkv, page_size, max_pages, window, scale_log2, status, 0, 1,    \
-                                          0.f, 0.f, 0, head_bias, pt::Unfolded{}, AttnForm{});                            \
+                                          0.f, 0.f, 0, head_bias, pt::Unfolded{}, AttnForm{}, order);                            \
     } while (0)
     if (dk == 64) { if (dv == 64) MI_PTL(64, 64); else MI_PTL(64, 128); }
     else { if (dv == 64) MI_PTL(128, 64); else MI_PTL(128, 128); }
@@ -625,17 +743,17 @@ int mi_attn_prefill_tc_shared(const void* q, const void* cache, const int* block
         return kLaunchFailed;
     }
     const int DKr = (dk + 63) / 64 * 64;
-    const dim3 grid(((int64_t)max_q_len * H + pt::BQ - 1) / pt::BQ, 1, B);
+    const pt::QueryTiles order = pt::query_order((int64_t)max_q_len * H, 1, B, DKr, window > 0);
+    const dim3 grid(pt::grid_x((int64_t)max_q_len * H, 1, order), 1, B);
     const float scale_log2 = scale * 1.4426950408889634f;
-    const size_t smem = (size_t)(DKr / 64) * pt::HALF_BYTES +
-                        (size_t)(pt::NK * (DKr / 64) + pt::NV * (dv / 64)) * pt::KV_HALF + 256;
 #define MI_PTS(KK, VV)                                                                                    \
     do {                                                                                                  \
         auto kern = pt::attn_prefill_tc_kernel<KK, VV>;                                                   \
+        const size_t smem = pt::smem_bytes(KK, VV);                                                       \
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);               \
-        kern<<<grid, 192, smem, stream>>>(maps, block_table, q_start, kv_len, (__nv_bfloat16*)out, 1, 1,  \
+        kern<<<grid, pt::THREADS, smem, stream>>>(maps, block_table, q_start, kv_len, (__nv_bfloat16*)out, 1, 1,  \
                                           page_size, max_pages, window, scale_log2, status, keep_first, H,  \
-                                          0.f, 0.f, 0, nullptr, pt::Unfolded{}, AttnForm{});                                \
+                                          0.f, 0.f, 0, nullptr, pt::Unfolded{}, AttnForm{}, order);                                \
     } while (0)
     if (dv == 64) {
         if (DKr == 64) MI_PTS(64, 64); else if (DKr == 128) MI_PTS(128, 64); else if (DKr == 192) MI_PTS(192, 64); else MI_PTS(256, 64);
@@ -685,23 +803,22 @@ int mi_attn_prefill_tc_unfolded(const void* q, const void* kv, const void* k_rot
         return kLaunchFailed;
     }
     const pt::Unfolded uf = {(d + 15) / 16, (r + 15) / 16, d, e, gate, ldg, gcol};
-    const dim3 grid((max_q_len + pt::BQ - 1) / pt::BQ, nh, B);
+    const pt::QueryTiles order = pt::query_order(max_q_len, nh, B, DKr, window > 0);
+    const dim3 grid(pt::grid_x(max_q_len, nh, order), 1, B);
     const float scale_log2 = scale * 1.4426950408889634f;
-    // two blocks share an SM wherever their tiles fit: from 192 key columns on with two K stages and one V stage
-#define MI_PTU(KK, VV, NKS, NVS)                                                                          \
+#define MI_PTU(KK, VV)                                                                                    \
     do {                                                                                                  \
-        const size_t smem = (size_t)(KK / 64) * pt::HALF_BYTES +                                          \
-                            (size_t)(NKS * (KK / 64) + NVS * (VV / 64)) * pt::KV_HALF + 256;              \
-        auto kern = pt::attn_prefill_tc_kernel<KK, VV, false, false, true, NKS, NVS>;                     \
+        const size_t smem = pt::smem_bytes(KK, VV);                                                       \
+        auto kern = pt::attn_prefill_tc_kernel<KK, VV, false, false, true>;                               \
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);               \
-        kern<<<grid, 192, smem, stream>>>(maps, nullptr, q_start, kv_len, (__nv_bfloat16*)out, nh, nh,    \
+        kern<<<grid, pt::THREADS, smem, stream>>>(maps, nullptr, q_start, kv_len, (__nv_bfloat16*)out, nh, nh, \
                                           pt::BN, 0, window, scale_log2, status, 0, 1, 0.f, 0.f, 0,       \
-                                          nullptr, uf, AttnForm{});                                                   \
+                                          nullptr, uf, AttnForm{}, order);                                                   \
     } while (0)
     if (DVr == 64) {
-        if (DKr == 128) MI_PTU(128, 64, 3, 2); else if (DKr == 192) MI_PTU(192, 64, 2, 2); else MI_PTU(256, 64, 2, 2);
+        if (DKr == 128) MI_PTU(128, 64); else if (DKr == 192) MI_PTU(192, 64); else MI_PTU(256, 64);
     } else {
-        if (DKr == 128) MI_PTU(128, 128, 3, 2); else if (DKr == 192) MI_PTU(192, 128, 2, 1); else MI_PTU(256, 128, 2, 2);
+        if (DKr == 128) MI_PTU(128, 128); else if (DKr == 192) MI_PTU(192, 128); else MI_PTU(256, 128);
     }
 #undef MI_PTU
     return finish_launch("attn_prefill_tc");
