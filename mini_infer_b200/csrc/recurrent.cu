@@ -412,6 +412,275 @@ delta_scan_kernel(const float* __restrict__ qkv, int ld_qkv, int64_t v_col0, con
         }
 }
 
+// ---------------------------------------------------------------------------
+// The delta rule with one decay per head, BLOCKS of 8 tokens at a time (long portions of the bfloat16 path; everything
+// float32).  Within a block that starts from S0, with G_t the product of the block's decays up to t,
+//   x_t = v_t - G_t S0^T k_t,   (I + L) u = beta x,   L_tj = beta_t (G_t / G_j) (k_t . k_j)  for j < t,
+//   o_t = G_t S0^T q_t + sum_{j <= t} (G_t / G_j) (q_t . k_j) u_j,   S = G_8 S0 + sum_t (G_8 / G_t) k_t u_t^T,
+// so the sums over S of eight tokens do not wait for one another.  delta_blocks_prepare_kernel makes ready, for all blocks
+// at once, unit q and k per key head and per head the 8 x 8 matrices that give (G_8 / G_t) u_t and the second term of o_t
+// from x; delta_blocks_scan_kernel walks.  The walk is bound by the reads of q and k from shared memory and the exchanges
+// of partial sums between lanes: a lane holds D / 16 rows of two columns of S (16 lanes to a column), so a row of
+// q or k that it reads serves two columns and a block's 32 sums take 30 exchanges.  2,048 tokens in prompts of 1,501 and
+// 547, 16 heads of 128 x 128: 512 us (454 walking, 58 making ready) token by token, 207 us (191 and 16) in blocks; the
+// distance from float64 is the same (1.0 of the other walk's over the tested forms).
+// ---------------------------------------------------------------------------
+constexpr int kBlockTokens = 8;
+constexpr int kBlockMats = 2 * kBlockTokens * kBlockTokens + kBlockTokens;     // floats per (block, head): W, O, G
+constexpr int kBlockCols = 16, kBlockStages = 3;
+
+// the first of a request's rows of block matrices: requests' blocks do not overlap, T / 8 + B rows hold them all
+__device__ __forceinline__ int64_t block_row0(int q0, int b) { return q0 / kBlockTokens + b; }
+
+// One warp per (block, key head); D = 64 or 128.  qk: [T][G][q D | k D]; mats: [row][H][W 8 x 8 | O 8 x 8 | G 8].
+template <int D>
+__global__ void __launch_bounds__(128)
+delta_blocks_prepare_kernel(const float* __restrict__ qkv, int ld_qkv, const float* __restrict__ beta_raw, int ld_beta,
+                            const float* __restrict__ a_raw, int ld_a, const float* __restrict__ a_log,
+                            const float* __restrict__ dt_bias, const int* __restrict__ q_start, float* __restrict__ qk,
+                            float* __restrict__ mats, int H, int G, float q_scale) {
+    constexpr int E = D / 32, N = kBlockTokens;          // numbers of a row per lane
+    __shared__ float sm[4][2][N][N + 1], inv_s[4][N][N + 1], rat_s[4][N][N + 1];
+    wait_for_earlier_kernels();
+    const int b = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int q0 = q_start[b], n = q_start[b + 1] - q0;
+    const int item = blockIdx.x * 4 + warp, blk = item / G, g = item - blk * G;
+    if (blk * N >= n) return;                            // uniform for the warp; no block barrier below
+    const int t0 = q0 + blk * N, nt = min(N, n - blk * N);
+    float q[N][E], k[N][E];
+#pragma unroll
+    for (int t = 0; t < N; ++t) {
+        float qq = 0.f, kk = 0.f;
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+            const float* row = qkv + (int64_t)(t0 + t) * ld_qkv + (int64_t)g * D + e * 32 + lane;
+            q[t][e] = t < nt ? row[0] : 0.f;
+            k[t][e] = t < nt ? row[(int64_t)G * D] : 0.f;
+            qq += q[t][e] * q[t][e]; kk += k[t][e] * k[t][e];
+        }
+        const float qn = q_scale / sqrtf(warp_sum(qq) + 1e-6f), kn = 1.0f / sqrtf(warp_sum(kk) + 1e-6f);
+        float* dst = qk + ((int64_t)(t0 + t) * G + g) * 2 * D + lane;
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+            q[t][e] *= qn; k[t][e] *= kn;
+            if (t < nt) { dst[e * 32] = q[t][e]; dst[D + e * 32] = k[t][e]; }
+        }
+    }
+    // k_t . k_j (j < t) and q_t . k_j (j <= t) to shared memory
+#pragma unroll
+    for (int t = 0; t < N; ++t) {
+#pragma unroll
+        for (int j = 0; j <= t; ++j) {
+            float kk = 0.f, qq = 0.f;
+#pragma unroll
+            for (int e = 0; e < E; ++e) { kk += k[t][e] * k[j][e]; qq += q[t][e] * k[j][e]; }
+            kk = warp_sum(kk); qq = warp_sum(qq);
+            if (lane == 0) { sm[warp][0][t][j] = kk; sm[warp][1][t][j] = qq; }
+        }
+    }
+    __syncwarp();
+    for (int h = g * (H / G); h < (g + 1) * (H / G); ++h) {
+        // lane t (of the first 8, repeated): its decay and write strength; a token past the end changes nothing
+        const int t = lane & 7;
+        float decay = 1.f, beta = 0.f;
+        if (t < nt) {
+            decay = expf(-expf(a_log[h]) * softplus_f(a_raw[(int64_t)(t0 + t) * ld_a + h] + dt_bias[h]));
+            beta = sigmoid_f(beta_raw[(int64_t)(t0 + t) * ld_beta + h]);
+        }
+        float* m = mats + ((block_row0(q0, b) + blk) * H + h) * kBlockMats;
+        // Every lane of a group of 8 holds column j = t of G_r / G_j (products of decays, not differences of logarithms,
+        // whose rounding would grow with their sum) and of (I + L)^-1 diag(beta), forward.
+        float x[N], ratio = 1.f, Gt = 1.f;
+#pragma unroll
+        for (int r = 0; r < N; ++r) {
+            const float gr = __shfl_sync(0xffffffffu, decay, r, 8);
+            ratio = r > t ? ratio * gr : 1.f;            // below the diagonal a product, on it 1
+            if (r <= t) Gt *= gr;
+            if (lane < 8) rat_s[warp][r][t] = r >= t ? ratio : 0.f;
+        }
+        __syncwarp();
+#pragma unroll
+        for (int r = 0; r < N; ++r) {
+            const float br = __shfl_sync(0xffffffffu, beta, r, 8);
+            float v = r == t ? beta : 0.f;
+#pragma unroll
+            for (int i = 0; i < r; ++i) v -= br * rat_s[warp][r][i] * sm[warp][0][r][i] * x[i];
+            x[r] = v;
+            if (lane < 8) inv_s[warp][r][t] = v;
+        }
+        __syncwarp();
+        for (int idx = lane; idx < N * N; idx += 32) {
+            const int r = idx >> 3, j = idx & 7;
+            float o = 0.f;
+#pragma unroll
+            for (int i = 0; i < N; ++i)
+                if (i <= r) o += rat_s[warp][r][i] * sm[warp][1][r][i] * inv_s[warp][i][j];
+            m[idx] = rat_s[warp][N - 1][r] * inv_s[warp][r][j];
+            m[N * N + idx] = o;
+        }
+        if (lane < 8) m[2 * N * N + lane] = Gt;
+        __syncwarp();                                    // both are written anew for the next head
+    }
+}
+
+template <int D> constexpr size_t delta_blocks_smem() {
+    return sizeof(float) * kBlockStages * (kBlockTokens * (2 * D + kBlockCols) + kBlockMats);
+}
+
+template <int D>
+__global__ void __launch_bounds__(128)
+delta_blocks_scan_kernel(const float* __restrict__ qkv, int ld_qkv, int64_t v_col0, const float* __restrict__ qk,
+                         const float* __restrict__ mats, float* __restrict__ state, int64_t state_stride,
+                         const int* __restrict__ q_start, const int* __restrict__ state_slot, float* __restrict__ out,
+                         int H, int G, int dv) {
+    extern __shared__ __align__(16) float sm[];
+    constexpr int N = kBlockTokens, MV = D / 64;         // 16-byte pieces of a row per lane
+    constexpr int STAGE = N * (2 * D + kBlockCols) + kBlockMats;
+    wait_for_earlier_kernels();
+    const int b = blockIdx.z, h = blockIdx.y, g = h / (H / G), col0 = blockIdx.x * kBlockCols;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int rg = lane & 15, cg = lane >> 4;
+    const int q0 = q_start[b], n = q_start[b + 1] - q0, blocks = (n + N - 1) / N;
+    const int64_t row0 = block_row0(q0, b);
+    const int wc = warp * 4 + cg * 2;                    // the lane's first column of the block's 16
+    float* S = state + (int64_t)state_slot[b] * state_stride + (int64_t)h * D * dv;
+    // rows 4 (rg + 16 m) + 2 p, + 1 of column wc + c
+    float2 s[2][2 * MV];
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+#pragma unroll
+        for (int m = 0; m < MV; ++m)
+#pragma unroll
+            for (int p = 0; p < 2; ++p) {
+                const int i = 4 * (rg + 16 * m) + 2 * p, col = col0 + wc + c;
+                s[c][2 * m + p] = col < dv ? make_float2(S[(int64_t)i * dv + col], S[(int64_t)(i + 1) * dv + col]) : make_float2(0.f, 0.f);
+            }
+    const int vt = tid >> 4, vc = tid & 15;              // the value this thread fetches
+    const bool v_ok = col0 + vc < dv;
+    auto fetch = [&](int blk) {
+        if (blk < blocks) {
+            float* st = sm + (blk % kBlockStages) * STAGE;
+            const int t0 = q0 + blk * N, nt = min(N, n - blk * N);
+            constexpr int PER = 2 * D / 4;               // 16-byte pieces of a token's q and k
+#pragma unroll
+            for (int i = 0; i < N * PER / 128; ++i) {
+                const int idx = tid + 128 * i, t = idx / PER, c = (idx - t * PER) * 4;
+                if (t < nt) copy_async_16(st + t * 2 * D + c, qk + ((int64_t)(t0 + t) * G + g) * 2 * D + c);
+                else *reinterpret_cast<float4*>(st + t * 2 * D + c) = make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+            float* vs = st + N * 2 * D;
+            if (vt < nt && v_ok) copy_async_f32(vs + tid, qkv + (int64_t)(t0 + vt) * ld_qkv + v_col0 + (int64_t)h * dv + col0 + vc);
+            else vs[tid] = 0.f;
+            if (tid < kBlockMats / 4) copy_async_16(vs + N * kBlockCols + 4 * tid, mats + ((row0 + blk) * H + h) * kBlockMats + 4 * tid);
+        }
+        copy_async_commit();
+    };
+    auto fma2 = [](float2 a, float2 x, float2 y) {       // a + x y, two numbers in one instruction
+        float2 r;
+        asm("{\n .reg .b64 a, x, y;\n mov.b64 a, {%2, %3};\n mov.b64 x, {%4, %5};\n mov.b64 y, {%6, %7};\n"
+            " fma.rn.f32x2 a, x, y, a;\n mov.b64 {%0, %1}, a;\n}"
+            : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(x.x), "f"(x.y), "f"(y.x), "f"(y.y));
+        return r;
+    };
+#pragma unroll
+    for (int i = 0; i < kBlockStages - 1; ++i) fetch(i);
+    for (int blk = 0; blk < blocks; ++blk) {
+        copy_async_wait_but_one();
+        __syncthreads();                                 // this block's rows are there; the stage before has been used
+        fetch(blk + kBlockStages - 1);
+        const float* st = sm + (blk % kBlockStages) * STAGE;
+        const float* vs = st + N * 2 * D;
+        const float* mt = vs + N * kBlockCols;
+        float pk[2][N], pq[2][N];
+        float4 k[N][MV];
+#pragma unroll
+        for (int t = 0; t < N; ++t) {
+            float4 q[MV];
+#pragma unroll
+            for (int m = 0; m < MV; ++m) {
+                q[m] = *reinterpret_cast<const float4*>(st + t * 2 * D + 4 * (rg + 16 * m));
+                k[t][m] = *reinterpret_cast<const float4*>(st + t * 2 * D + D + 4 * (rg + 16 * m));
+            }
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                float2 ak = make_float2(0.f, 0.f), aq = ak;
+#pragma unroll
+                for (int m = 0; m < MV; ++m) {
+                    ak = fma2(ak, s[c][2 * m], make_float2(k[t][m].x, k[t][m].y));
+                    aq = fma2(aq, s[c][2 * m], make_float2(q[m].x, q[m].y));
+                    ak = fma2(ak, s[c][2 * m + 1], make_float2(k[t][m].z, k[t][m].w));
+                    aq = fma2(aq, s[c][2 * m + 1], make_float2(q[m].z, q[m].w));
+                }
+                pk[c][t] = ak.x + ak.y; pq[c][t] = aq.x + aq.y;
+            }
+        }
+        // Sums over the 16 lanes of a column group, halving what a lane holds at each exchange: lane rg ends with token
+        // rg & 7 of column rg >> 3.
+        const bool hi8 = rg & 8, hi4 = rg & 4, hi2 = rg & 2, hi1 = rg & 1;
+#pragma unroll
+        for (int t = 0; t < N; ++t) {
+            pk[0][t] = (hi8 ? pk[1][t] : pk[0][t]) + __shfl_xor_sync(0xffffffffu, hi8 ? pk[0][t] : pk[1][t], 8);
+            pq[0][t] = (hi8 ? pq[1][t] : pq[0][t]) + __shfl_xor_sync(0xffffffffu, hi8 ? pq[0][t] : pq[1][t], 8);
+        }
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            pk[0][t] = (hi4 ? pk[0][t + 4] : pk[0][t]) + __shfl_xor_sync(0xffffffffu, hi4 ? pk[0][t] : pk[0][t + 4], 4);
+            pq[0][t] = (hi4 ? pq[0][t + 4] : pq[0][t]) + __shfl_xor_sync(0xffffffffu, hi4 ? pq[0][t] : pq[0][t + 4], 4);
+        }
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+            pk[0][t] = (hi2 ? pk[0][t + 2] : pk[0][t]) + __shfl_xor_sync(0xffffffffu, hi2 ? pk[0][t] : pk[0][t + 2], 2);
+            pq[0][t] = (hi2 ? pq[0][t + 2] : pq[0][t]) + __shfl_xor_sync(0xffffffffu, hi2 ? pq[0][t] : pq[0][t + 2], 2);
+        }
+        const float sk = (hi1 ? pk[0][1] : pk[0][0]) + __shfl_xor_sync(0xffffffffu, hi1 ? pk[0][0] : pk[0][1], 1);
+        const float sq = (hi1 ? pq[0][1] : pq[0][0]) + __shfl_xor_sync(0xffffffffu, hi1 ? pq[0][0] : pq[0][1], 1);
+        const int t = rg & 7, mc = wc + (rg >> 3);       // this lane's token and column
+        const float Gt = mt[2 * N * N + t];
+        const float x = vs[t * kBlockCols + mc] - Gt * sk;
+        float w = 0.f, o = Gt * sq;
+        float wm[N], om[N];
+#pragma unroll
+        for (int j = 0; j < N; j += 4) {
+            *reinterpret_cast<float4*>(wm + j) = *reinterpret_cast<const float4*>(mt + t * N + j);
+            *reinterpret_cast<float4*>(om + j) = *reinterpret_cast<const float4*>(mt + N * N + t * N + j);
+        }
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+            const float xj = __shfl_sync(0xffffffffu, x, (lane & 24) + j);
+            w += wm[j] * xj; o += om[j] * xj;
+        }
+        const int tok = blk * N + t, col = col0 + mc;
+        if (tok < n && col < dv) out[(int64_t)(q0 + tok) * H * dv + (int64_t)h * dv + col] = o;
+        const float Ge = mt[2 * N * N + N - 1];
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+#pragma unroll
+            for (int p = 0; p < 2 * MV; ++p) { s[c][p].x *= Ge; s[c][p].y *= Ge; }
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                const float wj = __shfl_sync(0xffffffffu, w, cg * 16 + c * 8 + j);
+                const float2 ww = make_float2(wj, wj);
+#pragma unroll
+                for (int m = 0; m < MV; ++m) {
+                    s[c][2 * m] = fma2(s[c][2 * m], ww, make_float2(k[j][m].x, k[j][m].y));
+                    s[c][2 * m + 1] = fma2(s[c][2 * m + 1], ww, make_float2(k[j][m].z, k[j][m].w));
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+#pragma unroll
+        for (int m = 0; m < MV; ++m)
+#pragma unroll
+            for (int p = 0; p < 2; ++p) {
+                const int i = 4 * (rg + 16 * m) + 2 * p, col = col0 + wc + c;
+                if (col < dv) { S[(int64_t)i * dv + col] = s[c][2 * m + p].x; S[(int64_t)(i + 1) * dv + col] = s[c][2 * m + p].y; }
+            }
+}
+
 // Gated linear attention walked in segments: for every token the query times the product of the decays since its
 // segment's start, qt[t][h][i] = q_t[i] * b_t[i] (what the start state must be read with), and per segment the whole
 // product bend[z][h][i].  A thread per (segment, head, key channel) multiplies its way through the segment.
@@ -908,6 +1177,41 @@ int mi_delta_scan_form(const float* qkv, int ld_qkv, const float* beta_raw, int 
     return delta_scan_launch(qkv, ld_qkv, beta_raw, ld_beta, a_raw, ld_a, a_log, dt_bias, state, state_stride, q_start,
                              state_slot, out, prep, T, B, H, G, d, dv, q_scale, form, tau, 1, 0, nullptr, nullptr, nullptr,
                              stream);
+}
+
+// The delta rule with one decay per head over blocks of 8 tokens (see delta_blocks_scan_kernel): keys of 64 or 128
+// numbers; qk holds T * G * 2 d floats, mats (T / 8 + B) * H * mi_delta_blocks_mats() floats, both 16-byte aligned.
+// The sums of a token run in another order than token by token: the two agree within rounding, not bit for bit.
+int mi_delta_blocks_supported(int d) { return d == 64 || d == 128; }
+int mi_delta_blocks_mats() { return kBlockMats; }
+
+int mi_delta_blocks(const float* qkv, int ld_qkv, const float* beta_raw, int ld_beta, const float* a_raw, int ld_a,
+                    const float* a_log, const float* dt_bias, float* state, int64_t state_stride, const int* q_start,
+                    const int* state_slot, float* out, float* qk, float* mats, int T, int B, int max_q_len, int H, int G,
+                    int d, int dv, float q_scale, cudaStream_t stream) {
+    if (B <= 0 || T <= 0) return kOk;
+    if (!mi_delta_blocks_supported(d) || dv < 1 || G < 1 || H % G || B > 65535 || H > 65535 || max_q_len < 1 || !beta_raw || !a_log) {
+        set_last_error("delta rule in blocks: %d heads over %d key heads of %d, values of %d, batch %d are not taken", H, G, d, dv, B);
+        return kBadShape;
+    }
+    if (!qk || !mats || ((reinterpret_cast<uintptr_t>(qk) | reinterpret_cast<uintptr_t>(mats)) & 15)) {
+        set_last_error("delta rule in blocks: the scratch is missing or not 16-byte aligned");
+        return kBadShape;
+    }
+    const int64_t items = ((int64_t)max_q_len + kBlockTokens - 1) / kBlockTokens * G;
+    const dim3 pgrid((unsigned)((items + 3) / 4), B), grid((dv + kBlockCols - 1) / kBlockCols, H, B);
+#define MI_DELTA_BLOCKS(D)                                                                                              \
+    do {                                                                                                                \
+        launch_dependent(delta_blocks_prepare_kernel<D>, pgrid, dim3(128), 0, stream, qkv, ld_qkv, beta_raw, ld_beta,    \
+                         a_raw, ld_a, a_log, dt_bias, q_start, qk, mats, H, G, q_scale);                                 \
+        const size_t smem = delta_blocks_smem<D>();                                                                     \
+        cudaFuncSetAttribute(delta_blocks_scan_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);       \
+        launch_dependent(delta_blocks_scan_kernel<D>, grid, dim3(128), smem, stream, qkv, ld_qkv, (int64_t)2 * G * d,    \
+                         (const float*)qk, (const float*)mats, state, state_stride, q_start, state_slot, out, H, G, dv); \
+    } while (0)
+    if (d == 64) MI_DELTA_BLOCKS(64); else MI_DELTA_BLOCKS(128);
+#undef MI_DELTA_BLOCKS
+    return finish_launch("delta_blocks", 2);
 }
 
 // Gated linear attention (form 2) with every request's portion walked as `segs` segments of seg_len tokens side by

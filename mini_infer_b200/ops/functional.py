@@ -1360,11 +1360,16 @@ def scan_segments(max_q_len: int, min_tokens: int, segment_tokens: int, max_segm
     return -(-max_q_len // per), per
 
 
+def delta_blocks_supported(d: int) -> bool:
+    """Whether :func:`delta_scan` walks keys of ``d`` numbers in blocks of tokens."""
+    return bool(library().mi_delta_blocks_supported(int(d)))
+
+
 def delta_scan(qkv: torch.Tensor, beta_raw: Optional[torch.Tensor], beta_col: int, a_raw: torch.Tensor, a_col: int,
                a_log: Optional[torch.Tensor], dt_bias: torch.Tensor, state: torch.Tensor, state_offset: int,
                q_start: torch.Tensor, state_slot: torch.Tensor, heads: int, key_heads: int, d: int, dv: int,
                q_scale: float, form: str = "channel_decay", tau: float = 1.0, segments: int = 1,
-               segment_tokens: int = 0) -> torch.Tensor:
+               segment_tokens: int = 0, blocks_of: int = 0) -> torch.Tensor:
     """Gated delta rule with a decay per head and key channel, token by token over every request's portion.
 
     ``form`` ``head_decay``: ONE decay per head (``a_raw`` holds ``heads`` columns and ``dt_bias`` ``heads``
@@ -1377,6 +1382,10 @@ def delta_scan(qkv: torch.Tensor, beta_raw: Optional[torch.Tensor], beta_col: in
     chained into every run's true start state and the read-outs corrected by ``(b_t q_t)^T S_start`` with ``b_t`` the
     product of the decays since the run's start.  The chain of dependent steps is a run's length, not the portion's;
     the sums of a token run in another order than in one piece, so the two agree within rounding, not bit for bit.
+
+    ``blocks_of`` > 0 (``head_decay`` only, keys of 64 or 128: :func:`delta_blocks_supported`): the length of the
+    longest portion; portions are walked in blocks of 8 tokens, whose sums over ``S`` do not wait for one another.
+    Again within rounding of the walk token by token, not bit for bit.
 
     ``qkv`` float32 ``[T, 2*key_heads*d + heads*dv]`` (q | k | v after their convolutions; the rows may go on
     with columns that are not read); ``beta_raw`` holds
@@ -1408,6 +1417,17 @@ def delta_scan(qkv: torch.Tensor, beta_raw: Optional[torch.Tensor], beta_col: in
     if DEBUG_BOUNDS:
         _dbg_range(state_slot, 0, state.shape[0], "delta_scan state_slot")
     out = torch.empty(T, heads * dv, dtype=F32, device=qkv.device)
+    if blocks_of > 0:
+        if form != "head_decay" or not delta_blocks_supported(d) or segments > 1:
+            raise ValueError(f"delta_scan: blocks of tokens are not built for '{form}' with keys of {d}")
+        qk = torch.empty(T * key_heads * 2 * d, dtype=F32, device=qkv.device)
+        mats = torch.empty((T // 8 + B) * heads * library().mi_delta_blocks_mats(), dtype=F32, device=qkv.device)
+        check(library().mi_delta_blocks(
+            _ptr(qkv), qkv.shape[1], beta_raw.data_ptr() + 4 * beta_col, beta_raw.shape[1], a_raw.data_ptr() + 4 * a_col,
+            a_raw.shape[1], _ptr(a_log), _ptr(dt_bias), state.data_ptr() + 4 * state_offset, state.shape[1],
+            _ptr(q_start), _ptr(state_slot), _ptr(out), _ptr(qk), _ptr(mats), T, B, int(blocks_of), heads, key_heads, d,
+            dv, float(q_scale), _stream()), "delta_scan")
+        return out
     # unit vectors, decays and write strengths of all tokens, made ready by a kernel before the walk
     prep = torch.empty(T * heads * library().mi_delta_scan_prep_row(d), dtype=F32, device=qkv.device)
     if segments > 1:

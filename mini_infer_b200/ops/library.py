@@ -46,6 +46,7 @@ _SIGNATURES = {
     "mi_grouped_gemm_tc": [P, P, P, P, P, I, I, I, I, I, I, F, F, P, P],
     "mi_grouped_gemm_tc_form": [P, P, P, P, P, I, I, I, I, I, I, I, F, F, P, P],
     "mi_random_fill": [P, I, L, ctypes.c_uint, ctypes.c_uint, F, F, P],
+    "mi_delta_blocks": [P, I, P, I, P, I, P, P, P, L, P, P, P, P, P, I, I, I, I, I, I, I, F, P],
     "mi_dense_f32": [P, P, P, I, I, I, P],
     "mi_l2_prefetch": [P, ctypes.c_ulonglong, P],
     "mi_causal_conv_silu": [P, I, P, P, I, P, L, P, P, P, P, I, I, I, I, I, P],
@@ -120,6 +121,8 @@ _OTHERS = {
     "mi_qkv_skinny_supported": ([I, I, I], c_int),
     "mi_dense_skinny_max_rows": ([], c_int),
     "mi_delta_scan_prep_row": ([I], c_int),
+    "mi_delta_blocks_supported": ([I], c_int),
+    "mi_delta_blocks_mats": ([], c_int),
     "mi_attn_mix_tc_supported": ([I, I, I, I], c_int),
     "mi_attn_mix_tc_splits": ([I], c_int),
     "mi_attn_mix_supported": ([I, I, I, I, I], c_int),

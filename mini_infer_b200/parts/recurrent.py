@@ -268,6 +268,13 @@ class GatedDelta(Mixer):
     def cache_need(self):
         return StateNeed((self.state_floats + max(self.conv_floats, 1),), torch.float32)
 
+    def _blocks_of(self, ctx: StepContext) -> int:
+        """The longest portion, if portions are walked in blocks of tokens.  (The float32 path walks token by token: its
+        sums run in one order however a prompt is cut.)"""
+        blocks = (self.rt.act == torch.bfloat16 and ctx.max_q_len >= TUNING.delta_blocks_min_tokens
+                  and F.delta_blocks_supported(self.d))
+        return ctx.max_q_len if blocks else 0
+
     def forward(self, x: torch.Tensor, ctx: StepContext, cache: CacheBinding) -> torch.Tensor:
         state = ctx.states[cache.group]
         proj = linear(x, self.w_in, torch.float32)
@@ -275,7 +282,7 @@ class GatedDelta(Mixer):
                                  ctx.q_start, ctx.req_of_token, ctx.state_slot)
         o = F.delta_scan(qkv, proj, self.col_beta, proj, self.col_decay, self.a_log, self.dt_bias, state, 0,
                          ctx.q_start, ctx.state_slot, self.nh, self.nkv, self.d, self.dv, self.d ** -0.5,
-                         form="head_decay")
+                         form="head_decay", blocks_of=self._blocks_of(ctx))
         y = F.gated_group_rmsnorm(o, proj, self.col_gate, self.norm_w, self.nh, False, self.eps, self.rt.act,
                                   silu_after=True)
         return linear(y, self.w_o, torch.float32)

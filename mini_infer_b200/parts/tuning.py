@@ -105,6 +105,10 @@ class Tuning:
     scan_segment_tokens: int = 128
     scan_max_segments: int = 32
 
+    # The delta rule with one decay per head (bfloat16 path): steps whose longest portion has at least this many tokens
+    # walk in blocks of 8 tokens.
+    delta_blocks_min_tokens: int = 8
+
     # Matrix memories with one gate per head and the gated linear recurrence per channel (bfloat16 path): portions of at
     # least so many tokens go over chunks of 64 tokens on the tensor cores, or in segments of 64 tokens side by side;
     # shorter ones are walked token by token.
