@@ -118,12 +118,6 @@ __device__ __forceinline__ bool pair_and(int id, bool ok) {
                  : "=r"(all) : "r"((uint32_t)ok), "r"(id) : "memory");
     return all != 0;
 }
-// one lane of a converged warp
-__device__ __forceinline__ bool elect_one() {
-    uint32_t is;
-    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(is));
-    return is != 0;
-}
 // two multiply-adds, two additions in one instruction (each rounded as by itself)
 __device__ __forceinline__ float2 fma_two(float2 a, float b, float c) {
     float2 r;
