@@ -122,6 +122,65 @@ causal_conv_silu_vec4_kernel(const float* __restrict__ x, int ldx, const float* 
     }
 }
 
+// The same for four taps (what the models use) over a window in registers: eleven rows are asked for at once and give
+// eight results, where a token by itself asked for its four rows after looking its request up.  2,048 tokens of 4,096
+// channels: 31.6 us, 28.4 us here.
+template <typename WT, typename OT, int FORM>
+__global__ void __launch_bounds__(128)
+causal_conv4_vec4_kernel(const float* __restrict__ x, int ldx, const float* __restrict__ in_bias, const WT* __restrict__ w, const WT* __restrict__ bias,
+                         const float* __restrict__ state, int64_t state_stride, const int* __restrict__ q_start,
+                         const int* __restrict__ req_of_token, const int* __restrict__ state_slot,
+                         OT* __restrict__ out, int ld_out, int C, int T) {
+    constexpr int N = 8, TAPS = 4;
+    wait_for_earlier_kernels();
+    const int c = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
+    if (c >= C) return;
+    float wt[4][TAPS];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+#pragma unroll
+        for (int j = 0; j < TAPS; ++j) wt[k][j] = to_float(w[(int64_t)(c + k) * TAPS + j]);
+    float4 bv = make_float4(0.f, 0.f, 0.f, 0.f), ib = bv;
+    if (bias) bv = make_float4(to_float(bias[c]), to_float(bias[c + 1]), to_float(bias[c + 2]), to_float(bias[c + 3]));
+    if (in_bias) ib = make_float4(in_bias[c], in_bias[c + 1], in_bias[c + 2], in_bias[c + 3]);
+    const int per = (T + gridDim.y - 1) / gridDim.y, t_end = min(T, ((int)blockIdx.y + 1) * per);
+    for (int t0 = blockIdx.y * per; t0 < t_end; t0 += N) {
+        float4 rows[N + TAPS - 1];                           // inputs of tokens t0 - 3 .. t0 + 7
+        int req[N], at[N];
+#pragma unroll
+        for (int u = 0; u < N + TAPS - 1; ++u) {
+            const int t = t0 - (TAPS - 1) + u;
+            rows[u] = t >= 0 && t < t_end ? __ldg(reinterpret_cast<const float4*>(x + (int64_t)t * ldx + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int u = 0; u < N; ++u) req[u] = __ldg(req_of_token + min(t0 + u, T - 1));
+#pragma unroll
+        for (int u = 0; u < N; ++u) at[u] = t0 + u - __ldg(q_start + req[u]);
+#pragma unroll
+        for (int u = 0; u < N; ++u) {
+            if (t0 + u >= t_end) break;
+            float4 acc = bv;
+#pragma unroll
+            for (int j = 0; j < TAPS; ++j) {
+                const int s = at[u] - (TAPS - 1 - j);        // position of the input of tap j in the request's portion
+                float4 v = rows[u + j];
+                if (s < 0) v = *reinterpret_cast<const float4*>(state + (int64_t)state_slot[req[u]] * state_stride + (int64_t)(s + TAPS - 1) * C + c);
+                else if (in_bias) { v.x += ib.x; v.y += ib.y; v.z += ib.z; v.w += ib.w; }
+                acc.x += wt[0][j] * v.x; acc.y += wt[1][j] * v.y; acc.z += wt[2][j] * v.z; acc.w += wt[3][j] * v.w;
+            }
+            OT* o = out + (int64_t)(t0 + u) * ld_out + c;
+            if (FORM == kConvResidual) {
+                const float4 xt = rows[u + TAPS - 1];
+                store4(o, make_float4(xt.x + acc.x, xt.y + acc.y, xt.z + acc.z, xt.w + acc.w));
+            } else if (FORM == kConvPlain) {
+                store4(o, acc);
+            } else {
+                store4(o, make_float4(silu_f(acc.x), silu_f(acc.y), silu_f(acc.z), silu_f(acc.w)));
+            }
+        }
+    }
+}
+
 // The last taps-1 inputs of every request after this step; one thread per (request, channel) moves its
 // entries in ascending order, so an entry is read before it is overwritten.
 __global__ void __launch_bounds__(256)
@@ -1005,6 +1064,37 @@ gated_group_rmsnorm_kernel(const float* __restrict__ y, const float* __restrict_
     }
 }
 
+// The same for groups of up to 128 columns on 16-byte boundaries, a warp per group and eight groups a block: a block of
+// one warp per group left the SMs waiting for blocks (2,048 rows of 16 groups of 128: 20 us, 12 us here for
+// 42 MB).  The sums run in the same order.
+template <typename AT, typename WT, int MODE>
+__global__ void __launch_bounds__(256)
+gated_group_rmsnorm_warp_kernel(const float* __restrict__ y, const float* __restrict__ gate, int ld_gate,
+                                const WT* __restrict__ w, int wlen, AT* __restrict__ out, int n, int gs, int groups,
+                                float eps, int64_t total) {
+    wait_for_earlier_kernels();
+    const int64_t item = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (item >= total) return;
+    const int64_t t = item / groups;
+    const int c0 = (int)(item - t * groups) * gs, i = 4 * (threadIdx.x & 31);
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f), g = v;
+    if (i < gs) {
+        v = *reinterpret_cast<const float4*>(y + t * n + c0 + i);
+        g = *reinterpret_cast<const float4*>(gate + t * ld_gate + c0 + i);
+        if (MODE == 0) { v.x *= silu_f(g.x); v.y *= silu_f(g.y); v.z *= silu_f(g.z); v.w *= silu_f(g.w); }
+    }
+    const float ss = warp_sum((v.x * v.x + v.y * v.y) + (v.z * v.z + v.w * v.w));
+    const float rr = 1.0f / sqrtf(ss / (float)gs + eps);
+    if (i >= gs) return;
+    const int wi = (c0 + i) % wlen;
+    v.x *= rr * to_float(w[wi]); v.y *= rr * to_float(w[wi + 1]);
+    v.z *= rr * to_float(w[wi + 2]); v.w *= rr * to_float(w[wi + 3]);
+    if (MODE == 1) { v.x *= sigmoid_f(g.x); v.y *= sigmoid_f(g.y); v.z *= sigmoid_f(g.z); v.w *= sigmoid_f(g.w); }
+    if (MODE == 2) { v.x *= silu_f(g.x); v.y *= silu_f(g.y); v.z *= silu_f(g.z); v.w *= silu_f(g.w); }
+    AT* o = out + t * n + c0 + i;
+    o[0] = from_float<AT>(v.x); o[1] = from_float<AT>(v.y); o[2] = from_float<AT>(v.z); o[3] = from_float<AT>(v.w);
+}
+
 }  // namespace mi
 
 using namespace mi;
@@ -1034,7 +1124,12 @@ static int launch_causal_conv(const float* x, int ldx, const float* in_bias, con
                       ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(state)) & 15) == 0;
 #define MI_CONV_LAUNCH(OT, FORM)                                                                                      \
     do {                                                                                                              \
-        if (vec4) {                                                                                                   \
+        if (vec4 && taps == 4) {                                                                                      \
+            MI_DISPATCH_1(wdtype, WT,                                                                                 \
+                launch_dependent(causal_conv4_vec4_kernel<WT, OT, FORM>, dim3((C / 4 + 127) / 128, ty), dim3(128), 0,     \
+                                 stream, x, ldx, in_bias, (const WT*)w, (const WT*)bias, (const float*)state, state_stride,    \
+                                 q_start, req_of_token, state_slot, (OT*)out, ld_out, C, T));                         \
+        } else if (vec4) {                                                                                            \
             MI_DISPATCH_1(wdtype, WT,                                                                                 \
                 launch_dependent(causal_conv_silu_vec4_kernel<WT, OT, FORM>, dim3((C / 4 + 127) / 128, ty), dim3(128), 0, \
                                  stream, x, ldx, in_bias, (const WT*)w, (const WT*)bias, (const float*)state, state_stride,    \
@@ -1266,6 +1361,16 @@ int mi_gated_group_rmsnorm(const float* y, const float* gate, int ld_gate, const
     const int work = vec ? gs / 4 : gs;      // a thread takes four floats where it can
     int threads = 32;
     while (threads < work && threads < 256) threads *= 2;
+    if (vec && threads == 32) {
+        const int64_t total = (int64_t)T * groups;
+        MI_DISPATCH_2(adtype, AT, wdtype, WT, {
+            auto kernel = mode == 0 ? gated_group_rmsnorm_warp_kernel<AT, WT, 0>
+                                    : (mode == 1 ? gated_group_rmsnorm_warp_kernel<AT, WT, 1> : gated_group_rmsnorm_warp_kernel<AT, WT, 2>);
+            launch_dependent(kernel, dim3((unsigned)((total + 7) / 8)), dim3(256), 0, stream, y, gate, ld_gate, (const WT*)w,
+                             wlen, (AT*)out, n, gs, groups, eps, total);
+        });
+        return finish_launch("gated_group_rmsnorm");
+    }
     MI_DISPATCH_2(adtype, AT, wdtype, WT,
         launch_dependent(gated_group_rmsnorm_kernel<AT, WT>, dim3(T, groups), dim3(threads), 0, stream, y, gate,
                          ld_gate, (const WT*)w, wlen, (AT*)out, n, gs, mode, eps, vec));
