@@ -81,6 +81,20 @@ __device__ __forceinline__ void store4(__nv_bfloat16* p, const float4& v) {
     u.y = *reinterpret_cast<unsigned int*>(&hi);
     *reinterpret_cast<uint2*>(p) = u;
 }
+// four consecutive values as floats; VEC: their address is a multiple of four elements
+template <bool VEC> __device__ __forceinline__ float4 load4f(const float* p) {
+    if (VEC) return __ldg(reinterpret_cast<const float4*>(p));
+    return make_float4(__ldg(p), __ldg(p + 1), __ldg(p + 2), __ldg(p + 3));
+}
+template <bool VEC> __device__ __forceinline__ float4 load4f(const __nv_bfloat16* p) {
+    if (VEC) {
+        const uint2 u = __ldg(reinterpret_cast<const uint2*>(p));
+        const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x));
+        const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
+        return make_float4(lo.x, lo.y, hi.x, hi.y);
+    }
+    return make_float4(to_float(p[0]), to_float(p[1]), to_float(p[2]), to_float(p[3]));
+}
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

@@ -274,9 +274,13 @@ qkv_post_kernel(const float* __restrict__ qkv, const WT* __restrict__ bias,
 
 // The same for many tokens in bfloat16 with the rotation over the whole head (or none) and
 // d a multiple of 8: one block per token, four pairs per thread and step (16-byte loads of the
-// float row, 8-byte stores), the angles' cosines and sines computed once when a thread keeps
-// its pair index for all heads.
-template <typename WT>
+// float row, 8-byte stores).  A block's threads form the token's cosines and sines once, a pair each, in shared
+// memory, and step through the heads without dividing: per thread these took more instructions than the rows
+// themselves.  2,048 tokens of 16 + 32 heads of 128: 22.4 us, 14.0 us with both and the bias four at a time
+// (75 MB; 17.4 us with its numbers one by one).
+constexpr int QKV_TABLE = 128;           // rotation pairs of a head that qkv_post_rows_kernel tables
+
+template <typename WT, bool BVEC>
 __global__ void __launch_bounds__(128)
 qkv_post_rows_kernel(const float* __restrict__ qkv, const WT* __restrict__ bias,
                      const int* __restrict__ positions, const float* __restrict__ inv_freq,
@@ -296,20 +300,23 @@ qkv_post_rows_kernel(const float* __restrict__ qkv, const WT* __restrict__ bias,
             kbase = (int64_t)page * nkv * page_size * d + (int64_t)off * d;
         }
     }
-    const bool same_i = (blockDim.x % per_head) == 0;
-    float cs[4] = {1.f, 1.f, 1.f, 1.f}, sn[4] = {0.f, 0.f, 0.f, 0.f};
-    if (same_i && inv_freq) {
-        const int i = 4 * (threadIdx.x % per_head);
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const float a = pos * inv_freq[i + u];
-            cs[u] = cosf(a); sn[u] = sinf(a);
+    // the token's angles, once for all heads, where a table holds them
+    __shared__ __align__(16) float cs_s[QKV_TABLE], sn_s[QKV_TABLE];
+    const bool tabled = inv_freq && half <= QKV_TABLE;
+    if (tabled) {
+        for (int i = threadIdx.x; i < half; i += blockDim.x) {
+            const float a = pos * inv_freq[i];
+            cs_s[i] = cosf(a); sn_s[i] = sinf(a);
         }
+        __syncthreads();
     }
+    // a thread's items lie `heads_step` heads apart at the same place of the head, unless the sizes are odd
+    const bool same_i = (blockDim.x % per_head) == 0;
+    const int my_head = threadIdx.x / per_head, my_i = 4 * (threadIdx.x - my_head * per_head), heads_step = blockDim.x / per_head;
     const int items = (nh + nkv) * per_head;
 #pragma unroll 4
-    for (int idx = threadIdx.x; idx < items; idx += blockDim.x) {
-        const int head = idx / per_head, i = 4 * (idx - head * per_head);
+    for (int idx = threadIdx.x, round = 0; idx < items; idx += blockDim.x, ++round) {
+        const int head = same_i ? my_head + round * heads_step : idx / per_head, i = same_i ? my_i : 4 * (idx - head * per_head);
         __nv_bfloat16* dst = nullptr;
         if (head < nh) dst = q_out + ((int64_t)t * nh + head) * d;
         else if (kbase >= 0) dst = k_cache + kbase + (int64_t)(head - nh) * page_size * d;
@@ -319,14 +326,16 @@ qkv_post_rows_kernel(const float* __restrict__ qkv, const WT* __restrict__ bias,
         const float4 h4 = *reinterpret_cast<const float4*>(row + c1);
         float lo[4] = {l4.x, l4.y, l4.z, l4.w}, hi[4] = {h4.x, h4.y, h4.z, h4.w};
         if (bias) {
-#pragma unroll
-            for (int u = 0; u < 4; ++u) { lo[u] += to_float(bias[c0 + u]); hi[u] += to_float(bias[c1 + u]); }
+            const float4 bl = load4f<BVEC>(bias + c0), bh = load4f<BVEC>(bias + c1);
+            lo[0] += bl.x; lo[1] += bl.y; lo[2] += bl.z; lo[3] += bl.w;
+            hi[0] += bh.x; hi[1] += bh.y; hi[2] += bh.z; hi[3] += bh.w;
         }
         float ylo[4], yhi[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-            float ca = cs[u], sa = sn[u];
-            if (!same_i && inv_freq) {
+            float ca = 1.f, sa = 0.f;
+            if (tabled) { ca = cs_s[i + u]; sa = sn_s[i + u]; }
+            else if (inv_freq) {
                 const float a = pos * inv_freq[i + u];
                 ca = cosf(a); sa = sinf(a);
             }
@@ -347,8 +356,8 @@ qkv_post_rows_kernel(const float* __restrict__ qkv, const WT* __restrict__ bias,
             const int c = (nh + nkv + hv) * d + i;
             float4 x = *reinterpret_cast<const float4*>(row + c);
             if (bias) {
-                x.x += to_float(bias[c]); x.y += to_float(bias[c + 1]);
-                x.z += to_float(bias[c + 2]); x.w += to_float(bias[c + 3]);
+                const float4 bv = load4f<BVEC>(bias + c);
+                x.x += bv.x; x.y += bv.y; x.z += bv.z; x.w += bv.w;
             }
             uint2 pk;
             pk.x = pack2(x.x, x.y); pk.y = pack2(x.z, x.w);
@@ -641,10 +650,13 @@ int mi_qkv_post(const float* qkv, const void* bias, int wdtype, const int* posit
     if (adtype == kBF16 && T >= 64 && d % 8 == 0 && (inv_freq == nullptr || rot_dim == d) &&
         (((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(q_out)) & 15) == 0) &&
         (nkv == 0 || ((reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache)) & 15) == 0)) {
-        MI_DISPATCH_1(wdtype, WT,
-            qkv_post_rows_kernel<WT><<<T, 128, 0, stream>>>(
-                qkv, (const WT*)bias, positions, inv_freq, slot_mapping, (__nv_bfloat16*)q_out,
-                (__nv_bfloat16*)k_cache, (__nv_bfloat16*)v_cache, nh, nkv, d, page_size));
+        // the bias four at a time where it lies on such a boundary
+        const bool bvec = (reinterpret_cast<uintptr_t>(bias) & (wdtype == kF32 ? 15 : 7)) == 0;
+        MI_DISPATCH_1(wdtype, WT, {
+            auto kernel = bvec ? qkv_post_rows_kernel<WT, true> : qkv_post_rows_kernel<WT, false>;
+            kernel<<<T, 128, 0, stream>>>(qkv, (const WT*)bias, positions, inv_freq, slot_mapping, (__nv_bfloat16*)q_out,
+                                          (__nv_bfloat16*)k_cache, (__nv_bfloat16*)v_cache, nh, nkv, d, page_size);
+        });
         return finish_launch("qkv_post");
     }
     // few tokens: many blocks of a few heads; many tokens: a block per token, which looks up its
