@@ -746,7 +746,7 @@ int mi_attn_decode_split_form(const void* q, const void* k_cache, const void* v_
         launch_dependent(attn_decode_split_kernel<AT, DD, SS>, grid, dim3(128), 0, stream,                \
             (const AT*)q, (const AT*)k_cache, (const AT*)v_cache, block_table, q_start, kv_len, part_o,  \
             part_ml, nh, nkv, page_size, max_pages, max_splits, window, scale, cap, chunk);               \
-        launch_dependent(attn_decode_merge_kernel<AT, DD, SS>, mgrid, dim3(DD <= 128 ? DD : 128), 0, stream, \
+        launch_behind(attn_decode_merge_kernel<AT, DD, SS>, mgrid, dim3(DD <= 128 ? DD : 128), 0, stream, \
             part_o, part_ml, q_start, kv_len, (AT*)out, nh, max_splits, window, sink, form);              \
     } while (0)
 #define MI_DEC_D(SS) do { if (d == 64) MI_DEC(64, SS); else if (d == 128) MI_DEC(128, SS); else MI_DEC(256, SS); } while (0)

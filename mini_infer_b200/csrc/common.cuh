@@ -149,8 +149,8 @@ __device__ __forceinline__ void allow_next_kernel() { asm volatile("griddepcontr
 bool dependent_launch_enabled();
 
 template <typename... P, typename... A>
-inline cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
-                                    A... args) {
+inline cudaError_t launch_placed_early(bool early, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
+                                       cudaStream_t stream, A... args) {
     cudaLaunchConfig_t lc = {};
     lc.gridDim = grid;
     lc.blockDim = block;
@@ -160,8 +160,19 @@ inline cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block,
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     lc.attrs = attr;
-    lc.numAttrs = dependent_launch_enabled() ? 1 : 0;
+    lc.numAttrs = early ? 1 : 0;
     return cudaLaunchKernelEx(&lc, kernel, static_cast<P>(args)...);
+}
+template <typename... P, typename... A>
+inline cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                                    A... args) {
+    return launch_placed_early(dependent_launch_enabled(), kernel, grid, block, smem, stream, args...);
+}
+// The same whatever the step's size, for the kernel behind another of the same call: a launch's latency (about a
+// microsecond between kernels of tens) overlaps the tail of the kernel before.
+template <typename... P, typename... A>
+inline cudaError_t launch_behind(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args) {
+    return launch_placed_early(true, kernel, grid, block, smem, stream, args...);
 }
 
 // What else an attention over the paged cache may be asked for (all zero: nothing).

@@ -1040,10 +1040,10 @@ int mi_memory_chunks(const void* proj, int ld, int col_q, int col_k, int col_v, 
         cudaFuncSetAttribute(mem::memory_chunk_outputs_kernel<LOG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_o); \
         launch_dependent(mem::memory_chunk_states_kernel<LOG>, dim3(chunks, H * tiles, B), dim3(128), smem_s, stream, in, \
                          (const float4*)gates, (const float4*)logs, decay, q_start, U, Un, keepc, H, d, dv, dvp, dp, tiles); \
-        launch_dependent(mem::memory_chunk_chain_kernel, dim3((d * (dvp / 8) + 255) / 256 + (LOG ? 1 : 0), H, B), dim3(256), \
+        launch_behind(mem::memory_chunk_chain_kernel, dim3((d * (dvp / 8) + 255) / 256 + (LOG ? 1 : 0), H, B), dim3(256), \
                          0, stream, U, LOG ? Un : nullptr, (const float*)keepc, state, stride, s_off, n_off, q_start,  \
                          state_slot, H, d, dv, dvp);                                                                   \
-        launch_dependent(mem::memory_chunk_outputs_kernel<LOG>, dim3(chunks, H * groups, B), dim3(256), smem_o, stream, in, \
+        launch_behind(mem::memory_chunk_outputs_kernel<LOG>, dim3(chunks, H * groups, B), dim3(256), smem_o, stream, in, \
                          (const float4*)gates, (const float4*)logs, decay, q_start, (const float*)U, (const float*)Un, out, \
                          den, H, d, dv, dvp, dp, tiles, per, groups);                                                  \
     } while (0)

@@ -130,16 +130,17 @@ __global__ void __launch_bounds__(128)
 causal_conv4_vec4_kernel(const float* __restrict__ x, int ldx, const float* __restrict__ in_bias, const WT* __restrict__ w, const WT* __restrict__ bias,
                          const float* __restrict__ state, int64_t state_stride, const int* __restrict__ q_start,
                          const int* __restrict__ req_of_token, const int* __restrict__ state_slot,
-                         OT* __restrict__ out, int ld_out, int C, int T) {
+                         OT* __restrict__ out, int ld_out, int C, int T, bool w_vec) {
     constexpr int N = 8, TAPS = 4;
     wait_for_earlier_kernels();
     const int c = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
     if (c >= C) return;
     float wt[4][TAPS];
 #pragma unroll
-    for (int k = 0; k < 4; ++k)
-#pragma unroll
-        for (int j = 0; j < TAPS; ++j) wt[k][j] = to_float(w[(int64_t)(c + k) * TAPS + j]);
+    for (int k = 0; k < 4; ++k) {                            // a channel's taps are four numbers side by side
+        const float4 f = w_vec ? load4f<true>(w + (int64_t)(c + k) * TAPS) : load4f<false>(w + (int64_t)(c + k) * TAPS);
+        wt[k][0] = f.x; wt[k][1] = f.y; wt[k][2] = f.z; wt[k][3] = f.w;
+    }
     float4 bv = make_float4(0.f, 0.f, 0.f, 0.f), ib = bv;
     if (bias) bv = make_float4(to_float(bias[c]), to_float(bias[c + 1]), to_float(bias[c + 2]), to_float(bias[c + 3]));
     if (in_bias) ib = make_float4(in_bias[c], in_bias[c + 1], in_bias[c + 2], in_bias[c + 3]);
@@ -1122,13 +1123,14 @@ static int launch_causal_conv(const float* x, int ldx, const float* in_bias, con
     if (ty > 65535) ty = 65535;
     const bool vec4 = C % 4 == 0 && ldx % 4 == 0 && ld_out % 4 == 0 && state_stride % 4 == 0 &&
                       ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(state)) & 15) == 0;
+    const bool w_vec = (reinterpret_cast<uintptr_t>(w) & (wdtype == kF32 ? 15 : 7)) == 0;
 #define MI_CONV_LAUNCH(OT, FORM)                                                                                      \
     do {                                                                                                              \
         if (vec4 && taps == 4) {                                                                                      \
             MI_DISPATCH_1(wdtype, WT,                                                                                 \
                 launch_dependent(causal_conv4_vec4_kernel<WT, OT, FORM>, dim3((C / 4 + 127) / 128, ty), dim3(128), 0,     \
                                  stream, x, ldx, in_bias, (const WT*)w, (const WT*)bias, (const float*)state, state_stride,    \
-                                 q_start, req_of_token, state_slot, (OT*)out, ld_out, C, T));                         \
+                                 q_start, req_of_token, state_slot, (OT*)out, ld_out, C, T, w_vec));                  \
         } else if (vec4) {                                                                                            \
             MI_DISPATCH_1(wdtype, WT,                                                                                 \
                 launch_dependent(causal_conv_silu_vec4_kernel<WT, OT, FORM>, dim3((C / 4 + 127) / 128, ty), dim3(128), 0, \
@@ -1149,7 +1151,7 @@ static int launch_causal_conv(const float* x, int ldx, const float* in_bias, con
 #undef MI_CONV_LAUNCH
     int launched = 1;
     if (taps > 1) {
-        launch_dependent(conv_state_update_kernel, dim3(cb, B), dim3(256), 0, stream, x, ldx, in_bias, state, state_stride,
+        launch_behind(conv_state_update_kernel, dim3(cb, B), dim3(256), 0, stream, x, ldx, in_bias, state, state_stride,
                          q_start, state_slot, C, taps);
         launched = 2;
     }
@@ -1301,7 +1303,7 @@ int mi_delta_blocks(const float* qkv, int ld_qkv, const float* beta_raw, int ld_
                          a_raw, ld_a, a_log, dt_bias, q_start, qk, mats, H, G, q_scale);                                 \
         const size_t smem = delta_blocks_smem<D>();                                                                     \
         cudaFuncSetAttribute(delta_blocks_scan_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);       \
-        launch_dependent(delta_blocks_scan_kernel<D>, grid, dim3(128), smem, stream, qkv, ld_qkv, (int64_t)2 * G * d,    \
+        launch_behind(delta_blocks_scan_kernel<D>, grid, dim3(128), smem, stream, qkv, ld_qkv, (int64_t)2 * G * d,    \
                          (const float*)qk, (const float*)mats, state, state_stride, q_start, state_slot, out, H, G, dv); \
     } while (0)
     if (d == 64) MI_DELTA_BLOCKS(64); else MI_DELTA_BLOCKS(128);
