@@ -1025,15 +1025,24 @@ int mi_memory_chunks(const void* proj, int ld, int col_q, int col_k, int col_v, 
     const int vec = d % 8 == 0 && dv % 8 == 0 && ld % 8 == 0 && col_q % 8 == 0 && col_k % 8 == 0 && col_v % 8 == 0 &&
                     (reinterpret_cast<uintptr_t>(proj) & 15) == 0;
     const mem::RowsB in = {(const __nv_bfloat16*)proj, ld, col_q, col_k, col_v, act, q_scale, vec};
-    // value tiles a block of the outputs walks over: as many as leave two blocks per SM
-    const int64_t blocks = (int64_t)chunks * H * tiles * B;
-    int per = (int)(blocks / 296);
-    per = per < 1 ? 1 : (per > tiles ? tiles : per);
-    const int groups = (tiles + per - 1) / per;
     const size_t rows_bytes = (size_t)mem::kC * (dp + 8) * 2, v_bytes = (size_t)mem::kC * mem::kVP * 2;
     const size_t s_bytes = (size_t)dp * (mem::kT * 4 + 16);
     const size_t smem_s = rows_bytes + 2 * v_bytes;
     const size_t smem_o = rows_bytes + v_bytes + (rows_bytes > s_bytes ? rows_bytes : s_bytes);
+    // Value tiles that a block of the outputs walks over: the number with the least work in turn, rounds of as many
+    // blocks as the device holds times a block's tiles and the queries, keys and scores before them (about one and a
+    // half tiles).  2,048 tokens, 4 heads of 8 tiles: 256 blocks of 4 in one round 36.5 us, 384 blocks of 3 in two 46.4 us.
+    // (The states' kernel, which is bound by what it writes, gains nothing from several tiles a block.)
+    int64_t held = 227 * 1024 / ((int64_t)smem_o + 2048);
+    held = 148 * (held < 1 ? 1 : (held > 8 ? 8 : held));
+    int per = 1;
+    float least = 0.f;
+    for (int p = 1; p <= tiles; ++p) {
+        const int64_t blocks = (int64_t)chunks * H * B * ((tiles + p - 1) / p);
+        const float cost = (float)((blocks + held - 1) / held) * ((float)p + 1.5f);
+        if (p == 1 || cost < least) { per = p; least = cost; }
+    }
+    const int groups = (tiles + per - 1) / per;
 #define MI_CHUNKS(LOG)                                                                                                 \
     do {                                                                                                               \
         cudaFuncSetAttribute(mem::memory_chunk_states_kernel<LOG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_s); \
