@@ -156,22 +156,24 @@ attn_tiled_kernel(const AT* __restrict__ q, const AT* __restrict__ k_cache, cons
 }
 
 // ---------------------------------------------------------------------------
-// The same in 32 bits for heads of 64 and 128: 32 queries of one head per block of 4 warps, key tiles of 32 at the same
+// The same in 32 bits for heads of 64 and 128: 32 queries of one head per block of 2 x 4 warps, key tiles of 32 at the same
 // absolute positions, one order of additions for every row whatever its step: a dot product is one chain of fused
-// multiply-adds over the head's numbers, an output one chain over the keys of a tile after its scaling.  Bound by the FMA
-// pipes and the reads of shared memory that feed them: a warp owns 8 queries through both products (no barrier
-// between them), with 2 x 4 scores and then 4 x (D / 16) outputs a thread, two of these per instruction; the next tile's
-// keys and values come by cp.async meanwhile; a warp passes over tiles that none of its queries sees.  512 queries of
-// 16 heads of 128 behind 700 keys: 876 us with the kernel above (one score or output per read pair of operands), 196 us.
+// multiply-adds over the head's numbers, an output one chain over the keys of a tile after its scaling; the tiles of even
+// and of odd number are walked side by side, by four warps each, and the two walks' rows meet at the end.  A warp owns 8
+// queries through both products (no block-wide barrier between them), with 2 x 4 scores and then 4 x (D / 16) outputs a
+// thread, two of these per instruction; it passes over tiles that none of its queries sees.  512 queries of 16 heads of
+// 128 behind 700 keys: 196 us in one walk of four warps with two buffers, 184 us in two with a buffer each (16 queries a
+// warp, with a third fewer reads of shared memory per product, 187 us); 876 us with the kernel above, which reads a pair of
+// operands per multiply-add.
 // ---------------------------------------------------------------------------
 constexpr int FQ = 32, FK = 32;
 
 template <int D> constexpr size_t rows_f32_smem() {
-    return sizeof(float) * (FQ * (D + 4) + 2 * (FK * (D + 4) + FK * D) + FQ * FK + FQ) + sizeof(int) * 2 * FK;
+    return sizeof(float) * (FQ * (D + 4) + 2 * (FK * (D + 4) + FK * D) + 2 * (FQ * FK + FQ)) + sizeof(int) * 2 * FK;
 }
 
 template <int D>
-__global__ void __launch_bounds__(128, 2)
+__global__ void __launch_bounds__(256, 2)
 attn_rows_f32_kernel(const float* __restrict__ q, const float* __restrict__ k_cache, const float* __restrict__ v_cache,
                      const int* __restrict__ block_table, const int* __restrict__ q_start, const int* __restrict__ kv_len,
                      float* __restrict__ out, int nh, int nkv, int page_size, int max_pages, int window, float scale) {
@@ -181,13 +183,15 @@ attn_rows_f32_kernel(const float* __restrict__ q, const float* __restrict__ k_ca
     const int q0 = q_start[b], q_len = q_start[b + 1] - q0;
     if (qt * FQ >= q_len) return;
     const int kvl = kv_len[b], hk = h / (nh / nkv);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int walk = threadIdx.x >> 7, tid = threadIdx.x & 127, warp = tid >> 5, lane = tid & 31;
     float* Qs = smem;                              // [FQ][QP]
-    float* Ks = Qs + FQ * QP;                      // [2][FK][QP]
-    float* Vs = Ks + 2 * FK * QP;                  // [2][FK][D]
-    float* Ps = Vs + 2 * FK * D + warp * 8 * FK;   // the warp's [FK][8]: key, query
-    float* As = Vs + 2 * FK * D + FQ * FK + warp * 8;     // the warp's 8 factors
-    int* there = reinterpret_cast<int*>(Vs + 2 * FK * D + FQ * FK + FQ);          // [2][FK]: the key has a page
+    float* Ks = Qs + FQ * QP + walk * FK * (QP + D);      // the walk's [FK][QP]
+    float* Vs = Ks + FK * QP;                      // ... and [FK][D]
+    float* behind = Qs + FQ * QP + 2 * FK * (QP + D);
+    float* Ps = behind + (walk * 4 + warp) * 8 * FK;      // the warp's [FK][8]: key, query
+    float* As = behind + 2 * FQ * FK + (walk * 4 + warp) * 8;     // the warp's 8 factors
+    int* there = reinterpret_cast<int*>(behind + 2 * FQ * FK + 2 * FQ) + walk * FK;      // [FK]: the key has a page
+    auto walk_sync = [&] { asm volatile("bar.sync %0, 128;" ::"r"(1 + walk) : "memory"); };
 
     const int nq = min(FQ, q_len - qt * FQ);
     const int p_lo = kvl - q_len + qt * FQ;        // position of the block's first query
@@ -196,15 +200,15 @@ attn_rows_f32_kernel(const float* __restrict__ q, const float* __restrict__ k_ca
     k_begin = (k_begin / FK) * FK;
     const int* table = block_table + (int64_t)b * max_pages;
 
-    auto ask = [&](int kt, int buf) {              // 4 threads a key row
+    auto ask = [&](int kt) {              // 4 threads a key row
         const int r = tid >> 2, kj = kt + r;
         int page = -1;
         if (kj < k_end) page = __ldg(table + kj / page_size);
         const bool in = page >= 0;
         const int64_t off = in ? (((int64_t)page * nkv + hk) * page_size + kj % page_size) * D : 0;
-        if ((tid & 3) == 0) there[buf * FK + r] = in;
-        const uint32_t kd = (uint32_t)__cvta_generic_to_shared(Ks + (buf * FK + r) * QP);
-        const uint32_t vd = (uint32_t)__cvta_generic_to_shared(Vs + (buf * FK + r) * D);
+        if ((tid & 3) == 0) there[r] = in;
+        const uint32_t kd = (uint32_t)__cvta_generic_to_shared(Ks + r * QP);
+        const uint32_t vd = (uint32_t)__cvta_generic_to_shared(Vs + r * D);
         const int n = in ? 16 : 0;                 // nothing read: zeros
 #pragma unroll
         for (int i = 0; i < D / 16; ++i) {
@@ -212,11 +216,9 @@ attn_rows_f32_kernel(const float* __restrict__ q, const float* __restrict__ k_ca
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(kd + c * 4), "l"(k_cache + off + c), "r"(n) : "memory");
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(vd + c * 4), "l"(v_cache + off + c), "r"(n) : "memory");
         }
-        asm volatile("cp.async.commit_group;" ::: "memory");
     };
 
-    ask(k_begin, 0);
-    for (int idx = tid; idx < FQ * (D / 4); idx += 128) {
+    for (int idx = threadIdx.x; idx < FQ * (D / 4); idx += 256) {
         const int i = idx / (D / 4), c = idx - i * (D / 4);
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
         if (i < nq) v = __ldg(reinterpret_cast<const float4*>(q + ((int64_t)(q0 + qt * FQ + i) * nh + h) * D) + c);
@@ -237,11 +239,13 @@ attn_rows_f32_kernel(const float* __restrict__ q, const float* __restrict__ k_ca
 #pragma unroll
         for (int j = 0; j < 2 * NC; ++j) acc[i][j] = 0ull;
 
-    int buf = 0;
-    for (int kt = k_begin; kt < k_end; kt += FK, buf ^= 1) {
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-        __syncthreads();                           // this tile is there, the other buffer has been used
-        if (kt + FK < k_end) ask(kt + FK, buf ^ 1);
+    __syncthreads();                               // the queries are there
+    // the walk's tiles: those whose number has its parity
+    for (int kt = k_begin + ((k_begin / FK ^ walk) & 1) * FK; kt < k_end; kt += 2 * FK) {
+        walk_sync();                               // the tile before has been used
+        ask(kt);
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        walk_sync();                               // this tile is there
         if (!busy || kt > w_last || (window > 0 && kt + FK <= w_first - window + 1)) continue;     // uniform for the warp
         float s[2][4];
 #pragma unroll
@@ -249,7 +253,7 @@ attn_rows_f32_kernel(const float* __restrict__ q, const float* __restrict__ k_ca
 #pragma unroll
             for (int j = 0; j < 4; ++j) s[i][j] = 0.f;
         const float* qrow = Qs + (wq + sr) * QP;
-        const float* krow = Ks + (buf * FK + sub) * QP;
+        const float* krow = Ks + sub * QP;
         float4 kv[2][4], qv[2][2];                 // the next four numbers are on their way while these are used
         auto pull = [&](int c, int at) {
 #pragma unroll
@@ -278,7 +282,7 @@ attn_rows_f32_kernel(const float* __restrict__ q, const float* __restrict__ k_ca
             for (int j = 0; j < 4; ++j) {
                 const int kj = kt + sub + 8 * j;
                 const bool vis = wq + sr + i < nq && kj <= p_i && (window == 0 || kj > p_i - window) &&
-                                 there[buf * FK + sub + 8 * j];
+                                 there[sub + 8 * j];
                 s[i][j] = vis ? s[i][j] : -INFINITY;
                 tmax = fmaxf(tmax, s[i][j]);
             }
@@ -311,7 +315,7 @@ attn_rows_f32_kernel(const float* __restrict__ q, const float* __restrict__ k_ca
                     acc[i][j] = f32t::pair_of(__fmul_rn(a.x, fs[i]), __fmul_rn(a.y, fs[i]));
                 }
         }
-        const float* vrow = Vs + buf * FK * D + oc;
+        const float* vrow = Vs + oc;
         float4 pn = *reinterpret_cast<const float4*>(Ps + orow);
         ulonglong2 vn[NC];
 #pragma unroll
@@ -338,20 +342,46 @@ attn_rows_f32_kernel(const float* __restrict__ q, const float* __restrict__ k_ca
         }
         __syncwarp();                              // the weights have been read
     }
-    if (!busy) return;
+    // The second walk leaves its rows where its tiles were: [FQ][D] outputs, then maxima and sums; the first takes them in.
+    __syncthreads();
+    float* theirs = Qs + FQ * QP + FK * (QP + D);
+    float* m_theirs = theirs + FQ * D;
+    float* l_theirs = m_theirs + FQ;
+    if (walk == 1 && busy) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+            if (sub == 0) { m_theirs[wq + sr + i] = m_run[i]; l_theirs[wq + sr + i] = l_run[i]; }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int c = 0; c < NC; ++c)
+                *reinterpret_cast<ulonglong2*>(theirs + (wq + orow + i) * D + oc + 64 * c) = make_ulonglong2(acc[i][2 * c], acc[i][2 * c + 1]);
+    }
+    __syncthreads();
+    if (walk == 1 || !busy) return;
+    // factors of the two walks' rows: exp(m - common maximum) over the common sum
 #pragma unroll
     for (int i = 0; i < 2; ++i)
-        if (sub == 0) As[sr + i] = l_run[i] > 0.f ? 1.f / l_run[i] : 0.f;
+        if (sub == 0) {
+            const float mt = m_theirs[wq + sr + i], lt = l_theirs[wq + sr + i], m = fmaxf(m_run[i], mt);
+            const float a = m == -INFINITY ? 0.f : expf(m_run[i] - m), b = m == -INFINITY ? 0.f : expf(mt - m);
+            const float l = fmaf(l_run[i], a, __fmul_rn(lt, b)), inv = l > 0.f ? 1.f / l : 0.f;
+            As[sr + i] = a * inv;
+            Ps[sr + i] = b * inv;
+        }
     __syncwarp();
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         if (wq + orow + i >= nq) break;
-        const float inv = As[orow + i];
+        const float a = As[orow + i], b = Ps[orow + i];
+        const float* r = theirs + (wq + orow + i) * D + oc;
         float* o = out + ((int64_t)(q0 + qt * FQ + wq + orow + i) * nh + h) * D + oc;
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
             const float2 lo = f32t::halves_of(acc[i][2 * c]), hi = f32t::halves_of(acc[i][2 * c + 1]);
-            *reinterpret_cast<float4*>(o + 64 * c) = make_float4(lo.x * inv, lo.y * inv, hi.x * inv, hi.y * inv);
+            const float4 y = *reinterpret_cast<const float4*>(r + 64 * c);
+            *reinterpret_cast<float4*>(o + 64 * c) = make_float4(fmaf(lo.x, a, __fmul_rn(y.x, b)), fmaf(lo.y, a, __fmul_rn(y.y, b)),
+                                                                 fmaf(hi.x, a, __fmul_rn(y.z, b)), fmaf(hi.y, a, __fmul_rn(y.w, b)));
         }
     }
 }
@@ -688,7 +718,7 @@ int mi_attn_tiled(const void* q, const void* k_cache, const void* v_cache, int a
         const size_t smem = d == 64 ? rows_f32_smem<64>() : rows_f32_smem<128>();
         auto kernel = d == 64 ? attn_rows_f32_kernel<64> : attn_rows_f32_kernel<128>;
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        kernel<<<grid, 128, smem, stream>>>((const float*)q, (const float*)k_cache, (const float*)v_cache, block_table,
+        kernel<<<grid, 256, smem, stream>>>((const float*)q, (const float*)k_cache, (const float*)v_cache, block_table,
                                             q_start, kv_len, (float*)out, nh, nkv, page_size, max_pages, window, scale);
         return finish_launch("attn_rows_f32");
     }
