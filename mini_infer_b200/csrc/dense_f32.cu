@@ -64,9 +64,10 @@ dense_f32_narrow_kernel(DenseF32 g) {
         if (r + i < rows) C[(int64_t)(row0 + r + i) * g.ldc + n] = acc[0][i];
 }
 
-// Which form: up to DF_NARROW_ROWS rows a product is bound by reading W, and the narrow tiles keep more of it in flight;
-// above, wide tiles of 128 columns, or of 64 where those of 128 would leave SMs without one.
-constexpr int DF_NARROW_ROWS = 16, DF_SMS = 148;
+// Which form: up to DF_NARROW_ROWS rows a product is bound by reading W, and the narrow tiles keep more of it in flight
+// (against [6144, 2048], narrow and wide: 16 rows 39 and 61 us, 32 rows 53 and 61, 48 rows 65 and 66; against [2048, 5632]:
+// 32 rows 66 and 163 us); above, wide tiles of 128 columns, or of 64 where those of 128 would leave SMs without one.
+constexpr int DF_NARROW_ROWS = 32, DF_SMS = 148;
 
 static int dense_f32_launch(const DenseF32& g, int batch, bool vec, cudaStream_t stream, const char* what) {
     const int64_t tiles_y = ((int64_t)g.T + f32t::BM - 1) / f32t::BM;
@@ -74,7 +75,7 @@ static int dense_f32_launch(const DenseF32& g, int batch, bool vec, cudaStream_t
     if (vec && g.T <= DF_NARROW_ROWS) {
         const size_t smem = f32t::narrow_smem(1);
         cudaFuncSetAttribute(dense_f32_narrow_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        dense_f32_narrow_kernel<<<dim3((g.N + f32t::NN - 1) / f32t::NN, 1, batch), f32t::THREADS, smem, stream>>>(g);
+        dense_f32_narrow_kernel<<<dim3((g.N + f32t::NN - 1) / f32t::NN, (g.T + f32t::NM - 1) / f32t::NM, batch), f32t::THREADS, smem, stream>>>(g);
         return finish_launch(what);
     }
     const int64_t wide = tiles_y * ((g.N + 127) / 128) * batch;

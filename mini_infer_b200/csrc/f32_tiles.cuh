@@ -9,7 +9,7 @@
 //              memory in registers meanwhile.  A warp covers 16 rows and is idle where its rows lie past the end; a
 //              block's warps take their rows in an order that turns with the block, so that the idle ones of several
 //              blocks do not all belong to one quarter of the SM.
-//   NarrowTile up to 16 rows x 32 columns by 128 threads, 4 rows a warp, one column (or gate and up column) a lane.
+//   NarrowTile 16 rows x 32 columns by 128 threads, 4 rows a warp, one column (or gate and up column) a lane.
 //              Bound by reading W: four tiles of 64 k arrive through cp.async while one is used.
 //
 // 512 rows against [6144, 2048] and [2048, 2048] (a q/k/v and an output product): 629 us with 64 x 64 tiles of 4 x 4

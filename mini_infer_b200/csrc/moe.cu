@@ -1025,8 +1025,10 @@ grouped_f32_narrow_kernel(GroupedF32 g) {
     }
 }
 
-// Narrow tiles up to so many rows per expert on average: there a product is bound by reading the experts' weights.
-constexpr int GF_NARROW_ROWS = 8;
+// Narrow tiles up to so many rows per expert on average: there a product is bound by reading the experts' weights (60 of
+// [2 x 1408, 2048], narrow and wide: 8 rows each 407 and 640 us, 12 rows 433 and 643; with 17 and more a second narrow tile
+// is needed: 20 rows each 790 and 650 us).
+constexpr int GF_NARROW_ROWS = 12;
 
 template <int MODE>
 static int grouped_f32_launch(const GroupedF32& g, int n_rows, cudaStream_t stream) {

@@ -106,8 +106,9 @@ class Tuning:
     scan_max_segments: int = 32
 
     # The delta rule with one decay per head (bfloat16 path): steps whose longest portion has at least this many tokens
-    # walk in blocks of 8 tokens.
-    delta_blocks_min_tokens: int = 8
+    # walk in blocks of 8 tokens.  A layer of 16 heads of 128 x 128, blocks against token by token: 8 tokens 28.6 and
+    # 23.7 us, 32 tokens 35.9 and 34.5, 64 tokens 40.1 and 43.5, 2,048 in two prompts 331 and 638.
+    delta_blocks_min_tokens: int = 48
 
     # Matrix memories with one gate per head and the gated linear recurrence per channel (bfloat16 path): portions of at
     # least so many tokens go over chunks of 64 tokens on the tensor cores, or in segments of 64 tokens side by side;

@@ -26,8 +26,8 @@ def within_chain(out, a, w):
     assert bool(((out.double() - ref).abs() <= bound).all())
 
 
-# rows: one, the narrow form's last, one more, a warp's and a tile's edges; columns and inner sizes that fill no tile
-@pytest.mark.parametrize("T", [1, 16, 17, 64, 65, 200])
+# rows: one, a narrow tile's last, one more, the narrow form's last, one more, a wide tile's edges; columns and inner sizes that fill no tile
+@pytest.mark.parametrize("T", [1, 16, 17, 32, 33, 64, 65, 200])
 @pytest.mark.parametrize("N,K", [(33, 4), (64, 68), (129, 100), (320, 63), (200, 2050), (19200, 36)])
 def test_dense_forms(T, N, K):
     a, w = rnd(T, K, seed=1), rnd(N, K, seed=2)
