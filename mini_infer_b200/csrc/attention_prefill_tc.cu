@@ -33,6 +33,7 @@
 // The reference computes prefill with one block per (request, head, query) and scalar dot
 // products over every page of the request (src/kernels/paged_attn_kernel.cu:102-288).
 
+#include "prefill_rules.h"
 #include "tcgen05.cuh"
 
 namespace mi {
@@ -476,12 +477,11 @@ attn_prefill_tc_kernel(const __grid_constant__ Maps maps, const int* __restrict_
                 }
                 l_run = l_run * alpha + ((sums[0].x + sums[0].y) + (sums[1].x + sums[1].y));
             }
-            // O is scaled only after O += P V of tile j - 1.  (S of tile j was issued after that of tile j - 2 was
-            // complete and that of tile j waits for this warp: the barrier is in phase j - 1 or j, which its
-            // parity tells apart, so the phases before need not have been followed one by one.)
+            // O is scaled only after O += P V of tile j - 1, and the last tile waits for that product in any case: see
+            // follows_product.
             const bool rescale = !LOGISTIC && j > 0 && !__all_sync(0xffffffffu, alpha == 1.f);
-            if (rescale) {
-                ok = mbar_wait(&o_done[t], (j - 1) & 1, abort_flag, 18);
+            if (follows_product(j, n_mine, rescale)) {
+                ok = mbar_wait(&o_done[t], (j - 1) & 1, abort_flag, rescale ? 18 : 19);
                 ok = __all_sync(0xffffffffu, ok);
             }
             if (ok && rescale) {
@@ -506,9 +506,8 @@ attn_prefill_tc_kernel(const __grid_constant__ Maps maps, const int* __restrict_
             }
         }
         if (together) {
-            // the last two products in turn: a parity tells only neighbouring phases apart
-            ok = ok && (n_mine < 2 || mbar_wait(&o_done[t], (n_mine - 2) & 1, abort_flag, 19)) &&
-                 mbar_wait(&o_done[t], (n_mine - 1) & 1, abort_flag, 20);
+            // the product before was seen complete ahead of the last hand-over: the barrier is in phase n - 1 or n
+            ok = ok && mbar_wait(&o_done[t], (n_mine - 1) & 1, abort_flag, 20);
             ok = __all_sync(0xffffffffu, ok);
             // the halves' sums meet where the maxima of a tile more would
             float* at = meet + (n_mine & 1) * 2 * BQ + r;
