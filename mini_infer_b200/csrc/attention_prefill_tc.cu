@@ -318,6 +318,7 @@ attn_prefill_tc_kernel(const __grid_constant__ Maps maps, const int* __restrict_
         const int t = warp - 18;
         if (t < tiles_q) {
             bool ok = *abort_flag == 0 && mbar_wait(&q_full[t], 0, abort_flag, 12);
+            ok = __all_sync(0xffffffffu, ok);             // the loops below are the whole warp's
             const int n_mine = tiles_of(t);
             const uint32_t tmem_t = tmem_base + t * COL_TILE;
             // descriptors of the tile origins; an offset of b bytes inside a tile adds b / 16 to the address field

@@ -4,6 +4,7 @@ barrier of O += P V, walked through in every interleaving."""
 import ctypes
 import itertools
 import os
+import re
 import subprocess
 
 import pytest
@@ -78,3 +79,15 @@ def test_the_walk_finds_a_wait_behind_the_last_hand_over():
     assert lost_or_early([late([False] * 3), late([False] * 3)], 3)
     none = lambda j, n, r: False
     assert lost_or_early([program(3, [False] * 3, none)] * 2, 3)
+
+
+def test_a_whole_warps_wait_is_agreed_upon():
+    """Lanes may give a wait up one by one (a limit each), and what follows is for whole warps: every wait that is not one
+    lane's alone is followed by a vote before anything else looks at its outcome."""
+    source = re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, "attention_prefill_tc.cu")).read())
+    statements = [re.sub(r"\s+", " ", s).strip() for s in source.split(";")]
+    waits = [i for i, s in enumerate(statements)
+             if re.search(r"\bok = .*(mbar_wait|k_there)\(", s) and "if (lane == 0) ok =" not in s]
+    assert len(waits) >= 7
+    for i in waits:
+        assert re.match(r"ok = (together = )?(__all_sync|pair_and)\(", statements[i + 1]), (statements[i], statements[i + 1])
