@@ -1085,8 +1085,8 @@ int mi_moe_router(const void* x, int adtype, const void* wr, const void* wsg, in
         const dim3 sgrid(ncols, token_tiles);
         if (adtype == kF32 && wdtype == kF32 && T > 4 * RT_TOK && H % 4 == 0 &&
             ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(wr) | reinterpret_cast<uintptr_t>(wsg)) & 15) == 0) {
-            if (smem_x > 48 * 1024)
-                cudaFuncSetAttribute(moe_router_logits_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_x);
+            // (asked for at every size: beside the kernel's static 1 KiB, 47 KiB of rows are too much by themselves)
+            cudaFuncSetAttribute(moe_router_logits_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_x);
             moe_router_logits_f32_kernel<<<dim3(token_tiles, (ncols + RL_ROWS - 1) / RL_ROWS), 256, smem_x, stream>>>(
                 (const float*)x, (const float*)wr, (const float*)wsg, z_scratch, T, H, E);
         } else

@@ -2,6 +2,10 @@
 eight queries of the attention): every form against float64 within the bound of a chain of additions, and the same bits
 from every form."""
 
+import os
+import subprocess
+import sys
+
 import pytest
 import torch
 
@@ -81,6 +85,24 @@ def test_router_of_many_tokens_adds_as_that_of_few(T, H, E, gated):
     for i, got in enumerate(whole):
         if got is not None:
             assert torch.equal(got, torch.cat([f[i] for f in few]))
+
+
+# the staged rows take H / 32 KiB of shared memory beside 1 KiB of the kernel's own: the sizes at which the two together
+# pass 48 KiB (1504, 1508), at which the rows alone do (1536, 1540), and the largest that the router takes
+@pytest.mark.parametrize("H", [1504, 1508, 1536, 1540, 6400])
+def test_router_rows_at_the_limits_of_shared_memory(H):
+    """In a process of its own: a larger size before it would have raised the kernel's limit for good."""
+    code = f"""
+import torch
+from mini_infer_b200.ops import functional as F
+x, w = torch.randn(40, {H}, device="cuda:0"), torch.randn(9, {H}, device="cuda:0") * 0.05
+whole = F.moe_router(x, w, None, 2, False, want_probs=True)
+few = [F.moe_router(x[lo:lo + 8].contiguous(), w, None, 2, False, want_probs=True) for lo in range(0, 40, 8)]
+for i, got in enumerate(whole):
+    assert got is None or torch.equal(got, torch.cat([f[i] for f in few]))
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    subprocess.run([sys.executable, "-c", code], check=True, cwd=root, timeout=300)
 
 
 @pytest.mark.parametrize("d,nh,nkv,page,window", [(64, 4, 2, 16, 0), (128, 2, 1, 16, 0), (128, 3, 3, 8, 40), (64, 2, 2, 32, 17)])
