@@ -1150,7 +1150,7 @@ int mi_moe_route_small(const void* x, int adtype, const void* wr, const void* ws
     const dim3 grid(ncols, (T + tok - 1) / tok);
 #define MI_ROUTE_LAUNCH(AT, WT, TOK)                                                                           \
     do {                                                                                                       \
-        if (smem > 48 * 1024)                                                                                  \
+        if (smem > 40 * 1024) /* (48 KiB with what the kernel has beside it) */                                \
             cudaFuncSetAttribute(moe_route_small_kernel<AT, WT, TOK>,                                          \
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                      \
         moe_route_small_kernel<AT, WT, TOK><<<grid, 256, smem, stream>>>(                                      \
@@ -1220,7 +1220,7 @@ int mi_moe_norm_route_small(float* hidden, const float* delta, const void* norm_
     lc.numAttrs = dependent_launch_enabled() ? 2 : 1;
 #define MI_NR_LAUNCH(AT, WT, NT)                                                                                 \
     do {                                                                                                         \
-        if (smem > 48 * 1024)                                                                                    \
+        if (smem > 40 * 1024) /* (48 KiB with what the kernel has beside it) */                                  \
             cudaFuncSetAttribute(moe_norm_route_small_kernel<AT, WT, NT>,                                        \
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                        \
         (void)cudaLaunchKernelEx(&lc, moe_norm_route_small_kernel<AT, WT, NT>, hidden, delta,             \

@@ -105,6 +105,25 @@ for i, got in enumerate(whole):
     subprocess.run([sys.executable, "-c", code], check=True, cwd=root, timeout=300)
 
 
+@pytest.mark.parametrize("d", [144, 146, 148])
+def test_tiled_attention_at_the_limit_of_shared_memory(d):
+    """Rows of 146 numbers and what the kernel has beside them pass 48 KiB together, neither by itself (a process of its
+    own, as above)."""
+    code = f"""
+import torch
+from mini_infer_b200.ops import functional as F
+q, k, v = (torch.randn(s, device="cuda:0") for s in ((16, 2, {d}), (1, 2, 16, {d}), (1, 2, 16, {d})))
+i32 = lambda t: torch.tensor(t, dtype=torch.int32, device="cuda:0")
+out = F.attention(q, k, v, i32([[0]]), i32([0, 16]), i32([16]), 16, 0)
+later = torch.ones(16, 16, dtype=torch.bool, device="cuda:0").triu(1)
+s = (torch.einsum("qhd,hkd->hqk", q.double(), k[0].double()) * {d} ** -0.5).masked_fill(later, -torch.inf)
+ref = torch.einsum("hqk,hkd->qhd", torch.softmax(s, -1), v[0].double())
+assert float((out - ref).abs().max()) <= 3e-6 * float(ref.abs().max())
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    subprocess.run([sys.executable, "-c", code], check=True, cwd=root, timeout=300)
+
+
 @pytest.mark.parametrize("d,nh,nkv,page,window", [(64, 4, 2, 16, 0), (128, 2, 1, 16, 0), (128, 3, 3, 8, 40), (64, 2, 2, 32, 17)])
 def test_attention_of_every_cut(d, nh, nkv, page, window):
     lengths, S = [1, 7, 8, 33, 64, 95], 95
