@@ -504,82 +504,84 @@ delta_blocks_prepare_kernel(const float* __restrict__ qkv, int ld_qkv, const flo
     wait_for_earlier_kernels();
     const int b = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int q0 = q_start[b], n = q_start[b + 1] - q0;
-    const int item = blockIdx.x * 4 + warp, blk = item / G, g = item - blk * G;
-    if (blk * N >= n) return;                            // uniform for the warp; no block barrier below
-    const int t0 = q0 + blk * N, nt = min(N, n - blk * N);
-    float q[N][E], k[N][E];
+    // (however many blocks the launch has; uniform for the warp, no block barrier below)
+    for (int item = blockIdx.x * 4 + warp, items = (n + N - 1) / N * G; item < items; item += gridDim.x * 4) {
+        const int blk = item / G, g = item - blk * G;
+        const int t0 = q0 + blk * N, nt = min(N, n - blk * N);
+        float q[N][E], k[N][E];
 #pragma unroll
-    for (int t = 0; t < N; ++t) {
-        float qq = 0.f, kk = 0.f;
+        for (int t = 0; t < N; ++t) {
+            float qq = 0.f, kk = 0.f;
 #pragma unroll
-        for (int e = 0; e < E; ++e) {
-            const float* row = qkv + (int64_t)(t0 + t) * ld_qkv + (int64_t)g * D + e * 32 + lane;
-            q[t][e] = t < nt ? row[0] : 0.f;
-            k[t][e] = t < nt ? row[(int64_t)G * D] : 0.f;
-            qq += q[t][e] * q[t][e]; kk += k[t][e] * k[t][e];
+            for (int e = 0; e < E; ++e) {
+                const float* row = qkv + (int64_t)(t0 + t) * ld_qkv + (int64_t)g * D + e * 32 + lane;
+                q[t][e] = t < nt ? row[0] : 0.f;
+                k[t][e] = t < nt ? row[(int64_t)G * D] : 0.f;
+                qq += q[t][e] * q[t][e]; kk += k[t][e] * k[t][e];
+            }
+            const float qn = q_scale / sqrtf(warp_sum(qq) + 1e-6f), kn = 1.0f / sqrtf(warp_sum(kk) + 1e-6f);
+            float* dst = qk + ((int64_t)(t0 + t) * G + g) * 2 * D + lane;
+#pragma unroll
+            for (int e = 0; e < E; ++e) {
+                q[t][e] *= qn; k[t][e] *= kn;
+                if (t < nt) { dst[e * 32] = q[t][e]; dst[D + e * 32] = k[t][e]; }
+            }
         }
-        const float qn = q_scale / sqrtf(warp_sum(qq) + 1e-6f), kn = 1.0f / sqrtf(warp_sum(kk) + 1e-6f);
-        float* dst = qk + ((int64_t)(t0 + t) * G + g) * 2 * D + lane;
+        // k_t . k_j (j < t) and q_t . k_j (j <= t) to shared memory
 #pragma unroll
-        for (int e = 0; e < E; ++e) {
-            q[t][e] *= qn; k[t][e] *= kn;
-            if (t < nt) { dst[e * 32] = q[t][e]; dst[D + e * 32] = k[t][e]; }
-        }
-    }
-    // k_t . k_j (j < t) and q_t . k_j (j <= t) to shared memory
+        for (int t = 0; t < N; ++t) {
 #pragma unroll
-    for (int t = 0; t < N; ++t) {
+            for (int j = 0; j <= t; ++j) {
+                float kk = 0.f, qq = 0.f;
 #pragma unroll
-        for (int j = 0; j <= t; ++j) {
-            float kk = 0.f, qq = 0.f;
-#pragma unroll
-            for (int e = 0; e < E; ++e) { kk += k[t][e] * k[j][e]; qq += q[t][e] * k[j][e]; }
-            kk = warp_sum(kk); qq = warp_sum(qq);
-            if (lane == 0) { sm[warp][0][t][j] = kk; sm[warp][1][t][j] = qq; }
-        }
-    }
-    __syncwarp();
-    for (int h = g * (H / G); h < (g + 1) * (H / G); ++h) {
-        // lane t (of the first 8, repeated): its decay and write strength; a token past the end changes nothing
-        const int t = lane & 7;
-        float decay = 1.f, beta = 0.f;
-        if (t < nt) {
-            decay = expf(-expf(a_log[h]) * softplus_f(a_raw[(int64_t)(t0 + t) * ld_a + h] + dt_bias[h]));
-            beta = sigmoid_f(beta_raw[(int64_t)(t0 + t) * ld_beta + h]);
-        }
-        float* m = mats + ((block_row0(q0, b) + blk) * H + h) * kBlockMats;
-        // Every lane of a group of 8 holds column j = t of G_r / G_j (products of decays, not differences of logarithms,
-        // whose rounding would grow with their sum) and of (I + L)^-1 diag(beta), forward.
-        float x[N], ratio = 1.f, Gt = 1.f;
-#pragma unroll
-        for (int r = 0; r < N; ++r) {
-            const float gr = __shfl_sync(0xffffffffu, decay, r, 8);
-            ratio = r > t ? ratio * gr : 1.f;            // below the diagonal a product, on it 1
-            if (r <= t) Gt *= gr;
-            if (lane < 8) rat_s[warp][r][t] = r >= t ? ratio : 0.f;
+                for (int e = 0; e < E; ++e) { kk += k[t][e] * k[j][e]; qq += q[t][e] * k[j][e]; }
+                kk = warp_sum(kk); qq = warp_sum(qq);
+                if (lane == 0) { sm[warp][0][t][j] = kk; sm[warp][1][t][j] = qq; }
+            }
         }
         __syncwarp();
+        for (int h = g * (H / G); h < (g + 1) * (H / G); ++h) {
+            // lane t (of the first 8, repeated): its decay and write strength; a token past the end changes nothing
+            const int t = lane & 7;
+            float decay = 1.f, beta = 0.f;
+            if (t < nt) {
+                decay = expf(-expf(a_log[h]) * softplus_f(a_raw[(int64_t)(t0 + t) * ld_a + h] + dt_bias[h]));
+                beta = sigmoid_f(beta_raw[(int64_t)(t0 + t) * ld_beta + h]);
+            }
+            float* m = mats + ((block_row0(q0, b) + blk) * H + h) * kBlockMats;
+            // Every lane of a group of 8 holds column j = t of G_r / G_j (products of decays, not differences of logarithms,
+            // whose rounding would grow with their sum) and of (I + L)^-1 diag(beta), forward.
+            float x[N], ratio = 1.f, Gt = 1.f;
 #pragma unroll
-        for (int r = 0; r < N; ++r) {
-            const float br = __shfl_sync(0xffffffffu, beta, r, 8);
-            float v = r == t ? beta : 0.f;
+            for (int r = 0; r < N; ++r) {
+                const float gr = __shfl_sync(0xffffffffu, decay, r, 8);
+                ratio = r > t ? ratio * gr : 1.f;            // below the diagonal a product, on it 1
+                if (r <= t) Gt *= gr;
+                if (lane < 8) rat_s[warp][r][t] = r >= t ? ratio : 0.f;
+            }
+            __syncwarp();
 #pragma unroll
-            for (int i = 0; i < r; ++i) v -= br * rat_s[warp][r][i] * sm[warp][0][r][i] * x[i];
-            x[r] = v;
-            if (lane < 8) inv_s[warp][r][t] = v;
+            for (int r = 0; r < N; ++r) {
+                const float br = __shfl_sync(0xffffffffu, beta, r, 8);
+                float v = r == t ? beta : 0.f;
+#pragma unroll
+                for (int i = 0; i < r; ++i) v -= br * rat_s[warp][r][i] * sm[warp][0][r][i] * x[i];
+                x[r] = v;
+                if (lane < 8) inv_s[warp][r][t] = v;
+            }
+            __syncwarp();
+            for (int idx = lane; idx < N * N; idx += 32) {
+                const int r = idx >> 3, j = idx & 7;
+                float o = 0.f;
+#pragma unroll
+                for (int i = 0; i < N; ++i)
+                    if (i <= r) o += rat_s[warp][r][i] * sm[warp][1][r][i] * inv_s[warp][i][j];
+                m[idx] = rat_s[warp][N - 1][r] * inv_s[warp][r][j];
+                m[N * N + idx] = o;
+            }
+            if (lane < 8) m[2 * N * N + lane] = Gt;
+            __syncwarp();                                    // both are written anew for the next head
         }
-        __syncwarp();
-        for (int idx = lane; idx < N * N; idx += 32) {
-            const int r = idx >> 3, j = idx & 7;
-            float o = 0.f;
-#pragma unroll
-            for (int i = 0; i < N; ++i)
-                if (i <= r) o += rat_s[warp][r][i] * sm[warp][1][r][i] * inv_s[warp][i][j];
-            m[idx] = rat_s[warp][N - 1][r] * inv_s[warp][r][j];
-            m[N * N + idx] = o;
-        }
-        if (lane < 8) m[2 * N * N + lane] = Gt;
-        __syncwarp();                                    // both are written anew for the next head
     }
 }
 
@@ -1277,7 +1279,8 @@ int mi_delta_scan_form(const float* qkv, int ld_qkv, const float* beta_raw, int 
 }
 
 // The delta rule with one decay per head over blocks of 8 tokens (see delta_blocks_scan_kernel): keys of 64 or 128
-// numbers; qk holds T * G * 2 d floats, mats (T / 8 + B) * H * mi_delta_blocks_mats() floats, both 16-byte aligned.
+// numbers; qk holds T * G * 2 d floats, mats (T / 8 + B) * H * mi_delta_blocks_mats() floats, both 16-byte aligned;
+// max_q_len sizes a launch only.
 // The sums of a token run in another order than token by token: the two agree within rounding, not bit for bit.
 int mi_delta_blocks_supported(int d) { return d == 64 || d == 128; }
 int mi_delta_blocks_mats() { return kBlockMats; }

@@ -1383,8 +1383,9 @@ def delta_scan(qkv: torch.Tensor, beta_raw: Optional[torch.Tensor], beta_col: in
     product of the decays since the run's start.  The chain of dependent steps is a run's length, not the portion's;
     the sums of a token run in another order than in one piece, so the two agree within rounding, not bit for bit.
 
-    ``blocks_of`` > 0 (``head_decay`` only, keys of 64 or 128: :func:`delta_blocks_supported`): the length of the
-    longest portion; portions are walked in blocks of 8 tokens, whose sums over ``S`` do not wait for one another.
+    ``blocks_of`` > 0 (``head_decay`` only, keys of 64 or 128: :func:`delta_blocks_supported`): portions are walked in
+    blocks of 8 tokens, whose sums over ``S`` do not wait for one another.  The number is the length of the longest
+    portion; it sizes a launch, and any other gives the same result.
     Again within rounding of the walk token by token, not bit for bit.
 
     ``qkv`` float32 ``[T, 2*key_heads*d + heads*dv]`` (q | k | v after their convolutions; the rows may go on

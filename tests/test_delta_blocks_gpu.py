@@ -58,6 +58,26 @@ def test_blocks_against_the_recurrence(lengths, H, G, d, dv, decay):
     assert error[True] <= max(1.5 * error[False], 2.0 ** -24 * d ** 0.5)
 
 
+@pytest.mark.parametrize("d", [64, 128])
+def test_the_length_given_sizes_the_launch_only(d):
+    from mini_infer_b200.ops import functional as F
+    g = torch.Generator().manual_seed(d)
+    rnd = lambda *s: torch.randn(*s, generator=g).to(DEV)
+    lengths, H, G, dv = [131, 9], 4, 2, 48
+    T, starts = sum(lengths), torch.tensor([0, 131, 140], dtype=torch.int32, device=DEV)
+    slots = torch.tensor([1, 0], dtype=torch.int32, device=DEV)
+    qkv, raw, a_log, dt_bias, state = rnd(T, 2 * G * d + H * dv), rnd(T, 2 * H), rnd(H) * 0.3, rnd(H), rnd(2, H * d * dv)
+    got = []
+    for blocks_of in (131, 1, 17, 1000):
+        st = state.clone()
+        junk = torch.full((1 << 22,), float("nan"), device=DEV)       # what the scratch finds
+        del junk
+        got.append((F.delta_scan(qkv, raw, 0, raw, H, a_log, dt_bias, st, 0, starts, slots, H, G, d, dv, d ** -0.5,
+                                 form="head_decay", blocks_of=blocks_of), st))
+    for out, st in got[1:]:
+        assert torch.equal(out, got[0][0]) and torch.equal(st, got[0][1])
+
+
 def test_blocks_are_refused_where_they_are_not_built():
     from mini_infer_b200.ops import functional as F
     z = torch.zeros(8, 400, device=DEV)
