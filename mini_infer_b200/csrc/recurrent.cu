@@ -708,7 +708,9 @@ delta_blocks_scan_kernel(const float* __restrict__ qkv, int ld_qkv, int64_t v_co
         }
 #pragma unroll
         for (int j = 0; j < N; ++j) {
-            const float xj = __shfl_sync(0xffffffffu, x, (lane & 24) + j);
+            // both matrices are zero behind the diagonal, but a later token's infinity must not meet that zero
+            float xj = __shfl_sync(0xffffffffu, x, (lane & 24) + j);
+            xj = j <= t ? xj : 0.f;
             w += wm[j] * xj; o += om[j] * xj;
         }
         const int tok = blk * N + t, col = col0 + mc;

@@ -78,6 +78,29 @@ def test_the_length_given_sizes_the_launch_only(d):
         assert torch.equal(out, got[0][0]) and torch.equal(st, got[0][1])
 
 
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+@pytest.mark.parametrize("where", ["value", "key", "query", "strength", "decay"])
+def test_tokens_before_one_that_is_not_finite_stay_as_they_are(where, bad):
+    from mini_infer_b200.ops import functional as F
+    g = torch.Generator().manual_seed(5)
+    rnd = lambda *s: torch.randn(*s, generator=g).to(DEV)
+    n, H, G, d, dv, at = 21, 2, 1, 64, 32, 13
+    i32 = lambda t: torch.tensor(t, dtype=torch.int32, device=DEV)
+    qkv, raw, a_log, dt_bias, state = rnd(n, 2 * G * d + H * dv), rnd(n, 2 * H), rnd(H) * 0.3, rnd(H), rnd(1, H * d * dv)
+    run = lambda: F.delta_scan(qkv, raw, 0, raw, H, a_log, dt_bias, state.clone(), 0, i32([0, n]), i32([0]), H, G, d, dv,
+                               d ** -0.5, form="head_decay", blocks_of=n)
+    clean = run()
+    if where in ("strength", "decay"):
+        raw[at, 0 if where == "strength" else H] = bad
+    else:
+        qkv[at, {"query": 7, "key": G * d + 7, "value": 2 * G * d + 7}[where]] = bad
+    out = run()
+    assert torch.equal(out[:at], clean[:at])
+    if where == "value":                # one column of one head
+        others = [c for c in range(H * dv) if c != 7]
+        assert not torch.isfinite(out[at, 7]) and torch.equal(out[:, others], clean[:, others])
+
+
 def test_blocks_are_refused_where_they_are_not_built():
     from mini_infer_b200.ops import functional as F
     z = torch.zeros(8, 400, device=DEV)
