@@ -269,9 +269,11 @@ class GatedDelta(Mixer):
         return StateNeed((self.state_floats + max(self.conv_floats, 1),), torch.float32)
 
     def _blocks_of(self, ctx: StepContext) -> int:
-        """The longest portion, if portions are walked in blocks of tokens.  (The float32 path walks token by token: its
-        sums run in one order however a prompt is cut.)"""
-        blocks = (self.rt.act == torch.bfloat16 and ctx.max_q_len >= TUNING.delta_blocks_min_tokens
+        """The longest portion, if the step's portions are walked in blocks of tokens.  (The float32 path walks token by
+        token: its sums run in one order however a prompt is cut.)"""
+        least = TUNING.delta_blocks_min_tokens
+        blocks = (self.rt.act == torch.bfloat16 and ctx.max_q_len >= least
+                  and ctx.num_tokens >= least + TUNING.delta_blocks_min_tokens_per_request * (ctx.num_requests - 1)
                   and F.delta_blocks_supported(self.d))
         return ctx.max_q_len if blocks else 0
 

@@ -106,9 +106,15 @@ class Tuning:
     scan_max_segments: int = 32
 
     # The delta rule with one decay per head (bfloat16 path): steps whose longest portion has at least this many tokens
-    # walk in blocks of 8 tokens.  A layer of 16 heads of 128 x 128, blocks against token by token: 8 tokens 28.6 and
-    # 23.7 us, 32 tokens 35.9 and 34.5, 64 tokens 40.1 and 43.5, 2,048 in two prompts 331 and 638.
+    # walk in blocks of 8 tokens.  Token by token and in blocks, us, one portion: 4 to 32 heads of keys of 128: 32 tokens
+    # 13-18 and 15-18, 48 tokens 18-25 and 16-21, 128 tokens 40-57 and 25-33; keys of 64: 32 tokens 13 and 13, 48
+    # tokens 16-18 and 14-15 (three portions alike: as much or more in favour of blocks).
     delta_blocks_min_tokens: int = 48
+    # ... and which bring this many tokens for every request more: in blocks a request of one token costs as much as one
+    # of eight.  One-token requests beside one portion, 16 heads of 128, token by token and in blocks: 7 beside 64 39 and
+    # 30, 15 beside 64 45 and 46, beside 96 59 and 51, 31 beside 96 69 and 78, beside 200 113 and 97, 63 beside 200 150
+    # and 149 (32 heads 238 and 267); 63 requests of 8 beside 48 135 and 122.
+    delta_blocks_min_tokens_per_request: int = 4
 
     # Matrix memories with one gate per head and the gated linear recurrence per channel (bfloat16 path): portions of at
     # least so many tokens go over chunks of 64 tokens on the tensor cores, or in segments of 64 tokens side by side;

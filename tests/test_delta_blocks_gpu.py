@@ -101,6 +101,19 @@ def test_tokens_before_one_that_is_not_finite_stay_as_they_are(where, bad):
         assert not torch.isfinite(out[at, 7]) and torch.equal(out[:, others], clean[:, others])
 
 
+@pytest.mark.parametrize("lengths,blocks", [([47], 0), ([48], 48), ([48, 48], 48), ([100, 1], 100), ([1] * 7 + [48], 0),
+                                             ([1] * 7 + [69], 69), ([1] * 31 + [100], 0), ([1] * 31 + [141], 141),
+                                             ([8] * 31 + [48], 48), ([40] * 8, 0)])
+def test_which_steps_walk_in_blocks(lengths, blocks):
+    from types import SimpleNamespace
+    from mini_infer_b200.parts.recurrent import GatedDelta
+    ctx = SimpleNamespace(num_tokens=sum(lengths), num_requests=len(lengths), max_q_len=max(lengths))
+    layer = lambda act, d: SimpleNamespace(rt=SimpleNamespace(act=act), d=d)
+    assert GatedDelta._blocks_of(layer(torch.bfloat16, 128), ctx) == blocks
+    assert GatedDelta._blocks_of(layer(torch.bfloat16, 96), ctx) == 0
+    assert GatedDelta._blocks_of(layer(torch.float32, 128), ctx) == 0
+
+
 def test_blocks_are_refused_where_they_are_not_built():
     from mini_infer_b200.ops import functional as F
     z = torch.zeros(8, 400, device=DEV)
