@@ -8,6 +8,7 @@ error; nothing falls back to PyTorch.
 from __future__ import annotations
 
 import ctypes
+import functools
 import math
 from typing import Optional, Tuple
 
@@ -1360,9 +1361,15 @@ def scan_segments(max_q_len: int, min_tokens: int, segment_tokens: int, max_segm
     return -(-max_q_len // per), per
 
 
+@functools.lru_cache(maxsize=None)
 def delta_blocks_supported(d: int) -> bool:
     """Whether :func:`delta_scan` walks keys of ``d`` numbers in blocks of tokens."""
     return bool(library().mi_delta_blocks_supported(int(d)))
+
+
+@functools.lru_cache(maxsize=None)
+def _delta_blocks_mats() -> int:
+    return int(library().mi_delta_blocks_mats())
 
 
 def delta_scan(qkv: torch.Tensor, beta_raw: Optional[torch.Tensor], beta_col: int, a_raw: torch.Tensor, a_col: int,
@@ -1421,13 +1428,13 @@ def delta_scan(qkv: torch.Tensor, beta_raw: Optional[torch.Tensor], beta_col: in
     if blocks_of > 0:
         if form != "head_decay" or not delta_blocks_supported(d) or segments > 1:
             raise ValueError(f"delta_scan: blocks of tokens are not built for '{form}' with keys of {d}")
-        qk = torch.empty(T * key_heads * 2 * d, dtype=F32, device=qkv.device)
-        mats = torch.empty((T // 8 + B) * heads * library().mi_delta_blocks_mats(), dtype=F32, device=qkv.device)
+        n_qk = T * key_heads * 2 * d                          # a multiple of 16 bytes: the matrices start behind it
+        qk = torch.empty(n_qk + (T // 8 + B) * heads * _delta_blocks_mats(), dtype=F32, device=qkv.device)
         check(library().mi_delta_blocks(
             _ptr(qkv), qkv.shape[1], beta_raw.data_ptr() + 4 * beta_col, beta_raw.shape[1], a_raw.data_ptr() + 4 * a_col,
             a_raw.shape[1], _ptr(a_log), _ptr(dt_bias), state.data_ptr() + 4 * state_offset, state.shape[1],
-            _ptr(q_start), _ptr(state_slot), _ptr(out), _ptr(qk), _ptr(mats), T, B, int(blocks_of), heads, key_heads, d,
-            dv, float(q_scale), _stream()), "delta_scan")
+            _ptr(q_start), _ptr(state_slot), _ptr(out), _ptr(qk), qk.data_ptr() + 4 * n_qk, T, B, int(blocks_of), heads,
+            key_heads, d, dv, float(q_scale), _stream()), "delta_scan")
         return out
     # unit vectors, decays and write strengths of all tokens, made ready by a kernel before the walk
     prep = torch.empty(T * heads * library().mi_delta_scan_prep_row(d), dtype=F32, device=qkv.device)
