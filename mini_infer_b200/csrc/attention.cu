@@ -320,8 +320,12 @@ attn_rows_f32_kernel(const float* __restrict__ q, const float* __restrict__ k_ca
         ulonglong2 vn[NC];
 #pragma unroll
         for (int c = 0; c < NC; ++c) vn[c] = *reinterpret_cast<const ulonglong2*>(vrow + 64 * c);
+        // Keys behind the warp's last query are left out: their weights are zeros, but values that are not finite must not
+        // meet those of queries before them.
+        const int n_keys = min(FK, w_last - kt + 1);
 #pragma unroll
         for (int kr = 0; kr < FK; ++kr) {
+            if (kr >= n_keys) break;
             const unsigned long long pp[4] = {f32t::pair_of(pn.x, pn.x), f32t::pair_of(pn.y, pn.y),
                                               f32t::pair_of(pn.z, pn.z), f32t::pair_of(pn.w, pn.w)};
             ulonglong2 v[NC];

@@ -152,3 +152,26 @@ def test_attention_of_every_cut(d, nh, nkv, page, window):
     two = F().attention(torch.cat([q[94:95], q[30:64]]).contiguous(), kc, vc, table.expand(2, -1).contiguous(), i32([0, 1, 35]),
                         i32([95, 64]), 34, window)
     assert torch.equal(two, torch.cat([whole[94:95], whole[30:64]]))
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("key,window", [(20, 0), (9, 0), (70, 24)])
+def test_values_that_are_not_finite_stay_with_their_queries(d, key, window):
+    """A query is as it was unless its block of 16 reaches the key: the tiles of the general kernel, which heads of other
+    sizes take, leave out what lies behind their 16 queries."""
+    S, nh, page = 96, 2, 16
+    q, k, v = rnd(S, nh, d, seed=15), rnd(S // page, nh, page, d, seed=16), rnd(S // page, nh, page, d, seed=17)
+    i32 = lambda t: torch.tensor(t, dtype=torch.int32, device=DEV)
+    run = lambda: F().attention(q, k, v, i32([list(range(S // page))]), i32([0, S]), i32([S]), S, window)
+    clean = run()
+    v[key // page, :, key % page, 3] = float("inf")
+    out = run()
+    before = key // 16 * 16
+    assert torch.equal(out[:before], clean[:before])
+    if window:                  # tiles of 32 keys that no query of a block of 16 sees any more
+        first = (key // 32 * 32 + 32 + window - 1) // 16 * 16 + 16
+        assert torch.equal(out[first:], clean[first:])
+    sees = slice(key, min(S, key + (window or S)))
+    assert not bool(torch.isfinite(out[sees, :, 3]).any())
+    rest = [c for c in range(d) if c != 3]
+    assert torch.equal(out[:, :, rest], clean[:, :, rest])
