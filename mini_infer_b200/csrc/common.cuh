@@ -145,8 +145,9 @@ __device__ __forceinline__ void wait_for_earlier_kernels() { asm volatile("gridd
 // at most one wave of blocks: a waiting block holds its SM's registers and shared memory).
 __device__ __forceinline__ void allow_next_kernel() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-// Whether launch_dependent() sets the attribute (mi_set_dependent_launch; off by default).
+// Whether launch_dependent() sets the attribute (mi_set_dependent_launch; off by default), and launch_behind() (on by default).
 bool dependent_launch_enabled();
+bool launch_behind_enabled();
 
 template <typename... P, typename... A>
 inline cudaError_t launch_placed_early(bool early, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
@@ -168,11 +169,11 @@ inline cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block,
                                     A... args) {
     return launch_placed_early(dependent_launch_enabled(), kernel, grid, block, smem, stream, args...);
 }
-// The same whatever the step's size, for the kernel behind another of the same call: a launch's latency (about a
-// microsecond between kernels of tens) overlaps the tail of the kernel before.
+// The same for the kernel behind another of the same call, whatever the step's size (unless early placement is switched
+// off): a launch's latency (about a microsecond between kernels of tens) overlaps the tail of the kernel before.
 template <typename... P, typename... A>
 inline cudaError_t launch_behind(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args) {
-    return launch_placed_early(true, kernel, grid, block, smem, stream, args...);
+    return launch_placed_early(launch_behind_enabled(), kernel, grid, block, smem, stream, args...);
 }
 
 // What else an attention over the paged cache may be asked for (all zero: nothing).

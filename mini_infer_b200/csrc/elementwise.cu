@@ -31,9 +31,11 @@ void set_last_error(const char* fmt, ...) {
 }
 
 static std::atomic<long long> g_launches{0};
-static std::atomic<int> g_dependent_launch{0};
+// 0: nothing is placed early; 1: every kernel that is written for it; 2: those behind another of the same call
+static std::atomic<int> g_dependent_launch{2};
 
-bool dependent_launch_enabled() { return g_dependent_launch.load(std::memory_order_relaxed) != 0; }
+bool dependent_launch_enabled() { return g_dependent_launch.load(std::memory_order_relaxed) == 1; }
+bool launch_behind_enabled() { return g_dependent_launch.load(std::memory_order_relaxed) != 0; }
 
 int finish_launch(const char* what, int n_kernels) {
     cudaError_t e = cudaGetLastError();
@@ -565,7 +567,9 @@ long long mi_launch_count() { return g_launches.load(std::memory_order_relaxed);
 
 // Switches programmatic dependent launch on (1) or off (0) for the kernels of decode-sized steps that
 // are written for it (see common.cuh); returns the setting before.
-int mi_set_dependent_launch(int on) { return g_dependent_launch.exchange(on ? 1 : 0, std::memory_order_relaxed); }
+int mi_set_dependent_launch(int which) {
+    return g_dependent_launch.exchange(which < 0 || which > 2 ? 2 : which, std::memory_order_relaxed);
+}
 
 int mi_embed_gather(const int* ids, const void* table, int wdtype, float* hidden, int T, int H, int V,
                     cudaStream_t stream) {

@@ -758,7 +758,10 @@ def l2_prefetch(t: torch.Tensor, max_bytes: Optional[int] = None) -> None:
 class dependent_launch:
     """``with dependent_launch(True):`` the kernels of decode-sized steps that are written for it (they wait
     for the kernels before them at their first line) are launched so that the device may place their blocks
-    while the kernel before them in the stream is still running; a pass captured under it replays so."""
+    while the kernel before them in the stream is still running; a pass captured under it replays so.
+    ``with dependent_launch(False):`` no kernel is.  Outside either, the kernels that stand behind another of the same
+    call are (the merge of a split decode attention, the walk behind its preparation, the chain and the read-outs of a
+    chunked memory, the state behind a convolution)."""
 
     def __init__(self, on: bool):
         self.on = bool(on)

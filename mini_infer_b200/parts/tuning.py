@@ -68,7 +68,8 @@ class Tuning:
     l2_prefetch_max_tokens: int = 15
 
     # Steps of at most this many tokens launch their kernels as programmatic dependents of the kernels before
-    # them (0 = off): a kernel's blocks are placed while the one before it drains.  At A2.7B sizes: batch 1
+    # them (0 = no step; kernels behind another of the same call are in steps of any size, see ``dependent_launch``): a
+    # kernel's blocks are placed while the one before it drains.  At A2.7B sizes: batch 1
     # +3.4 %, 2 +0.6 %, 4 +2.1 %, 8 +1.6 %; nothing either way from 16 tokens on, where library products stand
     # between the kernels that are written for it.  (Letting the next kernel's blocks in at a kernel's first
     # line instead of at its blocks' exit lost 5 to 8 % at batch 1 and 2: waiting blocks crowd the running ones.)

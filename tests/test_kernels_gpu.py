@@ -925,6 +925,42 @@ def test_debug_bounds_mode_names_the_bad_index(monkeypatch):
     assert f.debug_checks_run > 0
 
 
+def early_edges(call):
+    """How many kernels of a captured call may be placed while the kernel before them runs."""
+    from cuda.bindings import runtime
+    call()                                                          # whatever is set up once
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        call()
+    raw = runtime.cudaGraph_t(init_value=graph.raw_cuda_graph())
+    edges = getattr(runtime, "cudaGraphGetEdges_v2", None) or runtime.cudaGraphGetEdges
+    err, _, _, _, n = edges(raw)
+    assert int(err) == 0 and n > 0
+    err, _, _, data, n = edges(raw, n)
+    assert int(err) == 0
+    kind = lambda d: ord(d.type) if isinstance(d.type, (bytes, str)) else int(d.type)
+    return sum(kind(d) == int(runtime.cudaGraphDependencyType.cudaGraphDependencyTypeProgrammatic) for d in data[:n])
+
+
+def test_early_placement_can_be_switched_off():
+    dec = paged_case([700], [1], 2, 1, 64, 16, torch.bfloat16)
+    po, pml, splits = decode_scratch(1, 2, 700, 64)
+    attend = lambda: F().decode_attention(dec["q"], dec["kc"], dec["vc"], dec["table"], dec["q_start"], dec["kv_len"], po,
+                                          pml, splits)
+    x, w = rnd(4, 256, dtype=torch.bfloat16, seed=1), rnd(64, 256, dtype=torch.bfloat16, seed=2)
+    multiply = lambda: F().dense_skinny(F().dense_skinny(x, w, None, False).to(torch.bfloat16).repeat(1, 4), w, None, False)
+    both = lambda: (attend(), attend(), multiply())
+    with F().dependent_launch(False):
+        assert early_edges(both) == 0
+    plain = early_edges(both)                                       # the two merges
+    with F().dependent_launch(True):
+        assert early_edges(both) > plain > 0
+        with F().dependent_launch(False):
+            assert early_edges(both) == 0
+    assert early_edges(both) == plain
+
+
 def test_dependent_launch_gives_the_same_bits():
     """A chain of decode-sized kernels launched as programmatic dependents of one another (each waits for
     the kernels before it at its first line), eagerly and replayed from a CUDA graph, against the same
