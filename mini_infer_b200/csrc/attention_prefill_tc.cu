@@ -41,9 +41,6 @@ namespace pt {
 
 using namespace mi::tc;
 
-constexpr int BQ = 128;            // queries per tile (MMA M)
-// query tiles per block: two, but one where the queries of two would leave no room for rings
-constexpr int query_tiles(int dk) { return dk > 192 ? 1 : 2; }
 constexpr int BN = 64;             // keys per tile
 constexpr int HK = BN / 2;         // keys of a tile that a softmax thread takes
 constexpr int THREADS = 640;       // 2 x 8 softmax warps, two producers, two that issue MMAs
@@ -53,7 +50,6 @@ constexpr int KV_HALF = BN * 64 * 2;       // a tile of BN keys x 64 columns: 8 
 constexpr int WORDS = 512;
 constexpr int tail(int dk) { return WORDS + query_tiles(dk) * 2 * 2 * BQ * 4; }
 constexpr int SMEM_MAX = 227 * 1024;
-constexpr int SMS = 148;
 // Stages of the rings: as many K and V tiles as fit beside the queries (8 of each at most).
 constexpr int stages(int dk, int dv) {
     const int per = (dk / 64 + dv / 64) * KV_HALF, room = SMEM_MAX - tail(dk) - query_tiles(dk) * (dk / 64) * HALF_BYTES;
@@ -63,19 +59,6 @@ constexpr size_t smem_bytes(int dk, int dv) {
     return (size_t)query_tiles(dk) * (dk / 64) * HALF_BYTES + (size_t)stages(dk, dv) * (dk / 64 + dv / 64) * KV_HALF + tail(dk);
 }
 static_assert(stages(256, 128) >= 3 && stages(192, 128) >= 3, "rings of three stages at the largest sizes");
-// Which query tiles share a block (and its key tiles):
-//   kSingle      one alone, where the tiles of all heads and requests find an SM each (or two do not fit): a chain by
-//                itself takes 0.80 us a key tile, two beside each other 1.05 us
-//   kApart       the last but i and the first but i, where the pairs find an SM each and all earlier keys are seen: no
-//                block has two long ones (2,048 queries of 16 heads, 128 blocks: 36 us, 45 us with neighbours)
-//   kNeighbours  2 i and 2 i + 1, whose keys are nearly the same, so that both chains run to the end (8,192 queries of 16
-//                heads: 263 us, 353 us apart)
-enum QueryTiles : int { kSingle = 0, kApart = 1, kNeighbours = 2 };
-inline QueryTiles query_order(int64_t rows, int heads, int requests, int dk, bool bounded) {
-    const int64_t tiles = (rows + BQ - 1) / BQ, each = (int64_t)heads * requests;
-    if (query_tiles(dk) == 1 || tiles * each <= SMS) return kSingle;
-    return !bounded && (tiles + 1) / 2 * each <= SMS ? kApart : kNeighbours;
-}
 // blocks along x: the query tiles of the longest portion, for every head
 inline unsigned grid_x(int64_t rows, int heads, QueryTiles order) {
     const int64_t tiles = (rows + BQ - 1) / BQ;
@@ -631,7 +614,7 @@ int mi_attn_prefill_tc(const void* q, const void* k_cache, const void* v_cache, 
         set_last_error("prefill attention (tcgen05): cuTensorMapEncodeTiled failed");
         return kLaunchFailed;
     }
-    const pt::QueryTiles order = pt::query_order(max_q_len, nh, B, d, window > 0 || chunk > 0);
+    const pt::QueryTiles order = pt::query_order(max_q_len, T, nh, B, d, window > 0 || chunk > 0);
     const dim3 grid(pt::grid_x(max_q_len, nh, order), 1, B);
     const float scale_log2 = scale * 1.4426950408889634f;
     const size_t smem = d == 64 ? pt::smem_bytes(64, 64) : pt::smem_bytes(128, 128);
@@ -684,7 +667,7 @@ int mi_attn_prefill_tc_logistic(const void* q, const void* k_cache, const void* 
         set_last_error("prefill attention (tcgen05): cuTensorMapEncodeTiled failed");
         return kLaunchFailed;
     }
-    const pt::QueryTiles order = pt::query_order(max_q_len, nh, B, dk, window > 0);
+    const pt::QueryTiles order = pt::query_order(max_q_len, T, nh, B, dk, window > 0);
     const dim3 grid(pt::grid_x(max_q_len, nh, order), 1, B);
     const float scale_log2 = scale * 1.4426950408889634f;
 #define MI_PTL(KK, VV)                                                                                    \
@@ -737,7 +720,7 @@ int mi_attn_prefill_tc_shared(const void* q, const void* cache, const int* block
         return kLaunchFailed;
     }
     const int DKr = (dk + 63) / 64 * 64;
-    const pt::QueryTiles order = pt::query_order((int64_t)max_q_len * H, 1, B, DKr, window > 0);
+    const pt::QueryTiles order = pt::query_order((int64_t)max_q_len * H, (int64_t)T * H, 1, B, DKr, window > 0);
     const dim3 grid(pt::grid_x((int64_t)max_q_len * H, 1, order), 1, B);
     const float scale_log2 = scale * 1.4426950408889634f;
 #define MI_PTS(KK, VV)                                                                                    \
@@ -797,7 +780,7 @@ int mi_attn_prefill_tc_unfolded(const void* q, const void* kv, const void* k_rot
         return kLaunchFailed;
     }
     const pt::Unfolded uf = {(d + 15) / 16, (r + 15) / 16, d, e, gate, ldg, gcol};
-    const pt::QueryTiles order = pt::query_order(max_q_len, nh, B, DKr, window > 0);
+    const pt::QueryTiles order = pt::query_order(max_q_len, T, nh, B, DKr, window > 0);
     const dim3 grid(pt::grid_x(max_q_len, nh, order), 1, B);
     const float scale_log2 = scale * 1.4426950408889634f;
 #define MI_PTU(KK, VV)                                                                                    \

@@ -4,6 +4,7 @@ barrier of O += P V, walked through in every interleaving."""
 import ctypes
 import itertools
 import os
+import random
 import re
 import subprocess
 
@@ -12,7 +13,11 @@ import pytest
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "mini_infer_b200", "csrc")
 SOURCE = """
 #include "prefill_rules.h"
-extern "C" int follows_product(int j, int n, int rescale) { return mi::pt::follows_product(j, n, rescale != 0); }
+using namespace mi;
+extern "C" int follows_product(int j, int n, int rescale) { return pt::follows_product(j, n, rescale != 0); }
+extern "C" int query_order(int64_t longest, int64_t total, int heads, int requests, int dk, int bounded) {
+    return pt::query_order(longest, total, heads, requests, dk, bounded != 0);
+}
 """
 
 
@@ -22,7 +27,9 @@ def rules(tmp_path_factory):
     (folder / "rules.cpp").write_text(SOURCE)
     subprocess.run(["g++", "-std=c++17", "-shared", "-fPIC", "-Wall", "-Werror", "-I", CSRC, str(folder / "rules.cpp"), "-o",
                     str(folder / "rules.so")], check=True)
-    return ctypes.CDLL(str(folder / "rules.so"))
+    lib = ctypes.CDLL(str(folder / "rules.so"))
+    lib.query_order.argtypes = [ctypes.c_int64, ctypes.c_int64] + [ctypes.c_int] * 4
+    return lib
 
 
 def program(n, rescales, follows):
@@ -93,3 +100,30 @@ def test_a_whole_warps_wait_is_agreed_upon():
         if "ok = __all_sync(0xffffffffu, k_there(" in statements[i]:         # the vote is around the wait
             continue
         assert re.match(r"ok = (together = )?(__all_sync|pair_and)\(", statements[i + 1]), (statements[i], statements[i + 1])
+
+
+SINGLE, APART, NEIGHBOURS = 0, 1, 2
+
+
+@pytest.mark.parametrize("lengths,heads,order", [
+    ([2048], 16, APART), ([2048], 8, SINGLE), ([8192], 16, NEIGHBOURS), ([1000] * 3, 16, NEIGHBOURS),
+    ([1000, 100, 100], 16, APART), ([1000, 100, 100], 12, SINGLE), ([600, 20, 20, 20], 16, SINGLE),
+    ([1500, 100, 100], 16, APART), ([2000, 100, 100], 16, NEIGHBOURS)])
+def test_query_tiles_of_ragged_steps(rules, lengths, heads, order):
+    """Short portions beside a long one are not counted as if they were as long."""
+    assert rules.query_order(max(lengths), sum(lengths), heads, len(lengths), 128, 0) == order
+    assert rules.query_order(max(lengths), sum(lengths), heads, len(lengths), 256, 0) == SINGLE
+    assert rules.query_order(max(lengths), sum(lengths), heads, len(lengths), 128, 1) == (order if order == SINGLE else NEIGHBOURS)
+
+
+def test_tiles_that_find_an_sm_each_do_so(rules):
+    rng = random.Random(3)
+    for _ in range(3000):
+        lengths = [rng.randint(1, rng.choice([2, 200, 3000])) for _ in range(rng.randint(1, 8))]
+        heads = rng.choice([1, 2, 4, 8, 16, 28, 40])
+        tiles = [-(-n // 128) for n in lengths]
+        order = rules.query_order(max(lengths), sum(lengths), heads, len(lengths), 128, 0)
+        if order == SINGLE:
+            assert sum(tiles) * heads <= 148
+        if order == APART:
+            assert sum(-(-n // 2) for n in tiles) * heads <= 148
