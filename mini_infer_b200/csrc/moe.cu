@@ -1291,15 +1291,17 @@ int mi_grouped_gemm_plain(const void* A, int adtype, const int* gather, const vo
         set_last_error("grouped product: %d row tiles exceed the grid limit", max_tiles);
         return kBadShape;
     }
-    if (adtype == kF32 && wdtype == kF32 && cdtype == kF32 && Kd > 0 && Nout > 0) {
+    if (adtype == kF32 && wdtype == kF32 && cdtype == kF32) {
         const GroupedF32 g{(const float*)A, gather, (const float*)W, offsets, (float*)C, E, Nout, Kd, glu};
         return mode == 0 ? grouped_f32_launch<0>(g, n_rows, stream) : grouped_f32_launch<1>(g, n_rows, stream);
     }
     const dim3 grid((Nout + GB - 1) / GB, max_tiles);
 #define MI_GG(MODE)                                                                                     \
-    MI_DISPATCH_2(adtype, AT, wdtype, WT, MI_DISPATCH_1(cdtype, CT,                                     \
-        grouped_gemm_plain_kernel<AT, WT, CT, MODE><<<grid, 256, 0, stream>>>(                          \
-            (const AT*)A, gather, (const WT*)W, offsets, (CT*)C, E, Nout, Kd, glu)))
+    MI_DISPATCH_2(adtype, AT, wdtype, WT, MI_DISPATCH_1(cdtype, CT, {                                   \
+        if constexpr (sizeof(AT) + sizeof(WT) + sizeof(CT) < 3 * sizeof(float)) /* (all float: above) */ \
+            grouped_gemm_plain_kernel<AT, WT, CT, MODE><<<grid, 256, 0, stream>>>(                      \
+                (const AT*)A, gather, (const WT*)W, offsets, (CT*)C, E, Nout, Kd, glu);                 \
+    }))
     if (mode == 0) MI_GG(0); else MI_GG(1);
 #undef MI_GG
     return finish_launch("grouped_gemm_plain");

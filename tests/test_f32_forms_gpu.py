@@ -76,6 +76,15 @@ def test_grouped_forms(counts, nout, K, paired):
             assert bool(((out[lo:hi].double() - ref).abs() <= 16 * UNIT * (g.abs() + 1) * u.abs() + 1e-30).all())
 
 
+@pytest.mark.parametrize("rows", [3, 200])
+@pytest.mark.parametrize("paired", [False, True])
+def test_grouped_product_over_nothing(rows, paired):
+    x, w = torch.empty(rows, 0, device=DEV), torch.empty(2, 40, 0, device=DEV)
+    offsets = torch.tensor([0, 1, rows], dtype=torch.int32, device=DEV)
+    out = F().grouped_gemm_plain(x, None, w, offsets, rows, paired, torch.float32)
+    assert torch.equal(out, torch.zeros(rows, 20 if paired else 40, device=DEV))
+
+
 @pytest.mark.parametrize("T", [33, 40, 77, 512])
 @pytest.mark.parametrize("H,E,gated", [(64, 5, True), (1028, 16, False), (2048, 60, True), (2052, 33, True)])
 def test_router_of_many_tokens_adds_as_that_of_few(T, H, E, gated):
