@@ -520,17 +520,19 @@ def _vizalix_kernel_work(cfg, T, B, ctx, decode):
             ch = 2 * m["kv_heads"] * d + H * e
             state = (B if decode else 1) * H * d * e * 4 * 2
             add("delta_scan_kernel", n * (rows * (ch + H * d + H + H * e) * 4 + state), n * rows * H * d * e * 6.0)
-            for name in ("causal_conv_silu_kernel", "causal_conv_silu_vec4_kernel"):
+            for name in ("causal_conv_silu_kernel", "causal_conv_silu_vec4_kernel", "causal_conv4_vec4_kernel"):
                 add(name, n * rows * ch * 8, n * rows * ch * 8.0)
-            add("gated_group_rmsnorm_kernel", n * rows * H * e * (4 + 4 + 2), 0)
+            for name in ("gated_group_rmsnorm_kernel", "gated_group_rmsnorm_warp_kernel"):
+                add(name, n * rows * H * e * (4 + 4 + 2), 0)
         elif L["type"] == "mamba2":
             H, P, N = m["heads"], m["vdim"], m["state"]
             ch = H * P + 2 * N
             state = (B if decode else 1) * H * N * P * 4 * 2
             add("ssd_scan_kernel", n * (rows * (ch + H + H * P) * 4 + state), n * rows * H * N * P * 4.0)
-            for name in ("causal_conv_silu_kernel", "causal_conv_silu_vec4_kernel"):
+            for name in ("causal_conv_silu_kernel", "causal_conv_silu_vec4_kernel", "causal_conv4_vec4_kernel"):
                 add(name, n * rows * ch * 8, n * rows * ch * 8.0)
-            add("gated_group_rmsnorm_kernel", n * rows * H * P * (4 + 4 + 2), 0)
+            for name in ("gated_group_rmsnorm_kernel", "gated_group_rmsnorm_warp_kernel"):
+                add(name, n * rows * H * P * (4 + 4 + 2), 0)
         else:
             H, G, d, e, win = m["heads"], m["kv_heads"], m["dim"], m["vdim"], m["mask"]["size"]
             if decode:
@@ -916,20 +918,25 @@ def _bogetar_kernel_work(cfg, T, B, ctx, decode):
         a[0] += by
         a[1] += fl
 
-    def walk(H, G, d, e, form_columns):
+    def walk(H, G, d, e, form_columns, in_blocks=False):
         # rows in (q, k, v, and what the decays are made of), the prepared rows written and read, results out; the
-        # state read and written once per request
+        # state read and written once per request.  In blocks of 8 tokens what is prepared is unit rows per key head and
+        # 136 floats per (block, head).
         state = (B if decode else 1) * H * d * e * 4 * 2
-        add("delta_scan_kernel", rows * (H * (3 * d + 4) + H * e * 2) * 4 + state, rows * H * d * e * 6.0)
-        add("delta_prepare_kernel", rows * ((2 * G * d + form_columns) * 4 + H * (3 * d + 4) * 4), 0)
-        add("gated_group_rmsnorm_kernel", rows * H * e * (4 + 4 + 2), 0)
+        prepared = (rows * 2 * G * d + (rows + 7) // 8 * H * 136 if in_blocks else rows * H * (3 * d + 4)) * 4
+        add("delta_blocks_scan_kernel" if in_blocks else "delta_scan_kernel", prepared + rows * H * e * 2 * 4 + state,
+            rows * H * d * e * 6.0)
+        add("delta_blocks_prepare_kernel" if in_blocks else "delta_prepare_kernel",
+            rows * (2 * G * d + form_columns) * 4 + prepared, 0)
+        for name in ("gated_group_rmsnorm_kernel", "gated_group_rmsnorm_warp_kernel"):
+            add(name, rows * H * e * (4 + 4 + 2), 0)
     for L in cfg["layers"]:
         m = L["mixer"]
         if L["type"] == "delta":
             H, G, d, e = m["heads"], m["kv_heads"], m["dim"], m["vdim"]
             ch = 2 * G * d + H * e
-            walk(H, G, d, e, 2 * H)
-            for name in ("causal_conv_silu_kernel", "causal_conv_silu_vec4_kernel"):
+            walk(H, G, d, e, 2 * H, in_blocks=not decode and T >= 48 and d in (64, 128))
+            for name in ("causal_conv_silu_kernel", "causal_conv_silu_vec4_kernel", "causal_conv4_vec4_kernel"):
                 add(name, rows * ch * 8, rows * ch * 8.0)
         else:
             a, r = m["left"], m["right"]
@@ -946,7 +953,7 @@ def _bogetar_kernel_work(cfg, T, B, ctx, decode):
         parts = 1 if L["mlp"] is None else 2
         # the residual's float32 row in, the normalised float32 row out; then the filter's taps and its rounded row
         add("group_rmsnorm_kernel", parts * rows * W * 8, 0)
-        for name in ("causal_conv_silu_kernel", "causal_conv_silu_vec4_kernel"):
+        for name in ("causal_conv_silu_kernel", "causal_conv_silu_vec4_kernel", "causal_conv4_vec4_kernel"):
             add(name, parts * rows * W * (4 + 2), parts * rows * W * 2.0 * taps)
         # a part's float32 output in (two mixers' outputs, or the experts' rows), the residual read and written
         for name in ("out_norm_add_kernel", "out_norm_add_vec_kernel"):
@@ -1156,7 +1163,7 @@ def _dedizen_kernel_work(cfg, T, B, ctx, decode):
             if decode:
                 add("lru::lru_decode_kernel", B * C * (8 + 2 + 8 + 8 * (m["conv"] - 1)) + 2 * C * n * 2, B * C * n * 4.0)
             else:
-                for name in ("causal_conv_silu_kernel", "causal_conv_silu_vec4_kernel"):
+                for name in ("causal_conv_silu_kernel", "causal_conv_silu_vec4_kernel", "causal_conv4_vec4_kernel"):
                     add(name, T * C * 8, T * C * 2.0 * m["conv"])
                 add("lru::lru_gates_tc_kernel", T * C * 12 + 2 * C * n * 2, T * C * n * 4.0)
                 add("lru::lru_segments_kernel", T * C * 8)
