@@ -1,12 +1,19 @@
 // Dense product of the true 32-bit path: C[T, N] = A[T, K] . W[N, K]^T, float in, float out.
 //
-// Every output element is one chain of fused multiply-adds over k in ascending order, whatever the number
+// The additions of an output element and their order follow from the inner size K alone, whatever the number
 // of rows and wherever a row lies in its tile, so a token's result does not depend on how many other
 // tokens share its step: the float32 path gives the same bits for every way of cutting and batching the
 // work.  (A library product picks other kernels, and other orders of summation, for other row counts.)
-// CUDA cores only, no reduced-precision mode: this path exists to show faults that bfloat16 hides.
+//   K < 512    one chain of fused multiply-adds over k in ascending order, on the CUDA cores (f32_tiles.cuh)
+//   K >= 512   operands in two halves of 11 bits on the tensor cores, sums of 32 terms added in 32 bits (f32_tc.cuh).
+//              Off the 64-bit result by, relative to its norm, 1.5e-7 at K = 512, 1.5e-7 at 2048 and 1.7e-7 at 5632; the chain
+//              is off by 4.0e-7, 8.0e-7 and 1.3e-6.  Below 512 the chain is as near and the products are small.
+// No reduced-precision mode: this path exists to show faults that bfloat16 hides.
+// Against [6144, 2048] and [2048, 5632], chain and tensor cores: 1 row 29 and 20 us, 57 and 23; 32 rows 56 and 24, 69 and 28;
+// 512 rows 291 and 100 us (129 TFLOP/s), 330 and 83.
 // The reference runs every dense product in FP16 through cuBLAS (src/layers/mlp.cpp:120-130).
 
+#include "f32_tc.cuh"
 #include "f32_tiles.cuh"
 
 namespace mi {
@@ -65,7 +72,7 @@ dense_f32_narrow_kernel(DenseF32 g) {
 }
 
 // Which form: up to DF_NARROW_ROWS rows a product is bound by reading W, and the narrow tiles keep more of it in flight
-// (against [6144, 2048], narrow and wide: 16 rows 39 and 61 us, 32 rows 53 and 61, 48 rows 65 and 66; against [2048, 5632]:
+// (measured when larger inner sizes came here too: against [6144, 2048], narrow and wide: 16 rows 39 and 61 us, 32 rows 53 and 61, 48 rows 65 and 66; against [2048, 5632]:
 // 32 rows 66 and 163 us); above, wide tiles of 128 columns, or of 64 where those of 128 would leave SMs without one.
 constexpr int DF_NARROW_ROWS = 32, DF_SMS = 148;
 
@@ -92,28 +99,162 @@ static int dense_f32_launch(const DenseF32& g, int batch, bool vec, cudaStream_t
     return finish_launch(what);
 }
 
+// ---- inner sizes from f32tc::TC_MIN_K on: the tensor cores (f32_tc.cuh) ----
+
+// Rows of activations per tile and blocks per tile (1: no cluster), -1: chosen here.
+struct TcForm { int nt, split; };
+struct TcLaunch {
+    CUtensorMap map_w;
+    f32tc::RowMaps map_rows;
+    dim3 grid;
+    int split;
+    cudaStream_t stream;
+    const char* what;
+};
+
+template <bool PAIRED, int NT, bool SPLIT, bool VEC>
+static int f32_tc_launch_one(const f32tc::Problem& g, const TcLaunch& l) {
+    auto kern = f32tc::f32_tc_kernel<PAIRED, NT, SPLIT, VEC>;
+    const size_t smem = f32tc::smem_bytes(NT, l.split);
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = l.grid;
+    lc.blockDim = dim3(f32tc::threads(NT));
+    lc.dynamicSmemBytes = smem;
+    lc.stream = l.stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)l.split;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    lc.attrs = attr;
+    lc.numAttrs = SPLIT ? 1 : 0;
+    cudaLaunchKernelEx(&lc, kern, l.map_w, l.map_rows, g);
+    return finish_launch(l.what);
+}
+template <bool PAIRED, int NT>
+static int f32_tc_launch_nt(const f32tc::Problem& g, const TcLaunch& l) {
+    if constexpr (NT < 128) {
+        if (l.split > 1) return f32_tc_launch_one<PAIRED, NT, true, true>(g, l);
+    }
+    return f32_tc_launch_one<PAIRED, NT, false, true>(g, l);
+}
+
+// floats that hi and lo of `rows` rows take
+static int64_t f32_tc_scratch(int64_t rows, int K) { return rows > 32 ? 2 * rows * K : 0; }
+
+// `rows`: rows in all; `groups`: experts (0: a dense product).  `scratch`: f32_tc_scratch(rows * batch, K) floats.
+template <bool PAIRED>
+static int f32_tc_launch(f32tc::Problem g, float* scratch, int rows, int groups, int batch, TcForm form, cudaStream_t stream,
+                         const char* what) {
+    // all rows of W in one map: those of the experts, or of products that lie whole rows apart
+    const int64_t w_rows = groups ? (int64_t)groups * (PAIRED ? 2 : 1) * g.N : (int64_t)(batch - 1) * (g.sW / g.K) + g.N;
+    const bool vec = g.K % 4 == 0 && g.lda % 4 == 0 && g.sA % 4 == 0 && (batch == 1 || (g.sW > 0 && g.sW % g.K == 0)) &&
+                     w_rows < (1ll << 31) - 128 && 2ll * rows * batch < (1ll << 31) - 128 &&
+                     ((reinterpret_cast<uintptr_t>(g.A) | reinterpret_cast<uintptr_t>(g.W) | reinterpret_cast<uintptr_t>(scratch)) & 15) == 0;
+    const int64_t tiles_m = PAIRED ? (g.N + 63) / 64 : (g.N + 127) / 128;
+    auto tiles_of = [&](int nt) -> int64_t {
+        return groups ? (rows < rows / nt + groups ? rows : rows / nt + groups) : ((int64_t)rows + nt - 1) / nt;
+    };
+    int nt = vec ? form.nt : 32;
+    if (nt < 0) {
+        // A tile of 128 takes 1.6 times the time of one of 64 (55 and 34 us at K = 2048), so it pays where it saves waves.  Against
+        // [6144, 2048], tiles of 64 and 128: 128 rows 39 and 57 us, 512 rows 101 and 111; against [11264, 2048]: 69 and 58, 169 and 163.
+        const auto waves = [&](int64_t tiles) { return (tiles * tiles_m * batch + DF_SMS - 1) / DF_SMS; };
+        nt = rows <= 16 ? 16 : rows <= 32 ? 32 : 64;
+        if (rows / (groups ? groups : 1) > 64 && 8 * waves(tiles_of(128)) < 5 * waves(tiles_of(64))) nt = 128;
+    }
+    const int64_t tiles_y = tiles_of(nt);
+    if (tiles_y > 65535 || batch > 65535) {
+        set_last_error("%s: %d rows (%d products) exceed the grid limit", what, rows, batch);
+        return kBadShape;
+    }
+    TcLaunch l = {};
+    l.split = form.split;
+    if (l.split < 0) {
+        // Up to four blocks share a tile where tiles alone leave SMs without work: one row against [6144, 2048] 28 us, by two
+        // 19, by four 22; against [2048, 2048] 28, 18, 13, by eight 15; against [2048, 5632] 68, 38, 23, by eight 26.
+        l.split = 1;
+        while (l.split < 4 && 2 * l.split * tiles_m * tiles_y * batch <= DF_SMS) l.split *= 2;
+    }
+    if (!vec || nt == 128) l.split = 1;
+    while (l.split > 1 && l.split < f32tc::PARTS && (f32tc::PARTS / l.split) * nt * 512u > f32tc::SLOT_LIMIT) l.split *= 2;
+    l.grid = dim3((unsigned)(tiles_m * l.split), (unsigned)tiles_y, (unsigned)batch);
+    l.stream = stream;
+    l.what = what;
+    if (vec && !tc::make_map_f32(&l.map_w, g.W, (uint64_t)w_rows, (uint64_t)g.K, PAIRED ? 64 : 128)) {
+        set_last_error("%s: cuTensorMapEncodeTiled failed", what);
+        return kLaunchFailed;
+    }
+    if (f32tc::split_before(nt)) {
+        if (!scratch) { set_last_error("%s: no room for the rows' halves", what); return kBadShape; }
+        g.split_rows = (int64_t)rows * batch;
+        f32tc::f32_split_rows_kernel<<<dim3(rows, batch), 256, 0, stream>>>(g.A, g.gather, (uint4*)scratch, rows, g.lda, g.K / 4, g.sA,
+                                                                            g.split_rows);
+        const int rc = finish_launch(what);
+        if (rc != kOk) return rc;
+        if (!tc::make_map_f32(&l.map_rows.m16, scratch, 2ull * g.split_rows, (uint64_t)g.K, 16) ||
+            !tc::make_map_f32(&l.map_rows.whole, scratch, 2ull * g.split_rows, (uint64_t)g.K, (uint32_t)nt)) {
+            set_last_error("%s: cuTensorMapEncodeTiled failed", what);
+            return kLaunchFailed;
+        }
+    }
+    if (!vec) return f32_tc_launch_one<PAIRED, 32, false, false>(g, l);
+    switch (nt) {
+        case 16: return f32_tc_launch_nt<PAIRED, 16>(g, l);
+        case 32: return f32_tc_launch_nt<PAIRED, 32>(g, l);
+        case 64: return f32_tc_launch_nt<PAIRED, 64>(g, l);
+        default: return f32_tc_launch_nt<PAIRED, 128>(g, l);
+    }
+}
+
 }  // namespace mi
 
-extern "C" int mi_dense_f32(const float* A, const float* W, float* C, int T, int N, int K, cudaStream_t stream) {
-    using namespace mi;
-    if (T <= 0 || N <= 0) return kOk;
-    if (K <= 0) { set_last_error("dense product (float32): inner size %d", K); return kBadShape; }
-    const bool vec = (K % 4 == 0) && (((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W)) & 15) == 0);
-    return dense_f32_launch(DenseF32{A, W, C, T, N, K, K, N, 0, 0, 0}, 1, vec, stream, "dense_f32");
-}
+extern "C" int mi_f32_tc_min_inner() { return mi::f32tc::TC_MIN_K; }
+
+// Floats of scratch (16-byte aligned) that a product of `rows` rows (of all products together) takes.
+extern "C" int64_t mi_f32_tc_scratch(int64_t rows, int K) { return K >= mi::f32tc::TC_MIN_K ? mi::f32_tc_scratch(rows, K) : 0; }
 
 // `batch` products at once: C_b[T, N] = A_b[T, K] . W_b[N, K]^T with rows of A and C `lda` and `ldc` floats
 // apart and the operands of product b at A + b * sA, W + b * sW (rows K apart), C + b * sC: the heads of a
 // row of activations, each with a matrix of its own.  The same chain of additions per element as above.
 extern "C" int mi_dense_f32_batched(const float* A, const float* W, float* C, int T, int N, int K, int lda, int ldc,
-                                    int batch, int64_t sA, int64_t sW, int64_t sC, cudaStream_t stream) {
+                                    int batch, int64_t sA, int64_t sW, int64_t sC, float* scratch, int* status, cudaStream_t stream) {
     using namespace mi;
     if (T <= 0 || N <= 0 || batch <= 0) return kOk;
     if (K <= 0 || lda < K || ldc < N || batch > 65535) {
-        set_last_error("batched dense product (float32): inner size %d, rows %d and %d apart, %d products", K, lda, ldc, batch);
+        set_last_error("dense product (float32): inner size %d, rows %d and %d apart, %d products", K, lda, ldc, batch);
         return kBadShape;
     }
+    if (K >= f32tc::TC_MIN_K)
+        return f32_tc_launch<false>(f32tc::Problem{A, W, C, nullptr, nullptr, T, N, K, lda, ldc, 0, sA, sW, sC, 0, GluForm{}, status}, scratch, T, 0,
+                                    batch, TcForm{-1, -1}, stream, "dense_f32");
     const bool vec = (K % 4 == 0) && (lda % 4 == 0) && (sA % 4 == 0) && (sW % 4 == 0) &&
                      (((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W)) & 15) == 0);
-    return dense_f32_launch(DenseF32{A, W, C, T, N, K, lda, ldc, sA, sW, sC}, batch, vec, stream, "dense_f32_batched");
+    return dense_f32_launch(DenseF32{A, W, C, T, N, K, lda, ldc, sA, sW, sC}, batch, vec, stream, "dense_f32");
+}
+
+// C[T, N] = A[T, K] . W[N, K]^T.  `status` (device int, zero before the first call) receives a non-zero code if a wait inside
+// the kernel ran out.
+extern "C" int mi_dense_f32(const float* A, const float* W, float* C, int T, int N, int K, float* scratch, int* status,
+                            cudaStream_t stream) {
+    return mi_dense_f32_batched(A, W, C, T, N, K, K, N, 1, 0, 0, 0, scratch, status, stream);
+}
+// Grouped product of float operands (contract of mi_grouped_gemm_plain) for K >= mi_f32_tc_min_inner(); nt, split: rows of
+// activations per tile and blocks per tile, or -1.  E 0 and no offsets: one dense product.
+extern "C" int mi_f32_tc_form(const float* A, const int* gather, const float* W, const int* offsets, float* C, int n_rows, int E,
+                              int Nout, int K, int mode, int nt, int split, int glu_kind, float glu_limit, float glu_slope,
+                              const float* row_scale, float* scratch, int* status, cudaStream_t stream) {
+    using namespace mi;
+    if (n_rows <= 0 || Nout <= 0) return kOk;
+    const bool nts = nt == -1 || nt == 16 || nt == 32 || nt == 64 || nt == 128;
+    const bool splits = split == -1 || split == 1 || ((split == 2 || split == 4 || split == 8) && nt > 0);
+    if (K < f32tc::TC_MIN_K || !nts || !splits || (E > 0) != (offsets != nullptr) || (mode == 1 && E <= 0)) {
+        set_last_error("float32 product on tensor cores: inner size %d, %d experts, tiles of %d rows by %d blocks", K, E, nt, split);
+        return kBadShape;
+    }
+    const GluForm glu{glu_kind, glu_limit, glu_slope, mode == 1 ? row_scale : nullptr};
+    const f32tc::Problem g{A, W, C, gather, offsets, n_rows, Nout, K, K, Nout, E, 0, 0, 0, 0, glu, status};
+    const TcForm form{nt, split};
+    return mode == 1 ? f32_tc_launch<true>(g, scratch, n_rows, E, 1, form, stream, "grouped_gemm_plain")
+                     : f32_tc_launch<false>(g, scratch, n_rows, E, 1, form, stream, E ? "grouped_gemm_plain" : "dense_f32");
 }

@@ -1,4 +1,5 @@
-// Tiles of products in true 32 bits on the CUDA cores: what the dense and the grouped float32 products share.
+// Tiles of products in true 32 bits on the CUDA cores: what the dense and the grouped float32 products share (inner sizes
+// below 512; larger ones go to the tensor cores, f32_tc.cuh).
 //
 // Every output element is ONE chain of fused multiply-adds over k in ascending order, in every form below, so a
 // result has the same bits whichever form, tile or row of a tile computes it.  Two forms:
@@ -12,7 +13,7 @@
 //   NarrowTile 16 rows x 32 columns by 128 threads, 4 rows a warp, one column (or gate and up column) a lane.
 //              Bound by reading W: four tiles of 64 k arrive through cp.async while one is used.
 //
-// 512 rows against [6144, 2048] and [2048, 2048] (a q/k/v and an output product): 629 us with 64 x 64 tiles of 4 x 4
+// Measured when larger inner sizes came here: 512 rows against [6144, 2048] and [2048, 2048] (a q/k/v and an output product): 629 us with 64 x 64 tiles of 4 x 4
 // outputs a thread, 415 us with these (43 and 35 TFLOP/s; the FMA pipes are 70 % busy where every SM has blocks).
 #pragma once
 

@@ -937,9 +937,10 @@ __device__ __forceinline__ int find_row_tile(const int* __restrict__ offsets, in
     return 0;
 }
 
-// The grouped product of the true 32-bit path (contract as above, everything float), in the two forms of f32_tiles.cuh.
+// The grouped product of the true 32-bit path (contract as above, everything float) for inner sizes below 512, in the two
+// forms of f32_tiles.cuh (above: mi_f32_tc_form, dense_f32.cu).
 // A tile of a paired product holds gate rows of W in its first half of columns and the up rows of the same outputs in
-// its second, so that a thread has both.  512 tokens x 4 of 60 experts at [2 x 1408, 2048] and [2048, 1408], beside the
+// its second, so that a thread has both.  Measured when larger inner sizes came here: 512 tokens x 4 of 60 experts at [2 x 1408, 2048] and [2048, 1408], beside the
 // shared expert: 2.01 and 1.14 ms in tiles of 32 x 32 with one column a thread, 1.22 and 0.42 ms in these.
 struct GroupedF32 {
     const float* A; const int* gather; const float* W; const int* offsets; float* C;
@@ -1025,7 +1026,7 @@ grouped_f32_narrow_kernel(GroupedF32 g) {
     }
 }
 
-// Narrow tiles up to so many rows per expert on average: there a product is bound by reading the experts' weights (60 of
+// Narrow tiles up to so many rows per expert on average: there a product is bound by reading the experts' weights (then 60 of
 // [2 x 1408, 2048], narrow and wide: 8 rows each 407 and 640 us, 12 rows 433 and 643; with 17 and more a second narrow tile
 // is needed: 20 rows each 790 and 650 us).
 constexpr int GF_NARROW_ROWS = 12;

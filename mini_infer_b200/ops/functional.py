@@ -736,6 +736,8 @@ def grouped_gemm_plain(a: torch.Tensor, gather: Optional[torch.Tensor], w: torch
         _dbg_range(gather, 0, a.shape[0], "grouped_gemm_plain gather")
         if gather is None and a.shape[0] < n_rows:
             _bad("grouped_gemm_plain", f"{n_rows} rows wanted, the input has {a.shape[0]}")
+    if a.dtype == F32 and w.dtype == F32 and out_dtype == F32 and Kd >= library().mi_f32_tc_min_inner():
+        return f32_tc_form(a, gather, w, offsets, out, n_rows, swiglu_pair, glu, row_scale)
     check(library().mi_grouped_gemm_plain(_ptr(a), _code(a, "grouped_gemm a"), _ptr(gather), _ptr(w),
                                           _code(w, "grouped_gemm w"), _ptr(offsets), _ptr(out),
                                           _code(out, "grouped_gemm out"), int(n_rows), E, nout, Kd,
@@ -775,16 +777,42 @@ class dependent_launch:
         return False
 
 
+def f32_tc_form(a: torch.Tensor, gather: Optional[torch.Tensor], w: torch.Tensor, offsets: Optional[torch.Tensor],
+                out: torch.Tensor, n_rows: int, swiglu_pair: bool, glu=None, row_scale: Optional[torch.Tensor] = None,
+                rows_per_tile: int = -1, blocks_per_tile: int = -1) -> torch.Tensor:
+    """:func:`grouped_gemm_plain` (without ``offsets``: :func:`dense_f32`) of float32 operands with an inner size from
+    ``mi_f32_tc_min_inner()`` up, into ``out``: tensor cores, every operand as two numbers of 11 bits.  All forms
+    (``rows_per_tile`` 16, 32, 64, 128; ``blocks_per_tile`` 1, 2, 4, 8; -1: chosen by the sizes) give the same bits."""
+    global _tc_pending
+    E = 0 if offsets is None else w.shape[0]
+    nout = w.shape[-2] // 2 if swiglu_pair else w.shape[-2]
+    check(library().mi_f32_tc_form(_ptr(a), _ptr(gather), _ptr(w), _ptr(offsets), _ptr(out), int(n_rows), E, nout, a.shape[1],
+                                   1 if swiglu_pair else 0, int(rows_per_tile), int(blocks_per_tile), *_glu_args(glu),
+                                   _row_scale(row_scale, int(n_rows), swiglu_pair, "grouped_gemm_plain"),
+                                   _ptr(_f32_scratch(a, int(n_rows))), _ptr(_status_word(a.device)), _stream()), "f32_tc")
+    _tc_pending = True
+    return out
+
+
+def _f32_scratch(x: torch.Tensor, rows: int, K: Optional[int] = None) -> Optional[torch.Tensor]:
+    """Room for the two halves of ``rows`` rows in a float32 product on tensor cores (None where it takes none)."""
+    n = library().mi_f32_tc_scratch(rows, x.shape[-1] if K is None else K)
+    return torch.empty(n, dtype=F32, device=x.device) if n else None
+
+
 def dense_f32(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
-    """``x @ w.T`` in true float32 (``x [T, K]``, ``w [N, K]``): every output element is one chain of
-    fused multiply-adds over ``k`` in ascending order, so a row's result does not depend on how many rows
-    there are.  The dense product of the float32 path."""
+    """``x @ w.T`` in true float32 (``x [T, K]``, ``w [N, K]``): the additions of an output element and their order follow from
+    ``K`` alone (one chain of fused multiply-adds over ``k``, or from ``mi_f32_tc_min_inner()`` on chunks of 32), so a
+    row's result does not depend on how many rows there are.  The dense product of the float32 path."""
+    global _tc_pending
     _chk(x, "dense_f32 x", F32)
     T, K = x.shape
     _chk(w, "dense_f32 w", F32, (None, K))
     N = w.shape[0]
     out = torch.empty(T, N, dtype=F32, device=x.device)
-    check(library().mi_dense_f32(_ptr(x), _ptr(w), _ptr(out), T, N, K, _stream()), "dense_f32")
+    check(library().mi_dense_f32(_ptr(x), _ptr(w), _ptr(out), T, N, K, _ptr(_f32_scratch(x, T)),
+                                 _ptr(_status_word(x.device)), _stream()), "dense_f32")
+    _tc_pending = _tc_pending or K >= library().mi_f32_tc_min_inner()
     return out
 
 
@@ -972,6 +1000,13 @@ def _row_scale(row_scale: Optional[torch.Tensor], rows: int, swiglu_pair: bool, 
 
 _tc_status = {}
 _tc_pending = False
+
+
+def _status_word(dev: torch.device) -> torch.Tensor:
+    """The word in which kernels with bounded waits on ``dev`` say that one ran out (:func:`check_tc_status`)."""
+    if dev not in _tc_status:
+        _tc_status[dev] = torch.zeros(1, dtype=I32, device=dev)
+    return _tc_status[dev]
 
 
 TC_FORMS = (0, 1, 2, 3)
@@ -2024,6 +2059,7 @@ def dense_f32_heads(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor
     ``[T, *]`` float32 rows in which head ``h`` starts at column ``x_col + h * x_head_stride`` (default: heads
     of ``K`` side by side); ``out`` likewise (default ``[T, H * N]``).  The same fixed chain of additions per
     element as :func:`dense_f32`."""
+    global _tc_pending
     _chk(x, "dense_f32_heads x", F32)
     _chk(w, "dense_f32_heads w", F32)
     H, N, K = w.shape
@@ -2038,7 +2074,10 @@ def dense_f32_heads(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor
     if x_col + (H - 1) * xs + K > lda or out_col + (H - 1) * os_ + N > ldc:
         raise ValueError("dense_f32_heads: the heads do not fit the rows")
     check(library().mi_dense_f32_batched(x.data_ptr() + 4 * x_col, _ptr(w), out.data_ptr() + 4 * out_col, T, N, K,
-                                         lda, ldc, H, xs, N * K, os_, _stream()), "dense_f32_heads")
+                                         lda, ldc, H, xs, N * K, os_, _ptr(_f32_scratch(x, T * H, K)), _ptr(_status_word(x.device)),
+                                         _stream()),
+          "dense_f32_heads")
+    _tc_pending = _tc_pending or K >= library().mi_f32_tc_min_inner()
     return out
 
 

@@ -47,7 +47,8 @@ _SIGNATURES = {
     "mi_grouped_gemm_tc_form": [P, P, P, P, P, I, I, I, I, I, I, I, F, F, P, P],
     "mi_random_fill": [P, I, L, ctypes.c_uint, ctypes.c_uint, F, F, P],
     "mi_delta_blocks": [P, I, P, I, P, I, P, P, P, L, P, P, P, P, P, I, I, I, I, I, I, I, F, P],
-    "mi_dense_f32": [P, P, P, I, I, I, P],
+    "mi_dense_f32": [P, P, P, I, I, I, P, P, P],
+    "mi_f32_tc_form": [P, P, P, P, P, I, I, I, I, I, I, I, I, F, F, P, P, P, P],
     "mi_l2_prefetch": [P, ctypes.c_ulonglong, P],
     "mi_causal_conv_silu": [P, I, P, P, I, P, L, P, P, P, P, I, I, I, I, I, P],
     "mi_delta_scan": [P, I, P, I, P, I, P, P, P, L, P, P, P, P, I, I, I, I, I, I, F, P],
@@ -66,7 +67,7 @@ _SIGNATURES = {
     "mi_rows_plus_vec": [P, P, P, I, I, I, P],
     "mi_attn_prefill_tc_shared": [P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, F, I, P],
     "mi_clamped_glu": [P, P, I, L, I, F, F, P],
-    "mi_dense_f32_batched": [P, P, P, I, I, I, I, I, I, L, L, L, P],
+    "mi_dense_f32_batched": [P, P, P, I, I, I, I, I, I, L, L, L, P, P, P],
     "mi_latent_rows": [P, I, I, P, F, P, P, P, I, I, P, I, I, P, I, I, P, P, F, I, I, I, I, I, I, P],
     "mi_streams_embed": [P, P, P, P, I, F, P, L, L, L, P, P, P, I, I, P, I, F, P, I, I, I, I, P],
     "mi_streams_read": [P, P, P, P, P, P, P, I, P, I, I, I, I, F, P],
@@ -120,6 +121,8 @@ _OTHERS = {
     "mi_attn_prefill_tc_supported": ([I, I], c_int),
     "mi_qkv_skinny_supported": ([I, I, I], c_int),
     "mi_dense_skinny_max_rows": ([], c_int),
+    "mi_f32_tc_min_inner": ([], c_int),
+    "mi_f32_tc_scratch": ([L, I], c_int64),
     "mi_delta_scan_prep_row": ([I], c_int),
     "mi_delta_blocks_supported": ([I], c_int),
     "mi_delta_blocks_mats": ([], c_int),

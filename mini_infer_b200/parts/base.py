@@ -522,7 +522,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype) -> torch.Te
     bfloat16 path: the library product the reference also uses for every dense projection (cuBLAS,
     src/layers/attention.cpp:45-55, src/layers/mlp.cpp:120-130), accumulating in float32, or the engine's
     own decode kernel for the smallest steps.  float32 path (both operands float32): the engine's own
-    CUDA-core kernel, which adds in one fixed order whatever the number of rows, so that this path gives
+    kernels, which add in one fixed order whatever the number of rows, so that this path gives
     the same bits however the work is cut and batched."""
     from ..ops import functional as F
     if x.is_cuda and x.dtype == torch.float32 and w.dtype == torch.float32 and out_dtype == torch.float32:
