@@ -10,7 +10,7 @@
 //              is off by 4.0e-7, 8.0e-7 and 1.3e-6.  Below 512 the chain is as near and the products are small.
 // No reduced-precision mode: this path exists to show faults that bfloat16 hides.
 // Against [6144, 2048] and [2048, 5632], chain and tensor cores: 1 row 29 and 20 us, 57 and 23; 32 rows 56 and 24, 69 and 28;
-// 512 rows 291 and 100 us (129 TFLOP/s), 330 and 83.
+// 512 rows 291 and 94 us (137 TFLOP/s), 330 and 82.
 // The reference runs every dense product in FP16 through cuBLAS (src/layers/mlp.cpp:120-130).
 
 #include "f32_tc.cuh"
@@ -147,7 +147,8 @@ template <bool PAIRED>
 static int f32_tc_launch(f32tc::Problem g, float* scratch, int rows, int groups, int batch, TcForm form, cudaStream_t stream,
                          const char* what) {
     // all rows of W in one map: those of the experts, or of products that lie whole rows apart
-    const int64_t w_rows = groups ? (int64_t)groups * (PAIRED ? 2 : 1) * g.N : (int64_t)(batch - 1) * (g.sW / g.K) + g.N;
+    const int64_t own_rows = (PAIRED ? 2 : 1) * (int64_t)g.N;
+    const int64_t w_rows = groups ? groups * own_rows : (int64_t)(batch - 1) * (g.sW / g.K) + own_rows;
     const bool vec = g.K % 4 == 0 && g.lda % 4 == 0 && g.sA % 4 == 0 && (batch == 1 || (g.sW > 0 && g.sW % g.K == 0)) &&
                      w_rows < (1ll << 31) - 128 && 2ll * rows * batch < (1ll << 31) - 128 &&
                      ((reinterpret_cast<uintptr_t>(g.A) | reinterpret_cast<uintptr_t>(g.W) | reinterpret_cast<uintptr_t>(scratch)) & 15) == 0;
@@ -157,11 +158,12 @@ static int f32_tc_launch(f32tc::Problem g, float* scratch, int rows, int groups,
     };
     int nt = vec ? form.nt : 32;
     if (nt < 0) {
-        // A tile of 128 takes 1.6 times the time of one of 64 (55 and 34 us at K = 2048), so it pays where it saves waves.  Against
-        // [6144, 2048], tiles of 64 and 128: 128 rows 39 and 57 us, 512 rows 101 and 111; against [11264, 2048]: 69 and 58, 169 and 163.
+        // A tile of 128 takes 1.5 times the time of one of 64 (52 and 34 us at K = 2048), so it pays where it saves waves: against
+        // [6144, 2048], tiles of 64 and 128: 128 rows 36 and 54 us, 512 rows 94 and 104; against [11264, 2048]: 65 and 56, 162 and 152.
+        // 60 experts of [2 x 1408, 2048]: 34 rows each 314 and 356 us, 68 rows 474 and 423.
         const auto waves = [&](int64_t tiles) { return (tiles * tiles_m * batch + DF_SMS - 1) / DF_SMS; };
         nt = rows <= 16 ? 16 : rows <= 32 ? 32 : 64;
-        if (rows / (groups ? groups : 1) > 64 && 8 * waves(tiles_of(128)) < 5 * waves(tiles_of(64))) nt = 128;
+        if (groups ? rows > 48ll * groups : rows > 64 && 3 * waves(tiles_of(128)) < 2 * waves(tiles_of(64))) nt = 128;
     }
     const int64_t tiles_y = tiles_of(nt);
     if (tiles_y > 65535 || batch > 65535) {
@@ -172,9 +174,9 @@ static int f32_tc_launch(f32tc::Problem g, float* scratch, int rows, int groups,
     l.split = form.split;
     if (l.split < 0) {
         // Up to four blocks share a tile where tiles alone leave SMs without work: one row against [6144, 2048] 28 us, by two
-        // 19, by four 22; against [2048, 2048] 28, 18, 13, by eight 15; against [2048, 5632] 68, 38, 23, by eight 26.
+        // 19, by four 22; against [2048, 2048] 28, 18 and 13; against [2048, 5632] 68, 38 and 23 (by eight 15 and 26).
         l.split = 1;
-        while (l.split < 4 && 2 * l.split * tiles_m * tiles_y * batch <= DF_SMS) l.split *= 2;
+        while (l.split < f32tc::PARTS && 2 * l.split * tiles_m * tiles_y * batch <= DF_SMS) l.split *= 2;
     }
     if (!vec || nt == 128) l.split = 1;
     while (l.split > 1 && l.split < f32tc::PARTS && (f32tc::PARTS / l.split) * nt * 512u > f32tc::SLOT_LIMIT) l.split *= 2;
@@ -192,8 +194,8 @@ static int f32_tc_launch(f32tc::Problem g, float* scratch, int rows, int groups,
                                                                             g.split_rows);
         const int rc = finish_launch(what);
         if (rc != kOk) return rc;
-        if (!tc::make_map_f32(&l.map_rows.m16, scratch, 2ull * g.split_rows, (uint64_t)g.K, 16) ||
-            !tc::make_map_f32(&l.map_rows.whole, scratch, 2ull * g.split_rows, (uint64_t)g.K, (uint32_t)nt)) {
+        for (int i = 0; i < 4; ++i) {
+            if (tc::make_map_f32(&l.map_rows.m[i], scratch, 2ull * g.split_rows, (uint64_t)g.K, 16 * (i + 1))) continue;
             set_last_error("%s: cuTensorMapEncodeTiled failed", what);
             return kLaunchFailed;
         }
@@ -247,8 +249,8 @@ extern "C" int mi_f32_tc_form(const float* A, const int* gather, const float* W,
     using namespace mi;
     if (n_rows <= 0 || Nout <= 0) return kOk;
     const bool nts = nt == -1 || nt == 16 || nt == 32 || nt == 64 || nt == 128;
-    const bool splits = split == -1 || split == 1 || ((split == 2 || split == 4 || split == 8) && nt > 0);
-    if (K < f32tc::TC_MIN_K || !nts || !splits || (E > 0) != (offsets != nullptr) || (mode == 1 && E <= 0)) {
+    const bool splits = split == -1 || split == 1 || ((split == 2 || split == 4) && nt > 0);
+    if (K < f32tc::TC_MIN_K || !nts || !splits || (E > 0) != (offsets != nullptr)) {
         set_last_error("float32 product on tensor cores: inner size %d, %d experts, tiles of %d rows by %d blocks", K, E, nt, split);
         return kBadShape;
     }

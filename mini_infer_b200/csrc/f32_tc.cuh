@@ -10,7 +10,7 @@
 // here: see dense_f32.cu).
 //
 // Every output element is the same sums in the same order in every form below: chunks of 32 k in ascending order within
-// each of eight parts of the inner dimension, then the parts in ascending order.  So a row has the same bits however many
+// each of four parts of the inner dimension, then the parts in ascending order.  So a row has the same bits however many
 // rows share the step, in whichever tile and form, as the chains of the CUDA-core kernels have for smaller K.  A result that
 // is not finite (an operand that is not, or a sum that overflows) is computed again as a chain of multiply-adds, so infinities and
 // NaN reach exactly the elements that they reach there.
@@ -27,7 +27,7 @@
 //   tiles of 16 and 32: warps 19-22 bring the activations (cp.async, four chunks ahead) and make hi and lo of them in shared memory
 // What bounds a chunk of a tile of 64 or 128 is shared memory: weights written and read, activations written, and read by
 // every MMA.
-// SPLIT: a cluster of 2, 4 or 8 blocks shares a tile's parts and adds them up through distributed shared memory, where tiles
+// SPLIT: a cluster of 2 or 4 blocks shares a tile's parts and adds them up through distributed shared memory, where tiles
 // alone would leave SMs without work (a decode step's few rows).
 //
 // Every wait on an mbarrier is bounded: one that runs out sets the status word, and all roles fall through to the exit.
@@ -42,7 +42,7 @@ using namespace tc;
 
 constexpr int TC_MIN_K = 512;
 constexpr int FK = 32;                                 // k per chunk: 32 floats are a swizzled row of 128 bytes
-constexpr int PARTS = 8;
+constexpr int PARTS = 4;
 constexpr int OUT_WARP = 8, MMA_WARP = 16, W_WARP = 18, ROWS_WARP = 19;        // first warps of the roles
 constexpr bool split_before(int nt) { return nt >= 64; }
 constexpr int threads(int nt) { return 32 * (split_before(nt) ? 20 : 23); }
@@ -83,7 +83,7 @@ struct Problem {
     GluForm glu;
     int* status;
 };
-struct RowMaps { CUtensorMap m16, whole; };            // hi and lo of the activations in boxes of 16 rows and of a tile's
+struct RowMaps { CUtensorMap m[4]; };                  // hi and lo of the activations in boxes of 16, 32, 48 and 64 rows
 
 __device__ __forceinline__ void umma_tf32_tmem_a(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
                                                  uint32_t accumulate) {
@@ -314,9 +314,6 @@ f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
         float part[OWN];
 #pragma unroll
         for (int i = 0; i < OWN; ++i) part[i] = 0.f;
-        if (!SPLIT)
-#pragma unroll
-            for (int i = 0; i < OWN; ++i) own[i * 128] = 0.f;
         bool ok = true;
         int in_part = 0, parts = 0;
 #pragma unroll 1
@@ -343,9 +340,12 @@ f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
             if (lane == 0) mbar_arrive(&empty_bar[it % D_SLOTS]);
             if (++in_part == per_part || it == count - 1) {
                 float* to = own + (SPLIT ? parts * NT * 128 : 0);
+                if (!SPLIT && parts > 0)
+#pragma unroll
+                    for (int i = 0; i < OWN; ++i) part[i] = to[i * 128] + part[i];
 #pragma unroll
                 for (int i = 0; i < OWN; ++i) {
-                    to[i * 128] = SPLIT ? part[i] : to[i * 128] + part[i];
+                    to[i * 128] = 0.f + part[i];       // (a cluster's sums begin at +0, too)
                     part[i] = 0.f;
                 }
                 in_part = 0;
@@ -398,6 +398,8 @@ f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
     } else if (BEFORE) {
         if (lane == 0) {
             const int y_hi = (int)(blockIdx.z * (int64_t)g.T + row0), y_lo = y_hi + (int)g.split_rows;
+            const int n_rest = NT > 64 && n_mma > 64 ? n_mma - 64 : n_mma, at_rest = (n_mma - n_rest) * 128;
+            const CUtensorMap* rest = &map_rows.m[n_rest / 16 - 1];
             int i = 0;
 #pragma unroll 1
             for (; i < count; ++i) {
@@ -407,15 +409,12 @@ f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
                 uint64_t* bar = &rows_full[slot];
                 uint8_t *hi = hi_ring + slot * B_BYTES, *lo = lo_ring + slot * B_BYTES;
                 mbar_expect_tx(bar, 2 * n_mma * 128);
-                if (n_mma == NT) {
-                    tma_load_2d(hi, &map_rows.whole, k, y_hi, bar);
-                    tma_load_2d(lo, &map_rows.whole, k, y_lo, bar);
-                } else {
-                    for (int at = 0; at < n_mma; at += 16) {
-                        tma_load_2d(hi + at * 128, &map_rows.m16, k, y_hi + at, bar);
-                        tma_load_2d(lo + at * 128, &map_rows.m16, k, y_lo + at, bar);
-                    }
+                if (NT > 64 && n_mma > 64) {
+                    tma_load_2d(hi, &map_rows.m[3], k, y_hi, bar);
+                    tma_load_2d(lo, &map_rows.m[3], k, y_lo, bar);
                 }
+                tma_load_2d(hi + at_rest, rest, k, y_hi + n_mma - n_rest, bar);
+                tma_load_2d(lo + at_rest, rest, k, y_lo + n_mma - n_rest, bar);
             }
             for (int j = max(0, i - LO_SLOTS); j < i; ++j)
                 for (uint32_t n = 0; n < WAIT_LIMIT && !mbar_try_wait(&rows_full[j % LO_SLOTS], (j / LO_SLOTS) & 1); ++n) {}

@@ -777,12 +777,18 @@ class dependent_launch:
         return False
 
 
+def f32_tc_takes(x: torch.Tensor, w: torch.Tensor) -> bool:
+    """Whether :func:`f32_tc_form` takes this dense product: contiguous float32 rows of an inner size that is large enough."""
+    return (x.dtype == w.dtype == F32 and x.dim() == w.dim() == 2 and x.shape[1] == w.shape[1] and x.is_contiguous()
+            and w.is_contiguous() and w.shape[0] % 2 == 0 and x.shape[1] >= library().mi_f32_tc_min_inner())
+
+
 def f32_tc_form(a: torch.Tensor, gather: Optional[torch.Tensor], w: torch.Tensor, offsets: Optional[torch.Tensor],
                 out: torch.Tensor, n_rows: int, swiglu_pair: bool, glu=None, row_scale: Optional[torch.Tensor] = None,
                 rows_per_tile: int = -1, blocks_per_tile: int = -1) -> torch.Tensor:
-    """:func:`grouped_gemm_plain` (without ``offsets``: :func:`dense_f32`) of float32 operands with an inner size from
+    """:func:`grouped_gemm_plain` (without ``offsets``: :func:`dense_f32`, also paired) of float32 operands with an inner size from
     ``mi_f32_tc_min_inner()`` up, into ``out``: tensor cores, every operand as two numbers of 11 bits.  All forms
-    (``rows_per_tile`` 16, 32, 64, 128; ``blocks_per_tile`` 1, 2, 4, 8; -1: chosen by the sizes) give the same bits."""
+    (``rows_per_tile`` 16, 32, 64, 128; ``blocks_per_tile`` 1, 2, 4; -1: chosen by the sizes) give the same bits."""
     global _tc_pending
     E = 0 if offsets is None else w.shape[0]
     nout = w.shape[-2] // 2 if swiglu_pair else w.shape[-2]

@@ -512,6 +512,8 @@ def linear_swiglu(x: torch.Tensor, w_gate_up: torch.Tensor, act_dtype: torch.dty
     from ..ops import functional as F
     if x.is_cuda and x.shape[0] <= TUNING.dense_skinny_max_tokens and F.dense_skinny_takes(x, w_gate_up):
         return F.dense_skinny(x, w_gate_up, swiglu_pair=True, activation=activation)
+    if activation == "silu" and x.is_cuda and x.dtype == w_gate_up.dtype == act_dtype == torch.float32 and F.f32_tc_takes(x, w_gate_up):
+        return F.f32_tc_form(x, None, w_gate_up, None, x.new_empty(x.shape[0], w_gate_up.shape[0] // 2), x.shape[0], True)
     gu = linear(x, w_gate_up, act_dtype)
     return F.relu_glu(gu) if activation == "relu" else F.swiglu(gu)
 
