@@ -236,11 +236,16 @@ grouped_gemm_tc_kernel(const __grid_constant__ RowMaps maps_a, const __grid_cons
 // once.  The table of row tiles is built by every block for itself from the experts' offsets.
 //   warp 0    builds the table; TMA producer
 //   warp 1    tensor memory, MMAs
-//   warps 2-5 epilogue, one TMEM lane quarter each; a warp turns its 32 features x 32 rows through its
-//             own patch of shared memory so that rows leave in 16-byte stores
+//   warps 2-9 epilogue, two to a TMEM lane quarter that take groups of 32 rows in turn; a warp turns its 32 features x
+//             32 rows through its own patch of shared memory so that rows leave in 16-byte stores
+// The epilogue of a wide tile is not hidden (two tiles of 144 rows do not fit the tensor memory side by side), so it has eight
+// warps and tells the plain gated unit from the other forms once per group of rows, not for every number.  Gate and up of 60
+// experts of [2816, 2048]: 8,192 rows 183 -> 130 us (with four warps the gap between two tiles of a block was 15 us), 16,384
+// rows 276 -> 191 us, 4,096 rows 125 -> 116 us; the weights alone take 106 us.
 // NB: feature tiles of 128 per block in mode 0 (they share the row tile); mode 1 has gate and up.
+constexpr int EPILOGUE_WARPS = 8;
 template <int MODE, int TN, int STAGES, int NB>
-__global__ void __launch_bounds__(192, 1)
+__global__ void __launch_bounds__(32 * (2 + EPILOGUE_WARPS), 1)
 grouped_gemm_tc_persistent_kernel(const __grid_constant__ RowMaps maps_a, const __grid_constant__ CUtensorMap map_w,
                                   const int* __restrict__ offsets, void* __restrict__ C, int E, int Nout, int Kd,
                                   int* __restrict__ status, GluForm glu) {
@@ -254,8 +259,8 @@ grouped_gemm_tc_persistent_kernel(const __grid_constant__ RowMaps maps_a, const 
     __shared__ uint64_t full_bar[STAGES], empty_bar[STAGES], accum_full[2], accum_empty[2];
     __shared__ uint32_t tmem_base_s;
     __shared__ int abort_s, row_tiles_s;
-    constexpr int TURN_ROWS = MODE == 1 ? 32 : 16;        // rows of a warp's patch: 2 KiB either way
-    __shared__ __align__(16) uint8_t turn_s[4][TURN_ROWS * 32 * OUT_BYTES];   // per epilogue warp: [rows][32 features]
+    constexpr int TURN_ROWS = MODE == 1 ? 16 : 8;         // rows of a warp's patch: 1 KiB either way
+    __shared__ __align__(16) uint8_t turn_s[EPILOGUE_WARPS][TURN_ROWS * 32 * OUT_BYTES];      // per epilogue warp: [rows][32 features]
 
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     int2* table = reinterpret_cast<int2*>(smem + (size_t)STAGES * STAGE_BYTES);   // .x first row, .y expert << 16 | rows
@@ -265,7 +270,7 @@ grouped_gemm_tc_persistent_kernel(const __grid_constant__ RowMaps maps_a, const 
     if (threadIdx.x == 0) {
         abort_s = 0;
         for (int s = 0; s < STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
-        for (int s = 0; s < 2; ++s) { mbar_init(&accum_full[s], 1); mbar_init(&accum_empty[s], 4); }
+        for (int s = 0; s < 2; ++s) { mbar_init(&accum_full[s], 1); mbar_init(&accum_empty[s], EPILOGUE_WARPS); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
@@ -309,8 +314,7 @@ grouped_gemm_tc_persistent_kernel(const __grid_constant__ RowMaps maps_a, const 
 
     // Producer and MMA warp walk through their loops as whole warps and one lane issues, so that descriptors and
     // coordinates stay in uniform registers and a row tile's boxes leave together.  60 experts of [2816, 2048] and
-    // [2048, 1408]: 48 tokens 117 -> 109 us (6.4 TB/s of weights) and 69 -> 63 us; 2,048 tokens 194 -> 184 and 84 -> 80 us,
-    // where an SM takes in 24 bytes a cycle, weights and rows together, as it does at 48 tokens.
+    // [2048, 1408], 48 tokens: 117 -> 109 us (6.4 TB/s of weights) and 69 -> 63 us.
     if (warp == 0) {
         uint32_t it = 0;                                  // k blocks so far, over all tiles of this block
         bool ok = true;
@@ -385,7 +389,9 @@ grouped_gemm_tc_persistent_kernel(const __grid_constant__ RowMaps maps_a, const 
         const int quarter = warp & 3;
         const int fl = quarter * 32 + lane;
         const bool staged = (Nout % PER16) == 0 && ((reinterpret_cast<uintptr_t>(C) & 15) == 0);
-        uint8_t* turn = turn_s[quarter];
+        const int c_first = ((warp - 2) >> 2) * 32;
+        uint8_t* turn = turn_s[warp - 2];
+        const bool plain_unit = MODE == 1 && glu.kind == 0 && !glu.row_scale;
         uint32_t i = 0;
         bool ok = true;
         for (int tile = blockIdx.x; tile < total && ok; tile += gridDim.x) {
@@ -406,13 +412,19 @@ grouped_gemm_tc_persistent_kernel(const __grid_constant__ RowMaps maps_a, const 
                 if (fbase >= Nout) break;
                 const int f = fbase + fl;
 #pragma unroll 1
-                for (int c0 = 0; c0 < rows; c0 += 32) {
+                for (int c0 = c_first; c0 < rows; c0 += 64) {
                     uint32_t g[32];
                     tmem_ld32(lane_addr + half * pitch + c0, g);
                     if (MODE == 1) {
                         uint32_t u[32];
                         tmem_ld32(lane_addr + pitch + c0, u);
                         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                        if (plain_unit) {
+#pragma unroll
+                            for (int j = 0; j < 32; ++j)
+                                g[j] = (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(
+                                    glu_join_fast(__uint_as_float(g[j]), __uint_as_float(u[j]), GluForm{0, 0.f, 0.f, nullptr})));
+                        } else {
 #pragma unroll
                         for (int j = 0; j < 32; ++j) {
                             // (rows beyond the tile's last hold nothing and are not stored)
@@ -421,6 +433,7 @@ grouped_gemm_tc_persistent_kernel(const __grid_constant__ RowMaps maps_a, const 
                             // the result is rounded to bfloat16: the fast exponential and division are exact enough
                             g[j] = (uint32_t)__bfloat16_as_ushort(
                                 __float2bfloat16_rn(glu_join_fast(gv, __uint_as_float(u[j]) * rs, glu)));
+                        }
                         }
                     } else {
                         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
@@ -603,7 +616,7 @@ int mi_grouped_gemm_tc_form(const void* A, const void* W, const int* offsets, vo
     do {                                                                                              \
         auto kern = tc::grouped_gemm_tc_persistent_kernel<MODE, TN, ST, NB>;                          \
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);           \
-        kern<<<blocks, 192, smem, stream>>>(maps_a, map_w, offsets, C, E, Nout, Kd, status, glu);     \
+        kern<<<blocks, 32 * (2 + tc::EPILOGUE_WARPS), smem, stream>>>(maps_a, map_w, offsets, C, E, Nout, Kd, status, glu); \
     } while (0)
         if (form == 3) { if (mode == 1) MI_TCP_LAUNCH(1, 256, 3, 2); else MI_TCP_LAUNCH(0, 256, 3, 2); }
         else if (mode == 1) MI_TCP_LAUNCH(1, 160, 4, 2);
