@@ -500,6 +500,14 @@ def decode_split_size() -> int:
 DECODE_SPLIT_SIZES = (128, 256, 512)      # the split sizes the decode attention is built for
 
 
+def decode_joined_split(requests: int, heads: int, d: int, longest: int) -> Optional[int]:
+    """The smallest split with which a bfloat16 decode attention over up to ``longest`` keys takes one launch (None: none does)."""
+    for split in DECODE_SPLIT_SIZES:
+        if library().mi_attn_decode_joined(int(d), int(requests) * int(heads), -(-int(longest) // split)):
+            return split
+    return None
+
+
 def decode_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, block_table: torch.Tensor,
                      q_start: torch.Tensor, kv_len: torch.Tensor, part_o: torch.Tensor, part_ml: torch.Tensor,
                      max_splits: int, window: int = 0, scale: Optional[float] = None,

@@ -130,8 +130,9 @@ class GQAttention(Mixer):
         if self.rt.act == torch.float32:
             a = F.attention(q, kc, vc, view.block_table, ctx.q_start, ctx.kv_len, ctx.max_q_len, self.window)
         elif ctx.all_decode and "attn_part_o" in ctx.scratch and F.decode_attention_supported(self.d):
-            # one or two requests alone cannot fill the device with splits of 512 keys
-            split = TUNING.decode_split(ctx.num_requests, F.decode_split_size())
+            # a few requests alone cannot fill the device with splits of 512 keys
+            split = TUNING.decode_split(ctx.num_requests, F.decode_split_size(),
+                                        F.decode_joined_split(ctx.num_requests, q.shape[1], q.shape[2], ctx.max_kv_len))
             splits = -(-ctx.max_kv_len // split)
             a = F.decode_attention(q, kc, vc, view.block_table, ctx.q_start, ctx.kv_len,
                                    ctx.scratch["attn_part_o"], ctx.scratch["attn_part_ml"], splits, self.window,

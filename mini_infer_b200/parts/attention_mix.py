@@ -259,8 +259,9 @@ class HeadMixAttention(Mixer):
                                 self.window, self.scale, self.softcap, self.keep_first, sink=self.sink,
                                 head_bias=self.head_bias, **form)
         elif ctx.all_decode and self._split_decode and "attn_part_o" in ctx.scratch:
-            # one or two requests alone cannot fill the device with splits of 512 keys
-            split = TUNING.decode_split(ctx.num_requests, F.decode_split_size())
+            # a few requests alone cannot fill the device with splits of 512 keys
+            split = TUNING.decode_split(ctx.num_requests, F.decode_split_size(),
+                                        F.decode_joined_split(ctx.num_requests, q.shape[1], q.shape[2], ctx.max_kv_len))
             a = F.decode_attention(q, kc, vc, view.block_table, ctx.q_start, ctx.kv_len, ctx.scratch["attn_part_o"],
                                    ctx.scratch["attn_part_ml"], -(-ctx.max_kv_len // split), self.window,
                                    scale=self.scale, split=split, softcap=self.softcap, sink=self.sink, **form)

@@ -11,7 +11,7 @@ Qwen2-57B-A14B sizes; another width, expert count or GPU should re-measure them 
 from __future__ import annotations
 
 from dataclasses import dataclass
-from typing import Tuple
+from typing import Optional, Tuple
 
 
 @dataclass
@@ -55,6 +55,10 @@ class Tuning:
     # cannot fill 148 SMs with splits of 512 keys; splits of 256 for every batch size gained 4 % at batch 1
     # and lost 6 % at batch 8, hence the steps.  (bfloat16 path only: the float32 path runs one attention
     # kernel for every step, so that a request's logits do not depend on its batch.)
+    # These hold where the splits of a head do not go as a cluster in one launch; where they do (heads of 128, up to eight
+    # splits, no more blocks than the device holds), the smallest such split: 128, 256 and 512 keys, us, 8 requests of 600 keys
+    # 7.9, 9.9, 13.7 (8 heads); 6 of 2,000 19.3, 15.4, 16.2 (16 heads, 128 does not go as a cluster); 4 of 2,000 20.2, 19.4, 18.2
+    # (28 heads, 512 alone does).
     decode_split_by_requests: Tuple[Tuple[int, int], ...] = ((2, 128), (4, 256))
 
     # Chunked prefill: every full portion of a long prompt has the same shape, so its forward pass is replayed
@@ -149,7 +153,9 @@ class Tuning:
         step = 2 if num_requests <= 32 else (4 if num_requests <= 64 else 8)
         return -(-num_requests // step) * step
 
-    def decode_split(self, num_requests: int, default: int) -> int:
+    def decode_split(self, num_requests: int, default: int, joined: Optional[int] = None) -> int:
+        if joined is not None:
+            return joined
         for limit, split in self.decode_split_by_requests:
             if num_requests <= limit:
                 return split
