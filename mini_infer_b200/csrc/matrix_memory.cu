@@ -84,18 +84,23 @@ __device__ __forceinline__ void log_gates(const LogGates& g, int64_t t, int h, f
 // gates [T][H] = (keep, write, exp(-m), f);  logs [T][H] = (i, m, m before, 0) or null.
 // SCAN: the step m -> max(f + m, i) as the pair (f, i), pairs composed by warps and then over the warps: the sums of f
 // run in another order than in the chain, which is what the chunks of long portions do with them anyway.
+// A round takes a token per thread, and a round's latency (projections, two hyperbolic tangents, logarithms) is most of its time:
+// with SCAN rounds of 1,024 (2,048 tokens: 12.2 us in rounds of 256, 8.8 in these).
+constexpr int gate_threads(bool scan) { return scan ? 1024 : 256; }
+
 template <bool SCAN>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(gate_threads(SCAN))
 memory_gates_kernel(LogGates lg, State st, const int* __restrict__ q_start, const int* __restrict__ state_slot,
                     float4* __restrict__ gates, float4* __restrict__ logs, int H) {
-    __shared__ float si[256], sf[256], sm[257], wf[8], wi[8];
+    constexpr int N = gate_threads(SCAN);
+    __shared__ float si[256], sf[256], sm[N + 1], wf[N / 32], wi[N / 32];
     wait_for_earlier_kernels();
     const int h = blockIdx.x, b = blockIdx.y, tid = threadIdx.x;
     const int q0 = q_start[b], n = q_start[b + 1] - q0;
     float* m_state = st.row(state_slot[b]) + st.m_off + h;
     if (tid == 0) sm[0] = *m_state;
-    for (int c0 = 0; c0 < n; c0 += 256) {
-        const int nc = min(256, n - c0);
+    for (int c0 = 0; c0 < n; c0 += N) {
+        const int nc = min(N, n - c0);
         float li = -INFINITY, lf = 0.f;                  // (beyond the portion: a step that changes nothing)
         if (tid < nc) log_gates(lg, q0 + c0 + tid, h, li, lf);
         if (SCAN) {
@@ -575,6 +580,12 @@ __device__ __forceinline__ void copy_async_16b(void* smem_dst, const void* src) 
 }
 __device__ __forceinline__ void copy_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
+__device__ __forceinline__ void activate8(uint4& r) {
+    __nv_bfloat16* e = reinterpret_cast<__nv_bfloat16*>(&r);
+#pragma unroll
+    for (int x = 0; x < 8; ++x) { const float f = __bfloat162float(e[x]); e[x] = __float2bfloat16_rn(__fdividef(f, 1.0f + __expf(-f))); }
+}
+
 // eight neighbouring numbers of a row through the activation (zeros from column n on)
 __device__ __forceinline__ uint4 load8(const __nv_bfloat16* p, int n, int act, bool vec) {
     uint4 r = make_uint4(0u, 0u, 0u, 0u);
@@ -584,10 +595,7 @@ __device__ __forceinline__ uint4 load8(const __nv_bfloat16* p, int n, int act, b
 #pragma unroll
         for (int x = 0; x < 8; ++x) if (x < n) e[x] = p[x];
     }
-    if (act) {
-#pragma unroll
-        for (int x = 0; x < 8; ++x) { const float f = __bfloat162float(e[x]); e[x] = __float2bfloat16_rn(__fdividef(f, 1.0f + __expf(-f))); }
-    }
+    if (act) activate8(r);
     return r;
 }
 
@@ -605,10 +613,11 @@ __device__ __forceinline__ void fill_rows(__nv_bfloat16* dst, int pitch, const _
 }
 
 // U [chunk][H][d][dvp] (dvp: dv rounded up to 8, zeros beyond dv), Un [chunk][H][d] (log gates), keepc [chunk][H].  A block
-// of 4 warps takes a value tile of 64 columns of one (chunk, head).  The weights go into the values, w_j v_j, as high part
+// of 8 warps takes a value tile of 64 columns of one (chunk, head).  The weights go into the values, w_j v_j, as high part
 // and remainder: a tile's values are its own, while its keys serve every tile of the head.  dp = d rounded up to 16.
+constexpr int kStateThreads = 256;
 template <bool LOG>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(kStateThreads)
 memory_chunk_states_kernel(RowsB in, const float4* __restrict__ gates, const float4* __restrict__ logs,
                            const float* __restrict__ decay, const int* __restrict__ q_start, float* __restrict__ U,
                            float* __restrict__ Un, float* __restrict__ keepc, int H, int d, int dv, int dvp, int dp,
@@ -627,13 +636,27 @@ memory_chunk_states_kernel(RowsB in, const float4* __restrict__ gates, const flo
     __nv_bfloat16* Vh = Ks + kC * kp;                               // [64][kVP] weighted values, high parts
     __nv_bfloat16* Vl = Vh + kC * kVP;                              // remainders
     const int v_lo = tile * kT, nv = min(kT, dv - v_lo);
+    // All that comes from memory is asked for before any of it is used: 2,048 tokens, 4 heads of 256 x 512 (67 MB written) 36 us
+    // with 4 warps and the values asked for behind the weights, 30 us here.
+    constexpr int VN = kC * (kT / 8) / kStateThreads;
+    uint4 v_raw[VN];
+#pragma unroll
+    for (int x = 0; x < VN; ++x) {
+        const int idx = tid + x * kStateThreads, j = idx / (kT / 8), i = 8 * (idx % (kT / 8));
+        v_raw[x] = make_uint4(0u, 0u, 0u, 0u);
+        if (j < nt) v_raw[x] = load8(in.p + (t0 + j) * in.ld + in.v + (int64_t)h * dv + v_lo + i, nv - i, 0, in.vec);
+    }
+    float4 lg = make_float4(0.f, 0.f, 0.f, 0.f);
+    float m_end = 0.f;
+    if (LOG && tid < kC) {
+        if (tid < nt) lg = logs[(t0 + tid) * H + h];
+        m_end = logs[(t0 + nt - 1) * H + h].y;
+    }
     fill_rows(Ks, kp, in.p + t0 * in.ld + in.k + h * d, in.ld, d, dp, nt, in.act, in.vec);
     if (LOG) {
         chunk_log_decays(gates, t0, nt, H, h, Fh, Fl);
         __syncthreads();
         if (tid < kC) {
-            const float4 lg = tid < nt ? logs[(t0 + tid) * H + h] : make_float4(0.f, 0.f, 0.f, 0.f);
-            const float m_end = logs[(t0 + nt - 1) * H + h].y;
             wj[tid] = tid < nt ? expf((Fh[nt - 1] - Fh[tid]) + (Fl[nt - 1] - Fl[tid]) + (lg.x - m_end)) : 0.f;
             if (tid == 0 && tile == 0) keepc[at] = expf(Fh[nt - 1] + (lg.z - m_end));
         }
@@ -643,10 +666,11 @@ memory_chunk_states_kernel(RowsB in, const float4* __restrict__ gates, const flo
         if (tid == 0 && tile == 0) keepc[at] = expf((float)nt * ld);
     }
     __syncthreads();
-    for (int idx = tid; idx < kC * (kT / 8); idx += 128) {
-        const int j = idx / (kT / 8), i = 8 * (idx % (kT / 8));
-        uint4 v = make_uint4(0u, 0u, 0u, 0u), lo8;
-        if (j < nt) v = load8(in.p + (t0 + j) * in.ld + in.v + (int64_t)h * dv + v_lo + i, nv - i, in.act, in.vec);
+#pragma unroll
+    for (int x8 = 0; x8 < VN; ++x8) {
+        const int idx = tid + x8 * kStateThreads, j = idx / (kT / 8), i = 8 * (idx % (kT / 8));
+        uint4 v = v_raw[x8], lo8;
+        if (in.act) activate8(v);
         __nv_bfloat16* hi = reinterpret_cast<__nv_bfloat16*>(&v);
         __nv_bfloat16* lo = reinterpret_cast<__nv_bfloat16*>(&lo8);
         const float w = wj[j];
@@ -659,7 +683,7 @@ memory_chunk_states_kernel(RowsB in, const float4* __restrict__ gates, const flo
     __syncthreads();
     float* Ub = U + at * d * dvp + v_lo;
     const int nvp = min(kT, dvp - v_lo);
-    for (int mt = warp; mt < dp / 16; mt += 4) {
+    for (int mt = warp; mt < dp / 16; mt += kStateThreads / 32) {
         float acc[8][4];
 #pragma unroll
         for (int x = 0; x < 8; ++x) acc[x][0] = acc[x][1] = acc[x][2] = acc[x][3] = 0.f;
@@ -691,7 +715,7 @@ memory_chunk_states_kernel(RowsB in, const float4* __restrict__ gates, const flo
         }
     }
     if (LOG && tile == 0)
-        for (int i = tid; i < d; i += 128) {
+        for (int i = tid; i < d; i += kStateThreads) {
             float s = 0.f;
             for (int j = 0; j < nt; ++j) s += wj[j] * __bfloat162float(Ks[j * kp + i]);
             Un[at * d + i] = s;
@@ -965,7 +989,7 @@ int mi_memory_gates(const float* proj, int ld, int col_i, int col_f, const float
     const mem::LogGates lg = {proj, ld, col_i, col_f, bi, bf, cap};
     const mem::State st = {state, stride, 0, 0, m_off};
     if (scan)
-        launch_dependent(mem::memory_gates_kernel<true>, dim3(H, B), dim3(256), 0, stream, lg, st, q_start, state_slot,
+        launch_dependent(mem::memory_gates_kernel<true>, dim3(H, B), dim3(mem::gate_threads(true)), 0, stream, lg, st, q_start, state_slot,
                          (float4*)gates, (float4*)logs, H);
     else
         launch_dependent(mem::memory_gates_kernel<false>, dim3(H, B), dim3(256), 0, stream, lg, st, q_start, state_slot,
@@ -1047,7 +1071,7 @@ int mi_memory_chunks(const void* proj, int ld, int col_q, int col_k, int col_v, 
     do {                                                                                                               \
         cudaFuncSetAttribute(mem::memory_chunk_states_kernel<LOG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_s); \
         cudaFuncSetAttribute(mem::memory_chunk_outputs_kernel<LOG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_o); \
-        launch_dependent(mem::memory_chunk_states_kernel<LOG>, dim3(chunks, H * tiles, B), dim3(128), smem_s, stream, in, \
+        launch_dependent(mem::memory_chunk_states_kernel<LOG>, dim3(chunks, H * tiles, B), dim3(mem::kStateThreads), smem_s, stream, in, \
                          (const float4*)gates, (const float4*)logs, decay, q_start, U, Un, keepc, H, d, dv, dvp, dp, tiles); \
         launch_behind(mem::memory_chunk_chain_kernel, dim3((d * (dvp / 8) + 255) / 256 + (LOG ? 1 : 0), H, B), dim3(256), \
                          0, stream, U, LOG ? Un : nullptr, (const float*)keepc, state, stride, s_off, n_off, q_start,  \
