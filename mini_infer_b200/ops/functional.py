@@ -800,16 +800,19 @@ def f32_tc_form(a: torch.Tensor, gather: Optional[torch.Tensor], w: torch.Tensor
     global _tc_pending
     E = 0 if offsets is None else w.shape[0]
     nout = w.shape[-2] // 2 if swiglu_pair else w.shape[-2]
+    status = _status_word(a.device)
+    scratch = _f32_scratch(a, int(n_rows))
     check(library().mi_f32_tc_form(_ptr(a), _ptr(gather), _ptr(w), _ptr(offsets), _ptr(out), int(n_rows), E, nout, a.shape[1],
                                    1 if swiglu_pair else 0, int(rows_per_tile), int(blocks_per_tile), *_glu_args(glu),
                                    _row_scale(row_scale, int(n_rows), swiglu_pair, "grouped_gemm_plain"),
-                                   _ptr(_f32_scratch(a, int(n_rows))), _ptr(_status_word(a.device)), _stream()), "f32_tc")
+                                   _ptr(scratch), _ptr(status), _stream()), "f32_tc")
     _tc_pending = True
     return out
 
 
 def _f32_scratch(x: torch.Tensor, rows: int, K: Optional[int] = None) -> Optional[torch.Tensor]:
-    """Room for the two halves of ``rows`` rows in a float32 product on tensor cores (None where it takes none)."""
+    """Room for the two halves of ``rows`` rows in a float32 product on tensor cores (None where it takes none).  The caller
+    holds it until the product is queued: a block that is given back before may be given out again, and written, ahead of it."""
     n = library().mi_f32_tc_scratch(rows, x.shape[-1] if K is None else K)
     return torch.empty(n, dtype=F32, device=x.device) if n else None
 
@@ -824,8 +827,9 @@ def dense_f32(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
     _chk(w, "dense_f32 w", F32, (None, K))
     N = w.shape[0]
     out = torch.empty(T, N, dtype=F32, device=x.device)
-    check(library().mi_dense_f32(_ptr(x), _ptr(w), _ptr(out), T, N, K, _ptr(_f32_scratch(x, T)),
-                                 _ptr(_status_word(x.device)), _stream()), "dense_f32")
+    status = _status_word(x.device)
+    scratch = _f32_scratch(x, T)
+    check(library().mi_dense_f32(_ptr(x), _ptr(w), _ptr(out), T, N, K, _ptr(scratch), _ptr(status), _stream()), "dense_f32")
     _tc_pending = _tc_pending or K >= library().mi_f32_tc_min_inner()
     return out
 
@@ -2087,9 +2091,10 @@ def dense_f32_heads(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor
     ldc = out.numel() // max(T, 1)
     if x_col + (H - 1) * xs + K > lda or out_col + (H - 1) * os_ + N > ldc:
         raise ValueError("dense_f32_heads: the heads do not fit the rows")
+    status = _status_word(x.device)
+    scratch = _f32_scratch(x, T * H, K)
     check(library().mi_dense_f32_batched(x.data_ptr() + 4 * x_col, _ptr(w), out.data_ptr() + 4 * out_col, T, N, K,
-                                         lda, ldc, H, xs, N * K, os_, _ptr(_f32_scratch(x, T * H, K)), _ptr(_status_word(x.device)),
-                                         _stream()),
+                                         lda, ldc, H, xs, N * K, os_, _ptr(scratch), _ptr(status), _stream()),
           "dense_f32_heads")
     _tc_pending = _tc_pending or K >= library().mi_f32_tc_min_inner()
     return out
