@@ -190,8 +190,8 @@ static int f32_tc_launch(f32tc::Problem g, float* scratch, int rows, int groups,
     if (f32tc::split_before(nt)) {
         if (!scratch) { set_last_error("%s: no room for the rows' halves", what); return kBadShape; }
         g.split_rows = (int64_t)rows * batch;
-        f32tc::f32_split_rows_kernel<<<dim3(rows, batch), 256, 0, stream>>>(g.A, g.gather, (uint4*)scratch, rows, g.lda, g.K / 4, g.sA,
-                                                                            g.split_rows);
+        f32tc::f32_split_rows_kernel<<<dim3(rows, batch), 256, 0, stream>>>(g.A, g.gather, g.offsets, g.E, (uint4*)scratch, rows, g.lda,
+                                                                            g.K / 4, g.sA, g.split_rows);
         const int rc = finish_launch(what);
         if (rc != kOk) return rc;
         for (int i = 0; i < 4; ++i) {

@@ -162,11 +162,13 @@ __device__ __forceinline__ int row_tile(const int* __restrict__ offsets, int E, 
     return 0;
 }
 
-// hi and lo of rows of activations (K a multiple of 4): out[r] and out[rows + r] of x[gather ? gather[r] : r]
+// hi and lo of rows of activations (K a multiple of 4): out[r] and out[rows + r] of x[gather ? gather[r] : r].  Grouped: only the
+// rows that an expert has; beyond them `gather` need not be written.
 __global__ void __launch_bounds__(256)
-f32_split_rows_kernel(const float* __restrict__ x, const int* __restrict__ gather, uint4* __restrict__ out, int rows, int lda,
-                      int K4, int64_t sA, int64_t all_rows) {
+f32_split_rows_kernel(const float* __restrict__ x, const int* __restrict__ gather, const int* __restrict__ offsets, int E,
+                      uint4* __restrict__ out, int rows, int lda, int K4, int64_t sA, int64_t all_rows) {
     const int r = blockIdx.x;
+    if (offsets && r >= __ldg(offsets + E)) return;
     const uint4* src = reinterpret_cast<const uint4*>(x + blockIdx.y * sA + (int64_t)(gather ? __ldg(gather + r) : r) * lda);
     uint4* hi = out + ((int64_t)blockIdx.y * rows + r) * K4;
     for (int i = threadIdx.x; i < K4; i += 256) {

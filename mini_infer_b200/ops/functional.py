@@ -798,13 +798,21 @@ def f32_tc_form(a: torch.Tensor, gather: Optional[torch.Tensor], w: torch.Tensor
     ``mi_f32_tc_min_inner()`` up, into ``out``: tensor cores, every operand as two numbers of 11 bits.  All forms
     (``rows_per_tile`` 16, 32, 64, 128; ``blocks_per_tile`` 1, 2, 4; -1: chosen by the sizes) give the same bits."""
     global _tc_pending
+    _chk(a, "f32_tc a", F32)
+    n_rows, Kd = int(n_rows), a.shape[1]
+    _chk(w, "f32_tc w", F32, (None, Kd) if offsets is None else (None, None, Kd))
     E = 0 if offsets is None else w.shape[0]
     nout = w.shape[-2] // 2 if swiglu_pair else w.shape[-2]
+    _chk(gather, "f32_tc gather", I32)
+    _chk(offsets, "f32_tc offsets", I32, (E + 1,))
+    _chk(out, "f32_tc out", F32, (n_rows, nout))
+    if offsets is None and (a if gather is None else gather).shape[0] < n_rows:
+        raise ValueError(f"f32_tc: the input has fewer than {n_rows} rows")
     status = _status_word(a.device)
-    scratch = _f32_scratch(a, int(n_rows))
-    check(library().mi_f32_tc_form(_ptr(a), _ptr(gather), _ptr(w), _ptr(offsets), _ptr(out), int(n_rows), E, nout, a.shape[1],
+    scratch = _f32_scratch(a, n_rows)
+    check(library().mi_f32_tc_form(_ptr(a), _ptr(gather), _ptr(w), _ptr(offsets), _ptr(out), n_rows, E, nout, Kd,
                                    1 if swiglu_pair else 0, int(rows_per_tile), int(blocks_per_tile), *_glu_args(glu),
-                                   _row_scale(row_scale, int(n_rows), swiglu_pair, "grouped_gemm_plain"),
+                                   _row_scale(row_scale, n_rows, swiglu_pair, "grouped_gemm_plain"),
                                    _ptr(scratch), _ptr(status), _stream()), "f32_tc")
     _tc_pending = True
     return out
