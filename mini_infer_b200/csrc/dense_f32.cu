@@ -133,14 +133,18 @@ static int f32_tc_launch_one(const f32tc::Problem& g, const TcLaunch& l) {
 }
 template <bool PAIRED, int NT>
 static int f32_tc_launch_nt(const f32tc::Problem& g, const TcLaunch& l) {
-    if constexpr (NT < 128) {
-        if (l.split > 1) return f32_tc_launch_one<PAIRED, NT, true, true>(g, l);
-    }
-    return f32_tc_launch_one<PAIRED, NT, false, true>(g, l);
+    return l.split > 1 ? f32_tc_launch_one<PAIRED, NT, true, true>(g, l) : f32_tc_launch_one<PAIRED, NT, false, true>(g, l);
 }
 
-// floats that hi and lo of `rows` rows take
-static int64_t f32_tc_scratch(int64_t rows, int K) { return rows > 32 ? 2 * rows * K : 0; }
+// Rows whose parts are made ahead of a product, at most so many bytes of them at a time: a product of more rows goes in bands of
+// whole tiles (its rows do not touch each other).
+constexpr int64_t TC_SCRATCH_BYTES = 128ll << 20;
+static int64_t f32_tc_pitch(int K) { return (K + 7) & ~7; }            // bfloat16 numbers from row to row: 16 bytes and more
+// floats that the parts of `rows` rows take
+static int64_t f32_tc_scratch(int64_t rows, int K) {
+    const int64_t band = TC_SCRATCH_BYTES / (6 * f32_tc_pitch(K)) / 64 * 64, most = band > 64 ? band : 64;
+    return rows > 32 ? (3 * (rows < most ? rows : most) * f32_tc_pitch(K) + 1) / 2 : 0;
+}
 
 // `rows`: rows in all; `groups`: experts (0: a dense product).  `scratch`: f32_tc_scratch(rows * batch, K) floats.
 template <bool PAIRED>
@@ -150,63 +154,63 @@ static int f32_tc_launch(f32tc::Problem g, float* scratch, int rows, int groups,
     const int64_t own_rows = (PAIRED ? 2 : 1) * (int64_t)g.N;
     const int64_t w_rows = groups ? groups * own_rows : (int64_t)(batch - 1) * (g.sW / g.K) + own_rows;
     const bool vec = g.K % 4 == 0 && g.lda % 4 == 0 && g.sA % 4 == 0 && (batch == 1 || (g.sW > 0 && g.sW % g.K == 0)) &&
-                     w_rows < (1ll << 31) - 128 && 2ll * rows * batch < (1ll << 31) - 128 &&
+                     w_rows < (1ll << 31) - 128 &&
                      ((reinterpret_cast<uintptr_t>(g.A) | reinterpret_cast<uintptr_t>(g.W) | reinterpret_cast<uintptr_t>(scratch)) & 15) == 0;
     const int64_t tiles_m = PAIRED ? (g.N + 63) / 64 : (g.N + 127) / 128;
-    auto tiles_of = [&](int nt) -> int64_t {
-        return groups ? (rows < rows / nt + groups ? rows : rows / nt + groups) : ((int64_t)rows + nt - 1) / nt;
-    };
-    int nt = vec ? form.nt : 32;
-    if (nt < 0) {
-        // A tile of 128 takes 1.5 times the time of one of 64 (52 and 34 us at K = 2048), so it pays where it saves waves: against
-        // [6144, 2048], tiles of 64 and 128: 128 rows 36 and 54 us, 512 rows 94 and 104; against [11264, 2048]: 65 and 56, 162 and 152.
-        // 60 experts of [2 x 1408, 2048]: 34 rows each 314 and 356 us, 68 rows 474 and 423.
-        const auto waves = [&](int64_t tiles) { return (tiles * tiles_m * batch + DF_SMS - 1) / DF_SMS; };
-        nt = rows <= 16 ? 16 : rows <= 32 ? 32 : 64;
-        if (groups ? rows > 48ll * groups : rows > 64 && 3 * waves(tiles_of(128)) < 2 * waves(tiles_of(64))) nt = 128;
+    if (batch > 65535) { set_last_error("%s: %d products exceed the grid limit", what, batch); return kBadShape; }
+    int nt = !vec ? 32 : form.nt > 64 ? 64 : form.nt > 0 ? form.nt : rows <= 16 ? 16 : rows <= 32 ? 32 : 64;
+    // rows of a launch: what the scratch holds, or the grid
+    int64_t band = 65535ll * nt;
+    if (f32tc::split_before(nt)) {
+        const int64_t room = f32_tc_scratch((int64_t)rows * batch, g.K) * 2 / 3 / f32_tc_pitch(g.K) / batch;
+        band = room < rows ? room / 64 * 64 : rows;
+        if (band == 0) nt = 32, band = 65535ll * nt;   // (many products of long rows)
     }
-    const int64_t tiles_y = tiles_of(nt);
-    if (tiles_y > 65535 || batch > 65535) {
-        set_last_error("%s: %d rows (%d products) exceed the grid limit", what, rows, batch);
-        return kBadShape;
-    }
+    if (f32tc::split_before(nt) && !scratch) { set_last_error("%s: no room for the rows' parts", what); return kBadShape; }
     TcLaunch l = {};
-    l.split = form.split;
-    if (l.split < 0) {
-        // Up to four blocks share a tile where tiles alone leave SMs without work: one row against [6144, 2048] 28 us, by two
-        // 19, by four 22; against [2048, 2048] 28, 18 and 13; against [2048, 5632] 68, 38 and 23 (by eight 15 and 26).
-        l.split = 1;
-        while (l.split < f32tc::PARTS && 2 * l.split * tiles_m * tiles_y * batch <= DF_SMS) l.split *= 2;
-    }
-    if (!vec || nt == 128) l.split = 1;
-    while (l.split > 1 && l.split < f32tc::PARTS && (f32tc::PARTS / l.split) * nt * 512u > f32tc::SLOT_LIMIT) l.split *= 2;
-    l.grid = dim3((unsigned)(tiles_m * l.split), (unsigned)tiles_y, (unsigned)batch);
     l.stream = stream;
     l.what = what;
     if (vec && !tc::make_map_f32(&l.map_w, g.W, (uint64_t)w_rows, (uint64_t)g.K, PAIRED ? 64 : 128)) {
         set_last_error("%s: cuTensorMapEncodeTiled failed", what);
         return kLaunchFailed;
     }
-    if (f32tc::split_before(nt)) {
-        if (!scratch) { set_last_error("%s: no room for the rows' halves", what); return kBadShape; }
-        g.split_rows = (int64_t)rows * batch;
-        f32tc::f32_split_rows_kernel<<<dim3(rows, batch), 256, 0, stream>>>(g.A, g.gather, g.offsets, g.E, (uint4*)scratch, rows, g.lda,
-                                                                            g.K / 4, g.sA, g.split_rows);
-        const int rc = finish_launch(what);
-        if (rc != kOk) return rc;
-        for (int i = 0; i < 4; ++i) {
-            if (tc::make_map_f32(&l.map_rows.m[i], scratch, 2ull * g.split_rows, (uint64_t)g.K, 16 * (i + 1))) continue;
-            set_last_error("%s: cuTensorMapEncodeTiled failed", what);
-            return kLaunchFailed;
+    for (int64_t r0 = 0; r0 < rows; r0 += band) {
+        const int n = (int)(rows - r0 < band ? rows - r0 : band);
+        const int64_t tiles_y = groups ? (n < n / nt + groups ? n : n / nt + groups) : ((int64_t)n + nt - 1) / nt;
+        if (tiles_y > 65535) {
+            set_last_error("%s: %d rows of %d experts exceed the grid limit", what, rows, groups);
+            return kBadShape;
         }
+        g.row_begin = (int)r0;
+        g.row_end = (int)r0 + n;
+        l.split = form.split;
+        if (l.split < 0) {
+            // Up to four blocks share a tile where tiles alone leave SMs without work: one row against [6144, 2048] 28 us, by two
+            // 19, by four 22; against [2048, 2048] 28, 18 and 13; against [2048, 5632] 68, 38 and 23 (by eight 15 and 26).
+            l.split = 1;
+            while (l.split < f32tc::PARTS && 2 * l.split * tiles_m * tiles_y * batch <= DF_SMS) l.split *= 2;
+        }
+        if (!vec) l.split = 1;
+        while (l.split > 1 && l.split < f32tc::PARTS && (f32tc::PARTS / l.split) * 2 * nt * 512u > f32tc::SLOT_LIMIT) l.split *= 2;
+        l.grid = dim3((unsigned)(tiles_m * l.split), (unsigned)tiles_y, (unsigned)batch);
+        if (f32tc::split_before(nt)) {
+            const int pitch = (int)f32_tc_pitch(g.K);
+            f32tc::f32_split_rows_kernel<<<dim3(n, batch), 256, 0, stream>>>(g.A, g.gather, g.offsets, g.E, (uint2*)scratch, (int)r0, n,
+                                                                             g.lda, g.K / 4, pitch / 4, g.sA);
+            const int rc = finish_launch(what);
+            if (rc != kOk) return rc;
+            for (int i = 0; i < 4; ++i) {
+                if (f32tc::make_map_parts(&l.map_rows.m[i], scratch, (uint64_t)n * batch, (uint64_t)g.K, (uint64_t)pitch, 16 * (i + 1))) continue;
+                set_last_error("%s: cuTensorMapEncodeTiled failed", what);
+                return kLaunchFailed;
+            }
+        }
+        const int rc = !vec ? f32_tc_launch_one<PAIRED, 32, false, false>(g, l)
+                     : nt == 16 ? f32_tc_launch_nt<PAIRED, 16>(g, l)
+                     : nt == 32 ? f32_tc_launch_nt<PAIRED, 32>(g, l) : f32_tc_launch_nt<PAIRED, 64>(g, l);
+        if (rc != kOk) return rc;
     }
-    if (!vec) return f32_tc_launch_one<PAIRED, 32, false, false>(g, l);
-    switch (nt) {
-        case 16: return f32_tc_launch_nt<PAIRED, 16>(g, l);
-        case 32: return f32_tc_launch_nt<PAIRED, 32>(g, l);
-        case 64: return f32_tc_launch_nt<PAIRED, 64>(g, l);
-        default: return f32_tc_launch_nt<PAIRED, 128>(g, l);
-    }
+    return kOk;
 }
 
 }  // namespace mi
@@ -228,7 +232,7 @@ extern "C" int mi_dense_f32_batched(const float* A, const float* W, float* C, in
         return kBadShape;
     }
     if (K >= f32tc::TC_MIN_K)
-        return f32_tc_launch<false>(f32tc::Problem{A, W, C, nullptr, nullptr, T, N, K, lda, ldc, 0, sA, sW, sC, 0, GluForm{}, status}, scratch, T, 0,
+        return f32_tc_launch<false>(f32tc::Problem{A, W, C, nullptr, nullptr, N, K, lda, ldc, 0, sA, sW, sC, 0, 0, GluForm{}, status}, scratch, T, 0,
                                     batch, TcForm{-1, -1}, stream, "dense_f32");
     const bool vec = (K % 4 == 0) && (lda % 4 == 0) && (sA % 4 == 0) && (sW % 4 == 0) &&
                      (((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W)) & 15) == 0);
@@ -255,7 +259,7 @@ extern "C" int mi_f32_tc_form(const float* A, const int* gather, const float* W,
         return kBadShape;
     }
     const GluForm glu{glu_kind, glu_limit, glu_slope, mode == 1 ? row_scale : nullptr};
-    const f32tc::Problem g{A, W, C, gather, offsets, n_rows, Nout, K, K, Nout, E, 0, 0, 0, 0, glu, status};
+    const f32tc::Problem g{A, W, C, gather, offsets, Nout, K, K, Nout, E, 0, 0, 0, 0, 0, glu, status};
     const TcForm form{nt, split};
     return mode == 1 ? f32_tc_launch<true>(g, scratch, n_rows, E, 1, form, stream, "grouped_gemm_plain")
                      : f32_tc_launch<false>(g, scratch, n_rows, E, 1, form, stream, E ? "grouped_gemm_plain" : "dense_f32");

@@ -2,31 +2,31 @@
 //
 //   C[t, n] = A[t, :] . W[n, :]   (dense, one of several independent products, or an expert's rows of a grouped one)
 //
-// A number x of 32 bits is taken as hi + lo: hi is x rounded to 11 bits of mantissa, lo = x - hi (exact, at most 2^-11 of x) is
-// read to 11 bits, both operands of kind::tf32, and a product is hi hi + hi lo + lo hi.  What is left out, lo lo and lo's
-// last bits, is at most 3 * 2^-21 of a term (on average a tenth of that) and of either sign; the tensor cores add without rounding to nearest, so 32 terms at most are added there (first the small products,
-// then hi hi) and every such sum goes through registers, where it is added in 32 bits as any number is.  Against 64 bits the
-// result is nearer than a chain of K fused multiply-adds, from K = 512 on (measured, relative to the result's norm, chain and
-// here: see dense_f32.cu).
+// A number x of 32 bits is taken apart exactly, into three bfloat16 numbers: 2^24 x = h + m + l, each the rest rounded to 8 bits
+// (the factor keeps the parts of the smallest x among the normal numbers).  Of the nine products of two numbers' parts all are formed but
+// that of the two l, which is at most 2^-34 of the whole.  They stand in three sums by their size: hh; hm, mh and lh; hl, mm, lm and ml.
+// The tensor cores add without rounding to nearest, so 32 terms at most are added there: hh's have 16 bits, of which few are cut
+// off, and the other sums are 2^-8 of it and less.  Then the sums go to registers and are added up there, hh and the others each by
+// itself, in 32 bits as any number is, and meet in the output alone.  Measured error: see dense_f32.cu.
 //
 // Every output element is the same sums in the same order in every form below: chunks of 32 k in ascending order within
 // each of four parts of the inner dimension, then the parts in ascending order.  So a row has the same bits however many
 // rows share the step, in whichever tile and form, as the chains of the CUDA-core kernels have for smaller K.  A result that
-// is not finite (an operand that is not, or a sum that overflows) is computed again as a chain of multiply-adds, so infinities and
-// NaN reach exactly the elements that they reach there.
+// is not finite (an operand that is not, or one from 2^104 or a sum from 2^80 on) is computed again as a chain of multiply-adds, so
+// infinities and NaN that operands bring reach exactly the elements that they reach there.
 //
 // Weights are the M operand (128 rows a tile; 64 gate rows and the up rows of the same outputs in a paired product) and lie in
 // tensor memory, rows of activations are the N operand in shared memory.  Roles:
-//   warps 0-3 and 4-7, chunks in turn: weights, ring -> hi and lo -> tensor memory
+//   warps 0-3 and 4-7, chunks in turn: weights, ring -> three parts -> tensor memory
 //   warps 8-15  the sums of a chunk: tensor memory -> registers, added up
-//   warps 16, 17, chunks in turn: MMAs (12 a chunk; the tensor cores take them one by one as they come, so a single warp
-//               would leave them idle while it waits for the next chunk's operands); warp 16 allocates tensor memory
+//   warps 16, 17, chunks in turn: MMAs (8 a chunk; the tensor cores take them one by one as they come, so a single warp
+//               would leave them idle while it waits for the next chunk's operands); warp 16 allocates tensor memory.
+//               The activations' parts stand one behind the other, so that one MMA multiplies a part of the weights with two
+//               or all three of them (an MMA of 64 rows takes as long as one of 128)
 //   warp 18     weights: memory -> ring (TMA; without it, where rows are not aligned for it, the warps that read them ask
 //               for them with cp.async)
-//   tiles of 64 and 128 rows: warp 19 brings hi and lo of the activations, which f32_split_rows_kernel has made (TMA)
-//   tiles of 16 and 32: warps 19-22 bring the activations (cp.async, four chunks ahead) and make hi and lo of them in shared memory
-// What bounds a chunk of a tile of 64 or 128 is shared memory: weights written and read, activations written, and read by
-// every MMA.
+//   tiles of 64 rows: warp 19 brings the parts of the activations, which f32_split_rows_kernel has made (TMA)
+//   tiles of 16 and 32: warps 19-22 bring the activations (cp.async, four chunks ahead) and take them apart in shared memory
 // SPLIT: a cluster of 2 or 4 blocks shares a tile's parts and adds them up through distributed shared memory, where tiles
 // alone would leave SMs without work (a decode step's few rows).
 //
@@ -41,25 +41,37 @@ namespace f32tc {
 using namespace tc;
 
 constexpr int TC_MIN_K = 512;
-constexpr int FK = 32;                                 // k per chunk: 32 floats are a swizzled row of 128 bytes
+constexpr int FK = 32;                                 // k per chunk: 32 floats are a swizzled row of 128 bytes, 32 bfloat16 one of 64
 constexpr int PARTS = 4;
 constexpr int OUT_WARP = 8, MMA_WARP = 16, W_WARP = 18, ROWS_WARP = 19;        // first warps of the roles
 constexpr bool split_before(int nt) { return nt >= 64; }
 constexpr int threads(int nt) { return 32 * (split_before(nt) ? 20 : 23); }
-constexpr int T_SLOTS = 4, ROWS_AHEAD = 4;             // chunks of weights in tensor memory; of activations asked for
+constexpr int T_SLOTS = 2, ROWS_AHEAD = 4;             // chunks of weights in tensor memory; of activations asked for
 constexpr uint32_t SLOT_LIMIT = 65536;                 // bytes of part sums of a SPLIT block
-// D float32, A and B tf32, both K-major, M = 128 (without N)
-constexpr uint32_t IDESC = (1u << 4) | (2u << 7) | (2u << 10) | ((128u >> 4) << 24);
+constexpr float UP = 16777216.f, DOWN = 1.f / (UP * UP);       // factors of operands and results
+// D float32, A and B bfloat16, both K-major, M = 128 (without N)
+constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((128u >> 4) << 24);
 
-// Rings, in chunks: weights; hi and lo of the activations (at most four: see the phases below; hi also holds what is on its
-// way where the block splits it itself); sums in tensor memory
-constexpr int w_slots(int nt, bool split) { return nt == 128 ? 4 : (nt == 64 ? 6 : 8) - (split ? 2 : 0); }
-constexpr int lo_slots(int nt) { return nt == 128 ? 3 : 4; }
-constexpr int hi_slots(int nt) { return split_before(nt) ? lo_slots(nt) : lo_slots(nt) + ROWS_AHEAD; }
-constexpr int d_slots(int nt) { return nt == 128 ? 2 : 4; }
+// Rings, in chunks: weights; parts of the activations (at most four: see the phases below); activations on their way, where the
+// block takes them apart; sums in tensor memory
+constexpr int w_slots(int nt, bool split) { return (nt == 64 ? 6 : 8) - (split ? 2 : 0); }
+constexpr int ROW_SLOTS = 4;
+constexpr int raw_slots(int nt) { return split_before(nt) ? 0 : ROWS_AHEAD + 1; }
+constexpr int d_slots(int nt) { return nt == 64 ? 2 : 4; }
 inline size_t smem_bytes(int nt, int split) {
-    return 1024 + (size_t)w_slots(nt, split > 1) * 16384 + (size_t)(hi_slots(nt) + lo_slots(nt)) * nt * 128 +
-           (size_t)(split > 1 ? PARTS / split : 1) * nt * 512;
+    return 1024 + (size_t)w_slots(nt, split > 1) * 16384 + (size_t)ROW_SLOTS * nt * 192 + (size_t)raw_slots(nt) * nt * 128 +
+           (size_t)(split > 1 ? PARTS / split : 1) * 2 * nt * 512;
+}
+
+// The parts of `rows` rows of activations, [3][rows][pitch] of bfloat16: boxes of 32 columns x box_rows rows x 3, 64-byte swizzle.
+inline bool make_map_parts(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint64_t pitch, uint32_t box_rows) {
+    EncodeTiledFn fn = encode_fn();
+    if (!fn) return false;
+    const cuuint64_t dims[3] = {cols, rows, 3};
+    const cuuint64_t strides[2] = {pitch * 2, rows * pitch * 2};
+    const cuuint32_t box[3] = {(cuuint32_t)FK, box_rows, 3}, estr[3] = {1, 1, 1};
+    return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+              CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 // mbar_wait of tcgen05.cuh, by a whole warp
@@ -77,20 +89,34 @@ struct Problem {
     const float* A; const float* W; float* C;
     const int* gather;                                 // grouped: row of A of a sorted row (or null)
     const int* offsets;                                // grouped: [E + 1]; dense: null
-    int T, N, K, lda, ldc, E;                          // N: outputs (a paired product has 2 N rows of W an expert)
+    int N, K, lda, ldc, E;                             // N: outputs (a paired product has 2 N rows of W an expert)
     int64_t sA, sW, sC;                                // dense: operands of product blockIdx.z
-    int64_t split_rows;                                // rows of `hi` (those of `lo` come behind them), of products in turn
+    int row_begin, row_end;                            // the (sorted) rows of this launch
     GluForm glu;
     int* status;
 };
-struct RowMaps { CUtensorMap m[4]; };                  // hi and lo of the activations in boxes of 16, 32, 48 and 64 rows
+struct RowMaps { CUtensorMap m[4]; };                  // the activations' parts in boxes of 16, 32, 48 and 64 rows x 3
 
-__device__ __forceinline__ void umma_tf32_tmem_a(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
-                                                 uint32_t accumulate) {
+__device__ __forceinline__ void umma_tmem_a(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-        " tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n}"
+        " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}"
         ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+}
+// K-major tile of rows of 64 bytes, 64-byte swizzle: groups of 8 rows 512 bytes apart
+__device__ __forceinline__ uint64_t umma_desc_64(uint32_t smem_addr) {
+    uint64_t d = 0;
+    d |= (uint64_t)((smem_addr & 0x3FFFFu) >> 4);
+    d |= (uint64_t)1 << 16;
+    d |= (uint64_t)(512 >> 4) << 32;
+    d |= (uint64_t)1 << 46;
+    d |= (uint64_t)4 << 61;
+    return d;
+}
+__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+        ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z) : "memory");
 }
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
@@ -111,11 +137,19 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
 }
 __device__ __forceinline__ void wait_tmem_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
-// hi and lo of x as operands of kind::tf32, which reads their upper 19 bits.  (x + 0x1000 may carry a NaN's bits into the sign:
-// then lo is the NaN.)
-__device__ __forceinline__ void split(uint32_t x, uint32_t& hi, uint32_t& lo) {
-    hi = (x + 0x1000u) & 0xffffe000u;
-    lo = __float_as_uint(__uint_as_float(x) - __uint_as_float(hi));
+// The parts of two neighbours, as pairs of bfloat16.  (Of an infinity, a NaN or a number whose h is an infinity, l is a NaN.)
+__device__ __forceinline__ uint32_t pack(float a, float b) {
+    const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<const uint32_t*>(&v);
+}
+__device__ __forceinline__ float first_of(uint32_t v) { return __uint_as_float(v << 16); }
+__device__ __forceinline__ float second_of(uint32_t v) { return __uint_as_float(v & 0xffff0000u); }
+__device__ __forceinline__ void take_apart(uint32_t x0, uint32_t x1, uint32_t& h, uint32_t& m, uint32_t& l) {
+    const float a = __uint_as_float(x0) * UP, b = __uint_as_float(x1) * UP;
+    h = pack(a, b);
+    const float ra = a - first_of(h), rb = b - second_of(h);
+    m = pack(ra, rb);
+    l = pack(ra - first_of(m), rb - second_of(m));
 }
 __device__ __forceinline__ void cp_async16(uint32_t dst, const char* src, bool there) {
     const int n = there ? 16 : 0;                      // nothing read: the bytes become zeros
@@ -134,12 +168,12 @@ __device__ __noinline__ float chain(const float* __restrict__ a, const float* __
     return s;
 }
 
-// An expert's rows are split evenly over its tiles of up to `nt` rows, whole groups of 16.  Uniform for the warp.
-__device__ __forceinline__ int row_tile(const int* __restrict__ offsets, int E, int nt, int slot, int& e, int& row0) {
+// An expert's rows among [begin, end) are split evenly over its tiles of up to `nt` rows, whole groups of 16.  Uniform for the warp.
+__device__ __forceinline__ int row_tile(const int* __restrict__ offsets, int E, int begin, int end, int nt, int slot, int& e, int& row0) {
     const int lane = threadIdx.x & 31;
     for (int base = 0; base < E; base += 32) {
         const int i = base + lane;
-        const int lo = i < E ? __ldg(offsets + i) : 0, cnt = i < E ? __ldg(offsets + i + 1) - lo : 0;
+        const int lo = i < E ? max(__ldg(offsets + i), begin) : 0, cnt = i < E ? max(0, min(__ldg(offsets + i + 1), end) - lo) : 0;
         const int own = (cnt + nt - 1) / nt;
         int through = own;
 #pragma unroll
@@ -162,21 +196,24 @@ __device__ __forceinline__ int row_tile(const int* __restrict__ offsets, int E, 
     return 0;
 }
 
-// hi and lo of rows of activations (K a multiple of 4): out[r] and out[rows + r] of x[gather ? gather[r] : r].  Grouped: only the
-// rows that an expert has; beyond them `gather` need not be written.
+// The parts of rows of activations (K a multiple of 4, read four at a time): out[part][z * rows + r][pitch] of
+// x_z[gather ? gather[first + r] : first + r].  Grouped: only the rows that an expert has; beyond them `gather` need not be written.
 __global__ void __launch_bounds__(256)
 f32_split_rows_kernel(const float* __restrict__ x, const int* __restrict__ gather, const int* __restrict__ offsets, int E,
-                      uint4* __restrict__ out, int rows, int lda, int K4, int64_t sA, int64_t all_rows) {
+                      uint2* __restrict__ out, int first, int rows, int lda, int K4, int pitch4, int64_t sA) {
     const int r = blockIdx.x;
-    if (offsets && r >= __ldg(offsets + E)) return;
-    const uint4* src = reinterpret_cast<const uint4*>(x + blockIdx.y * sA + (int64_t)(gather ? __ldg(gather + r) : r) * lda);
-    uint4* hi = out + ((int64_t)blockIdx.y * rows + r) * K4;
+    if (offsets && first + r >= __ldg(offsets + E)) return;
+    const int64_t row = gather ? __ldg(gather + first + r) : first + r, part = (int64_t)gridDim.y * rows * pitch4;
+    const uint4* src = reinterpret_cast<const uint4*>(x + blockIdx.y * sA + row * lda);
+    uint2* to = out + ((int64_t)blockIdx.y * rows + r) * pitch4;
     for (int i = threadIdx.x; i < K4; i += 256) {
         const uint4 v = __ldg(src + i);
-        uint4 h, l;
-        split(v.x, h.x, l.x); split(v.y, h.y, l.y); split(v.z, h.z, l.z); split(v.w, h.w, l.w);
-        hi[i] = h;
-        hi[all_rows * K4 + i] = l;
+        uint2 h, m, l;
+        take_apart(v.x, v.y, h.x, m.x, l.x);
+        take_apart(v.z, v.w, h.y, m.y, l.y);
+        to[i] = h;
+        to[part + i] = m;
+        to[2 * part + i] = l;
     }
 }
 
@@ -187,13 +224,14 @@ __global__ void __launch_bounds__(threads(NT), 1)
 f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ RowMaps map_rows, Problem g) {
     constexpr bool BEFORE = split_before(NT);
     static_assert(!BEFORE || VEC, "rows that are split before are aligned");
-    constexpr int THREADS = threads(NT), W_SLOTS = w_slots(NT, SPLIT), LO_SLOTS = lo_slots(NT), HI_SLOTS = hi_slots(NT), D_SLOTS = d_slots(NT);
-    constexpr int B_BYTES = NT * 128;
+    constexpr int THREADS = threads(NT), W_SLOTS = w_slots(NT, SPLIT), RAW_SLOTS = raw_slots(NT), D_SLOTS = d_slots(NT);
+    constexpr int D_STEP = 384 / D_SLOTS;              // columns of tensor memory of a chunk's three sums
+    constexpr int ROW_BYTES = NT * 192;                // a chunk's activations: [part][rows][64 bytes], swizzled
     constexpr int FEATS = PAIRED ? 64 : 128;           // outputs of a tile
     constexpr int OWN = NT / 2;                        // rows of activations of an adding warp
     constexpr int PER = NT / 16;                       // 16-byte pieces of activations per thread and chunk
     extern __shared__ uint8_t smem_raw[];
-    __shared__ uint64_t full_bar[4], done_bar[4], empty_bar[D_SLOTS], w_full[W_SLOTS], w_read[W_SLOTS], rows_full[LO_SLOTS];
+    __shared__ uint64_t full_bar[4], done_bar[4], empty_bar[D_SLOTS], w_full[W_SLOTS], w_read[W_SLOTS], rows_full[ROW_SLOTS];
     __shared__ uint32_t tmem_base_s;
     __shared__ int abort_s;
 
@@ -205,11 +243,11 @@ f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
     const int n0 = (int)(blockIdx.x / ranks) * FEATS;
     int e = 0, row0, rows;
     if (g.offsets) {
-        rows = row_tile(g.offsets, g.E, NT, blockIdx.y, e, row0);
+        rows = row_tile(g.offsets, g.E, g.row_begin, g.row_end, NT, blockIdx.y, e, row0);
         if (rows == 0) return;                         // uniform for the block and its cluster
     } else {
-        row0 = blockIdx.y * NT;
-        rows = min(NT, g.T - row0);
+        row0 = g.row_begin + blockIdx.y * NT;
+        rows = min(NT, g.row_end - row0);
     }
     const float* A = g.A + blockIdx.z * g.sA;
     const float* W = g.W + blockIdx.z * g.sW + (int64_t)e * (PAIRED ? 2 : 1) * g.N * g.K;
@@ -220,10 +258,11 @@ f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
     const int first = min(chunks, (int)rank * own_parts * per_part), count = min(chunks, first + own_parts * per_part) - first;
 
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    uint8_t* hi_ring = smem;                           // [slot][NT][128 bytes], swizzled
-    uint8_t* lo_ring = hi_ring + HI_SLOTS * B_BYTES;
-    uint8_t* w_ring = lo_ring + LO_SLOTS * B_BYTES;    // [slot][128 rows][128 bytes], swizzled
-    float* sums = reinterpret_cast<float*>(w_ring + W_SLOTS * 16384);      // [part][NT][128]: SPLIT parts, otherwise their total
+    uint8_t* rows_ring = smem;
+    uint8_t* raw_ring = rows_ring + ROW_SLOTS * ROW_BYTES;                 // [slot][NT][128 bytes]
+    uint8_t* w_ring = raw_ring + RAW_SLOTS * NT * 128;                     // [slot][128 rows][128 bytes], swizzled
+    float* sums = reinterpret_cast<float*>(w_ring + W_SLOTS * 16384);      // [part][hh, others][NT][128]: SPLIT parts, otherwise their total
+    const uint32_t part_bytes = (uint32_t)n_mma * 64;
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     volatile int* abort_flag = &abort_s;
 
@@ -231,7 +270,7 @@ f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
         abort_s = 0;
         for (int s = 0; s < 4; ++s) { mbar_init(&full_bar[s], BEFORE ? 4 : 8); mbar_init(&done_bar[s], 1); }
         for (int s = 0; s < D_SLOTS; ++s) mbar_init(&empty_bar[s], 8);
-        for (int s = 0; s < LO_SLOTS; ++s) mbar_init(&rows_full[s], 1);
+        for (int s = 0; s < ROW_SLOTS; ++s) mbar_init(&rows_full[s], 1);
         for (int s = 0; s < W_SLOTS; ++s) { mbar_init(&w_full[s], 1); mbar_init(&w_read[s], 4); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -244,7 +283,7 @@ f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = tmem_base_s;                 // columns 0-255: four chunks' sums; 256-511: four of weights
+    const uint32_t tmem = tmem_base_s;                 // columns 0-383: two or four chunks' sums; 384-511: two of weights
 
     // Phases of the barriers of four (full, done): whoever waits for chunk i there has itself to act before chunk i + 4
     // can complete, so a parity never stands for the phase after the next.
@@ -270,7 +309,7 @@ f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
 #pragma unroll 1
         for (int i = 0; i < SLOTS - 1; ++i) ask(turn + 2 * i);
         const uint8_t* w_lane = w_ring + quarter * 4096 + lane * 128;
-        const uint32_t t_lane = tmem + ((uint32_t)(quarter * 32) << 16) + 256;
+        const uint32_t t_lane = tmem + ((uint32_t)(quarter * 32) << 16) + 384;
 #pragma unroll 1
         for (int i = turn; i < count; i += 2) {
             const int slot = i % W_SLOTS;
@@ -282,30 +321,29 @@ f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
                 asm volatile("cp.async.wait_group %0;" ::"n"(SLOTS - 1) : "memory");
                 __syncwarp();
             }
-            // the MMAs of chunk i - T_SLOTS have read its place in tensor memory
-            if (i >= T_SLOTS && !wait_for(&done_bar[i & 3], ((i - T_SLOTS) >> 2) & 1, abort_flag, 32)) break;
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint8_t* w = w_lane + slot * 16384;
             const uint32_t at = t_lane + (i % T_SLOTS) * 64;
+            uint32_t h[16], m[16], l[16];
 #pragma unroll
-            for (int k = 0; k < 2; ++k) {
-                uint32_t hi[16], lo[16];
-#pragma unroll
-                for (int p = 0; p < 4; ++p) {
-                    const uint4 v = *reinterpret_cast<const uint4*>(w + (((4 * k + p) ^ (lane & 7)) << 4));
-                    split(v.x, hi[4 * p], lo[4 * p]); split(v.y, hi[4 * p + 1], lo[4 * p + 1]);
-                    split(v.z, hi[4 * p + 2], lo[4 * p + 2]); split(v.w, hi[4 * p + 3], lo[4 * p + 3]);
-                }
-                tmem_st16(at + 16 * k, hi);
-                tmem_st16(at + 32 + 16 * k, lo);
+            for (int p = 0; p < 8; ++p) {
+                const uint4 v = *reinterpret_cast<const uint4*>(w + ((p ^ (lane & 7)) << 4));
+                take_apart(v.x, v.y, h[2 * p], m[2 * p], l[2 * p]);
+                take_apart(v.z, v.w, h[2 * p + 1], m[2 * p + 1], l[2 * p + 1]);
             }
+            if (VEC) {
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&w_read[slot]);
+            }
+            // the MMAs of chunk i - T_SLOTS have read its place in tensor memory
+            if (i >= T_SLOTS && !wait_for(&done_bar[(i - T_SLOTS) & 3], ((i - T_SLOTS) >> 2) & 1, abort_flag, 32)) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            tmem_st16(at, h);
+            tmem_st16(at + 16, m);
+            tmem_st16(at + 32, l);
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
-            if (lane == 0) {
-                mbar_arrive(&full_bar[i & 3]);
-                if (VEC) mbar_arrive(&w_read[slot]);
-            }
+            if (lane == 0) mbar_arrive(&full_bar[i & 3]);
         }
         asm volatile("cp.async.wait_group 0;" ::: "memory");
     } else if (warp < MMA_WARP) {
@@ -313,9 +351,9 @@ f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
         const int quarter = warp & 3, c_lo = ((warp - OUT_WARP) >> 2) * OWN, feat = quarter * 32 + lane;
         const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16) + c_lo;
         float* own = sums + c_lo * 128 + feat;         // of the first part; columns 128 apart
-        float part[OWN];
+        float part[2][OWN];                            // hh, others
 #pragma unroll
-        for (int i = 0; i < OWN; ++i) part[i] = 0.f;
+        for (int i = 0; i < OWN; ++i) part[0][i] = part[1][i] = 0.f;
         bool ok = true;
         int in_part = 0, parts = 0;
 #pragma unroll 1
@@ -324,32 +362,35 @@ f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             if (c_lo < n_mma) {                        // uniform
-                const uint32_t d = lane_addr + (it % D_SLOTS) * (256 / D_SLOTS);
-                constexpr int GROUP = OWN < 32 ? OWN : OWN == 32 ? 32 : 16;
+                const uint32_t d = lane_addr + (it % D_SLOTS) * D_STEP;
+                constexpr int GROUP = OWN < 16 ? OWN : 16;
 #pragma unroll
-                for (int i0 = 0; i0 < OWN; i0 += GROUP) {
-                    uint32_t v[GROUP];
-                    if constexpr (GROUP == 32) tmem_ld32(d + i0, v);
-                    else if constexpr (GROUP == 16) tmem_ld16(d + i0, v);
-                    else tmem_ld8(d + i0, v);
-                    wait_tmem_ld();
+                for (int x = 0; x < 3; ++x)
 #pragma unroll
-                    for (int i = 0; i < GROUP; ++i) part[i0 + i] += __uint_as_float(v[i]);
-                }
+                    for (int i0 = 0; i0 < OWN; i0 += GROUP) {
+                        uint32_t v[GROUP];
+                        if constexpr (GROUP == 16) tmem_ld16(d + x * n_mma + i0, v);
+                        else tmem_ld8(d + x * n_mma + i0, v);
+                        wait_tmem_ld();
+#pragma unroll
+                        for (int i = 0; i < GROUP; ++i) part[x > 0][i0 + i] += __uint_as_float(v[i]);
+                    }
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) mbar_arrive(&empty_bar[it % D_SLOTS]);
             if (++in_part == per_part || it == count - 1) {
-                float* to = own + (SPLIT ? parts * NT * 128 : 0);
-                if (!SPLIT && parts > 0)
+                float* to = own + (SPLIT ? parts * 2 * NT * 128 : 0);
 #pragma unroll
-                    for (int i = 0; i < OWN; ++i) part[i] = to[i * 128] + part[i];
+                for (int x = 0; x < 2; ++x)
 #pragma unroll
-                for (int i = 0; i < OWN; ++i) {
-                    to[i * 128] = 0.f + part[i];       // (a cluster's sums begin at +0, too)
-                    part[i] = 0.f;
-                }
+                    for (int i = 0; i < OWN; ++i) {
+                        float* at = to + (x * NT + i) * 128;
+                        if (!SPLIT && parts > 0) part[x][i] = *at + part[x][i];
+                        *at = 0.f + part[x][i];        // (a cluster's sums begin at +0, too)
+                        part[x][i] = 0.f;
+                        if (i % 8 == 7) asm volatile("" ::: "memory");     // (all loads at once would take registers that are not there)
+                    }
                 in_part = 0;
                 ++parts;
             }
@@ -357,26 +398,27 @@ f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
         if (SPLIT)
             for (; parts < own_parts; ++parts)         // past the last chunk
 #pragma unroll
-                for (int i = 0; i < OWN; ++i) own[(parts * NT + i) * 128] = 0.f;
+                for (int i = 0; i < OWN; ++i) own[(parts * 2 * NT + i) * 128] = own[((parts * 2 + 1) * NT + i) * 128] = 0.f;
     } else if (warp < W_WARP) {
-        const uint32_t idesc = IDESC | ((uint32_t)(n_mma >> 3) << 17);
-        const uint64_t hi_desc = umma_desc(smem_u32(hi_ring)), lo_desc = umma_desc(smem_u32(lo_ring));
+        const uint32_t by_n = (uint32_t)(n_mma >> 3) << 17, idesc1 = IDESC | by_n, idesc2 = IDESC | 2 * by_n, idesc3 = IDESC | 3 * by_n;
+        const uint64_t rows_desc = umma_desc_64(smem_u32(rows_ring));
+        const uint32_t step = part_bytes >> 4;
 #pragma unroll 1
         for (int i = warp - MMA_WARP; i < count; i += 2) {
             if (!wait_for(&empty_bar[i % D_SLOTS], ((i / D_SLOTS) & 1) ^ 1, abort_flag, 35)) break;
-            if (BEFORE && !wait_for(&rows_full[i % LO_SLOTS], (i / LO_SLOTS) & 1, abort_flag, 38)) break;
+            if (BEFORE && !wait_for(&rows_full[i % ROW_SLOTS], (i / ROW_SLOTS) & 1, abort_flag, 38)) break;
             if (!wait_for(&full_bar[i & 3], (i >> 2) & 1, abort_flag, 36)) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint64_t bh = hi_desc + (uint32_t)(((i % HI_SLOTS) * B_BYTES) >> 4), bl = lo_desc + (uint32_t)(((i % LO_SLOTS) * B_BYTES) >> 4);
-            const uint32_t wh = tmem + 256 + (i % T_SLOTS) * 64, wl = wh + 32, d = tmem + (i % D_SLOTS) * (256 / D_SLOTS);
+            const uint64_t bh = rows_desc + (uint32_t)(((i % ROW_SLOTS) * ROW_BYTES) >> 4), bl = bh + 2 * step;
+            const uint32_t wh = tmem + 384 + (i % T_SLOTS) * 64, wm = wh + 16, wl = wm + 16, d = tmem + (i % D_SLOTS) * D_STEP;
             if (elect_one()) {
 #pragma unroll
-                for (int k = 0; k < FK / 8; ++k) {
-                    umma_tf32_tmem_a(d, wl + k * 8, bh + k * 2, idesc, k > 0);
-                    umma_tf32_tmem_a(d, wh + k * 8, bl + k * 2, idesc, 1);
+                for (int k = 0; k < FK / 16; ++k) {    // 16 k: 8 columns of weights, 32 bytes of a row
+                    umma_tmem_a(d, wh + k * 8, bh + k * 2, idesc3, k > 0);                   // hh, hm, hl
+                    umma_tmem_a(d + n_mma, wm + k * 8, bh + k * 2, idesc2, 1);               //     mh, mm
+                    umma_tmem_a(d + n_mma, wl + k * 8, bh + k * 2, idesc2, 1);               //     lh, lm
+                    umma_tmem_a(d + 2 * n_mma, wm + k * 8, bl + k * 2, idesc1, 1);           //         ml
                 }
-#pragma unroll
-                for (int k = 0; k < FK / 8; ++k) umma_tf32_tmem_a(d, wh + k * 8, bh + k * 2, idesc, 1);
                 umma_commit(&done_bar[i & 3]);
             }
             __syncwarp();
@@ -397,46 +439,40 @@ f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
             for (int j = max(0, i - W_SLOTS); j < i; ++j)          // nothing is on its way when the block ends, also after an abort
                 for (uint32_t n = 0; n < WAIT_LIMIT && !mbar_try_wait(&w_full[j % W_SLOTS], (j / W_SLOTS) & 1); ++n) {}
         }
-    } else if (BEFORE) {
+    } else if constexpr (BEFORE) {
         if (lane == 0) {
-            const int y_hi = (int)(blockIdx.z * (int64_t)g.T + row0), y_lo = y_hi + (int)g.split_rows;
-            const int n_rest = NT > 64 && n_mma > 64 ? n_mma - 64 : n_mma, at_rest = (n_mma - n_rest) * 128;
-            const CUtensorMap* rest = &map_rows.m[n_rest / 16 - 1];
+            const int y = (int)(blockIdx.z * (int64_t)(g.row_end - g.row_begin)) + row0 - g.row_begin;
+            const CUtensorMap* map = &map_rows.m[n_mma / 16 - 1];
             int i = 0;
 #pragma unroll 1
             for (; i < count; ++i) {
-                // the MMAs of chunk i - LO_SLOTS have read its place
-                if (i >= LO_SLOTS && !mbar_wait(&done_bar[(i - LO_SLOTS) & 3], ((i - LO_SLOTS) >> 2) & 1, abort_flag, 33)) break;
-                const int slot = i % LO_SLOTS, k = (first + i) * FK;
-                uint64_t* bar = &rows_full[slot];
-                uint8_t *hi = hi_ring + slot * B_BYTES, *lo = lo_ring + slot * B_BYTES;
-                mbar_expect_tx(bar, 2 * n_mma * 128);
-                if (NT > 64 && n_mma > 64) {
-                    tma_load_2d(hi, &map_rows.m[3], k, y_hi, bar);
-                    tma_load_2d(lo, &map_rows.m[3], k, y_lo, bar);
-                }
-                tma_load_2d(hi + at_rest, rest, k, y_hi + n_mma - n_rest, bar);
-                tma_load_2d(lo + at_rest, rest, k, y_lo + n_mma - n_rest, bar);
+                // the MMAs of chunk i - ROW_SLOTS have read its place
+                if (i >= ROW_SLOTS && !mbar_wait(&done_bar[i & 3], ((i - ROW_SLOTS) >> 2) & 1, abort_flag, 33)) break;
+                const int slot = i % ROW_SLOTS;
+                mbar_expect_tx(&rows_full[slot], 3 * part_bytes);
+                tma_load_3d(rows_ring + slot * ROW_BYTES, map, (first + i) * FK, y, 0, &rows_full[slot]);
             }
-            for (int j = max(0, i - LO_SLOTS); j < i; ++j)
-                for (uint32_t n = 0; n < WAIT_LIMIT && !mbar_try_wait(&rows_full[j % LO_SLOTS], (j / LO_SLOTS) & 1); ++n) {}
+            for (int j = max(0, i - ROW_SLOTS); j < i; ++j)
+                for (uint32_t n = 0; n < WAIT_LIMIT && !mbar_try_wait(&rows_full[j % ROW_SLOTS], (j / ROW_SLOTS) & 1); ++n) {}
         }
     } else {
         // this thread's pieces of a chunk are rows tid / 8 + 16 j at piece tid % 8; it alone reads what it asked for
         const int tid = threadIdx.x - 32 * ROWS_WARP, piece = tid & 7, r_lo = tid >> 3;
-        const uint32_t pitch = (uint32_t)g.lda * 4u, b_lane = r_lo * 128 + ((piece ^ (r_lo & 7)) << 4);
+        const uint32_t pitch = (uint32_t)g.lda * 4u, raw_lane = tid * 16;
+        // 8 bytes of each part: in 16-byte piece (piece / 2) of the row, swizzled by bits 7 and 8 of the address
+        const uint32_t rows_lane = r_lo * 64 + (((piece >> 1) ^ ((r_lo >> 1) & 3)) << 4) + (piece & 1) * 8;
         uint32_t row_of[PER];
 #pragma unroll
         for (int j = 0; j < PER; ++j) {
             const int r = r_lo + 16 * j;
             row_of[j] = r >= rows ? 0xffffffffu : g.gather ? (uint32_t)__ldg(g.gather + row0 + r) : (uint32_t)(row0 + r);
         }
-        const uint32_t hi_at = smem_u32(hi_ring) + b_lane;
+        const uint32_t raw_at = smem_u32(raw_ring) + raw_lane;
         auto ask = [&](int i) {
             if (i < count) {
                 const int k = (first + i) * FK + piece * 4, left = g.K - k;
                 const char* base = reinterpret_cast<const char*>(A + k);
-                const uint32_t at = hi_at + (i % HI_SLOTS) * B_BYTES;
+                const uint32_t at = raw_at + (i % RAW_SLOTS) * (NT * 128);
 #pragma unroll
                 for (int j = 0; j < PER; ++j) {
                     if (16 * j >= n_mma) break;        // uniform; no MMA reads these rows
@@ -460,20 +496,22 @@ f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
         for (int i = 0; i < ROWS_AHEAD; ++i) ask(i);
 #pragma unroll 1
         for (int i = 0; i < count; ++i) {
-            // the MMAs of chunk i - 4 have read its place in the ring of lo, and that of chunk i + 4 in the ring of hi
-            if (i >= LO_SLOTS && !wait_for(&done_bar[i & 3], ((i - LO_SLOTS) >> 2) & 1, abort_flag, 33)) break;
-            ask(i + ROWS_AHEAD);
+            ask(i + ROWS_AHEAD);                       // into the place of chunk i - 1, which this thread has read
             asm volatile("cp.async.wait_group %0;" ::"n"(ROWS_AHEAD) : "memory");
-            uint8_t* hi_p = hi_ring + b_lane + (i % HI_SLOTS) * B_BYTES;
-            uint8_t* lo_p = lo_ring + b_lane + (i % LO_SLOTS) * B_BYTES;
+            // the MMAs of chunk i - ROW_SLOTS have read its place
+            if (i >= ROW_SLOTS && !wait_for(&done_bar[i & 3], ((i - ROW_SLOTS) >> 2) & 1, abort_flag, 33)) break;
+            const uint8_t* from = raw_ring + raw_lane + (i % RAW_SLOTS) * (NT * 128);
+            uint8_t* to = rows_ring + rows_lane + (i % ROW_SLOTS) * ROW_BYTES;
 #pragma unroll
             for (int j = 0; j < PER; ++j) {
                 if (16 * j >= n_mma) break;
-                const uint4 v = *reinterpret_cast<const uint4*>(hi_p + j * 2048);
-                uint4 hi, lo;
-                split(v.x, hi.x, lo.x); split(v.y, hi.y, lo.y); split(v.z, hi.z, lo.z); split(v.w, hi.w, lo.w);
-                *reinterpret_cast<uint4*>(hi_p + j * 2048) = hi;
-                *reinterpret_cast<uint4*>(lo_p + j * 2048) = lo;
+                const uint4 v = *reinterpret_cast<const uint4*>(from + j * 2048);
+                uint2 h, m, l;
+                take_apart(v.x, v.y, h.x, m.x, l.x);
+                take_apart(v.z, v.w, h.y, m.y, l.y);
+                *reinterpret_cast<uint2*>(to + j * 1024) = h;
+                *reinterpret_cast<uint2*>(to + j * 1024 + part_bytes) = m;
+                *reinterpret_cast<uint2*>(to + j * 1024 + 2 * part_bytes) = l;
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
@@ -490,7 +528,7 @@ f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
     if (abort_s == 0) {
         const uint32_t sums_at = smem_u32(sums);
-        auto total = [&](int feat, int r) {
+        auto sum = [&](int feat, int r) {
             if (!SPLIT) return sums[r * 128 + feat];
             float v = 0.f;
 #pragma unroll
@@ -498,12 +536,13 @@ f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
                 uint32_t there;
                 float s;
                 asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there)
-                             : "r"(sums_at + (uint32_t)(((p % own_parts) * NT + r) * 128 + feat) * 4), "r"(p / own_parts));
+                             : "r"(sums_at + (uint32_t)(((p % own_parts) * 2 * NT + r) * 128 + feat) * 4), "r"(p / own_parts));
                 asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(s) : "r"(there));
                 v += s;
             }
             return v;
         };
+        auto total = [&](int feat, int r) { return (sum(feat, r) + sum(feat, NT + r)) * DOWN; };
         // rows rank, rank + ranks, ... of the tile are this block's
         for (int idx = threadIdx.x; idx < FEATS * ((rows - (int)rank + (int)ranks - 1) / (int)ranks); idx += THREADS) {
             const int feat = idx % FEATS, r = (idx / FEATS) * (int)ranks + (int)rank, n = n0 + feat, t = row0 + r;
