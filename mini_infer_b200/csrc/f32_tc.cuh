@@ -4,10 +4,10 @@
 //
 // A number x of 32 bits is taken apart exactly, into three bfloat16 numbers: 2^24 x = h + m + l, each the rest rounded to 8 bits
 // (the factor keeps the parts of the smallest x among the normal numbers).  Of the nine products of two numbers' parts all are formed but
-// that of the two l, which is at most 2^-34 of the whole.  They stand in three sums by their size: hh; hm, mh and lh; hl, mm, lm and ml.
-// The tensor cores add without rounding to nearest, so 32 terms at most are added there: hh's have 16 bits, of which few are cut
-// off, and the other sums are 2^-8 of it and less.  Then the sums go to registers and are added up there, hh and the others each by
-// itself, in 32 bits as any number is, and meet in the output alone.  Measured error: see dense_f32.cu.
+// that of the two l, which is at most 2^-34 of the whole.  They stand in two sums by their size: hh; and the others, hm, mh and lh beside
+// hl, mm, lm and ml, 2^-8 of it and less.  The tensor cores add without rounding to nearest.  hh's terms have 16 bits, of which
+// few are cut off, but 32 of them at most are added there: then the sum goes to registers and is added up in 32 bits as any
+// number is.  The others stay for a part of the inner dimension.  Both meet in the output alone.  Measured error: see dense_f32.cu.
 //
 // Every output element is the same sums in the same order in every form below: chunks of 32 k in ascending order within
 // each of four parts of the inner dimension, then the parts in ascending order.  So a row has the same bits however many
@@ -19,14 +19,13 @@
 // tensor memory, rows of activations are the N operand in shared memory.  Roles:
 //   warps 0-3 and 4-7, chunks in turn: weights, ring -> three parts -> tensor memory
 //   warps 8-15  the sums of a chunk: tensor memory -> registers, added up
-//   warps 16, 17, chunks in turn: MMAs (8 a chunk; the tensor cores take them one by one as they come, so a single warp
-//               would leave them idle while it waits for the next chunk's operands); warp 16 allocates tensor memory.
-//               The activations' parts stand one behind the other, so that one MMA multiplies a part of the weights with two
-//               or all three of them (an MMA of 64 rows takes as long as one of 128)
-//   warp 18     weights: memory -> ring (TMA; without it, where rows are not aligned for it, the warps that read them ask
+//   warp 16     MMAs, 10 a chunk (the next chunk is waited for before the last two are given out, so that the tensor cores do
+//               not run dry); tensor memory.  The activations' parts stand one behind the other, so that one MMA multiplies a
+//               part of the weights with two of them (an MMA of 64 rows takes 62 cycles, as long as one of 128)
+//   warp 17     weights: memory -> ring (TMA; without it, where rows are not aligned for it, the warps that read them ask
 //               for them with cp.async)
-//   tiles of 64 rows: warp 19 brings the parts of the activations, which f32_split_rows_kernel has made (TMA)
-//   tiles of 16 and 32: warps 19-22 bring the activations (cp.async, four chunks ahead) and take them apart in shared memory
+//   tiles of 64 rows: warp 18 brings the parts of the activations, which f32_split_rows_kernel has made (TMA)
+//   tiles of 16 and 32: warps 18-21 bring the activations (cp.async, four chunks ahead) and take them apart in shared memory
 // SPLIT: a cluster of 2 or 4 blocks shares a tile's parts and adds them up through distributed shared memory, where tiles
 // alone would leave SMs without work (a decode step's few rows).
 //
@@ -43,21 +42,21 @@ using namespace tc;
 constexpr int TC_MIN_K = 512;
 constexpr int FK = 32;                                 // k per chunk: 32 floats are a swizzled row of 128 bytes, 32 bfloat16 one of 64
 constexpr int PARTS = 4;
-constexpr int OUT_WARP = 8, MMA_WARP = 16, W_WARP = 18, ROWS_WARP = 19;        // first warps of the roles
+constexpr int OUT_WARP = 8, MMA_WARP = 16, W_WARP = 17, ROWS_WARP = 18;        // first warps of the roles
 constexpr bool split_before(int nt) { return nt >= 64; }
-constexpr int threads(int nt) { return 32 * (split_before(nt) ? 20 : 23); }
-constexpr int T_SLOTS = 2, ROWS_AHEAD = 4;             // chunks of weights in tensor memory; of activations asked for
+constexpr int threads(int nt) { return 32 * (split_before(nt) ? 19 : 22); }
+constexpr int ROWS_AHEAD = 4;                          // chunks of activations asked for
 constexpr uint32_t SLOT_LIMIT = 65536;                 // bytes of part sums of a SPLIT block
 constexpr float UP = 16777216.f, DOWN = 1.f / (UP * UP);       // factors of operands and results
 // D float32, A and B bfloat16, both K-major, M = 128 (without N)
 constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((128u >> 4) << 24);
 
 // Rings, in chunks: weights; parts of the activations (at most four: see the phases below); activations on their way, where the
-// block takes them apart; sums in tensor memory
+// block takes them apart; in tensor memory weights and sums of hh
 constexpr int w_slots(int nt, bool split) { return (nt == 64 ? 6 : 8) - (split ? 2 : 0); }
 constexpr int ROW_SLOTS = 4;
 constexpr int raw_slots(int nt) { return split_before(nt) ? 0 : ROWS_AHEAD + 1; }
-constexpr int d_slots(int nt) { return nt == 64 ? 2 : 4; }
+constexpr int t_slots(int nt) { return nt == 64 ? 2 : 4; }
 inline size_t smem_bytes(int nt, int split) {
     return 1024 + (size_t)w_slots(nt, split > 1) * 16384 + (size_t)ROW_SLOTS * nt * 192 + (size_t)raw_slots(nt) * nt * 128 +
            (size_t)(split > 1 ? PARTS / split : 1) * 2 * nt * 512;
@@ -144,12 +143,22 @@ __device__ __forceinline__ uint32_t pack(float a, float b) {
 }
 __device__ __forceinline__ float first_of(uint32_t v) { return __uint_as_float(v << 16); }
 __device__ __forceinline__ float second_of(uint32_t v) { return __uint_as_float(v & 0xffff0000u); }
+__device__ __forceinline__ void add2(float& a, float& b, float x, float y) {
+    asm("{\n .reg .b64 s, t;\n mov.b64 s, {%0, %1};\n mov.b64 t, {%2, %3};\n add.rn.f32x2 s, s, t;\n mov.b64 {%0, %1}, s;\n}"
+        : "+f"(a), "+f"(b) : "f"(x), "f"(y));
+}
+// (a, b) - (x, y), exact here
+__device__ __forceinline__ void less2(float& a, float& b, float x, float y) {
+    asm("{\n .reg .b64 s, t, u;\n mov.b64 s, {%0, %1};\n mov.b64 t, {%2, %3};\n mov.b64 u, {%4, %4};\n fma.rn.f32x2 s, t, u, s;\n"
+        " mov.b64 {%0, %1}, s;\n}" : "+f"(a), "+f"(b) : "f"(x), "f"(y), "f"(-1.f));
+}
 __device__ __forceinline__ void take_apart(uint32_t x0, uint32_t x1, uint32_t& h, uint32_t& m, uint32_t& l) {
-    const float a = __uint_as_float(x0) * UP, b = __uint_as_float(x1) * UP;
+    float a = __uint_as_float(x0) * UP, b = __uint_as_float(x1) * UP;
     h = pack(a, b);
-    const float ra = a - first_of(h), rb = b - second_of(h);
-    m = pack(ra, rb);
-    l = pack(ra - first_of(m), rb - second_of(m));
+    less2(a, b, first_of(h), second_of(h));
+    m = pack(a, b);
+    less2(a, b, first_of(m), second_of(m));
+    l = pack(a, b);
 }
 __device__ __forceinline__ void cp_async16(uint32_t dst, const char* src, bool there) {
     const int n = there ? 16 : 0;                      // nothing read: the bytes become zeros
@@ -224,14 +233,16 @@ __global__ void __launch_bounds__(threads(NT), 1)
 f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ RowMaps map_rows, Problem g) {
     constexpr bool BEFORE = split_before(NT);
     static_assert(!BEFORE || VEC, "rows that are split before are aligned");
-    constexpr int THREADS = threads(NT), W_SLOTS = w_slots(NT, SPLIT), RAW_SLOTS = raw_slots(NT), D_SLOTS = d_slots(NT);
-    constexpr int D_STEP = 384 / D_SLOTS;              // columns of tensor memory of a chunk's three sums
+    constexpr int THREADS = threads(NT), W_SLOTS = w_slots(NT, SPLIT), RAW_SLOTS = raw_slots(NT), T_SLOTS = t_slots(NT);
+    // columns of tensor memory: T_SLOTS chunks' hh; the others' two sums, of even and of odd parts; T_SLOTS chunks of weights
+    constexpr int OTHERS_AT = 128, W_AT = 512 - T_SLOTS * 64;
+    static_assert(T_SLOTS * NT <= OTHERS_AT && OTHERS_AT + 4 * NT <= W_AT, "tensor memory");
     constexpr int ROW_BYTES = NT * 192;                // a chunk's activations: [part][rows][64 bytes], swizzled
     constexpr int FEATS = PAIRED ? 64 : 128;           // outputs of a tile
     constexpr int OWN = NT / 2;                        // rows of activations of an adding warp
     constexpr int PER = NT / 16;                       // 16-byte pieces of activations per thread and chunk
     extern __shared__ uint8_t smem_raw[];
-    __shared__ uint64_t full_bar[4], done_bar[4], empty_bar[D_SLOTS], w_full[W_SLOTS], w_read[W_SLOTS], rows_full[ROW_SLOTS];
+    __shared__ uint64_t full_bar[4], done_bar[4], empty_bar[T_SLOTS], w_full[W_SLOTS], w_read[W_SLOTS], rows_full[ROW_SLOTS];
     __shared__ uint32_t tmem_base_s;
     __shared__ int abort_s;
 
@@ -269,7 +280,7 @@ f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
     if (threadIdx.x == 0) {
         abort_s = 0;
         for (int s = 0; s < 4; ++s) { mbar_init(&full_bar[s], BEFORE ? 4 : 8); mbar_init(&done_bar[s], 1); }
-        for (int s = 0; s < D_SLOTS; ++s) mbar_init(&empty_bar[s], 8);
+        for (int s = 0; s < T_SLOTS; ++s) mbar_init(&empty_bar[s], 8);
         for (int s = 0; s < ROW_SLOTS; ++s) mbar_init(&rows_full[s], 1);
         for (int s = 0; s < W_SLOTS; ++s) { mbar_init(&w_full[s], 1); mbar_init(&w_read[s], 4); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -283,7 +294,7 @@ f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = tmem_base_s;                 // columns 0-383: two or four chunks' sums; 384-511: two of weights
+    const uint32_t tmem = tmem_base_s;
 
     // Phases of the barriers of four (full, done): whoever waits for chunk i there has itself to act before chunk i + 4
     // can complete, so a parity never stands for the phase after the next.
@@ -309,7 +320,7 @@ f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
 #pragma unroll 1
         for (int i = 0; i < SLOTS - 1; ++i) ask(turn + 2 * i);
         const uint8_t* w_lane = w_ring + quarter * 4096 + lane * 128;
-        const uint32_t t_lane = tmem + ((uint32_t)(quarter * 32) << 16) + 384;
+        const uint32_t t_lane = tmem + ((uint32_t)(quarter * 32) << 16) + W_AT;
 #pragma unroll 1
         for (int i = turn; i < count; i += 2) {
             const int slot = i % W_SLOTS;
@@ -351,9 +362,9 @@ f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
         const int quarter = warp & 3, c_lo = ((warp - OUT_WARP) >> 2) * OWN, feat = quarter * 32 + lane;
         const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16) + c_lo;
         float* own = sums + c_lo * 128 + feat;         // of the first part; columns 128 apart
-        float part[2][OWN];                            // hh, others
+        float part[OWN];                               // hh
 #pragma unroll
-        for (int i = 0; i < OWN; ++i) part[0][i] = part[1][i] = 0.f;
+        for (int i = 0; i < OWN; ++i) part[i] = 0.f;
         bool ok = true;
         int in_part = 0, parts = 0;
 #pragma unroll 1
@@ -362,35 +373,38 @@ f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             if (c_lo < n_mma) {                        // uniform
-                const uint32_t d = lane_addr + (it % D_SLOTS) * D_STEP;
-                constexpr int GROUP = OWN < 16 ? OWN : 16;
+                const uint32_t d = lane_addr + (it % T_SLOTS) * NT;
+                uint32_t v[OWN];
+                if constexpr (OWN == 32) tmem_ld32(d, v);
+                else if constexpr (OWN == 16) tmem_ld16(d, v);
+                else tmem_ld8(d, v);
+                wait_tmem_ld();
 #pragma unroll
-                for (int x = 0; x < 3; ++x)
-#pragma unroll
-                    for (int i0 = 0; i0 < OWN; i0 += GROUP) {
-                        uint32_t v[GROUP];
-                        if constexpr (GROUP == 16) tmem_ld16(d + x * n_mma + i0, v);
-                        else tmem_ld8(d + x * n_mma + i0, v);
-                        wait_tmem_ld();
-#pragma unroll
-                        for (int i = 0; i < GROUP; ++i) part[x > 0][i0 + i] += __uint_as_float(v[i]);
-                    }
+                for (int i = 0; i < OWN; i += 2) add2(part[i], part[i + 1], __uint_as_float(v[i]), __uint_as_float(v[i + 1]));
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
-            if (lane == 0) mbar_arrive(&empty_bar[it % D_SLOTS]);
+            if (lane == 0) mbar_arrive(&empty_bar[it % T_SLOTS]);
             if (++in_part == per_part || it == count - 1) {
+                // The others' columns are written anew two parts on, by MMAs that wait for a chunk of the part between to be
+                // read here (a part that another follows has at least T_SLOTS chunks: inner sizes from 512 up).
                 float* to = own + (SPLIT ? parts * 2 * NT * 128 : 0);
+                const uint32_t d = lane_addr + OTHERS_AT + (parts & 1) * 2 * NT;
 #pragma unroll
-                for (int x = 0; x < 2; ++x)
+                for (int i0 = 0; i0 < OWN; i0 += 8) {
+                    uint32_t x[8], y[8];
+                    tmem_ld8(d + i0, x);
+                    tmem_ld8(d + n_mma + i0, y);
+                    wait_tmem_ld();
 #pragma unroll
-                    for (int i = 0; i < OWN; ++i) {
-                        float* at = to + (x * NT + i) * 128;
-                        if (!SPLIT && parts > 0) part[x][i] = *at + part[x][i];
-                        *at = 0.f + part[x][i];        // (a cluster's sums begin at +0, too)
-                        part[x][i] = 0.f;
-                        if (i % 8 == 7) asm volatile("" ::: "memory");     // (all loads at once would take registers that are not there)
+                    for (int i = 0; i < 8; ++i) {
+                        float *hh = to + (i0 + i) * 128, *others = hh + NT * 128, o = __uint_as_float(x[i]) + __uint_as_float(y[i]);
+                        if (!SPLIT && parts > 0) part[i0 + i] = *hh + part[i0 + i], o = *others + o;
+                        *hh = 0.f + part[i0 + i];      // (a cluster's sums begin at +0, too)
+                        *others = 0.f + o;
+                        part[i0 + i] = 0.f;
                     }
+                }
                 in_part = 0;
                 ++parts;
             }
@@ -400,28 +414,41 @@ f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
 #pragma unroll
                 for (int i = 0; i < OWN; ++i) own[(parts * 2 * NT + i) * 128] = own[((parts * 2 + 1) * NT + i) * 128] = 0.f;
     } else if (warp < W_WARP) {
-        const uint32_t by_n = (uint32_t)(n_mma >> 3) << 17, idesc1 = IDESC | by_n, idesc2 = IDESC | 2 * by_n, idesc3 = IDESC | 3 * by_n;
+        const uint32_t by_n = (uint32_t)(n_mma >> 3) << 17, idesc1 = IDESC | by_n, idesc2 = IDESC | 2 * by_n;
         const uint64_t rows_desc = umma_desc_64(smem_u32(rows_ring));
         const uint32_t step = part_bytes >> 4;
+        auto ready = [&](int i) {
+            return wait_for(&empty_bar[i % T_SLOTS], ((i / T_SLOTS) & 1) ^ 1, abort_flag, 35) &&
+                   (!BEFORE || wait_for(&rows_full[i % ROW_SLOTS], (i / ROW_SLOTS) & 1, abort_flag, 38)) &&
+                   wait_for(&full_bar[i & 3], (i >> 2) & 1, abort_flag, 36);
+        };
+        bool ok = count > 0 && ready(0);
+        int in_part = 0, odd = 0;
 #pragma unroll 1
-        for (int i = warp - MMA_WARP; i < count; i += 2) {
-            if (!wait_for(&empty_bar[i % D_SLOTS], ((i / D_SLOTS) & 1) ^ 1, abort_flag, 35)) break;
-            if (BEFORE && !wait_for(&rows_full[i % ROW_SLOTS], (i / ROW_SLOTS) & 1, abort_flag, 38)) break;
-            if (!wait_for(&full_bar[i & 3], (i >> 2) & 1, abort_flag, 36)) break;
+        for (int i = 0; i < count && ok; ++i) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint64_t bh = rows_desc + (uint32_t)(((i % ROW_SLOTS) * ROW_BYTES) >> 4), bl = bh + 2 * step;
-            const uint32_t wh = tmem + 384 + (i % T_SLOTS) * 64, wm = wh + 16, wl = wm + 16, d = tmem + (i % D_SLOTS) * D_STEP;
+            // 16 k: 8 columns of weights, 32 bytes of a row
+            const uint64_t bh = rows_desc + (uint32_t)(((i % ROW_SLOTS) * ROW_BYTES) >> 4), bm = bh + step, bl = bm + step;
+            const uint32_t wh = tmem + W_AT + (i % T_SLOTS) * 64, wm = wh + 16, wl = wm + 16;
+            const uint32_t hh = tmem + (i % T_SLOTS) * NT, o1 = tmem + OTHERS_AT + odd * 2 * NT, o2 = o1 + n_mma;
             if (elect_one()) {
 #pragma unroll
-                for (int k = 0; k < FK / 16; ++k) {    // 16 k: 8 columns of weights, 32 bytes of a row
-                    umma_tmem_a(d, wh + k * 8, bh + k * 2, idesc3, k > 0);                   // hh, hm, hl
-                    umma_tmem_a(d + n_mma, wm + k * 8, bh + k * 2, idesc2, 1);               //     mh, mm
-                    umma_tmem_a(d + n_mma, wl + k * 8, bh + k * 2, idesc2, 1);               //     lh, lm
-                    umma_tmem_a(d + 2 * n_mma, wm + k * 8, bl + k * 2, idesc1, 1);           //         ml
+                for (int k = 0; k < FK / 16; ++k) {
+                    umma_tmem_a(o1, wh + k * 8, bm + k * 2, idesc2, in_part + k > 0);        // hm, hl
+                    umma_tmem_a(o1, wm + k * 8, bh + k * 2, idesc2, 1);                      // mh, mm
+                    umma_tmem_a(o1, wl + k * 8, bh + k * 2, idesc2, 1);                      // lh, lm
+                    umma_tmem_a(o2, wm + k * 8, bl + k * 2, idesc1, 1);                      //     ml
                 }
+            }
+            __syncwarp();
+            if (i + 1 < count) ok = ready(i + 1);      // (it waits for no chunk behind i - 1)
+            if (elect_one()) {
+#pragma unroll
+                for (int k = 0; k < FK / 16; ++k) umma_tmem_a(hh, wh + k * 8, bh + k * 2, idesc1, k > 0);
                 umma_commit(&done_bar[i & 3]);
             }
             __syncwarp();
+            if (++in_part == per_part) in_part = 0, odd ^= 1;
         }
     } else if (warp == W_WARP) {
         if (VEC && lane == 0) {
