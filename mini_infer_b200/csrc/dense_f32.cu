@@ -105,7 +105,6 @@ static int dense_f32_launch(const DenseF32& g, int batch, bool vec, cudaStream_t
 struct TcForm { int nt, split; };
 struct TcLaunch {
     CUtensorMap map_w;
-    f32tc::RowMaps map_rows;
     dim3 grid;
     int split;
     cudaStream_t stream;
@@ -128,7 +127,7 @@ static int f32_tc_launch_one(const f32tc::Problem& g, const TcLaunch& l) {
     attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
     lc.attrs = attr;
     lc.numAttrs = SPLIT ? 1 : 0;
-    cudaLaunchKernelEx(&lc, kern, l.map_w, l.map_rows, g);
+    cudaLaunchKernelEx(&lc, kern, l.map_w, g);
     return finish_launch(l.what);
 }
 template <bool PAIRED, int NT>
@@ -136,17 +135,22 @@ static int f32_tc_launch_nt(const f32tc::Problem& g, const TcLaunch& l) {
     return l.split > 1 ? f32_tc_launch_one<PAIRED, NT, true, true>(g, l) : f32_tc_launch_one<PAIRED, NT, false, true>(g, l);
 }
 
-// Rows whose parts are made ahead of a product, at most so many bytes of them at a time: a product of more rows goes in bands of
-// whole tiles (its rows do not touch each other).
+// Rows whose parts are made ahead of a product, at most so many bytes of them at a time: a product of more rows goes in bands
+// (its rows do not touch each other).
 constexpr int64_t TC_SCRATCH_BYTES = 128ll << 20;
-static int64_t f32_tc_pitch(int K) { return (K + 7) & ~7; }            // bfloat16 numbers from row to row: 16 bytes and more
-// floats that the parts of `rows` rows take
-static int64_t f32_tc_scratch(int64_t rows, int K) {
-    const int64_t band = TC_SCRATCH_BYTES / (6 * f32_tc_pitch(K)) / 64 * 64, most = band > 64 ? band : 64;
-    return rows > 32 ? (3 * (rows < most ? rows : most) * f32_tc_pitch(K) + 1) / 2 : 0;
+static int64_t f32_tc_row_bytes(int K) { return 6ll * ((K + f32tc::FK - 1) / f32tc::FK * f32tc::FK); }
+// tiles of up to nt rows that n rows make at most
+static int64_t f32_tc_tiles(int64_t n, int groups, int nt) { return groups ? (n < n / nt + groups ? n : n / nt + groups) : (n + nt - 1) / nt; }
+// floats that the parts of `rows` rows of `batch` products each, or of `groups` experts together, take
+static int64_t f32_tc_scratch(int64_t rows, int K, int groups, int batch) {
+    if (rows <= 32) return 0;
+    const int64_t own = f32_tc_row_bytes(K), most = TC_SCRATCH_BYTES / own / batch;
+    int64_t all = rows + 16 * f32_tc_tiles(rows, groups, 64);
+    if (all > most) all = most > 64 ? most : 64;
+    return all * batch * (own / 4);
 }
 
-// `rows`: rows in all; `groups`: experts (0: a dense product).  `scratch`: f32_tc_scratch(rows * batch, K) floats.
+// `rows`: rows in all; `groups`: experts (0: a dense product).  `scratch`: f32_tc_scratch(rows, K, groups, batch) floats.
 template <bool PAIRED>
 static int f32_tc_launch(f32tc::Problem g, float* scratch, int rows, int groups, int batch, TcForm form, cudaStream_t stream,
                          const char* what) {
@@ -159,12 +163,13 @@ static int f32_tc_launch(f32tc::Problem g, float* scratch, int rows, int groups,
     const int64_t tiles_m = PAIRED ? (g.N + 63) / 64 : (g.N + 127) / 128;
     if (batch > 65535) { set_last_error("%s: %d products exceed the grid limit", what, batch); return kBadShape; }
     int nt = !vec ? 32 : form.nt > 64 ? 64 : form.nt > 0 ? form.nt : rows <= 16 ? 16 : rows <= 32 ? 32 : 64;
-    // rows of a launch: what the scratch holds, or the grid
+    // rows of a launch: what the scratch holds (16 rows more for a tile), or the grid
     int64_t band = 65535ll * nt;
     if (f32tc::split_before(nt)) {
-        const int64_t room = f32_tc_scratch((int64_t)rows * batch, g.K) * 2 / 3 / f32_tc_pitch(g.K) / batch;
-        band = room < rows ? room / 64 * 64 : rows;
-        if (band == 0) nt = 32, band = 65535ll * nt;   // (many products of long rows)
+        const int64_t room = f32_tc_scratch(rows, g.K, groups, batch) / (f32_tc_row_bytes(g.K) / 4) / batch;
+        band = rows;
+        while (band > 0 && band + 16 * f32_tc_tiles(band, groups, nt) > room) band = band / 2 / 64 * 64;
+        if (band == 0) nt = 32, band = 65535ll * nt;   // (rows that are too long, or too many experts)
     }
     if (f32tc::split_before(nt) && !scratch) { set_last_error("%s: no room for the rows' parts", what); return kBadShape; }
     TcLaunch l = {};
@@ -176,7 +181,7 @@ static int f32_tc_launch(f32tc::Problem g, float* scratch, int rows, int groups,
     }
     for (int64_t r0 = 0; r0 < rows; r0 += band) {
         const int n = (int)(rows - r0 < band ? rows - r0 : band);
-        const int64_t tiles_y = groups ? (n < n / nt + groups ? n : n / nt + groups) : ((int64_t)n + nt - 1) / nt;
+        const int64_t tiles_y = f32_tc_tiles(n, groups, nt);
         if (tiles_y > 65535) {
             set_last_error("%s: %d rows of %d experts exceed the grid limit", what, rows, groups);
             return kBadShape;
@@ -194,16 +199,10 @@ static int f32_tc_launch(f32tc::Problem g, float* scratch, int rows, int groups,
         while (l.split > 1 && l.split < f32tc::PARTS && (f32tc::PARTS / l.split) * 2 * nt * 512u > f32tc::SLOT_LIMIT) l.split *= 2;
         l.grid = dim3((unsigned)(tiles_m * l.split), (unsigned)tiles_y, (unsigned)batch);
         if (f32tc::split_before(nt)) {
-            const int pitch = (int)f32_tc_pitch(g.K);
-            f32tc::f32_split_rows_kernel<<<dim3(n, batch), 256, 0, stream>>>(g.A, g.gather, g.offsets, g.E, (uint2*)scratch, (int)r0, n,
-                                                                             g.lda, g.K / 4, pitch / 4, g.sA);
+            g.parts = (uint8_t*)scratch;
+            f32tc::f32_split_rows_kernel<<<dim3(tiles_y, (g.K + f32tc::SPLIT_K - 1) / f32tc::SPLIT_K, batch), 256, 0, stream>>>(g, nt);
             const int rc = finish_launch(what);
             if (rc != kOk) return rc;
-            for (int i = 0; i < 4; ++i) {
-                if (f32tc::make_map_parts(&l.map_rows.m[i], scratch, (uint64_t)n * batch, (uint64_t)g.K, (uint64_t)pitch, 16 * (i + 1))) continue;
-                set_last_error("%s: cuTensorMapEncodeTiled failed", what);
-                return kLaunchFailed;
-            }
         }
         const int rc = !vec ? f32_tc_launch_one<PAIRED, 32, false, false>(g, l)
                      : nt == 16 ? f32_tc_launch_nt<PAIRED, 16>(g, l)
@@ -217,8 +216,10 @@ static int f32_tc_launch(f32tc::Problem g, float* scratch, int rows, int groups,
 
 extern "C" int mi_f32_tc_min_inner() { return mi::f32tc::TC_MIN_K; }
 
-// Floats of scratch (16-byte aligned) that a product of `rows` rows (of all products together) takes.
-extern "C" int64_t mi_f32_tc_scratch(int64_t rows, int K) { return K >= mi::f32tc::TC_MIN_K ? mi::f32_tc_scratch(rows, K) : 0; }
+// Floats of scratch (16-byte aligned) that a product of `rows` rows, of `groups` experts or (0) in each of `batch` products, takes.
+extern "C" int64_t mi_f32_tc_scratch(int64_t rows, int K, int groups, int batch) {
+    return K >= mi::f32tc::TC_MIN_K && rows > 0 && batch > 0 ? mi::f32_tc_scratch(rows, K, groups, batch) : 0;
+}
 
 // `batch` products at once: C_b[T, N] = A_b[T, K] . W_b[N, K]^T with rows of A and C `lda` and `ldc` floats
 // apart and the operands of product b at A + b * sA, W + b * sW (rows K apart), C + b * sC: the heads of a
@@ -232,7 +233,7 @@ extern "C" int mi_dense_f32_batched(const float* A, const float* W, float* C, in
         return kBadShape;
     }
     if (K >= f32tc::TC_MIN_K)
-        return f32_tc_launch<false>(f32tc::Problem{A, W, C, nullptr, nullptr, N, K, lda, ldc, 0, sA, sW, sC, 0, 0, GluForm{}, status}, scratch, T, 0,
+        return f32_tc_launch<false>(f32tc::Problem{A, W, C, nullptr, nullptr, N, K, lda, ldc, 0, sA, sW, sC, 0, 0, nullptr, GluForm{}, status}, scratch, T, 0,
                                     batch, TcForm{-1, -1}, stream, "dense_f32");
     const bool vec = (K % 4 == 0) && (lda % 4 == 0) && (sA % 4 == 0) && (sW % 4 == 0) &&
                      (((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W)) & 15) == 0);
@@ -259,7 +260,7 @@ extern "C" int mi_f32_tc_form(const float* A, const int* gather, const float* W,
         return kBadShape;
     }
     const GluForm glu{glu_kind, glu_limit, glu_slope, mode == 1 ? row_scale : nullptr};
-    const f32tc::Problem g{A, W, C, gather, offsets, Nout, K, K, Nout, E, 0, 0, 0, 0, 0, glu, status};
+    const f32tc::Problem g{A, W, C, gather, offsets, Nout, K, K, Nout, E, 0, 0, 0, 0, 0, nullptr, glu, status};
     const TcForm form{nt, split};
     return mode == 1 ? f32_tc_launch<true>(g, scratch, n_rows, E, 1, form, stream, "grouped_gemm_plain")
                      : f32_tc_launch<false>(g, scratch, n_rows, E, 1, form, stream, E ? "grouped_gemm_plain" : "dense_f32");

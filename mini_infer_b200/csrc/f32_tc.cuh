@@ -17,14 +17,14 @@
 //
 // Weights are the M operand (128 rows a tile; 64 gate rows and the up rows of the same outputs in a paired product) and lie in
 // tensor memory, rows of activations are the N operand in shared memory.  Roles:
-//   warps 0-3 and 4-7, chunks in turn: weights, ring -> three parts -> tensor memory
-//   warps 8-15  the sums of a chunk: tensor memory -> registers, added up
-//   warp 16     MMAs, 10 a chunk (the next chunk is waited for before the last two are given out, so that the tensor cores do
-//               not run dry); tensor memory.  The activations' parts stand one behind the other, so that one MMA multiplies a
-//               part of the weights with two of them (an MMA of 64 rows takes 62 cycles, as long as one of 128)
+//   warps 0-7 (tiles of 64 rows) or 0-11, four for a chunk, in turn: weights, ring -> three parts -> tensor memory
+//   warps 8-15 or 12-15  the sums of a chunk: tensor memory -> registers, added up
+//   warp 16     MMAs, 10 a chunk; tensor memory.  The activations' parts stand one behind the other, so that one MMA multiplies a
+//               part of the weights with two of them
 //   warp 17     weights: memory -> ring (TMA; without it, where rows are not aligned for it, the warps that read them ask
 //               for them with cp.async)
-//   tiles of 64 rows: warp 18 brings the parts of the activations, which f32_split_rows_kernel has made (TMA)
+//   tiles of 64 rows: warp 18 brings the parts of the activations, which f32_split_rows_kernel has laid out as they stand here
+//               (one plain copy a chunk; as boxes of rows of 64 bytes they held the tile up)
 //   tiles of 16 and 32: warps 18-21 bring the activations (cp.async, four chunks ahead) and take them apart in shared memory
 // SPLIT: a cluster of 2 or 4 blocks shares a tile's parts and adds them up through distributed shared memory, where tiles
 // alone would leave SMs without work (a decode step's few rows).
@@ -40,10 +40,11 @@ namespace f32tc {
 using namespace tc;
 
 constexpr int TC_MIN_K = 512;
-constexpr int FK = 32;                                 // k per chunk: 32 floats are a swizzled row of 128 bytes, 32 bfloat16 one of 64
+constexpr int FK = 32;                                 // k per chunk: 32 floats are a swizzled row of 128 bytes
 constexpr int PARTS = 4;
-constexpr int OUT_WARP = 8, MMA_WARP = 16, W_WARP = 17, ROWS_WARP = 18;        // first warps of the roles
+constexpr int MMA_WARP = 16, W_WARP = 17, ROWS_WARP = 18;        // first warps of the roles
 constexpr bool split_before(int nt) { return nt >= 64; }
+constexpr int w_turns(int nt) { return split_before(nt) ? 2 : 3; }             // groups of four warps that take chunks of weights in turn
 constexpr int threads(int nt) { return 32 * (split_before(nt) ? 19 : 22); }
 constexpr int ROWS_AHEAD = 4;                          // chunks of activations asked for
 constexpr uint32_t SLOT_LIMIT = 65536;                 // bytes of part sums of a SPLIT block
@@ -53,7 +54,7 @@ constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((128u >> 4) << 
 
 // Rings, in chunks: weights; parts of the activations (at most four: see the phases below); activations on their way, where the
 // block takes them apart; in tensor memory weights and sums of hh
-constexpr int w_slots(int nt, bool split) { return (nt == 64 ? 6 : 8) - (split ? 2 : 0); }
+constexpr int w_slots(int nt, bool split) { return nt == 64 ? (split ? 4 : 6) : (split ? 6 : 9); }        // (a multiple of w_turns)
 constexpr int ROW_SLOTS = 4;
 constexpr int raw_slots(int nt) { return split_before(nt) ? 0 : ROWS_AHEAD + 1; }
 constexpr int t_slots(int nt) { return nt == 64 ? 2 : 4; }
@@ -62,22 +63,23 @@ inline size_t smem_bytes(int nt, int split) {
            (size_t)(split > 1 ? PARTS / split : 1) * 2 * nt * 512;
 }
 
-// The parts of `rows` rows of activations, [3][rows][pitch] of bfloat16: boxes of 32 columns x box_rows rows x 3, 64-byte swizzle.
-inline bool make_map_parts(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint64_t pitch, uint32_t box_rows) {
-    EncodeTiledFn fn = encode_fn();
-    if (!fn) return false;
-    const cuuint64_t dims[3] = {cols, rows, 3};
-    const cuuint64_t strides[2] = {pitch * 2, rows * pitch * 2};
-    const cuuint32_t box[3] = {(cuuint32_t)FK, box_rows, 3}, estr[3] = {1, 1, 1};
-    return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-              CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
 // mbar_wait of tcgen05.cuh, by a whole warp
 __device__ __forceinline__ bool wait_for(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int code) {
     bool there = false;
     for (uint32_t i = 0; i < WAIT_LIMIT && !there; ++i) {
         there = __all_sync(0xffffffffu, mbar_try_wait(bar, parity));
+        if (!there && *abort_flag) return false;
+    }
+    if (!there) *abort_flag = code;
+    return there;
+}
+// ... for three at once: one behind the other they take 230 cycles each in a busy SM, also where nothing is left to wait for
+__device__ __forceinline__ bool wait_for3(uint64_t* a, uint32_t pa, uint64_t* b, uint32_t pb, uint64_t* c, uint32_t pc,
+                                          volatile int* abort_flag, int code) {
+    bool there = false;
+    for (uint32_t i = 0; i < WAIT_LIMIT && !there; ++i) {
+        const bool ta = mbar_try_wait(a, pa), tb = mbar_try_wait(b, pb), tc = mbar_try_wait(c, pc);
+        there = __all_sync(0xffffffffu, ta & tb & tc);
         if (!there && *abort_flag) return false;
     }
     if (!there) *abort_flag = code;
@@ -91,31 +93,25 @@ struct Problem {
     int N, K, lda, ldc, E;                             // N: outputs (a paired product has 2 N rows of W an expert)
     int64_t sA, sW, sC;                                // dense: operands of product blockIdx.z
     int row_begin, row_end;                            // the (sorted) rows of this launch
+    uint8_t* parts;                                    // of their activations, tile by tile as tile_at says
     GluForm glu;
     int* status;
 };
-struct RowMaps { CUtensorMap m[4]; };                  // the activations' parts in boxes of 16, 32, 48 and 64 rows x 3
 
-__device__ __forceinline__ void umma_tmem_a(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+// (the descriptor's halves: only the lower one moves with the tile)
+__device__ __forceinline__ void umma_tmem_a(uint32_t tmem_d, uint32_t tmem_a, uint32_t b_lo, uint32_t b_hi, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-        " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}"
-        ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+        "{\n .reg .pred p;\n .reg .b64 b;\n setp.ne.b32 p, %5, 0;\n mov.b64 b, {%2, %3};\n"
+        " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %4, p;\n}"
+        ::"r"(tmem_d), "r"(tmem_a), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate) : "memory");
 }
-// K-major tile of rows of 64 bytes, 64-byte swizzle: groups of 8 rows 512 bytes apart
-__device__ __forceinline__ uint64_t umma_desc_64(uint32_t smem_addr) {
-    uint64_t d = 0;
-    d |= (uint64_t)((smem_addr & 0x3FFFFu) >> 4);
-    d |= (uint64_t)1 << 16;
-    d |= (uint64_t)(512 >> 4) << 32;
-    d |= (uint64_t)1 << 46;
-    d |= (uint64_t)4 << 61;
-    return d;
+// K-major tile in core matrices of 8 rows x 16 bytes, one behind the other along the rows, k_bytes apart along k
+__device__ __forceinline__ uint64_t umma_desc_plain(uint32_t smem_addr, uint32_t k_bytes) {
+    return (uint64_t)((smem_addr & 0x3FFFFu) >> 4) | (uint64_t)(k_bytes >> 4) << 16 | (uint64_t)(128 >> 4) << 32 | (uint64_t)1 << 46;
 }
-__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
-        ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z) : "memory");
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
 }
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
@@ -205,24 +201,42 @@ __device__ __forceinline__ int row_tile(const int* __restrict__ offsets, int E, 
     return 0;
 }
 
-// The parts of rows of activations (K a multiple of 4, read four at a time): out[part][z * rows + r][pitch] of
-// x_z[gather ? gather[first + r] : first + r].  Grouped: only the rows that an expert has; beyond them `gather` need not be written.
+// The rows of tile `slot` of product z among the launch's: first and number.  Uniform for the warp.
+__device__ __forceinline__ int tile_rows(const Problem& g, int nt, int slot, int& e, int& row0) {
+    if (g.offsets) return row_tile(g.offsets, g.E, g.row_begin, g.row_end, nt, slot, e, row0);
+    e = 0;
+    row0 = g.row_begin + slot * nt;
+    return min(nt, g.row_end - row0);
+}
+// Where its parts lie: chunks in turn, [8 k][part][n rows][16 bytes] each with n the tile's rows rounded up to 16 (hence room for
+// 16 rows more than there are for every tile before it).
+__device__ __forceinline__ int64_t tile_at(const Problem& g, int z, int slots, int slot, int row0, int chunks) {
+    return ((int64_t)z * (g.row_end - g.row_begin + 16 * slots) + (row0 - g.row_begin) + 16 * slot) * chunks * (FK * 6);
+}
+
+// The parts of a tile's rows of activations, zeros from K (a multiple of 4) to the end of its chunk.  Grouped: rows that no expert
+// has are not read (`gather` need not be written there).  A warp's lanes are 32 rows: 32 bytes of each are read, 512 bytes of
+// a part written.
+constexpr int SPLIT_K = 64;                            // k of a block: 8 warps x 8
 __global__ void __launch_bounds__(256)
-f32_split_rows_kernel(const float* __restrict__ x, const int* __restrict__ gather, const int* __restrict__ offsets, int E,
-                      uint2* __restrict__ out, int first, int rows, int lda, int K4, int pitch4, int64_t sA) {
-    const int r = blockIdx.x;
-    if (offsets && first + r >= __ldg(offsets + E)) return;
-    const int64_t row = gather ? __ldg(gather + first + r) : first + r, part = (int64_t)gridDim.y * rows * pitch4;
-    const uint4* src = reinterpret_cast<const uint4*>(x + blockIdx.y * sA + row * lda);
-    uint2* to = out + ((int64_t)blockIdx.y * rows + r) * pitch4;
-    for (int i = threadIdx.x; i < K4; i += 256) {
-        const uint4 v = __ldg(src + i);
-        uint2 h, m, l;
-        take_apart(v.x, v.y, h.x, m.x, l.x);
-        take_apart(v.z, v.w, h.y, m.y, l.y);
-        to[i] = h;
-        to[part + i] = m;
-        to[2 * part + i] = l;
+f32_split_rows_kernel(Problem g, int nt) {
+    const int k = blockIdx.y * SPLIT_K + (threadIdx.x >> 5) * 8, chunks = (g.K + FK - 1) / FK;
+    int e = 0, row0 = 0;
+    const int rows = tile_rows(g, nt, blockIdx.x, e, row0), n = (rows + 15) & ~15;
+    if (k >= chunks * FK) return;
+    uint4* to = reinterpret_cast<uint4*>(g.parts + tile_at(g, blockIdx.z, gridDim.x, blockIdx.x, row0, chunks)) + (int64_t)(k / 8) * 3 * n;
+    for (int r = threadIdx.x & 31; r < rows; r += 32) {
+        const int64_t row = g.gather ? __ldg(g.gather + row0 + r) : row0 + r;
+        const uint4* src = reinterpret_cast<const uint4*>(g.A + blockIdx.z * g.sA + row * g.lda + k);
+        const uint4 none = make_uint4(0u, 0u, 0u, 0u), a = k < g.K ? __ldg(src) : none, b = k + 4 < g.K ? __ldg(src + 1) : none;
+        uint4 h, m, l;
+        take_apart(a.x, a.y, h.x, m.x, l.x);
+        take_apart(a.z, a.w, h.y, m.y, l.y);
+        take_apart(b.x, b.y, h.z, m.z, l.z);
+        take_apart(b.z, b.w, h.w, m.w, l.w);
+        to[r] = h;
+        to[n + r] = m;
+        to[2 * n + r] = l;
     }
 }
 
@@ -230,16 +244,18 @@ f32_split_rows_kernel(const float* __restrict__ x, const int* __restrict__ gathe
 // rows of W (boxes of 32 floats x 128 rows, 64 in a paired product, 128-byte swizzle).
 template <bool PAIRED, int NT, bool SPLIT, bool VEC>
 __global__ void __launch_bounds__(threads(NT), 1)
-f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ RowMaps map_rows, Problem g) {
+f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, Problem g) {
     constexpr bool BEFORE = split_before(NT);
     static_assert(!BEFORE || VEC, "rows that are split before are aligned");
     constexpr int THREADS = threads(NT), W_SLOTS = w_slots(NT, SPLIT), RAW_SLOTS = raw_slots(NT), T_SLOTS = t_slots(NT);
+    constexpr int TURNS = w_turns(NT), OUT_WARP = 4 * TURNS;
+    static_assert(W_SLOTS % TURNS == 0, "a turn's own slots");
     // columns of tensor memory: T_SLOTS chunks' hh; the others' two sums, of even and of odd parts; T_SLOTS chunks of weights
     constexpr int OTHERS_AT = 128, W_AT = 512 - T_SLOTS * 64;
     static_assert(T_SLOTS * NT <= OTHERS_AT && OTHERS_AT + 4 * NT <= W_AT, "tensor memory");
-    constexpr int ROW_BYTES = NT * 192;                // a chunk's activations: [part][rows][64 bytes], swizzled
+    constexpr int ROW_BYTES = NT * 192;                // a chunk's activations: [8 k][part][rows][16 bytes]
     constexpr int FEATS = PAIRED ? 64 : 128;           // outputs of a tile
-    constexpr int OWN = NT / 2;                        // rows of activations of an adding warp
+    constexpr int OWN = NT / ((MMA_WARP - OUT_WARP) / 4);                  // rows of activations of an adding warp
     constexpr int PER = NT / 16;                       // 16-byte pieces of activations per thread and chunk
     extern __shared__ uint8_t smem_raw[];
     __shared__ uint64_t full_bar[4], done_bar[4], empty_bar[T_SLOTS], w_full[W_SLOTS], w_read[W_SLOTS], rows_full[ROW_SLOTS];
@@ -252,14 +268,9 @@ f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
         asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(ranks));
     }
     const int n0 = (int)(blockIdx.x / ranks) * FEATS;
-    int e = 0, row0, rows;
-    if (g.offsets) {
-        rows = row_tile(g.offsets, g.E, g.row_begin, g.row_end, NT, blockIdx.y, e, row0);
-        if (rows == 0) return;                         // uniform for the block and its cluster
-    } else {
-        row0 = g.row_begin + blockIdx.y * NT;
-        rows = min(NT, g.row_end - row0);
-    }
+    int e = 0, row0 = 0;
+    const int rows = tile_rows(g, NT, blockIdx.y, e, row0);
+    if (rows == 0) return;                             // uniform for the block and its cluster
     const float* A = g.A + blockIdx.z * g.sA;
     const float* W = g.W + blockIdx.z * g.sW + (int64_t)e * (PAIRED ? 2 : 1) * g.N * g.K;
     float* C = g.C + blockIdx.z * g.sC;
@@ -273,14 +284,14 @@ f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
     uint8_t* raw_ring = rows_ring + ROW_SLOTS * ROW_BYTES;                 // [slot][NT][128 bytes]
     uint8_t* w_ring = raw_ring + RAW_SLOTS * NT * 128;                     // [slot][128 rows][128 bytes], swizzled
     float* sums = reinterpret_cast<float*>(w_ring + W_SLOTS * 16384);      // [part][hh, others][NT][128]: SPLIT parts, otherwise their total
-    const uint32_t part_bytes = (uint32_t)n_mma * 64;
+    const uint32_t part_bytes = (uint32_t)n_mma * 16;  // of 8 k
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     volatile int* abort_flag = &abort_s;
 
     if (threadIdx.x == 0) {
         abort_s = 0;
         for (int s = 0; s < 4; ++s) { mbar_init(&full_bar[s], BEFORE ? 4 : 8); mbar_init(&done_bar[s], 1); }
-        for (int s = 0; s < T_SLOTS; ++s) mbar_init(&empty_bar[s], 8);
+        for (int s = 0; s < T_SLOTS; ++s) mbar_init(&empty_bar[s], MMA_WARP - OUT_WARP);
         for (int s = 0; s < ROW_SLOTS; ++s) mbar_init(&rows_full[s], 1);
         for (int s = 0; s < W_SLOTS; ++s) { mbar_init(&w_full[s], 1); mbar_init(&w_read[s], 4); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -316,19 +327,19 @@ f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
             }
             asm volatile("cp.async.commit_group;" ::: "memory");
         };
-        constexpr int SLOTS = W_SLOTS / 2;             // of this turn
+        constexpr int SLOTS = W_SLOTS / TURNS;         // of this turn
 #pragma unroll 1
-        for (int i = 0; i < SLOTS - 1; ++i) ask(turn + 2 * i);
+        for (int i = 0; i < SLOTS - 1; ++i) ask(turn + TURNS * i);
         const uint8_t* w_lane = w_ring + quarter * 4096 + lane * 128;
         const uint32_t t_lane = tmem + ((uint32_t)(quarter * 32) << 16) + W_AT;
 #pragma unroll 1
-        for (int i = turn; i < count; i += 2) {
+        for (int i = turn; i < count; i += TURNS) {
             const int slot = i % W_SLOTS;
             if (VEC) {
                 if (!wait_for(&w_full[slot], (i / W_SLOTS) & 1, abort_flag, 31)) break;
             } else {
                 __syncwarp();                          // the whole warp has read its chunk before: that slot is asked for anew
-                ask(i + 2 * (SLOTS - 1));
+                ask(i + TURNS * (SLOTS - 1));
                 asm volatile("cp.async.wait_group %0;" ::"n"(SLOTS - 1) : "memory");
                 __syncwarp();
             }
@@ -415,36 +426,31 @@ f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
                 for (int i = 0; i < OWN; ++i) own[(parts * 2 * NT + i) * 128] = own[((parts * 2 + 1) * NT + i) * 128] = 0.f;
     } else if (warp < W_WARP) {
         const uint32_t by_n = (uint32_t)(n_mma >> 3) << 17, idesc1 = IDESC | by_n, idesc2 = IDESC | 2 * by_n;
-        const uint64_t rows_desc = umma_desc_64(smem_u32(rows_ring));
-        const uint32_t step = part_bytes >> 4;
+        const uint64_t rows_desc = umma_desc_plain(smem_u32(rows_ring), 3 * part_bytes);
+        const uint32_t desc_lo = (uint32_t)rows_desc, desc_hi = (uint32_t)(rows_desc >> 32);
+        // room for the sums, rows (where no copy brings them: the room once more), weights (and rows)
         auto ready = [&](int i) {
-            return wait_for(&empty_bar[i % T_SLOTS], ((i / T_SLOTS) & 1) ^ 1, abort_flag, 35) &&
-                   (!BEFORE || wait_for(&rows_full[i % ROW_SLOTS], (i / ROW_SLOTS) & 1, abort_flag, 38)) &&
-                   wait_for(&full_bar[i & 3], (i >> 2) & 1, abort_flag, 36);
+            const uint32_t room = ((i / T_SLOTS) & 1) ^ 1;
+            return wait_for3(&empty_bar[i % T_SLOTS], room, BEFORE ? &rows_full[i % ROW_SLOTS] : &empty_bar[i % T_SLOTS],
+                             BEFORE ? (i / ROW_SLOTS) & 1 : room, &full_bar[i & 3], (i >> 2) & 1, abort_flag, 35);
         };
-        bool ok = count > 0 && ready(0);
         int in_part = 0, odd = 0;
 #pragma unroll 1
-        for (int i = 0; i < count && ok; ++i) {
+        for (int i = 0; i < count && ready(i); ++i) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            // 16 k: 8 columns of weights, 32 bytes of a row
-            const uint64_t bh = rows_desc + (uint32_t)(((i % ROW_SLOTS) * ROW_BYTES) >> 4), bm = bh + step, bl = bm + step;
+            const uint32_t bh = desc_lo + (i % ROW_SLOTS) * (ROW_BYTES >> 4), bm = bh + n_mma, bl = bm + n_mma;
+            const uint32_t k_step = 6 * n_mma;         // 16 k of rows; of weights 8 columns
             const uint32_t wh = tmem + W_AT + (i % T_SLOTS) * 64, wm = wh + 16, wl = wm + 16;
             const uint32_t hh = tmem + (i % T_SLOTS) * NT, o1 = tmem + OTHERS_AT + odd * 2 * NT, o2 = o1 + n_mma;
             if (elect_one()) {
 #pragma unroll
                 for (int k = 0; k < FK / 16; ++k) {
-                    umma_tmem_a(o1, wh + k * 8, bm + k * 2, idesc2, in_part + k > 0);        // hm, hl
-                    umma_tmem_a(o1, wm + k * 8, bh + k * 2, idesc2, 1);                      // mh, mm
-                    umma_tmem_a(o1, wl + k * 8, bh + k * 2, idesc2, 1);                      // lh, lm
-                    umma_tmem_a(o2, wm + k * 8, bl + k * 2, idesc1, 1);                      //     ml
+                    umma_tmem_a(o1, wh + k * 8, bm + k * k_step, desc_hi, idesc2, in_part + k > 0);   // hm, hl
+                    umma_tmem_a(o1, wm + k * 8, bh + k * k_step, desc_hi, idesc2, 1);                 // mh, mm
+                    umma_tmem_a(o1, wl + k * 8, bh + k * k_step, desc_hi, idesc2, 1);                 // lh, lm
+                    umma_tmem_a(o2, wm + k * 8, bl + k * k_step, desc_hi, idesc1, 1);                 //     ml
+                    umma_tmem_a(hh, wh + k * 8, bh + k * k_step, desc_hi, idesc1, k > 0);
                 }
-            }
-            __syncwarp();
-            if (i + 1 < count) ok = ready(i + 1);      // (it waits for no chunk behind i - 1)
-            if (elect_one()) {
-#pragma unroll
-                for (int k = 0; k < FK / 16; ++k) umma_tmem_a(hh, wh + k * 8, bh + k * 2, idesc1, k > 0);
                 umma_commit(&done_bar[i & 3]);
             }
             __syncwarp();
@@ -468,16 +474,16 @@ f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
         }
     } else if constexpr (BEFORE) {
         if (lane == 0) {
-            const int y = (int)(blockIdx.z * (int64_t)(g.row_end - g.row_begin)) + row0 - g.row_begin;
-            const CUtensorMap* map = &map_rows.m[n_mma / 16 - 1];
+            const uint32_t bytes = 12 * part_bytes;
+            const uint8_t* from = g.parts + tile_at(g, blockIdx.z, gridDim.y, blockIdx.y, row0, chunks) + (int64_t)first * bytes;
             int i = 0;
 #pragma unroll 1
             for (; i < count; ++i) {
                 // the MMAs of chunk i - ROW_SLOTS have read its place
                 if (i >= ROW_SLOTS && !mbar_wait(&done_bar[i & 3], ((i - ROW_SLOTS) >> 2) & 1, abort_flag, 33)) break;
                 const int slot = i % ROW_SLOTS;
-                mbar_expect_tx(&rows_full[slot], 3 * part_bytes);
-                tma_load_3d(rows_ring + slot * ROW_BYTES, map, (first + i) * FK, y, 0, &rows_full[slot]);
+                mbar_expect_tx(&rows_full[slot], bytes);
+                bulk_load(rows_ring + slot * ROW_BYTES, from + (int64_t)i * bytes, bytes, &rows_full[slot]);
             }
             for (int j = max(0, i - ROW_SLOTS); j < i; ++j)
                 for (uint32_t n = 0; n < WAIT_LIMIT && !mbar_try_wait(&rows_full[j % ROW_SLOTS], (j / ROW_SLOTS) & 1); ++n) {}
@@ -486,8 +492,7 @@ f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
         // this thread's pieces of a chunk are rows tid / 8 + 16 j at piece tid % 8; it alone reads what it asked for
         const int tid = threadIdx.x - 32 * ROWS_WARP, piece = tid & 7, r_lo = tid >> 3;
         const uint32_t pitch = (uint32_t)g.lda * 4u, raw_lane = tid * 16;
-        // 8 bytes of each part: in 16-byte piece (piece / 2) of the row, swizzled by bits 7 and 8 of the address
-        const uint32_t rows_lane = r_lo * 64 + (((piece >> 1) ^ ((r_lo >> 1) & 3)) << 4) + (piece & 1) * 8;
+        const uint32_t rows_lane = (piece >> 1) * 3 * part_bytes + r_lo * 16 + (piece & 1) * 8;       // 8 bytes of each part
         uint32_t row_of[PER];
 #pragma unroll
         for (int j = 0; j < PER; ++j) {
@@ -536,9 +541,9 @@ f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
                 uint2 h, m, l;
                 take_apart(v.x, v.y, h.x, m.x, l.x);
                 take_apart(v.z, v.w, h.y, m.y, l.y);
-                *reinterpret_cast<uint2*>(to + j * 1024) = h;
-                *reinterpret_cast<uint2*>(to + j * 1024 + part_bytes) = m;
-                *reinterpret_cast<uint2*>(to + j * 1024 + 2 * part_bytes) = l;
+                *reinterpret_cast<uint2*>(to + j * 256) = h;
+                *reinterpret_cast<uint2*>(to + j * 256 + part_bytes) = m;
+                *reinterpret_cast<uint2*>(to + j * 256 + 2 * part_bytes) = l;
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();

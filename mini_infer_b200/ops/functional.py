@@ -809,7 +809,7 @@ def f32_tc_form(a: torch.Tensor, gather: Optional[torch.Tensor], w: torch.Tensor
     if offsets is None and (a if gather is None else gather).shape[0] < n_rows:
         raise ValueError(f"f32_tc: the input has fewer than {n_rows} rows")
     status = _status_word(a.device)
-    scratch = _f32_scratch(a, n_rows)
+    scratch = _f32_scratch(a, n_rows, Kd, E)
     check(library().mi_f32_tc_form(_ptr(a), _ptr(gather), _ptr(w), _ptr(offsets), _ptr(out), n_rows, E, nout, Kd,
                                    1 if swiglu_pair else 0, int(rows_per_tile), int(blocks_per_tile), *_glu_args(glu),
                                    _row_scale(row_scale, n_rows, swiglu_pair, "grouped_gemm_plain"),
@@ -818,10 +818,11 @@ def f32_tc_form(a: torch.Tensor, gather: Optional[torch.Tensor], w: torch.Tensor
     return out
 
 
-def _f32_scratch(x: torch.Tensor, rows: int, K: Optional[int] = None) -> Optional[torch.Tensor]:
-    """Room for the two halves of ``rows`` rows in a float32 product on tensor cores (None where it takes none).  The caller
-    holds it until the product is queued: a block that is given back before may be given out again, and written, ahead of it."""
-    n = library().mi_f32_tc_scratch(rows, x.shape[-1] if K is None else K)
+def _f32_scratch(x: torch.Tensor, rows: int, K: int, experts: int = 0, products: int = 1) -> Optional[torch.Tensor]:
+    """Room for the parts of the rows of float32 products on tensor cores (None where they take none): ``rows`` of all experts, or of
+    each of several products.  The caller holds it until the product is queued: a block that is given back before may be given out
+    again, and written, ahead of it."""
+    n = library().mi_f32_tc_scratch(rows, K, experts, products)
     return torch.empty(n, dtype=F32, device=x.device) if n else None
 
 
@@ -836,7 +837,7 @@ def dense_f32(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
     N = w.shape[0]
     out = torch.empty(T, N, dtype=F32, device=x.device)
     status = _status_word(x.device)
-    scratch = _f32_scratch(x, T)
+    scratch = _f32_scratch(x, T, K)
     check(library().mi_dense_f32(_ptr(x), _ptr(w), _ptr(out), T, N, K, _ptr(scratch), _ptr(status), _stream()), "dense_f32")
     _tc_pending = _tc_pending or K >= library().mi_f32_tc_min_inner()
     return out
@@ -2100,7 +2101,7 @@ def dense_f32_heads(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor
     if x_col + (H - 1) * xs + K > lda or out_col + (H - 1) * os_ + N > ldc:
         raise ValueError("dense_f32_heads: the heads do not fit the rows")
     status = _status_word(x.device)
-    scratch = _f32_scratch(x, T * H, K)
+    scratch = _f32_scratch(x, T, K, 0, H)
     check(library().mi_dense_f32_batched(x.data_ptr() + 4 * x_col, _ptr(w), out.data_ptr() + 4 * out_col, T, N, K,
                                          lda, ldc, H, xs, N * K, os_, _ptr(scratch), _ptr(status), _stream()),
           "dense_f32_heads")
