@@ -17,15 +17,17 @@
 //
 // Weights are the M operand (128 rows a tile; 64 gate rows and the up rows of the same outputs in a paired product) and lie in
 // tensor memory, rows of activations are the N operand in shared memory.  Roles:
-//   warps 0-7 (tiles of 64 rows) or 0-11, four for a chunk, in turn: weights, ring -> three parts -> tensor memory
+//   warps 0-7 or (tiles of 16 rows) 0-11, four for a chunk, in turn: weights, ring -> three parts -> tensor memory
 //   warps 8-15 or 12-15  the sums of a chunk: tensor memory -> registers, added up
-//   warp 16     MMAs, 10 a chunk; tensor memory.  The activations' parts stand one behind the other, so that one MMA multiplies a
-//               part of the weights with two of them
-//   warp 17     weights: memory -> ring (TMA; without it, where rows are not aligned for it, the warps that read them ask
+//   warps 16, 17, chunks in turn: MMAs, 10 a chunk (a warp takes 800 cycles for one in a busy SM, twice the MMAs' own time), the
+//               others into sums of its own; warp 16 allocates tensor memory.  The activations' parts stand one behind the
+//               other, so that one MMA multiplies a part of the weights with two of them
+//   warp 18     weights: memory -> ring (TMA; without it, where rows are not aligned for it, the warps that read them ask
 //               for them with cp.async)
-//   tiles of 64 rows: warp 18 brings the parts of the activations, which f32_split_rows_kernel has laid out as they stand here
+//   tiles of 64 rows: warp 19 brings the parts of the activations, which f32_split_rows_kernel has laid out as they stand here
 //               (one plain copy a chunk; as boxes of rows of 64 bytes they held the tile up)
-//   tiles of 16 and 32: warps 18-21 bring the activations (cp.async, four chunks ahead) and take them apart in shared memory
+//   tiles of 16 and 32: warps 19-22, chunks in turn: activations, memory -> ring (cp.async, a warp's next two chunks ahead) ->
+//               three parts in shared memory
 // SPLIT: a cluster of 2 or 4 blocks shares a tile's parts and adds them up through distributed shared memory, where tiles
 // alone would leave SMs without work (a decode step's few rows).
 //
@@ -33,6 +35,8 @@
 #pragma once
 
 #include "tcgen05.cuh"
+
+#include <type_traits>
 
 namespace mi {
 namespace f32tc {
@@ -42,11 +46,11 @@ using namespace tc;
 constexpr int TC_MIN_K = 512;
 constexpr int FK = 32;                                 // k per chunk: 32 floats are a swizzled row of 128 bytes
 constexpr int PARTS = 4;
-constexpr int MMA_WARP = 16, W_WARP = 17, ROWS_WARP = 18;        // first warps of the roles
+constexpr int MMA_WARP = 16, W_WARP = 18, ROWS_WARP = 19;        // first warps of the roles
 constexpr bool split_before(int nt) { return nt >= 64; }
-constexpr int w_turns(int nt) { return split_before(nt) ? 2 : 3; }             // groups of four warps that take chunks of weights in turn
-constexpr int threads(int nt) { return 32 * (split_before(nt) ? 19 : 22); }
-constexpr int ROWS_AHEAD = 4;                          // chunks of activations asked for
+constexpr int w_turns(int nt) { return nt == 16 ? 3 : 2; }                   // groups of four warps that take chunks of weights in turn
+constexpr int threads(int nt) { return 32 * (split_before(nt) ? 20 : 23); }
+constexpr int ROWS_WARPS = 4, ROWS_AHEAD = 2;          // of tiles that bring the activations themselves; a warp's chunks asked for
 constexpr uint32_t SLOT_LIMIT = 65536;                 // bytes of part sums of a SPLIT block
 constexpr float UP = 16777216.f, DOWN = 1.f / (UP * UP);       // factors of operands and results
 // D float32, A and B bfloat16, both K-major, M = 128 (without N)
@@ -54,9 +58,9 @@ constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((128u >> 4) << 
 
 // Rings, in chunks: weights; parts of the activations (at most four: see the phases below); activations on their way, where the
 // block takes them apart; in tensor memory weights and sums of hh
-constexpr int w_slots(int nt, bool split) { return nt == 64 ? (split ? 4 : 6) : (split ? 6 : 9); }        // (a multiple of w_turns)
+constexpr int w_slots(int nt, bool split) { return nt == 64 ? (split ? 4 : 6) : w_turns(nt) == 3 || split ? 6 : 8; }       // (a multiple of w_turns)
 constexpr int ROW_SLOTS = 4;
-constexpr int raw_slots(int nt) { return split_before(nt) ? 0 : ROWS_AHEAD + 1; }
+constexpr int raw_slots(int nt) { return split_before(nt) ? 0 : ROWS_WARPS * ROWS_AHEAD; }
 constexpr int t_slots(int nt) { return nt == 64 ? 2 : 4; }
 inline size_t smem_bytes(int nt, int split) {
     return 1024 + (size_t)w_slots(nt, split > 1) * 16384 + (size_t)ROW_SLOTS * nt * 192 + (size_t)raw_slots(nt) * nt * 128 +
@@ -250,15 +254,15 @@ f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, Problem g) {
     constexpr int THREADS = threads(NT), W_SLOTS = w_slots(NT, SPLIT), RAW_SLOTS = raw_slots(NT), T_SLOTS = t_slots(NT);
     constexpr int TURNS = w_turns(NT), OUT_WARP = 4 * TURNS;
     static_assert(W_SLOTS % TURNS == 0, "a turn's own slots");
-    // columns of tensor memory: T_SLOTS chunks' hh; the others' two sums, of even and of odd parts; T_SLOTS chunks of weights
+    // columns of tensor memory: T_SLOTS chunks' hh; the others' two sums of either MMA warp; T_SLOTS chunks of weights
     constexpr int OTHERS_AT = 128, W_AT = 512 - T_SLOTS * 64;
     static_assert(T_SLOTS * NT <= OTHERS_AT && OTHERS_AT + 4 * NT <= W_AT, "tensor memory");
     constexpr int ROW_BYTES = NT * 192;                // a chunk's activations: [8 k][part][rows][16 bytes]
     constexpr int FEATS = PAIRED ? 64 : 128;           // outputs of a tile
     constexpr int OWN = NT / ((MMA_WARP - OUT_WARP) / 4);                  // rows of activations of an adding warp
-    constexpr int PER = NT / 16;                       // 16-byte pieces of activations per thread and chunk
+    constexpr int PER = NT / 4;                        // 16-byte pieces of activations per lane and chunk
     extern __shared__ uint8_t smem_raw[];
-    __shared__ uint64_t full_bar[4], done_bar[4], empty_bar[T_SLOTS], w_full[W_SLOTS], w_read[W_SLOTS], rows_full[ROW_SLOTS];
+    __shared__ uint64_t full_bar[4], done_bar[8], empty_bar[T_SLOTS], others_read, w_full[W_SLOTS], w_read[W_SLOTS], rows_full[ROW_SLOTS];
     __shared__ uint32_t tmem_base_s;
     __shared__ int abort_s;
 
@@ -290,8 +294,10 @@ f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, Problem g) {
 
     if (threadIdx.x == 0) {
         abort_s = 0;
-        for (int s = 0; s < 4; ++s) { mbar_init(&full_bar[s], BEFORE ? 4 : 8); mbar_init(&done_bar[s], 1); }
+        for (int s = 0; s < 4; ++s) mbar_init(&full_bar[s], BEFORE ? 4 : 5);
+        for (int s = 0; s < 8; ++s) mbar_init(&done_bar[s], 1);
         for (int s = 0; s < T_SLOTS; ++s) mbar_init(&empty_bar[s], MMA_WARP - OUT_WARP);
+        mbar_init(&others_read, MMA_WARP - OUT_WARP);
         for (int s = 0; s < ROW_SLOTS; ++s) mbar_init(&rows_full[s], 1);
         for (int s = 0; s < W_SLOTS; ++s) { mbar_init(&w_full[s], 1); mbar_init(&w_read[s], 4); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -307,8 +313,9 @@ f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, Problem g) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tmem_base_s;
 
-    // Phases of the barriers of four (full, done): whoever waits for chunk i there has itself to act before chunk i + 4
-    // can complete, so a parity never stands for the phase after the next.
+    // Phases of full and done: whoever waits for chunk i there has itself to act before chunk i + 4 can complete, so a parity never
+    // stands for the phase after the next.  Nor for the one before: done has eight barriers, since the two MMA warps' chunks complete
+    // in either order and a warp of the weights, which waits for every third chunk, then knows of all chunks eight before alone.
     if (warp < OUT_WARP) {
         const int turn = warp >> 2, quarter = warp & 3;
         // !VEC: this warp's 32 rows of chunk i, a row's lanes beside each other
@@ -357,7 +364,7 @@ f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, Problem g) {
                 if (lane == 0) mbar_arrive(&w_read[slot]);
             }
             // the MMAs of chunk i - T_SLOTS have read its place in tensor memory
-            if (i >= T_SLOTS && !wait_for(&done_bar[(i - T_SLOTS) & 3], ((i - T_SLOTS) >> 2) & 1, abort_flag, 32)) break;
+            if (i >= T_SLOTS && !wait_for(&done_bar[(i - T_SLOTS) & 7], ((i - T_SLOTS) >> 3) & 1, abort_flag, 32)) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             tmem_st16(at, h);
             tmem_st16(at + 16, m);
@@ -380,7 +387,7 @@ f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, Problem g) {
         int in_part = 0, parts = 0;
 #pragma unroll 1
         for (int it = 0; it < count; ++it) {
-            ok = wait_for(&done_bar[it & 3], (it >> 2) & 1, abort_flag, 37);
+            ok = wait_for(&done_bar[it & 7], (it >> 3) & 1, abort_flag, 37);
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             if (c_lo < n_mma) {                        // uniform
@@ -397,23 +404,40 @@ f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, Problem g) {
             __syncwarp();
             if (lane == 0) mbar_arrive(&empty_bar[it % T_SLOTS]);
             if (++in_part == per_part || it == count - 1) {
-                // The others' columns are written anew two parts on, by MMAs that wait for a chunk of the part between to be
-                // read here (a part that another follows has at least T_SLOTS chunks: inner sizes from 512 up).
+                // the others of both MMA warps, the next part's may follow
                 float* to = own + (SPLIT ? parts * 2 * NT * 128 : 0);
-                const uint32_t d = lane_addr + OTHERS_AT + (parts & 1) * 2 * NT;
+                constexpr int GROUP = OWN < 16 ? OWN : 16;
+                float others[OWN];
 #pragma unroll
-                for (int i0 = 0; i0 < OWN; i0 += 8) {
-                    uint32_t x[8], y[8];
-                    tmem_ld8(d + i0, x);
-                    tmem_ld8(d + n_mma + i0, y);
+                for (int i0 = 0; i0 < OWN; i0 += GROUP) {
+                    const uint32_t d = lane_addr + OTHERS_AT + i0;
+                    uint32_t x[GROUP], y[GROUP];
+                    if constexpr (GROUP == 16) { tmem_ld16(d, x); tmem_ld16(d + n_mma, y); }
+                    else { tmem_ld8(d, x); tmem_ld8(d + n_mma, y); }
                     wait_tmem_ld();
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        float *hh = to + (i0 + i) * 128, *others = hh + NT * 128, o = __uint_as_float(x[i]) + __uint_as_float(y[i]);
-                        if (!SPLIT && parts > 0) part[i0 + i] = *hh + part[i0 + i], o = *others + o;
-                        *hh = 0.f + part[i0 + i];      // (a cluster's sums begin at +0, too)
-                        *others = 0.f + o;
-                        part[i0 + i] = 0.f;
+                    for (int i = 0; i < GROUP; ++i) others[i0 + i] = __uint_as_float(x[i]) + __uint_as_float(y[i]);
+                    if constexpr (GROUP == 16) { tmem_ld16(d + 2 * NT, x); tmem_ld16(d + 2 * NT + n_mma, y); }
+                    else { tmem_ld8(d + 2 * NT, x); tmem_ld8(d + 2 * NT + n_mma, y); }
+                    wait_tmem_ld();
+#pragma unroll
+                    for (int i = 0; i < GROUP; ++i) others[i0 + i] += __uint_as_float(x[i]) + __uint_as_float(y[i]);
+                }
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&others_read);
+                const bool more = !SPLIT && parts > 0;
+#pragma unroll
+                for (int i0 = 0; i0 < 2 * OWN; i0 += GROUP) {                // hh, others
+                    const bool hh = i0 < OWN;
+                    float* at = to + (hh ? i0 : NT + i0 - OWN) * 128;
+                    float before[GROUP];               // (all loads ahead of the additions)
+#pragma unroll
+                    for (int i = 0; i < GROUP; ++i) before[i] = more ? at[i * 128] : 0.f;      // (a cluster's sums begin at +0, too)
+#pragma unroll
+                    for (int i = 0; i < GROUP; ++i) {
+                        at[i * 128] = before[i] + (hh ? part[i0 + i] : others[i0 - OWN + i]);
+                        if (hh) part[i0 + i] = 0.f;
                     }
                 }
                 in_part = 0;
@@ -425,37 +449,48 @@ f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, Problem g) {
 #pragma unroll
                 for (int i = 0; i < OWN; ++i) own[(parts * 2 * NT + i) * 128] = own[((parts * 2 + 1) * NT + i) * 128] = 0.f;
     } else if (warp < W_WARP) {
-        const uint32_t by_n = (uint32_t)(n_mma >> 3) << 17, idesc1 = IDESC | by_n, idesc2 = IDESC | 2 * by_n;
-        const uint64_t rows_desc = umma_desc_plain(smem_u32(rows_ring), 3 * part_bytes);
-        const uint32_t desc_lo = (uint32_t)rows_desc, desc_hi = (uint32_t)(rows_desc >> 32);
-        // room for the sums, rows (where no copy brings them: the room once more), weights (and rows)
-        auto ready = [&](int i) {
-            const uint32_t room = ((i / T_SLOTS) & 1) ^ 1;
-            return wait_for3(&empty_bar[i % T_SLOTS], room, BEFORE ? &rows_full[i % ROW_SLOTS] : &empty_bar[i % T_SLOTS],
-                             BEFORE ? (i / ROW_SLOTS) & 1 : room, &full_bar[i & 3], (i >> 2) & 1, abort_flag, 35);
-        };
-        int in_part = 0, odd = 0;
+        // The rows' number is a constant in here: with the operands formed from a variable one the warp took 450 cycles a chunk to
+        // give the products out, and more than that to wait for what was there.
+        auto give = [&](auto rows_c) {
+            constexpr uint32_t n = decltype(rows_c)::value, IDESC1 = IDESC | (n >> 3) << 17, IDESC2 = IDESC | (n >> 2) << 17;
+            constexpr uint32_t K_STEP = 6 * n;         // 16 k of rows; of weights 8 columns
+            const uint64_t rows_desc = umma_desc_plain(smem_u32(rows_ring), 48 * n);
+            const uint32_t desc_lo = (uint32_t)rows_desc, desc_hi = (uint32_t)(rows_desc >> 32);
+            const uint32_t t = __reduce_max_sync(0xffffffffu, tmem);       // (the same in all lanes also for the compiler)
+            // (every part has two chunks and more: inner sizes from 512 up)
+            int in_part = warp - MMA_WARP, parts = 0;
+            const uint32_t o1 = t + OTHERS_AT + in_part * 2 * NT;
 #pragma unroll 1
-        for (int i = 0; i < count && ready(i); ++i) {
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t bh = desc_lo + (i % ROW_SLOTS) * (ROW_BYTES >> 4), bm = bh + n_mma, bl = bm + n_mma;
-            const uint32_t k_step = 6 * n_mma;         // 16 k of rows; of weights 8 columns
-            const uint32_t wh = tmem + W_AT + (i % T_SLOTS) * 64, wm = wh + 16, wl = wm + 16;
-            const uint32_t hh = tmem + (i % T_SLOTS) * NT, o1 = tmem + OTHERS_AT + odd * 2 * NT, o2 = o1 + n_mma;
-            if (elect_one()) {
+            for (int i = in_part; i < count; i += 2) {
+                if (in_part < 2 && parts > 0 && !wait_for(&others_read, (parts - 1) & 1, abort_flag, 36)) break;
+                // room for the sums, rows (where no copy brings them: the room once more), weights (and rows)
+                const uint32_t room = ((i / T_SLOTS) & 1) ^ 1;
+                uint64_t* empty = &empty_bar[i % T_SLOTS];
+                if (!wait_for3(empty, room, BEFORE ? &rows_full[i % ROW_SLOTS] : empty, BEFORE ? (i / ROW_SLOTS) & 1 : room,
+                               &full_bar[i & 3], (i >> 2) & 1, abort_flag, 35)) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t bh = desc_lo + (i % ROW_SLOTS) * (ROW_BYTES >> 4), bm = bh + n, bl = bm + n;
+                const uint32_t wh = t + W_AT + (i % T_SLOTS) * 64, wm = wh + 16, wl = wm + 16, hh = t + (i % T_SLOTS) * NT;
+                if (elect_one()) {
 #pragma unroll
-                for (int k = 0; k < FK / 16; ++k) {
-                    umma_tmem_a(o1, wh + k * 8, bm + k * k_step, desc_hi, idesc2, in_part + k > 0);   // hm, hl
-                    umma_tmem_a(o1, wm + k * 8, bh + k * k_step, desc_hi, idesc2, 1);                 // mh, mm
-                    umma_tmem_a(o1, wl + k * 8, bh + k * k_step, desc_hi, idesc2, 1);                 // lh, lm
-                    umma_tmem_a(o2, wm + k * 8, bl + k * k_step, desc_hi, idesc1, 1);                 //     ml
-                    umma_tmem_a(hh, wh + k * 8, bh + k * k_step, desc_hi, idesc1, k > 0);
+                    for (int k = 0; k < FK / 16; ++k) {
+                        umma_tmem_a(o1, wh + k * 8, bm + k * K_STEP, desc_hi, IDESC2, in_part > 1 || k > 0);      // hm, hl
+                        umma_tmem_a(o1, wm + k * 8, bh + k * K_STEP, desc_hi, IDESC2, 1);                    // mh, mm
+                        umma_tmem_a(o1, wl + k * 8, bh + k * K_STEP, desc_hi, IDESC2, 1);                    // lh, lm
+                        umma_tmem_a(o1 + n, wm + k * 8, bl + k * K_STEP, desc_hi, IDESC1, 1);                //     ml
+                        umma_tmem_a(hh, wh + k * 8, bh + k * K_STEP, desc_hi, IDESC1, k > 0);
+                    }
+                    umma_commit(&done_bar[i & 7]);
                 }
-                umma_commit(&done_bar[i & 3]);
+                __syncwarp();
+                in_part += 2;
+                if (in_part >= per_part) in_part -= per_part, ++parts;
             }
-            __syncwarp();
-            if (++in_part == per_part) in_part = 0, odd ^= 1;
-        }
+        };
+        if (NT == 16 || n_mma == 16) give(std::integral_constant<uint32_t, 16>());
+        else if (NT == 32 || n_mma == 32) give(std::integral_constant<uint32_t, NT < 32 ? 16 : 32>());
+        else if (n_mma == 48) give(std::integral_constant<uint32_t, NT < 64 ? 16 : 48>());
+        else give(std::integral_constant<uint32_t, NT < 64 ? 16 : 64>());
     } else if (warp == W_WARP) {
         if (VEC && lane == 0) {
             const int row_w = (int)((blockIdx.z * g.sW) / g.K) + e * (PAIRED ? 2 : 1) * g.N + n0;          // (sW: whole rows)
@@ -480,7 +515,7 @@ f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, Problem g) {
 #pragma unroll 1
             for (; i < count; ++i) {
                 // the MMAs of chunk i - ROW_SLOTS have read its place
-                if (i >= ROW_SLOTS && !mbar_wait(&done_bar[i & 3], ((i - ROW_SLOTS) >> 2) & 1, abort_flag, 33)) break;
+                if (i >= ROW_SLOTS && !mbar_wait(&done_bar[(i - ROW_SLOTS) & 7], ((i - ROW_SLOTS) >> 3) & 1, abort_flag, 33)) break;
                 const int slot = i % ROW_SLOTS;
                 mbar_expect_tx(&rows_full[slot], bytes);
                 bulk_load(rows_ring + slot * ROW_BYTES, from + (int64_t)i * bytes, bytes, &rows_full[slot]);
@@ -489,17 +524,17 @@ f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, Problem g) {
                 for (uint32_t n = 0; n < WAIT_LIMIT && !mbar_try_wait(&rows_full[j % ROW_SLOTS], (j / ROW_SLOTS) & 1); ++n) {}
         }
     } else {
-        // this thread's pieces of a chunk are rows tid / 8 + 16 j at piece tid % 8; it alone reads what it asked for
-        const int tid = threadIdx.x - 32 * ROWS_WARP, piece = tid & 7, r_lo = tid >> 3;
-        const uint32_t pitch = (uint32_t)g.lda * 4u, raw_lane = tid * 16;
+        // a lane's pieces of a chunk are rows lane / 8 + 4 j at piece lane % 8; it alone reads what it asked for
+        const int own = warp - ROWS_WARP, piece = lane & 7, r_lo = lane >> 3;
+        const uint32_t pitch = (uint32_t)g.lda * 4u;
         const uint32_t rows_lane = (piece >> 1) * 3 * part_bytes + r_lo * 16 + (piece & 1) * 8;       // 8 bytes of each part
         uint32_t row_of[PER];
 #pragma unroll
         for (int j = 0; j < PER; ++j) {
-            const int r = r_lo + 16 * j;
+            const int r = r_lo + 4 * j;
             row_of[j] = r >= rows ? 0xffffffffu : g.gather ? (uint32_t)__ldg(g.gather + row0 + r) : (uint32_t)(row0 + r);
         }
-        const uint32_t raw_at = smem_u32(raw_ring) + raw_lane;
+        const uint32_t raw_at = smem_u32(raw_ring) + lane * 16;
         auto ask = [&](int i) {
             if (i < count) {
                 const int k = (first + i) * FK + piece * 4, left = g.K - k;
@@ -507,17 +542,17 @@ f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, Problem g) {
                 const uint32_t at = raw_at + (i % RAW_SLOTS) * (NT * 128);
 #pragma unroll
                 for (int j = 0; j < PER; ++j) {
-                    if (16 * j >= n_mma) break;        // uniform; no MMA reads these rows
+                    if (4 * j >= n_mma) break;         // uniform; no MMA reads these rows
                     const bool row = row_of[j] != 0xffffffffu;
                     const char* src = base + (uint64_t)row_of[j] * pitch;
                     if (VEC) {
                         const bool in = row && left > 0;
-                        cp_async16(at + j * 2048, in ? src : reinterpret_cast<const char*>(g.W), in);
+                        cp_async16(at + j * 512, in ? src : reinterpret_cast<const char*>(g.W), in);
                     } else {
 #pragma unroll
                         for (int x = 0; x < 4; ++x) {
                             const bool in = row && left > x;
-                            cp_async4(at + j * 2048 + 4 * x, in ? src + 4 * x : reinterpret_cast<const char*>(g.W), in);
+                            cp_async4(at + j * 512 + 4 * x, in ? src + 4 * x : reinterpret_cast<const char*>(g.W), in);
                         }
                     }
                 }
@@ -525,29 +560,29 @@ f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, Problem g) {
             asm volatile("cp.async.commit_group;" ::: "memory");
         };
 #pragma unroll 1
-        for (int i = 0; i < ROWS_AHEAD; ++i) ask(i);
+        for (int i = 0; i < ROWS_AHEAD; ++i) ask(own + i * ROWS_WARPS);
 #pragma unroll 1
-        for (int i = 0; i < count; ++i) {
-            ask(i + ROWS_AHEAD);                       // into the place of chunk i - 1, which this thread has read
-            asm volatile("cp.async.wait_group %0;" ::"n"(ROWS_AHEAD) : "memory");
+        for (int i = own; i < count; i += ROWS_WARPS) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(ROWS_AHEAD - 1) : "memory");
             // the MMAs of chunk i - ROW_SLOTS have read its place
-            if (i >= ROW_SLOTS && !wait_for(&done_bar[i & 3], ((i - ROW_SLOTS) >> 2) & 1, abort_flag, 33)) break;
-            const uint8_t* from = raw_ring + raw_lane + (i % RAW_SLOTS) * (NT * 128);
+            if (i >= ROW_SLOTS && !wait_for(&done_bar[(i - ROW_SLOTS) & 7], ((i - ROW_SLOTS) >> 3) & 1, abort_flag, 33)) break;
+            const uint8_t* from = raw_ring + lane * 16 + (i % RAW_SLOTS) * (NT * 128);
             uint8_t* to = rows_ring + rows_lane + (i % ROW_SLOTS) * ROW_BYTES;
 #pragma unroll
             for (int j = 0; j < PER; ++j) {
-                if (16 * j >= n_mma) break;
-                const uint4 v = *reinterpret_cast<const uint4*>(from + j * 2048);
+                if (4 * j >= n_mma) break;
+                const uint4 v = *reinterpret_cast<const uint4*>(from + j * 512);
                 uint2 h, m, l;
                 take_apart(v.x, v.y, h.x, m.x, l.x);
                 take_apart(v.z, v.w, h.y, m.y, l.y);
-                *reinterpret_cast<uint2*>(to + j * 256) = h;
-                *reinterpret_cast<uint2*>(to + j * 256 + part_bytes) = m;
-                *reinterpret_cast<uint2*>(to + j * 256 + 2 * part_bytes) = l;
+                *reinterpret_cast<uint2*>(to + j * 64) = h;
+                *reinterpret_cast<uint2*>(to + j * 64 + part_bytes) = m;
+                *reinterpret_cast<uint2*>(to + j * 64 + 2 * part_bytes) = l;
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
             if (lane == 0) mbar_arrive(&full_bar[i & 3]);
+            ask(i + ROWS_AHEAD * ROWS_WARPS);          // into the place of this chunk, which this lane has read
         }
         asm volatile("cp.async.wait_group 0;" ::: "memory");
     }
