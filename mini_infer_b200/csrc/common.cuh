@@ -201,6 +201,13 @@ void set_last_error(const char* fmt, ...);
 // Checks cudaGetLastError after a launcher queued `n_kernels` kernels and counts them.
 int finish_launch(const char* what, int n_kernels = 1);
 
+// Multiprocessors of the current device (0 where there is none).
+inline int sm_count() {
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+    return n;
+}
+
 }  // namespace mi
 
 // Dispatch helpers: run `BODY` with `AT`/`WT` bound to the C++ types of the codes.

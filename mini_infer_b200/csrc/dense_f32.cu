@@ -5,12 +5,16 @@
 // tokens share its step: the float32 path gives the same bits for every way of cutting and batching the
 // work.  (A library product picks other kernels, and other orders of summation, for other row counts.)
 //   K < 512    one chain of fused multiply-adds over k in ascending order, on the CUDA cores (f32_tiles.cuh)
-//   K >= 512   operands in two halves of 11 bits on the tensor cores, sums of 32 terms added in 32 bits (f32_tc.cuh).
-//              Off the 64-bit result by, relative to its norm, 1.5e-7 at K = 512, 1.5e-7 at 2048 and 1.7e-7 at 5632; the chain
-//              is off by 4.0e-7, 8.0e-7 and 1.3e-6.  Below 512 the chain is as near and the products are small.
-// No reduced-precision mode: this path exists to show faults that bfloat16 hides.
-// Against [6144, 2048] and [2048, 5632], chain and tensor cores: 1 row 29 and 20 us, 57 and 23; 32 rows 56 and 24, 69 and 28;
-// 512 rows 291 and 94 us (137 TFLOP/s), 330 and 82.
+//   K >= 512   operands taken apart exactly, into three bfloat16 numbers each, on the tensor cores; sums of 32 terms added in
+//              32 bits (f32_tc.cuh).
+// Off the 64-bit result, relative to its norm, here and as a chain: normal numbers 7.3e-8 and 4.0e-7 at K = 512, 9.9e-8 and 8.0e-7
+// at 2048, 1.4e-7 and 1.3e-6 at 5632; positive ones 6.1e-8 and 3.1e-7, 6.5e-8 and 6.1e-7, 7.8e-8 and 1.2e-6; rows of one number 2.5e-8 both
+// (a row of a single 1.0 gives the weight's bits), of 2 2.5e-8 and 3.1e-8, of 8 2.8e-8 and 5.5e-8, of 64 4.8e-8 and 1.4e-7; numbers
+// of 1e-41 1.8e-6 and 4.1e-5.
+// Times in us with a cold L2, tensor cores and chain.  Against [6144, 2048]: 1 row 24 and 30, 32 rows 27 and 58, 64 rows 42 and 95,
+// 512 rows 122 and 295 (106 TFLOP/s), 2,048 rows 402 and 1,011; against [2048, 5632]: 26 and 60, 30 and 73, 40 and 265, 99 and 336, 361 and 1,033.
+// The line at 512: there the two meet (against [2048, 512]: 1 row 12 and 11, 48 rows 21 and 30, 256 rows 32 and 28, 512 rows 30 and 38, 2,048
+// rows 79 and 105), and the tensor cores' four parts of the inner dimension need four chunks of 32 each.
 // The reference runs every dense product in FP16 through cuBLAS (src/layers/mlp.cpp:120-130).
 
 #include "f32_tc.cuh"
@@ -74,7 +78,7 @@ dense_f32_narrow_kernel(DenseF32 g) {
 // Which form: up to DF_NARROW_ROWS rows a product is bound by reading W, and the narrow tiles keep more of it in flight
 // (measured when larger inner sizes came here too: against [6144, 2048], narrow and wide: 16 rows 39 and 61 us, 32 rows 53 and 61, 48 rows 65 and 66; against [2048, 5632]:
 // 32 rows 66 and 163 us); above, wide tiles of 128 columns, or of 64 where those of 128 would leave SMs without one.
-constexpr int DF_NARROW_ROWS = 32, DF_SMS = 148;
+constexpr int DF_NARROW_ROWS = 32;
 
 static int dense_f32_launch(const DenseF32& g, int batch, bool vec, cudaStream_t stream, const char* what) {
     const int64_t tiles_y = ((int64_t)g.T + f32t::BM - 1) / f32t::BM;
@@ -86,7 +90,7 @@ static int dense_f32_launch(const DenseF32& g, int batch, bool vec, cudaStream_t
         return finish_launch(what);
     }
     const int64_t wide = tiles_y * ((g.N + 127) / 128) * batch;
-    const bool half = wide < DF_SMS;
+    const bool half = wide < sm_count();
     const int bn = half ? 64 : 128;
     const dim3 grid((g.N + bn - 1) / bn, (unsigned)tiles_y, batch);
     if (half) {
@@ -141,16 +145,23 @@ constexpr int64_t TC_SCRATCH_BYTES = 128ll << 20;
 static int64_t f32_tc_row_bytes(int K) { return 6ll * ((K + f32tc::FK - 1) / f32tc::FK * f32tc::FK); }
 // tiles of up to nt rows that n rows make at most
 static int64_t f32_tc_tiles(int64_t n, int groups, int nt) { return groups ? (n < n / nt + groups ? n : n / nt + groups) : (n + nt - 1) / nt; }
+// Rows of a tile at most.  Of 60 experts' rows, tiles of 16, 32 and 64 against [2 x 1408, 2048]: 8 rows each 268, 274 and 312 us, 13 rows 311,
+// 281 and 314, 17 rows 383, 285 and 319, 34 rows 610, 424 and 345.
+static int f32_tc_tile(int64_t rows, int groups, int wanted) {
+    if (wanted > 0) return wanted < 64 ? wanted : 64;
+    const int64_t few = groups ? 9ll * groups : 16, more = groups ? 20ll * groups : 32;
+    return rows <= few ? 16 : rows <= more ? 32 : 64;
+}
 // floats that the parts of `rows` rows of `batch` products each, or of `groups` experts together, take
-static int64_t f32_tc_scratch(int64_t rows, int K, int groups, int batch) {
-    if (rows <= 32) return 0;
+static int64_t f32_tc_scratch(int64_t rows, int K, int groups, int batch, int wanted) {
+    if (!f32tc::split_before(f32_tc_tile(rows, groups, wanted))) return 0;
     const int64_t own = f32_tc_row_bytes(K), most = TC_SCRATCH_BYTES / own / batch;
     int64_t all = rows + 16 * f32_tc_tiles(rows, groups, 64);
-    if (all > most) all = most > 64 ? most : 64;
+    if (all > most) all = most > 80 ? most : 80;
     return all * batch * (own / 4);
 }
 
-// `rows`: rows in all; `groups`: experts (0: a dense product).  `scratch`: f32_tc_scratch(rows, K, groups, batch) floats.
+// `rows`: rows in all; `groups`: experts (0: a dense product).  `scratch`: f32_tc_scratch(rows, K, groups, batch, form.nt) floats.
 template <bool PAIRED>
 static int f32_tc_launch(f32tc::Problem g, float* scratch, int rows, int groups, int batch, TcForm form, cudaStream_t stream,
                          const char* what) {
@@ -159,19 +170,21 @@ static int f32_tc_launch(f32tc::Problem g, float* scratch, int rows, int groups,
     const int64_t w_rows = groups ? groups * own_rows : (int64_t)(batch - 1) * (g.sW / g.K) + own_rows;
     const bool vec = g.K % 4 == 0 && g.lda % 4 == 0 && g.sA % 4 == 0 && (batch == 1 || (g.sW > 0 && g.sW % g.K == 0)) &&
                      w_rows < (1ll << 31) - 128 &&
-                     ((reinterpret_cast<uintptr_t>(g.A) | reinterpret_cast<uintptr_t>(g.W) | reinterpret_cast<uintptr_t>(scratch)) & 15) == 0;
+                     ((reinterpret_cast<uintptr_t>(g.A) | reinterpret_cast<uintptr_t>(g.W)) & 15) == 0;
+    const int sms = sm_count();
     const int64_t tiles_m = PAIRED ? (g.N + 63) / 64 : (g.N + 127) / 128;
     if (batch > 65535) { set_last_error("%s: %d products exceed the grid limit", what, batch); return kBadShape; }
-    int nt = !vec ? 32 : form.nt > 64 ? 64 : form.nt > 0 ? form.nt : rows <= 16 ? 16 : rows <= 32 ? 32 : 64;
+    int nt = f32_tc_tile(rows, groups, form.nt);
+    if (!vec && nt < 32) nt = 32;
     // rows of a launch: what the scratch holds (16 rows more for a tile), or the grid
     int64_t band = 65535ll * nt;
     if (f32tc::split_before(nt)) {
-        const int64_t room = f32_tc_scratch(rows, g.K, groups, batch) / (f32_tc_row_bytes(g.K) / 4) / batch;
+        const int64_t room = f32_tc_scratch(rows, g.K, groups, batch, form.nt) / (f32_tc_row_bytes(g.K) / 4) / batch;
         band = rows;
         while (band > 0 && band + 16 * f32_tc_tiles(band, groups, nt) > room) band = band / 2 / 64 * 64;
-        if (band == 0) nt = 32, band = 65535ll * nt;   // (rows that are too long, or too many experts)
+        if (band == 0) nt = 32, band = 65535ll * nt;   // (rows that are too long, or too many experts or products)
     }
-    if (f32tc::split_before(nt) && !scratch) { set_last_error("%s: no room for the rows' parts", what); return kBadShape; }
+    if (f32tc::split_before(nt) && (!scratch || (reinterpret_cast<uintptr_t>(scratch) & 15))) { set_last_error("%s: no room for the rows' parts", what); return kBadShape; }
     TcLaunch l = {};
     l.stream = stream;
     l.what = what;
@@ -193,18 +206,20 @@ static int f32_tc_launch(f32tc::Problem g, float* scratch, int rows, int groups,
             // Up to four blocks share a tile where tiles alone leave SMs without work: one row against [6144, 2048] 28 us, by two
             // 19, by four 22; against [2048, 2048] 28, 18 and 13; against [2048, 5632] 68, 38 and 23 (by eight 15 and 26).
             l.split = 1;
-            while (l.split < f32tc::PARTS && 2 * l.split * tiles_m * tiles_y * batch <= DF_SMS) l.split *= 2;
+            while (l.split < f32tc::PARTS && 2 * l.split * tiles_m * tiles_y * batch <= sms) l.split *= 2;
         }
         if (!vec) l.split = 1;
         while (l.split > 1 && l.split < f32tc::PARTS && (f32tc::PARTS / l.split) * 2 * nt * 512u > f32tc::SLOT_LIMIT) l.split *= 2;
         l.grid = dim3((unsigned)(tiles_m * l.split), (unsigned)tiles_y, (unsigned)batch);
         if (f32tc::split_before(nt)) {
             g.parts = (uint8_t*)scratch;
-            f32tc::f32_split_rows_kernel<<<dim3(tiles_y, (g.K + f32tc::SPLIT_K - 1) / f32tc::SPLIT_K, batch), 256, 0, stream>>>(g, nt);
+            auto split_rows = vec ? f32tc::f32_split_rows_kernel<true> : f32tc::f32_split_rows_kernel<false>;
+            split_rows<<<dim3((unsigned)tiles_y, (g.K + f32tc::SPLIT_K - 1) / f32tc::SPLIT_K, batch), 256, 0, stream>>>(g, nt);
             const int rc = finish_launch(what);
             if (rc != kOk) return rc;
         }
-        const int rc = !vec ? f32_tc_launch_one<PAIRED, 32, false, false>(g, l)
+        const int rc = !vec && nt == 64 ? f32_tc_launch_one<PAIRED, 64, false, false>(g, l)
+                     : !vec ? f32_tc_launch_one<PAIRED, 32, false, false>(g, l)
                      : nt == 16 ? f32_tc_launch_nt<PAIRED, 16>(g, l)
                      : nt == 32 ? f32_tc_launch_nt<PAIRED, 32>(g, l) : f32_tc_launch_nt<PAIRED, 64>(g, l);
         if (rc != kOk) return rc;
@@ -216,9 +231,10 @@ static int f32_tc_launch(f32tc::Problem g, float* scratch, int rows, int groups,
 
 extern "C" int mi_f32_tc_min_inner() { return mi::f32tc::TC_MIN_K; }
 
-// Floats of scratch (16-byte aligned) that a product of `rows` rows, of `groups` experts or (0) in each of `batch` products, takes.
-extern "C" int64_t mi_f32_tc_scratch(int64_t rows, int K, int groups, int batch) {
-    return K >= mi::f32tc::TC_MIN_K && rows > 0 && batch > 0 ? mi::f32_tc_scratch(rows, K, groups, batch) : 0;
+// Floats of scratch (16-byte aligned) that a product of `rows` rows, of `groups` experts or (0) in each of `batch` products, takes;
+// nt: rows per tile, or -1 (mi_f32_tc_form).
+extern "C" int64_t mi_f32_tc_scratch(int64_t rows, int K, int groups, int batch, int nt) {
+    return K >= mi::f32tc::TC_MIN_K && rows > 0 && batch > 0 ? mi::f32_tc_scratch(rows, K, groups, batch, nt) : 0;
 }
 
 // `batch` products at once: C_b[T, N] = A_b[T, K] . W_b[N, K]^T with rows of A and C `lda` and `ldc` floats

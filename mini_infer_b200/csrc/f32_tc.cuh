@@ -218,10 +218,11 @@ __device__ __forceinline__ int64_t tile_at(const Problem& g, int z, int slots, i
     return ((int64_t)z * (g.row_end - g.row_begin + 16 * slots) + (row0 - g.row_begin) + 16 * slot) * chunks * (FK * 6);
 }
 
-// The parts of a tile's rows of activations, zeros from K (a multiple of 4) to the end of its chunk.  Grouped: rows that no expert
-// has are not read (`gather` need not be written there).  A warp's lanes are 32 rows: 32 bytes of each are read, 512 bytes of
-// a part written.
+// The parts of a tile's rows of activations, zeros from K to the end of its chunk.  Grouped: rows that no expert has are not read
+// (`gather` need not be written there).  A warp's lanes are 32 rows: 32 bytes of each are read, 512 bytes of a part written.
+// VEC: rows are 16-byte aligned, K is a multiple of 4.
 constexpr int SPLIT_K = 64;                            // k of a block: 8 warps x 8
+template <bool VEC>
 __global__ void __launch_bounds__(256)
 f32_split_rows_kernel(Problem g, int nt) {
     const int k = blockIdx.y * SPLIT_K + (threadIdx.x >> 5) * 8, chunks = (g.K + FK - 1) / FK;
@@ -231,8 +232,16 @@ f32_split_rows_kernel(Problem g, int nt) {
     uint4* to = reinterpret_cast<uint4*>(g.parts + tile_at(g, blockIdx.z, gridDim.x, blockIdx.x, row0, chunks)) + (int64_t)(k / 8) * 3 * n;
     for (int r = threadIdx.x & 31; r < rows; r += 32) {
         const int64_t row = g.gather ? __ldg(g.gather + row0 + r) : row0 + r;
-        const uint4* src = reinterpret_cast<const uint4*>(g.A + blockIdx.z * g.sA + row * g.lda + k);
-        const uint4 none = make_uint4(0u, 0u, 0u, 0u), a = k < g.K ? __ldg(src) : none, b = k + 4 < g.K ? __ldg(src + 1) : none;
+        const float* src = g.A + blockIdx.z * g.sA + row * g.lda + k;
+        uint4 a = make_uint4(0u, 0u, 0u, 0u), b = a;
+        if (VEC) {
+            if (k < g.K) a = __ldg(reinterpret_cast<const uint4*>(src));
+            if (k + 4 < g.K) b = __ldg(reinterpret_cast<const uint4*>(src) + 1);
+        } else {
+            auto at = [&](int x) { return k + x < g.K ? __float_as_uint(__ldg(src + x)) : 0u; };
+            a = make_uint4(at(0), at(1), at(2), at(3));
+            b = make_uint4(at(4), at(5), at(6), at(7));
+        }
         uint4 h, m, l;
         take_apart(a.x, a.y, h.x, m.x, l.x);
         take_apart(a.z, a.w, h.y, m.y, l.y);
@@ -244,13 +253,13 @@ f32_split_rows_kernel(Problem g, int nt) {
     }
 }
 
-// NT: rows of activations per tile at most.  VEC: rows are 16-byte aligned, K is a multiple of 4 and `map_w` describes all
-// rows of W (boxes of 32 floats x 128 rows, 64 in a paired product, 128-byte swizzle).
+// NT: rows of activations per tile at most.  VEC: rows (of weights, and of activations that the block brings itself) are 16-byte
+// aligned, K is a multiple of 4 and `map_w` describes all rows of W (boxes of 32 floats x 128 rows, 64 in a paired product,
+// 128-byte swizzle).
 template <bool PAIRED, int NT, bool SPLIT, bool VEC>
 __global__ void __launch_bounds__(threads(NT), 1)
 f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, Problem g) {
     constexpr bool BEFORE = split_before(NT);
-    static_assert(!BEFORE || VEC, "rows that are split before are aligned");
     constexpr int THREADS = threads(NT), W_SLOTS = w_slots(NT, SPLIT), RAW_SLOTS = raw_slots(NT), T_SLOTS = t_slots(NT);
     constexpr int TURNS = w_turns(NT), OUT_WARP = 4 * TURNS;
     static_assert(W_SLOTS % TURNS == 0, "a turn's own slots");

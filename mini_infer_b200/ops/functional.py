@@ -795,8 +795,9 @@ def f32_tc_form(a: torch.Tensor, gather: Optional[torch.Tensor], w: torch.Tensor
                 out: torch.Tensor, n_rows: int, swiglu_pair: bool, glu=None, row_scale: Optional[torch.Tensor] = None,
                 rows_per_tile: int = -1, blocks_per_tile: int = -1) -> torch.Tensor:
     """:func:`grouped_gemm_plain` (without ``offsets``: :func:`dense_f32`, also paired) of float32 operands with an inner size from
-    ``mi_f32_tc_min_inner()`` up, into ``out``: tensor cores, every operand as two numbers of 11 bits.  All forms
-    (``rows_per_tile`` 16, 32, 64, 128; ``blocks_per_tile`` 1, 2, 4; -1: chosen by the sizes) give the same bits."""
+    ``mi_f32_tc_min_inner()`` up, into ``out``: tensor cores, every operand as the exact sum of three
+    bfloat16 numbers.  All forms (``rows_per_tile`` 16, 32, 64, or more, which is taken as 64; ``blocks_per_tile`` 1, 2, 4;
+    -1: chosen by the sizes) give the same bits."""
     global _tc_pending
     _chk(a, "f32_tc a", F32)
     n_rows, Kd = int(n_rows), a.shape[1]
@@ -809,7 +810,7 @@ def f32_tc_form(a: torch.Tensor, gather: Optional[torch.Tensor], w: torch.Tensor
     if offsets is None and (a if gather is None else gather).shape[0] < n_rows:
         raise ValueError(f"f32_tc: the input has fewer than {n_rows} rows")
     status = _status_word(a.device)
-    scratch = _f32_scratch(a, n_rows, Kd, E)
+    scratch = _f32_scratch(a, n_rows, Kd, E, 1, int(rows_per_tile))
     check(library().mi_f32_tc_form(_ptr(a), _ptr(gather), _ptr(w), _ptr(offsets), _ptr(out), n_rows, E, nout, Kd,
                                    1 if swiglu_pair else 0, int(rows_per_tile), int(blocks_per_tile), *_glu_args(glu),
                                    _row_scale(row_scale, n_rows, swiglu_pair, "grouped_gemm_plain"),
@@ -818,11 +819,12 @@ def f32_tc_form(a: torch.Tensor, gather: Optional[torch.Tensor], w: torch.Tensor
     return out
 
 
-def _f32_scratch(x: torch.Tensor, rows: int, K: int, experts: int = 0, products: int = 1) -> Optional[torch.Tensor]:
+def _f32_scratch(x: torch.Tensor, rows: int, K: int, experts: int = 0, products: int = 1,
+                 rows_per_tile: int = -1) -> Optional[torch.Tensor]:
     """Room for the parts of the rows of float32 products on tensor cores (None where they take none): ``rows`` of all experts, or of
     each of several products.  The caller holds it until the product is queued: a block that is given back before may be given out
     again, and written, ahead of it."""
-    n = library().mi_f32_tc_scratch(rows, K, experts, products)
+    n = library().mi_f32_tc_scratch(rows, K, experts, products, rows_per_tile)
     return torch.empty(n, dtype=F32, device=x.device) if n else None
 
 

@@ -122,7 +122,7 @@ _OTHERS = {
     "mi_qkv_skinny_supported": ([I, I, I], c_int),
     "mi_dense_skinny_max_rows": ([], c_int),
     "mi_f32_tc_min_inner": ([], c_int),
-    "mi_f32_tc_scratch": ([L, I, I, I], c_int64),
+    "mi_f32_tc_scratch": ([L, I, I, I, I], c_int64),
     "mi_delta_scan_prep_row": ([I], c_int),
     "mi_delta_blocks_supported": ([I], c_int),
     "mi_delta_blocks_mats": ([], c_int),
