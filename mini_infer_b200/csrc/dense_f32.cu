@@ -75,9 +75,10 @@ dense_f32_narrow_kernel(DenseF32 g) {
         if (r + i < rows) C[(int64_t)(row0 + r + i) * g.ldc + n] = acc[0][i];
 }
 
-// Which form: up to DF_NARROW_ROWS rows a product is bound by reading W, and the narrow tiles keep more of it in flight
-// (measured when larger inner sizes came here too: against [6144, 2048], narrow and wide: 16 rows 39 and 61 us, 32 rows 53 and 61, 48 rows 65 and 66; against [2048, 5632]:
-// 32 rows 66 and 163 us); above, wide tiles of 128 columns, or of 64 where those of 128 would leave SMs without one.
+// Which form: up to DF_NARROW_ROWS rows a product is bound by reading W, and the narrow tiles keep more of it in flight; above,
+// wide tiles of 128 columns, or of 64 where those of 128 would leave SMs without one.  Narrow and wide in us: 32 rows against
+// [6144, 256] 14 and 18, [2048, 480] 12 and 27, [512, 384] 10 and 23; 64 rows 21 and 18, 16 and 29, 10 and 23; 256 rows 53 and 33, 39 and 27,
+// 14 and 23: at 32 rows the narrow tiles are faster for any number of columns, further on only for few.
 constexpr int DF_NARROW_ROWS = 32;
 
 static int dense_f32_launch(const DenseF32& g, int batch, bool vec, cudaStream_t stream, const char* what) {
@@ -203,8 +204,8 @@ static int f32_tc_launch(f32tc::Problem g, float* scratch, int rows, int groups,
         g.row_end = (int)r0 + n;
         l.split = form.split;
         if (l.split < 0) {
-            // Up to four blocks share a tile where tiles alone leave SMs without work: one row against [6144, 2048] 28 us, by two
-            // 19, by four 22; against [2048, 2048] 28, 18 and 13; against [2048, 5632] 68, 38 and 23 (by eight 15 and 26).
+            // Up to four blocks share a tile where tiles alone leave SMs without work.  By one, two and four blocks, us: one row against
+            // [6144, 2048] 31, 23, 29; [2048, 2048] 29, 21, 16; [2048, 5632] 62, 37, 25; 32 rows 35, 27, 33; 35, 25, 19; 76, 45, 29.
             l.split = 1;
             while (l.split < f32tc::PARTS && 2 * l.split * tiles_m * tiles_y * batch <= sms) l.split *= 2;
         }

@@ -1026,9 +1026,9 @@ grouped_f32_narrow_kernel(GroupedF32 g) {
     }
 }
 
-// Narrow tiles up to so many rows per expert on average: there a product is bound by reading the experts' weights (then 60 of
-// [2 x 1408, 2048], narrow and wide: 8 rows each 407 and 640 us, 12 rows 433 and 643; with 17 and more a second narrow tile
-// is needed: 20 rows each 790 and 650 us).
+// Narrow tiles up to so many rows per expert on average: there a product is bound by reading the experts' weights (60 of
+// [2 x 704, 480], narrow and wide: 4 rows each 59 and 98 us, 12 rows 74 and 113, 16 rows 78 and 100, 20 rows 123 and 123, 32 rows 137 and 125;
+// with 17 and more an expert needs a second narrow tile, and of an average of 12 few experts have them).
 constexpr int GF_NARROW_ROWS = 12;
 
 template <int MODE>
