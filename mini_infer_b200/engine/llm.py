@@ -77,6 +77,12 @@ class GPUExecutor:
         self._drop_ahead()
         self.runner.release(rid)
 
+    def _sample(self, logits: torch.Tensor, requests: Sequence[Request], ahead: int) -> int:
+        """Queue the sampling of a token for each request, and with it the check of what was replayed since the last."""
+        waits, self.runner.waits_unchecked = self.runner.waits_unchecked, False
+        return self.sampler.launch(logits, [r.params for r in requests], [r.stream for r in requests],
+                                   [len(r.generated) + ahead for r in requests], waits)
+
     def run(self, entries: Sequence[StepEntry], sample_for: Sequence[Request],
             lookahead: bool = False) -> Dict[Hashable, int]:
         rids = [r.rid for r in sample_for]
@@ -99,16 +105,14 @@ class GPUExecutor:
             if not sample_for:
                 return {}
             assert [rid for rid, _ in res.index] == rids
-            handle = self.sampler.launch(res.logits, [r.params for r in sample_for],
-                                         [r.stream for r in sample_for], [len(r.generated) for r in sample_for])
+            handle = self._sample(res.logits, sample_for, 0)
         if lookahead and self.runner.can_step_ahead(rids):
             try:
                 logits = self.runner.step_ahead(rids, self.sampler.device_tokens(handle))
             except OutOfPages:
                 pass                # the scheduler decides what makes room
             else:
-                nxt = self.sampler.launch(logits, [r.params for r in sample_for], [r.stream for r in sample_for],
-                                          [len(r.generated) + 1 for r in sample_for])
+                nxt = self._sample(logits, sample_for, 1)
                 note = self.observer.after_forward(rids, [1] * len(rids), logits) if self.observer is not None else None
                 self._ahead = (rids, nxt, None, note)
         toks = self.sampler.fetch(handle)

@@ -145,6 +145,7 @@ class ModelRunner:
         self._launches_follow_context = any(getattr(p, "launches_follow_context", False) for p in model.all_parts())
         self._graph_pool = None
         self.graph_replays = 0
+        self.waits_unchecked = False        # a replay since the last check held kernels with bounded waits
         self.graph_kernel_launches = 0      # kernels of this library launched through graph replays
 
     # ------------------------------------------------------------------ #
@@ -432,14 +433,16 @@ class ModelRunner:
             torch.cuda.synchronize(self.rt.device)
             if self._graph_pool is None:
                 self._graph_pool = torch.cuda.graph_pool_handle()
+            from ..ops.functional import tc_launches
             from ..ops.library import launch_count
-            before = launch_count()
+            before, waits = launch_count(), tc_launches()
             g = torch.cuda.CUDAGraph()
             with torch.cuda.graph(g, pool=self._graph_pool):
                 out = self.model.forward(ctx, logit_rows)
-            self._graphs[key] = (g, out, launch_count() - before, [p.side_outputs() for p in parts])
-        g, out, kernels, side = self._graphs[key]
+            self._graphs[key] = (g, out, launch_count() - before, [p.side_outputs() for p in parts], tc_launches() > waits)
+        g, out, kernels, side, waits = self._graphs[key]
         g.replay()
+        self.waits_unchecked |= waits
         for p, outputs in zip(parts, side):
             if outputs is not None:
                 p.adopt_side_outputs(outputs)
@@ -451,6 +454,8 @@ class ModelRunner:
 
     @torch.no_grad()
     def step(self, entries: Sequence[StepEntry]) -> StepResult:
+        """Run one step.  A pass that is replayed is not waited for: if it holds kernels with bounded waits, ``waits_unchecked`` is
+        set, and who reads the results next reads ``ops.functional.wait_status`` with them (the sampler does)."""
         decode_graph = self._graph_eligible(entries)
         ctx, logit_rows, index = self.prepare(entries, pad_to=self._graph_batch(len(entries)) if decode_graph else 0)
         # What a failed step wrote into the paged caches lies beyond every request's committed tokens and

@@ -379,7 +379,6 @@ def prefill_attention_tc(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.
     scaled score becomes ``softcap * tanh(score / softcap)``; ``sink``: the softmax counts one key more, of
     score 0 and without a value; ``chunk``, ``sink_score``, ``gate``: as in :func:`attention_mix`.  Call
     :func:`check_tc_status` after the step: a wait inside the kernel that ran out is reported there."""
-    global _tc_pending
     _chk(q, "prefill_attention_tc q", BF16)
     T, nh, d = q.shape
     _chk(k_cache, "prefill_attention_tc k_cache", BF16)
@@ -409,7 +408,7 @@ def prefill_attention_tc(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.
                                        *_attn_form("prefill_attention_tc", nh, T, int(window), bool(sink), int(chunk),
                                                    sink_score, gate, gate_col), _stream()),
           "prefill_attention_tc")
-    _tc_pending = True
+    _tc_launched()
     return out
 
 
@@ -424,7 +423,6 @@ def prefill_attention_tc_logistic(q: torch.Tensor, k_cache: torch.Tensor, v_cach
     head_bias[h])`` by itself, not normalised over the keys (what :func:`attention_mix` computes with
     ``head_bias``).  bfloat16; key and value heads of 64 or 128 numbers each, not necessarily alike.  Returns
     ``[T, nh, dv]``.  Call :func:`check_tc_status` after the step."""
-    global _tc_pending
     _chk(q, "prefill_attention_tc_logistic q", BF16)
     T, nh, dk = q.shape
     _chk(k_cache, "prefill_attention_tc_logistic k_cache", BF16, (None, None, None, dk))
@@ -448,7 +446,7 @@ def prefill_attention_tc_logistic(q: torch.Tensor, k_cache: torch.Tensor, v_cach
                                                 nh, nkv, dk, dv, page_size, num_pages, max_pages, int(window),
                                                 float(scale), _ptr(head_bias), _stream()),
           "prefill_attention_tc_logistic")
-    _tc_pending = True
+    _tc_launched()
     return out
 
 
@@ -463,7 +461,6 @@ def prefill_attention_tc_shared(q: torch.Tensor, cache: torch.Tensor, block_tabl
     ``value_dim`` numbers of its key rows: ``q [T, H, dk]``, ``cache [pages, 1, page_size, dk]``, result
     ``[T, H, value_dim]``.  The rows of a query tile are (query, head) pairs, so a tile of keys is fetched once
     for all heads.  Sizes: :func:`prefill_attention_tc_shared_supported`."""
-    global _tc_pending
     _chk(q, "prefill_attention_tc_shared q", BF16)
     T, H, dk = q.shape
     _chk(cache, "prefill_attention_tc_shared cache", BF16, (None, 1, None, dk))
@@ -484,7 +481,7 @@ def prefill_attention_tc_shared(q: torch.Tensor, cache: torch.Tensor, block_tabl
                                               int(value_dim), page_size, num_pages, max_pages, int(window),
                                               float(scale), int(keep_first), _stream()),
           "prefill_attention_tc_shared")
-    _tc_pending = True
+    _tc_launched()
     return out
 
 
@@ -798,7 +795,6 @@ def f32_tc_form(a: torch.Tensor, gather: Optional[torch.Tensor], w: torch.Tensor
     ``mi_f32_tc_min_inner()`` up, into ``out``: tensor cores, every operand as the exact sum of three
     bfloat16 numbers.  All forms (``rows_per_tile`` 16, 32, 64, or more, which is taken as 64; ``blocks_per_tile`` 1, 2, 4;
     -1: chosen by the sizes) give the same bits."""
-    global _tc_pending
     _chk(a, "f32_tc a", F32)
     n_rows, Kd = int(n_rows), a.shape[1]
     _chk(w, "f32_tc w", F32, (None, Kd) if offsets is None else (None, None, Kd))
@@ -815,7 +811,7 @@ def f32_tc_form(a: torch.Tensor, gather: Optional[torch.Tensor], w: torch.Tensor
                                    1 if swiglu_pair else 0, int(rows_per_tile), int(blocks_per_tile), *_glu_args(glu),
                                    _row_scale(row_scale, n_rows, swiglu_pair, "grouped_gemm_plain"),
                                    _ptr(scratch), _ptr(status), _stream()), "f32_tc")
-    _tc_pending = True
+    _tc_launched()
     return out
 
 
@@ -832,7 +828,6 @@ def dense_f32(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
     """``x @ w.T`` in true float32 (``x [T, K]``, ``w [N, K]``): the additions of an output element and their order follow from
     ``K`` alone (one chain of fused multiply-adds over ``k``, or from ``mi_f32_tc_min_inner()`` on chunks of 32), so a
     row's result does not depend on how many rows there are.  The dense product of the float32 path."""
-    global _tc_pending
     _chk(x, "dense_f32 x", F32)
     T, K = x.shape
     _chk(w, "dense_f32 w", F32, (None, K))
@@ -841,7 +836,8 @@ def dense_f32(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
     status = _status_word(x.device)
     scratch = _f32_scratch(x, T, K)
     check(library().mi_dense_f32(_ptr(x), _ptr(w), _ptr(out), T, N, K, _ptr(scratch), _ptr(status), _stream()), "dense_f32")
-    _tc_pending = _tc_pending or K >= library().mi_f32_tc_min_inner()
+    if K >= library().mi_f32_tc_min_inner():
+        _tc_launched()
     return out
 
 
@@ -1029,6 +1025,19 @@ def _row_scale(row_scale: Optional[torch.Tensor], rows: int, swiglu_pair: bool, 
 
 _tc_status = {}
 _tc_pending = False
+_tc_launches = 0
+
+
+def _tc_launched() -> None:
+    global _tc_pending, _tc_launches
+    _tc_pending = True
+    _tc_launches += 1
+
+
+def tc_launches() -> int:
+    """How many kernels with bounded waits this process has launched, or recorded into a graph: a pass during whose capture the
+    number grew holds such kernels, and each of its replays has to be checked too (:func:`wait_status`)."""
+    return _tc_launches
 
 
 def _status_word(dev: torch.device) -> torch.Tensor:
@@ -1051,7 +1060,6 @@ def grouped_gemm_tc(a_sorted: torch.Tensor, w: torch.Tensor, offsets: torch.Tens
     kernel's forms (``TC_FORMS``: one block per tile with row tiles of 128 or 256, persistent with
     row tiles of 160 or 256); the library chooses by the rows per expert when it is None.
     """
-    global _tc_pending
     _chk(a_sorted, "grouped_gemm_tc a", BF16)
     n_rows, Kd = a_sorted.shape
     _chk(w, "grouped_gemm_tc w", BF16, (None, None, Kd))
@@ -1069,7 +1077,7 @@ def grouped_gemm_tc(a_sorted: torch.Tensor, w: torch.Tensor, offsets: torch.Tens
                                             -1 if form is None else int(form), *_glu_args(glu),
                                             _row_scale(row_scale, n_rows, swiglu_pair, "grouped_gemm_tc"), _stream()),
           "grouped_gemm_tc")
-    _tc_pending = True
+    _tc_launched()
     return out
 
 
@@ -1083,6 +1091,22 @@ def grouped_gemm_tc_inject_wait_fault(skip_k_block: int, wait_limit: int) -> Non
     lib.mi_grouped_gemm_tc_test_fault(int(skip_k_block), int(wait_limit))
 
 
+def wait_status(dev: torch.device) -> torch.Tensor:
+    """The word of :func:`_status_word`, for a caller that reads it behind its own synchronisation (a replayed pass runs none of the
+    launchers here, so :func:`check_tc_status` does not know of it); :func:`raise_wait_status` if it is not zero."""
+    return _status_word(dev)
+
+
+def raise_wait_status(dev: torch.device, code: int) -> None:
+    _status_word(dev).zero_()
+    from .library import KernelError
+    raise KernelError(f"tcgen05 kernel on {dev}: a wait ran out (code {code}; grouped product: "
+                      f"1 = producer waiting for a free stage, 2 = MMA waiting for data, "
+                      f"3 = epilogue waiting for the accumulators; prefill attention: 11-19; float32 product: 31 = weights, "
+                      f"32 = their place in tensor memory, 33 = place of the activations, 34 = place of the weights, 35 and 36 = MMA "
+                      f"waiting for operands or read sums, 37 = sums); results of that step are invalid")
+
+
 def check_tc_status() -> None:
     """Raise if a bounded wait inside a tensor-core kernel gave up since the last check (synchronises
     only when such a kernel was launched)."""
@@ -1093,12 +1117,7 @@ def check_tc_status() -> None:
     for dev, st in _tc_status.items():
         code = int(st.item())
         if code:
-            st.zero_()
-            from .library import KernelError
-            raise KernelError(f"tcgen05 kernel on {dev}: a wait ran out (code {code}; grouped product: "
-                              f"1 = producer waiting for a free stage, 2 = MMA waiting for data, "
-                              f"3 = epilogue waiting for the accumulators; prefill attention: 11-19); "
-                              f"results of that step are invalid")
+            raise_wait_status(dev, code)
 
 
 def random_fill(out: torch.Tensor, key: Tuple[int, int], scale: float, offset: float) -> torch.Tensor:
@@ -2088,7 +2107,6 @@ def dense_f32_heads(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor
     ``[T, *]`` float32 rows in which head ``h`` starts at column ``x_col + h * x_head_stride`` (default: heads
     of ``K`` side by side); ``out`` likewise (default ``[T, H * N]``).  The same fixed chain of additions per
     element as :func:`dense_f32`."""
-    global _tc_pending
     _chk(x, "dense_f32_heads x", F32)
     _chk(w, "dense_f32_heads w", F32)
     H, N, K = w.shape
@@ -2107,7 +2125,8 @@ def dense_f32_heads(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor
     check(library().mi_dense_f32_batched(x.data_ptr() + 4 * x_col, _ptr(w), out.data_ptr() + 4 * out_col, T, N, K,
                                          lda, ldc, H, xs, N * K, os_, _ptr(scratch), _ptr(status), _stream()),
           "dense_f32_heads")
-    _tc_pending = _tc_pending or K >= library().mi_f32_tc_min_inner()
+    if K >= library().mi_f32_tc_min_inner():
+        _tc_launched()
     return out
 
 
@@ -2294,7 +2313,6 @@ def prefill_attention_tc_unfolded(q: torch.Tensor, kv: torch.Tensor, k_rot: torc
     _chk(kv_len, "prefill_attention_tc_unfolded kv_len", I32, (B,))
     _chk(out, "prefill_attention_tc_unfolded out", BF16, (T, H * value_dim))
     _chk(gate, "prefill_attention_tc_unfolded gate", F32, (T, None))
-    global _tc_pending
     dev = q.device
     if dev not in _tc_status:
         _tc_status[dev] = torch.zeros(1, dtype=I32, device=dev)
@@ -2307,7 +2325,7 @@ def prefill_attention_tc_unfolded(q: torch.Tensor, kv: torch.Tensor, k_rot: torc
         int(max_q_len), H, int(dim), int(rot_dim), int(value_dim), rows, pitch, H * int(dim), k_rot.shape[1],
         int(window), float(scale), _ptr(gate), gate.shape[1] if gate is not None else 0, int(gate_col), _stream()),
         "prefill_attention_tc_unfolded")
-    _tc_pending = True
+    _tc_launched()
     return out
 
 

@@ -30,20 +30,24 @@ class Sampler:
         self._out = [torch.zeros(max_rows, dtype=torch.int32, device=device) for _ in range(2)]
         self._out_host = [torch.zeros(max_rows, dtype=torch.int32).pin_memory() for _ in range(2)]
         self._fetched = [torch.cuda.Event(), torch.cuda.Event()]
+        self._waits_host = [torch.zeros(1, dtype=torch.int32).pin_memory() for _ in range(2)]
+        self._waits = [False, False]
         self._rows = [0, 0]
         self._turn = 0
 
     def launch(self, logits: torch.Tensor, params: Sequence[SamplingParams], streams: Sequence[int],
-               indices: Sequence[int]) -> int:
+               indices: Sequence[int], waits: bool = False) -> int:
         """Queue the sampling of ``logits [R, V]`` (float32; row ``r`` is token number ``indices[r]``
         of stream ``streams[r]``) and the copy of the token ids to the host.  Returns the handle
-        for :meth:`device_tokens` and :meth:`fetch`."""
+        for :meth:`device_tokens` and :meth:`fetch`.  ``waits``: whether a bounded wait of a kernel before ran out comes with
+        the tokens, and :meth:`fetch` raises then."""
         R = logits.shape[0]
         if R > self.max_rows:
             raise ValueError(f"Sampler: {R} rows exceed the {self.max_rows} it was built for")
         k = self._turn
         self._turn ^= 1
         self._rows[k] = R
+        self._waits[k] = waits
         if R == 0:
             return k
         out = self._out[k][:R]
@@ -62,6 +66,8 @@ class Sampler:
                                           device=self.device)
             F.sample_rows(logits, dev[0, :R], dev[1, :R], dev[2, :R], self._probs[:R], out)
         self._out_host[k][:R].copy_(out, non_blocking=True)
+        if waits:
+            self._waits_host[k].copy_(F.wait_status(out.device), non_blocking=True)
         self._fetched[k].record()
         return k
 
@@ -75,6 +81,10 @@ class Sampler:
         if R == 0:
             return []
         self._fetched[handle].synchronize()
+        if self._waits[handle]:
+            code = int(self._waits_host[handle][0])
+            if code:
+                F.raise_wait_status(self._out[handle].device, code)
         return self._out_host[handle][:R].tolist()
 
     def sample(self, logits: torch.Tensor, params: Sequence[SamplingParams], streams: Sequence[int],
