@@ -476,7 +476,7 @@ __device__ __forceinline__ float capped_tanh(float x) {
 
 constexpr int DEC_SPLIT = 512;      // keys per split by default; smaller splits spread one or two requests over the device
 constexpr int DEC_GROUPS = 16;
-constexpr int DEC_JOIN_MAX = 8, DEC_JOIN_BLOCKS = 4 * 148;
+constexpr int DEC_JOIN_MAX = 8, DEC_JOIN_PER_SM = 4;
 
 // JOIN: the splits of a head are a cluster of at most DEC_JOIN_MAX blocks, and the first of them adds the others' results up
 // from their shared memory, as the merge kernel below does from the scratch (which is then not touched): one launch instead of
@@ -835,7 +835,7 @@ int mi_attn_decode_split_supported(int split) { return (split == 128 || split ==
 // 1 if the splits of a decode attention over a bfloat16 cache go as clusters, in one launch: heads of `d` numbers, `heads` of all
 // requests together, up to `splits` each.
 int mi_attn_decode_joined(int d, int64_t heads, int splits) {
-    return d == 128 && splits <= DEC_JOIN_MAX && heads * splits <= DEC_JOIN_BLOCKS ? 1 : 0;
+    return d == 128 && splits <= DEC_JOIN_MAX && heads * splits <= DEC_JOIN_PER_SM * (int64_t)sm_count() ? 1 : 0;
 }
 
 // Decode attention: every request has exactly one query token.  `part_o` needs

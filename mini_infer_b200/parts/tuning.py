@@ -55,10 +55,12 @@ class Tuning:
     # cannot fill 148 SMs with splits of 512 keys; splits of 256 for every batch size gained 4 % at batch 1
     # and lost 6 % at batch 8, hence the steps.  (bfloat16 path only: the float32 path runs one attention
     # kernel for every step, so that a request's logits do not depend on its batch.)
-    # These hold where the splits of a head do not go as a cluster in one launch; where they do (heads of 128, up to eight
-    # splits, no more blocks than the device holds), the smallest such split: 128, 256 and 512 keys, us, 8 requests of 600 keys
-    # 7.9, 9.9, 13.7 (8 heads); 6 of 2,000 19.3, 15.4, 16.2 (16 heads, 128 does not go as a cluster); 4 of 2,000 20.2, 19.4, 18.2
-    # (28 heads, 512 alone does).
+    # Where a smaller split lets a head's splits go as a cluster in one launch (heads of 128, up to eight splits of the longest context, no
+    # more blocks than the device holds), the smallest such.  This split in two launches and that one in one, us with a cold L2: 8
+    # requests of up to 600 keys 20.0 and 10.3 (8 heads; by 512 and 128), 23.6 and 15.4 (16 heads; 512 and 256), 3 of 1,000 15.9 and
+    # 12.9 (28 heads; 256 both).  Never a larger one: 1 request of 3,000 keys, 8 heads, 12.5 by 128 in two launches, 16.0 by 512 in one;
+    # 4 of 4,096 behind a window of 1,024, 16 heads, 18.3 by 256, 21.1 by 512.  Of 240 steps (1 to 16 requests, 300 to 4,096 keys, with
+    # and without a window) none is slower than by the number of requests alone.
     decode_split_by_requests: Tuple[Tuple[int, int], ...] = ((2, 128), (4, 256))
 
     # Chunked prefill: every full portion of a long prompt has the same shape, so its forward pass is replayed
@@ -154,12 +156,8 @@ class Tuning:
         return -(-num_requests // step) * step
 
     def decode_split(self, num_requests: int, default: int, joined: Optional[int] = None) -> int:
-        if joined is not None:
-            return joined
-        for limit, split in self.decode_split_by_requests:
-            if num_requests <= limit:
-                return split
-        return default
+        split = next((s for limit, s in self.decode_split_by_requests if num_requests <= limit), default)
+        return split if joined is None else min(split, joined)
 
 
 def _from_environment(t: Tuning) -> Tuning:
