@@ -160,7 +160,7 @@ __device__ __forceinline__ void store_pair(__nv_bfloat16* p, float a, float b) {
     *reinterpret_cast<__nv_bfloat162*>(p) = __floats2bfloat162_rn(a, b);
 }
 
-// (c, s) turns the pair (a, b); rounded alike in every kernel that does it
+// (c, s) turns the pair (a, b); rounded alike in both kernels of this file (few tokens and many)
 __device__ __forceinline__ void rotate_pair(float a, float b, float c, float s, float& ya, float& yb) {
     ya = __fmaf_rn(a, c, -__fmul_rn(b, s));
     yb = __fmaf_rn(b, c, __fmul_rn(a, s));

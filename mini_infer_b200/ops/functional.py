@@ -396,13 +396,11 @@ def prefill_attention_tc(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.
     if scale is None:
         scale = 1.0 / math.sqrt(d)
     dev = q.device
-    if dev not in _tc_status:
-        _tc_status[dev] = torch.zeros(1, dtype=I32, device=dev)
     if DEBUG_BOUNDS:
         _dbg_batch("prefill_attention_tc", q_start, kv_len, block_table, T, num_pages, page_size, int(window),
                    int(max_q_len), int(chunk))
     check(library().mi_attn_prefill_tc(_ptr(q), _ptr(k_cache), _ptr(v_cache), _ptr(block_table), _ptr(q_start),
-                                       _ptr(kv_len), _ptr(out), _ptr(_tc_status[dev]), T, B, int(max_q_len), nh, nkv,
+                                       _ptr(kv_len), _ptr(out), _ptr(_status_word(dev)), T, B, int(max_q_len), nh, nkv,
                                        d, page_size, num_pages, max_pages, int(window), float(scale),
                                        int(keep_first), float(softcap), int(bool(sink)),
                                        *_attn_form("prefill_attention_tc", nh, T, int(window), bool(sink), int(chunk),
@@ -436,13 +434,11 @@ def prefill_attention_tc_logistic(q: torch.Tensor, k_cache: torch.Tensor, v_cach
     _chk(kv_len, "prefill_attention_tc_logistic kv_len", I32, (B,))
     out = torch.empty(T, nh, dv, dtype=BF16, device=q.device)
     dev = q.device
-    if dev not in _tc_status:
-        _tc_status[dev] = torch.zeros(1, dtype=I32, device=dev)
     if DEBUG_BOUNDS:
         _dbg_batch("prefill_attention_tc_logistic", q_start, kv_len, block_table, T, num_pages, page_size, int(window),
                    int(max_q_len))
     check(library().mi_attn_prefill_tc_logistic(_ptr(q), _ptr(k_cache), _ptr(v_cache), _ptr(block_table), _ptr(q_start),
-                                                _ptr(kv_len), _ptr(out), _ptr(_tc_status[dev]), T, B, int(max_q_len),
+                                                _ptr(kv_len), _ptr(out), _ptr(_status_word(dev)), T, B, int(max_q_len),
                                                 nh, nkv, dk, dv, page_size, num_pages, max_pages, int(window),
                                                 float(scale), _ptr(head_bias), _stream()),
           "prefill_attention_tc_logistic")
@@ -471,13 +467,11 @@ def prefill_attention_tc_shared(q: torch.Tensor, cache: torch.Tensor, block_tabl
     _chk(kv_len, "prefill_attention_tc_shared kv_len", I32, (B,))
     out = torch.empty(T, H, int(value_dim), dtype=BF16, device=q.device)
     dev = q.device
-    if dev not in _tc_status:
-        _tc_status[dev] = torch.zeros(1, dtype=I32, device=dev)
     if DEBUG_BOUNDS:
         _dbg_batch("prefill_attention_tc_shared", q_start, kv_len, block_table, T, num_pages, page_size, int(window),
                    int(max_q_len))
     check(library().mi_attn_prefill_tc_shared(_ptr(q), _ptr(cache), _ptr(block_table), _ptr(q_start), _ptr(kv_len),
-                                              _ptr(out), _ptr(_tc_status[dev]), T, B, int(max_q_len), H, dk,
+                                              _ptr(out), _ptr(_status_word(dev)), T, B, int(max_q_len), H, dk,
                                               int(value_dim), page_size, num_pages, max_pages, int(window),
                                               float(scale), int(keep_first), _stream()),
           "prefill_attention_tc_shared")
@@ -833,10 +827,11 @@ def dense_f32(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
     _chk(w, "dense_f32 w", F32, (None, K))
     N = w.shape[0]
     out = torch.empty(T, N, dtype=F32, device=x.device)
-    status = _status_word(x.device)
+    on_tc = K >= library().mi_f32_tc_min_inner()
+    status = _status_word(x.device) if on_tc else None
     scratch = _f32_scratch(x, T, K)
     check(library().mi_dense_f32(_ptr(x), _ptr(w), _ptr(out), T, N, K, _ptr(scratch), _ptr(status), _stream()), "dense_f32")
-    if K >= library().mi_f32_tc_min_inner():
+    if on_tc:
         _tc_launched()
     return out
 
@@ -1041,7 +1036,8 @@ def tc_launches() -> int:
 
 
 def _status_word(dev: torch.device) -> torch.Tensor:
-    """The word in which kernels with bounded waits on ``dev`` say that one ran out (:func:`check_tc_status`)."""
+    """The word in which kernels with bounded waits on ``dev`` say that one ran out (:func:`check_tc_status`).  As for every library
+    that keeps something on the device, a first call belongs before a capture."""
     if dev not in _tc_status:
         _tc_status[dev] = torch.zeros(1, dtype=I32, device=dev)
     return _tc_status[dev]
@@ -1067,12 +1063,10 @@ def grouped_gemm_tc(a_sorted: torch.Tensor, w: torch.Tensor, offsets: torch.Tens
     nout = wrows // 2 if swiglu_pair else wrows
     _chk(offsets, "grouped_gemm_tc offsets", I32, (E + 1,))
     dev = a_sorted.device
-    if dev not in _tc_status:
-        _tc_status[dev] = torch.zeros(1, dtype=I32, device=dev)
     out = torch.empty(n_rows, nout, dtype=BF16 if swiglu_pair else F32, device=dev)
     if DEBUG_BOUNDS:
         _dbg_offsets(offsets, int(n_rows), "grouped_gemm_tc")
-    check(library().mi_grouped_gemm_tc_form(_ptr(a_sorted), _ptr(w), _ptr(offsets), _ptr(out), _ptr(_tc_status[dev]),
+    check(library().mi_grouped_gemm_tc_form(_ptr(a_sorted), _ptr(w), _ptr(offsets), _ptr(out), _ptr(_status_word(dev)),
                                             n_rows, E, nout, Kd, 1 if swiglu_pair else 0,
                                             -1 if form is None else int(form), *_glu_args(glu),
                                             _row_scale(row_scale, n_rows, swiglu_pair, "grouped_gemm_tc"), _stream()),
@@ -2120,12 +2114,13 @@ def dense_f32_heads(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor
     ldc = out.numel() // max(T, 1)
     if x_col + (H - 1) * xs + K > lda or out_col + (H - 1) * os_ + N > ldc:
         raise ValueError("dense_f32_heads: the heads do not fit the rows")
-    status = _status_word(x.device)
+    on_tc = K >= library().mi_f32_tc_min_inner()
+    status = _status_word(x.device) if on_tc else None
     scratch = _f32_scratch(x, T, K, 0, H)
     check(library().mi_dense_f32_batched(x.data_ptr() + 4 * x_col, _ptr(w), out.data_ptr() + 4 * out_col, T, N, K,
                                          lda, ldc, H, xs, N * K, os_, _ptr(scratch), _ptr(status), _stream()),
           "dense_f32_heads")
-    if K >= library().mi_f32_tc_min_inner():
+    if on_tc:
         _tc_launched()
     return out
 
@@ -2314,14 +2309,12 @@ def prefill_attention_tc_unfolded(q: torch.Tensor, kv: torch.Tensor, k_rot: torc
     _chk(out, "prefill_attention_tc_unfolded out", BF16, (T, H * value_dim))
     _chk(gate, "prefill_attention_tc_unfolded gate", F32, (T, None))
     dev = q.device
-    if dev not in _tc_status:
-        _tc_status[dev] = torch.zeros(1, dtype=I32, device=dev)
     if DEBUG_BOUNDS:
         total = int(kv_len.sum())
         if total > rows:
             _bad("prefill_attention_tc_unfolded", f"contexts of {total} tokens in {rows} rows")
     check(library().mi_attn_prefill_tc_unfolded(
-        _ptr(q), _ptr(kv), _ptr(k_rot), _ptr(q_start), _ptr(kv_len), _ptr(out), _ptr(_tc_status[dev]), T, B,
+        _ptr(q), _ptr(kv), _ptr(k_rot), _ptr(q_start), _ptr(kv_len), _ptr(out), _ptr(_status_word(dev)), T, B,
         int(max_q_len), H, int(dim), int(rot_dim), int(value_dim), rows, pitch, H * int(dim), k_rot.shape[1],
         int(window), float(scale), _ptr(gate), gate.shape[1] if gate is not None else 0, int(gate_col), _stream()),
         "prefill_attention_tc_unfolded")

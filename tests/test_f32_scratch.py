@@ -69,3 +69,10 @@ def test_first_product_of_a_device(monkeypatch):
     out = F.dense_f32(x, w)
     assert float((out.double() - x.double() @ w.double().T).norm()) < 1e-6 * float(out.norm())
     F.check_tc_status()
+
+
+@pytest.mark.gpu
+def test_small_inner_sizes_need_no_word(monkeypatch):
+    monkeypatch.setattr(F, "_tc_status", {})
+    F.dense_f32(torch.randn(3, 64, device="cuda:0"), torch.randn(5, 64, device="cuda:0"))
+    assert not F._tc_status
