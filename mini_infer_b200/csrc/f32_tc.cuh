@@ -4,10 +4,11 @@
 //
 // A number x of 32 bits is taken apart exactly, into three bfloat16 numbers: 2^24 x = h + m + l, each the rest rounded to 8 bits
 // (the factor keeps the parts of the smallest x among the normal numbers).  Of the nine products of two numbers' parts all are formed but
-// that of the two l, which is at most 2^-34 of the whole.  They stand in two sums by their size: hh; and the others, hm, mh and lh beside
-// hl, mm, lm and ml, 2^-8 of it and less.  The tensor cores add without rounding to nearest.  hh's terms have 16 bits, of which
-// few are cut off, but 32 of them at most are added there: then the sum goes to registers and is added up in 32 bits as any
-// number is.  The others stay for a part of the inner dimension.  Both meet in the output alone.  Measured error: see dense_f32.cu.
+// that of the two l, which is at most 2^-34 of the whole, in two sums: hh; and the others, which are 2^-8 of it and less.  The tensor
+// cores add without rounding to nearest.  hh's terms have 16 bits, of which few are cut off, but 32 of them at most are added
+// there: then the sum goes to registers and is added up in 32 bits as any number is.  The others stay for a part of the
+// inner dimension.  Both meet in the output alone.  Measured error: see dense_f32.cu.  (Three bfloat16 parts instead of a float32:
+// G. Henry, P. T. P. Tang, A. Heinecke, ARITH 2019.)
 //
 // Every output element is the same sums in the same order in every form below: chunks of 32 k in ascending order within
 // each of four parts of the inner dimension, then the parts in ascending order.  So a row has the same bits however many
@@ -19,9 +20,8 @@
 // tensor memory, rows of activations are the N operand in shared memory.  Roles:
 //   warps 0-7 or (tiles of 16 rows) 0-11, four for a chunk, in turn: weights, ring -> three parts -> tensor memory
 //   warps 8-15 or 12-15  the sums of a chunk: tensor memory -> registers, added up
-//   warps 16, 17, chunks in turn: MMAs, 10 a chunk (a warp takes 800 cycles for one in a busy SM, twice the MMAs' own time), the
-//               others into sums of its own; warp 16 allocates tensor memory.  The activations' parts stand one behind the
-//               other, so that one MMA multiplies a part of the weights with two of them
+//   warps 16, 17, chunks in turn: MMAs, 16 a chunk (a warp takes 800 cycles for one in a busy SM, more than the MMAs' own time), the
+//               others into a sum of its own; warp 16 allocates tensor memory.
 //   warp 18     weights: memory -> ring (TMA; without it, where rows are not aligned for it, the warps that read them ask
 //               for them with cp.async)
 //   tiles of 64 rows: warp 19 brings the parts of the activations, which f32_split_rows_kernel has laid out as they stand here
@@ -61,7 +61,8 @@ constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((128u >> 4) << 
 constexpr int w_slots(int nt, bool split) { return nt == 64 ? (split ? 4 : 6) : w_turns(nt) == 3 || split ? 6 : 8; }       // (a multiple of w_turns)
 constexpr int ROW_SLOTS = 4;
 constexpr int raw_slots(int nt) { return split_before(nt) ? 0 : ROWS_WARPS * ROWS_AHEAD; }
-constexpr int t_slots(int nt) { return nt == 64 ? 2 : 4; }
+constexpr int T_SLOTS = 4;
+constexpr int h_slots(int nt) { return nt == 64 ? 3 : 4; }
 inline size_t smem_bytes(int nt, int split) {
     return 1024 + (size_t)w_slots(nt, split > 1) * 16384 + (size_t)ROW_SLOTS * nt * 192 + (size_t)raw_slots(nt) * nt * 128 +
            (size_t)(split > 1 ? PARTS / split : 1) * 2 * nt * 512;
@@ -253,18 +254,18 @@ template <bool PAIRED, int NT, bool SPLIT, bool VEC>
 __global__ void __launch_bounds__(threads(NT), 1)
 f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, Problem g) {
     constexpr bool BEFORE = split_before(NT);
-    constexpr int THREADS = threads(NT), W_SLOTS = w_slots(NT, SPLIT), RAW_SLOTS = raw_slots(NT), T_SLOTS = t_slots(NT);
+    constexpr int THREADS = threads(NT), W_SLOTS = w_slots(NT, SPLIT), RAW_SLOTS = raw_slots(NT), H_SLOTS = h_slots(NT);
     constexpr int TURNS = w_turns(NT), OUT_WARP = 4 * TURNS;
     static_assert(W_SLOTS % TURNS == 0, "a turn's own slots");
-    // columns of tensor memory: T_SLOTS chunks' hh; the others' two sums of either MMA warp; T_SLOTS chunks of weights
-    constexpr int OTHERS_AT = 128, W_AT = 512 - T_SLOTS * 64;
-    static_assert(T_SLOTS * NT <= OTHERS_AT && OTHERS_AT + 4 * NT <= W_AT, "tensor memory");
+    // columns of tensor memory: H_SLOTS chunks' hh; the others of either MMA warp; T_SLOTS chunks of weights, 16 columns a part
+    constexpr int OTHERS_AT = 192, W_AT = 320;
+    static_assert(H_SLOTS * NT <= OTHERS_AT && OTHERS_AT + 2 * NT <= W_AT && W_AT + T_SLOTS * 48 <= 512, "tensor memory");
     constexpr int ROW_BYTES = NT * 192;                // a chunk's activations: [8 k][part][rows][16 bytes]
     constexpr int FEATS = PAIRED ? 64 : 128;           // outputs of a tile
     constexpr int OWN = NT / ((MMA_WARP - OUT_WARP) / 4);                  // rows of activations of an adding warp
     constexpr int PER = NT / 4;                        // 16-byte pieces of activations per lane and chunk
     extern __shared__ uint8_t smem_raw[];
-    __shared__ uint64_t full_bar[4], done_bar[8], empty_bar[T_SLOTS], others_read, w_full[W_SLOTS], w_read[W_SLOTS], rows_full[ROW_SLOTS];
+    __shared__ uint64_t full_bar[4], done_bar[8], empty_bar[H_SLOTS], others_read, w_full[W_SLOTS], w_read[W_SLOTS], rows_full[ROW_SLOTS];
     __shared__ uint32_t tmem_base_s;
     __shared__ int abort_s;
 
@@ -298,7 +299,7 @@ f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, Problem g) {
         abort_s = 0;
         for (int s = 0; s < 4; ++s) mbar_init(&full_bar[s], BEFORE ? 4 : 5);
         for (int s = 0; s < 8; ++s) mbar_init(&done_bar[s], 1);
-        for (int s = 0; s < T_SLOTS; ++s) mbar_init(&empty_bar[s], MMA_WARP - OUT_WARP);
+        for (int s = 0; s < H_SLOTS; ++s) mbar_init(&empty_bar[s], MMA_WARP - OUT_WARP);
         mbar_init(&others_read, MMA_WARP - OUT_WARP);
         for (int s = 0; s < ROW_SLOTS; ++s) mbar_init(&rows_full[s], 1);
         for (int s = 0; s < W_SLOTS; ++s) { mbar_init(&w_full[s], 1); mbar_init(&w_read[s], 4); }
@@ -353,7 +354,7 @@ f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, Problem g) {
                 __syncwarp();
             }
             const uint8_t* w = w_lane + slot * 16384;
-            const uint32_t at = t_lane + (i % T_SLOTS) * 64;
+            const uint32_t at = t_lane + (i % T_SLOTS) * 48;
             uint32_t h[16], m[16], l[16];
 #pragma unroll
             for (int p = 0; p < 8; ++p) {
@@ -393,7 +394,7 @@ f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, Problem g) {
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             if (c_lo < n_mma) {                        // uniform
-                const uint32_t d = lane_addr + (it % T_SLOTS) * NT;
+                const uint32_t d = lane_addr + (it % H_SLOTS) * NT;
                 uint32_t v[OWN];
                 if constexpr (OWN == 32) tmem_ld32(d, v);
                 else if constexpr (OWN == 16) tmem_ld16(d, v);
@@ -404,7 +405,7 @@ f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, Problem g) {
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
-            if (lane == 0) mbar_arrive(&empty_bar[it % T_SLOTS]);
+            if (lane == 0) mbar_arrive(&empty_bar[it % H_SLOTS]);
             if (++in_part == per_part || it == count - 1) {
                 // the others of both MMA warps, the next part's may follow
                 float* to = own + (SPLIT ? parts * 2 * NT * 128 : 0);
@@ -414,16 +415,11 @@ f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, Problem g) {
                 for (int i0 = 0; i0 < OWN; i0 += GROUP) {
                     const uint32_t d = lane_addr + OTHERS_AT + i0;
                     uint32_t x[GROUP], y[GROUP];
-                    if constexpr (GROUP == 16) { tmem_ld16(d, x); tmem_ld16(d + n_mma, y); }
-                    else { tmem_ld8(d, x); tmem_ld8(d + n_mma, y); }
+                    if constexpr (GROUP == 16) { tmem_ld16(d, x); tmem_ld16(d + NT, y); }
+                    else { tmem_ld8(d, x); tmem_ld8(d + NT, y); }
                     wait_tmem_ld();
 #pragma unroll
                     for (int i = 0; i < GROUP; ++i) others[i0 + i] = __uint_as_float(x[i]) + __uint_as_float(y[i]);
-                    if constexpr (GROUP == 16) { tmem_ld16(d + 2 * NT, x); tmem_ld16(d + 2 * NT + n_mma, y); }
-                    else { tmem_ld8(d + 2 * NT, x); tmem_ld8(d + 2 * NT + n_mma, y); }
-                    wait_tmem_ld();
-#pragma unroll
-                    for (int i = 0; i < GROUP; ++i) others[i0 + i] += __uint_as_float(x[i]) + __uint_as_float(y[i]);
                 }
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
@@ -454,33 +450,36 @@ f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, Problem g) {
         // The rows' number is a constant in here: with the operands formed from a variable one the warp took 450 cycles a chunk to
         // give the products out, and more than that to wait for what was there.
         auto give = [&](auto rows_c) {
-            constexpr uint32_t n = decltype(rows_c)::value, IDESC1 = IDESC | (n >> 3) << 17, IDESC2 = IDESC | (n >> 2) << 17;
+            constexpr uint32_t n = decltype(rows_c)::value, DESC = IDESC | (n >> 3) << 17;
             constexpr uint32_t K_STEP = 6 * n;         // 16 k of rows; of weights 8 columns
             const uint64_t rows_desc = umma_desc_plain(smem_u32(rows_ring), 48 * n);
             const uint32_t desc_lo = (uint32_t)rows_desc, desc_hi = (uint32_t)(rows_desc >> 32);
             const uint32_t t = __reduce_max_sync(0xffffffffu, tmem);       // (the same in all lanes also for the compiler)
             // (every part has two chunks and more: inner sizes from 512 up)
             int in_part = warp - MMA_WARP, parts = 0;
-            const uint32_t o1 = t + OTHERS_AT + in_part * 2 * NT;
+            const uint32_t others = t + OTHERS_AT + in_part * NT;
 #pragma unroll 1
             for (int i = in_part; i < count; i += 2) {
                 if (in_part < 2 && parts > 0 && !wait_for(&others_read, (parts - 1) & 1, abort_flag, 36)) break;
                 // room for the sums, rows (where no copy brings them: the room once more), weights (and rows)
-                const uint32_t room = ((i / T_SLOTS) & 1) ^ 1;
-                uint64_t* empty = &empty_bar[i % T_SLOTS];
+                const uint32_t room = ((i / H_SLOTS) & 1) ^ 1;
+                uint64_t* empty = &empty_bar[i % H_SLOTS];
                 if (!wait_for3(empty, room, BEFORE ? &rows_full[i % ROW_SLOTS] : empty, BEFORE ? (i / ROW_SLOTS) & 1 : room,
                                &full_bar[i & 3], (i >> 2) & 1, abort_flag, 35)) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t bh = desc_lo + (i % ROW_SLOTS) * (ROW_BYTES >> 4), bm = bh + n, bl = bm + n;
-                const uint32_t wh = t + W_AT + (i % T_SLOTS) * 64, wm = wh + 16, wl = wm + 16, hh = t + (i % T_SLOTS) * NT;
+                const uint32_t wh = t + W_AT + (i % T_SLOTS) * 48, wm = wh + 16, wl = wm + 16, hh = t + (i % H_SLOTS) * NT;
                 if (elect_one()) {
 #pragma unroll
                     for (int k = 0; k < FK / 16; ++k) {
-                        umma_tmem_a(o1, wh + k * 8, bm + k * K_STEP, desc_hi, IDESC2, in_part > 1 || k > 0);      // hm, hl
-                        umma_tmem_a(o1, wm + k * 8, bh + k * K_STEP, desc_hi, IDESC2, 1);                    // mh, mm
-                        umma_tmem_a(o1, wl + k * 8, bh + k * K_STEP, desc_hi, IDESC2, 1);                    // lh, lm
-                        umma_tmem_a(o1 + n, wm + k * 8, bl + k * K_STEP, desc_hi, IDESC1, 1);                //     ml
-                        umma_tmem_a(hh, wh + k * 8, bh + k * K_STEP, desc_hi, IDESC1, k > 0);
+                        umma_tmem_a(hh, wh + k * 8, bh + k * K_STEP, desc_hi, DESC, k > 0);
+                        umma_tmem_a(others, wh + k * 8, bm + k * K_STEP, desc_hi, DESC, in_part > 1 || k > 0);
+                        umma_tmem_a(others, wm + k * 8, bh + k * K_STEP, desc_hi, DESC, 1);
+                        umma_tmem_a(others, wh + k * 8, bl + k * K_STEP, desc_hi, DESC, 1);
+                        umma_tmem_a(others, wm + k * 8, bm + k * K_STEP, desc_hi, DESC, 1);
+                        umma_tmem_a(others, wl + k * 8, bh + k * K_STEP, desc_hi, DESC, 1);
+                        umma_tmem_a(others, wm + k * 8, bl + k * K_STEP, desc_hi, DESC, 1);
+                        umma_tmem_a(others, wl + k * 8, bm + k * K_STEP, desc_hi, DESC, 1);
                     }
                     umma_commit(&done_bar[i & 7]);
                 }
