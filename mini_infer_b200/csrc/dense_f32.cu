@@ -240,7 +240,7 @@ extern "C" int64_t mi_f32_tc_scratch(int64_t rows, int K, int groups, int batch,
 
 // `batch` products at once: C_b[T, N] = A_b[T, K] . W_b[N, K]^T with rows of A and C `lda` and `ldc` floats
 // apart and the operands of product b at A + b * sA, W + b * sW (rows K apart), C + b * sC: the heads of a
-// row of activations, each with a matrix of its own.  The same chain of additions per element as above.
+// row of activations, each with a matrix of its own.  The same additions in the same order per element as above.
 extern "C" int mi_dense_f32_batched(const float* A, const float* W, float* C, int T, int N, int K, int lda, int ldc,
                                     int batch, int64_t sA, int64_t sW, int64_t sC, float* scratch, int* status, cudaStream_t stream) {
     using namespace mi;

@@ -2099,8 +2099,8 @@ def dense_f32_heads(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor
                     out_head_stride: Optional[int] = None) -> torch.Tensor:
     """A product per head in true float32: ``out[t, h] = w[h] @ x[t, h]`` with ``w [H, N, K]``.  ``x`` is
     ``[T, *]`` float32 rows in which head ``h`` starts at column ``x_col + h * x_head_stride`` (default: heads
-    of ``K`` side by side); ``out`` likewise (default ``[T, H * N]``).  The same fixed chain of additions per
-    element as :func:`dense_f32`."""
+    of ``K`` side by side); ``out`` likewise (default ``[T, H * N]``).  The same additions in the same order per
+    element as in :func:`dense_f32`."""
     _chk(x, "dense_f32_heads x", F32)
     _chk(w, "dense_f32_heads w", F32)
     H, N, K = w.shape

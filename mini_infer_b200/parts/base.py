@@ -59,8 +59,9 @@ class TensorDecl:
 class Precision:
     """One of the two paths through the whole model.
 
-    ``float32``: weights, activations, cache and every product in true 32-bit
-    (TF32 and reduced-precision reductions are switched off).
+    ``float32``: weights, activations, cache, every operand and every sum in 32 bits (TF32 and reduced-precision
+    reductions of library products are switched off; the tensor cores take an operand as the exact sum of three
+    bfloat16 numbers).
     ``bfloat16``: matrices, activations between products and the cache in
     bfloat16; the residual stream, norms, softmax, router, rotation angles and
     every accumulation in float32.
