@@ -11,10 +11,10 @@
 // at 2048, 1.4e-7 and 1.3e-6 at 5632; positive ones 6.1e-8 and 3.1e-7, 6.5e-8 and 6.1e-7, 7.8e-8 and 1.2e-6; rows of one number 2.5e-8 both
 // (a row of a single 1.0 gives the weight's bits), of 2 2.5e-8 and 3.1e-8, of 8 2.8e-8 and 5.5e-8, of 64 4.8e-8 and 1.4e-7; numbers
 // of 1e-41 1.8e-6 and 4.1e-5.
-// Times in us with a cold L2, tensor cores and chain.  Against [6144, 2048]: 1 row 24 and 30, 32 rows 27 and 58, 64 rows 42 and 95,
-// 512 rows 122 and 295 (106 TFLOP/s), 2,048 rows 402 and 1,011; against [2048, 5632]: 26 and 60, 30 and 73, 40 and 265, 99 and 336, 361 and 1,033.
-// The line at 512: there the two meet (against [2048, 512]: 1 row 12 and 11, 48 rows 21 and 30, 256 rows 32 and 28, 512 rows 30 and 38, 2,048
-// rows 79 and 105), and the tensor cores' four parts of the inner dimension need four chunks of 32 each.
+// Times in us with a cold L2, tensor cores and chain.  Against [6144, 2048]: 1 row 24 and 30, 32 rows 26 and 58, 64 rows 42 and 95,
+// 512 rows 114 and 295 (113 TFLOP/s), 2,048 rows 372 and 1,011; against [2048, 5632]: 26 and 60, 30 and 73, 40 and 265, 95 and 336, 337 and 1,033.
+// The line at 512: there the two meet (against [2048, 512]: 1 row 11 and 11, 48 rows 21 and 30, 256 rows 30 and 28, 512 rows 28 and 38, 2,048
+// rows 71 and 105), and the tensor cores' four parts of the inner dimension need four chunks of 32 each.
 // The reference runs every dense product in FP16 through cuBLAS (src/layers/mlp.cpp:120-130).
 
 #include "f32_tc.cuh"
@@ -147,7 +147,8 @@ static int64_t f32_tc_row_bytes(int K) { return 6ll * ((K + f32tc::FK - 1) / f32
 // tiles of up to nt rows that n rows make at most
 static int64_t f32_tc_tiles(int64_t n, int groups, int nt) { return groups ? (n < n / nt + groups ? n : n / nt + groups) : (n + nt - 1) / nt; }
 // Rows of a tile at most.  Of 60 experts' rows, tiles of 16, 32 and 64 against [2 x 1408, 2048]: 8 rows each 268, 274 and 312 us, 13 rows 311,
-// 281 and 314, 17 rows 383, 285 and 319, 34 rows 610, 424 and 345.
+// 281 and 314, 17 rows 383, 285 and 319, 34 rows 610, 424 and 337.  Chains: 1 row each (16 tokens of 4 experts) 241 us, 183 here;
+// 3 rows 337 and 263; 8 rows 429 and 269; 34 rows 800 and 337; against [2048, 1408] 113 and 116, 163 and 151, 230 and 155, 431 and 198.
 static int f32_tc_tile(int64_t rows, int groups, int wanted) {
     if (wanted > 0) return wanted < 64 ? wanted : 64;
     const int64_t few = groups ? 9ll * groups : 16, more = groups ? 20ll * groups : 32;

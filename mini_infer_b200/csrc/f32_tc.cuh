@@ -640,7 +640,7 @@ f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, Problem g) {
         }
         if (__syncthreads_or((again | again_up) != 0)) {
             // ... once more as the CUDA-core kernels compute them, the tile's operands by way of the rings.  512 rows against
-            // [6144, 2048]: 0.12 ms; one of them NaN 0.30 ms; all of them 2.3 ms (43.7 with a thread's operands from memory).
+            // [6144, 2048]: 0.11 ms; one of them NaN 0.28 ms; all of them 2.3 ms (43.7 with a thread's operands from memory).
             constexpr int PITCH = FK + 1;
             float* w_s = reinterpret_cast<float*>(smem);
             float* a_s = w_s + 128 * PITCH;
